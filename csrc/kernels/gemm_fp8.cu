@@ -314,67 +314,133 @@ __device__ __forceinline__ uint32_t to_e4m3x4(float a, float b, float c, float d
   return static_cast<uint32_t>(lo) | (static_cast<uint32_t>(hi) << 16);
 }
 
-// One warp per row; a lane covers 16 consecutive elements (two 16-byte loads, one 16-byte
-// store), eight lanes one 128-element block, so a warp moves 512 elements per step. Every lane
-// runs every step (the shuffles name the whole warp); K is a multiple of 128, so the eight lanes
-// of a block are active or idle together.
-// rows_dev (may be null): device-side count of the rows in use; the scale table keeps its row
-// stride M whatever that count.
-__device__ __forceinline__ uint4 quant16(const float (&f)[16], bool active, float* scale_out) {
-  float amax = 0.f;
-#pragma unroll
-  for (int j = 0; j < 16; ++j) amax = fmaxf(amax, fabsf(f[j]));
-  amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-  amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-  amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
-  const float scale = amax > 0.f ? amax / 448.f : 1.f;
-  *scale_out = scale;
-  uint4 pk = make_uint4(0u, 0u, 0u, 0u);
-  if (active) {
-    // true division (not a reciprocal multiply): ties must round as in x / scale
-    pk.x = to_e4m3x4(__fdiv_rn(f[0], scale), __fdiv_rn(f[1], scale), __fdiv_rn(f[2], scale), __fdiv_rn(f[3], scale));
-    pk.y = to_e4m3x4(__fdiv_rn(f[4], scale), __fdiv_rn(f[5], scale), __fdiv_rn(f[6], scale), __fdiv_rn(f[7], scale));
-    pk.z = to_e4m3x4(__fdiv_rn(f[8], scale), __fdiv_rn(f[9], scale), __fdiv_rn(f[10], scale), __fdiv_rn(f[11], scale));
-    pk.w = to_e4m3x4(__fdiv_rn(f[12], scale), __fdiv_rn(f[13], scale), __fdiv_rn(f[14], scale), __fdiv_rn(f[15], scale));
+// Every quantiser below gives a warp R consecutive rows x 256 columns: a lane covers 8 consecutive
+// columns of each row (one 16-byte access of bf16), 16 lanes one 128-column block, and the R row
+// loads are all in flight before the first use. What bounds them is memory once the arithmetic is
+// out of the way: a warp per row with one 512-column step at a time left one load latency per step
+// exposed, and a compiler division per element (about ten instructions) made the kernels
+// issue-bound. 73984 x 2048, 73984 x 1408 and the 66 x (2816 + 1408) x 2048 expert weights, before ->
+// after: see the figures at each kernel.
+//
+// e4m3(x / scale) must round as the correctly rounded quotient does (a reciprocal multiply moves
+// some ties). Markstein (1990): with r = RN(1 / s) and q0 = RN(x r), the residual x - q0 s is exact in
+// one FMA and RN(q0 + r residual) is RN(x / s): three operations. The range check keeps every
+// quotient that does not round to zero clear of underflow and r clear of overflow; other scales
+// take the division. The sign of a zero quotient is the numerator's. All 128 x 128 pairs of bf16
+// significands at every exponent distance that matters give the quotient's bits.
+struct Quot {
+  float s, r;
+  bool fast;
+  __device__ __forceinline__ explicit Quot(float scale)
+      : s(scale), r(1.f / scale), fast(scale > 8.6736174e-19f && scale < 1.1529215e18f) {}
+  __device__ __forceinline__ float markstein(float x) const {
+    const float q0 = x * r;
+    return copysignf(fmaf(fmaf(-q0, s, x), r, q0), x);
   }
-  return pk;
+  // e4m3 of 8 bf16 values
+  __device__ __forceinline__ uint2 operator()(const bf16x8& p) const {
+    float f[8];
+    unpack8(p, f);
+    if (fast) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[j] = markstein(f[j]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[j] = __fdiv_rn(f[j], s);
+    }
+    return make_uint2(to_e4m3x4(f[0], f[1], f[2], f[3]), to_e4m3x4(f[4], f[5], f[6], f[7]));
+  }
+};
+// bf16(e4m3 * scale) of 8 values
+__device__ __forceinline__ bf16x8 dequant8(uint2 q, float s) {
+  const uint32_t w2[2] = {q.x, q.y};
+  float f[8];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const __half2_raw h2 = __nv_cvt_fp8x2_to_halfraw2(
+        static_cast<__nv_fp8x2_storage_t>((w2[j >> 1] >> (16 * (j & 1))) & 0xffffu), __NV_E4M3);
+    const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&h2));
+    f[2 * j] = v.x * s;
+    f[2 * j + 1] = v.y * s;
+  }
+  return pack8(f);
+}
+// largest magnitude of 8 bf16 values (exact; NaN is ignored, as fmaxf ignores it)
+__device__ __forceinline__ bf16 amax8(const bf16x8& p) {
+  const __nv_bfloat162 m = __hmax2(__hmax2(__habs2(p.v[0]), __habs2(p.v[1])),
+                                   __hmax2(__habs2(p.v[2]), __habs2(p.v[3])));
+  return __hmax(__hmax(__low2bfloat16(m), __high2bfloat16(m)), __ushort_as_bfloat16(0));
+}
+__device__ __forceinline__ float block_scale(float amax) { return amax > 0.f ? amax / 448.f : 1.f; }
+__device__ __forceinline__ bf16x8 zero8() {
+  bf16x8 z;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) z.v[j] = __floats2bfloat162_rn(0.f, 0.f);
+  return z;
 }
 
+// Quantises R rows x 256 columns held one bf16x8 per row and lane (zeros outside the matrix) and
+// stores bytes and scales: row0 is the first row, c the lane's first column. Every lane takes part
+// in the shuffles; two rows share one as a bf16 pair.
+template <int R>
+__device__ __forceinline__ void quant_tile(const bf16x8 (&v)[R], int row0, int m_eff, int M, int c, int K,
+                                           int lane, uint8_t* __restrict__ q, float* __restrict__ scales) {
+  float keep = 1.f;
+#pragma unroll
+  for (int i = 0; i < R; i += 2) {
+    __nv_bfloat162 m = __halves2bfloat162(amax8(v[i]), amax8(v[i + 1]));
+#pragma unroll
+    for (int o = 1; o < 16; o <<= 1) m = __hmax2(m, __shfl_xor_sync(0xffffffffu, m, o));
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const float scale = block_scale(bf16_to_f32(h ? __high2bfloat16(m) : __low2bfloat16(m)));
+      if ((lane & 15) == i + h) keep = scale;
+      if (row0 + i + h < m_eff && c < K)
+        *reinterpret_cast<uint2*>(q + static_cast<size_t>(row0 + i + h) * K + c) = Quot(scale)(v[i + h]);
+    }
+  }
+  // lane j of a block's 16 holds the scale of row j: R consecutive floats of the table's row
+  if ((lane & 15) < R && row0 + (lane & 15) < m_eff && c < K)
+    scales[static_cast<size_t>(c >> 7) * M + row0 + (lane & 15)] = keep;
+}
+
+constexpr int QR = 8;       // rows of a warp in the plain row kernels
+constexpr int QR_SWI = 4;   // two operands per element: half the rows for the same registers
+
+// first row and column group of this warp; column groups of the same rows are neighbours
+__device__ __forceinline__ bool warp_tile(int rows_per, int M, int K, int& row0, int& c, int lane) {
+  const int ncg = (K + 255) >> 8;
+  const long w = (static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  row0 = static_cast<int>(w / ncg) * rows_per;
+  c = static_cast<int>(w % ncg) * 256 + lane * 8;
+  return w < static_cast<long>((M + rows_per - 1) / rows_per) * ncg;
+}
+
+// rows_dev (may be null): device-side count of the rows in use; the scale table keeps its row
+// stride M whatever that count.
+// 73984 x 2048: 132 us -> 100 us (read 2, write 1 byte an element: 4560 GB/s).
 __global__ void __launch_bounds__(256) quant_rows_kernel(const bf16* __restrict__ x, long ld, int M,
                                                          int K, uint8_t* __restrict__ q,
                                                          float* __restrict__ scales,
                                                          const int* __restrict__ rows_dev) {
   const int lane = threadIdx.x & 31;
   const int m_eff = rows_dev != nullptr ? min(M, *rows_dev) : M;
-  const long warps = (static_cast<long>(gridDim.x) * blockDim.x) >> 5;
-  for (long row = (static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; row < m_eff;
-       row += warps) {
-    const bf16* src = x + static_cast<size_t>(row) * ld;
-    for (int c0 = 0; c0 < K; c0 += 512) {
-      const int c = c0 + lane * 16;
-      const bool active = c < K;
-      float f[16];
-      if (active) {
-        unpack8(*reinterpret_cast<const bf16x8*>(src + c), f);
-        unpack8(*reinterpret_cast<const bf16x8*>(src + c + 8), f + 8);
-      } else {
+  int row0, c;
+  if (!warp_tile(QR, M, K, row0, c, lane) || row0 >= m_eff) return;
+  bf16x8 v[QR];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) f[j] = 0.f;
-      }
-      float scale;
-      const uint4 pk = quant16(f, active, &scale);
-      if (active) {
-        *reinterpret_cast<uint4*>(q + static_cast<size_t>(row) * K + c) = pk;
-        if ((lane & 7) == 0) scales[static_cast<size_t>(c >> 7) * M + row] = scale;
-      }
-    }
-  }
+  for (int i = 0; i < QR; ++i)
+    v[i] = row0 + i < m_eff && c < K
+               ? *reinterpret_cast<const bf16x8*>(x + static_cast<size_t>(row0 + i) * ld + c)
+               : zero8();
+  quant_tile<QR>(v, row0, m_eff, M, c, K, lane, q, scales);
 }
 
 // SwiGLU fused with the row quantiser: h = silu(gate) * up is written as bf16 (the backward
 // and the weight gradient of the next product need it) and, from those bf16 values, as e4m3 +
 // 1 x 128 scales for the FP8 product that consumes it. One pass over gu instead of a SwiGLU
 // pass and a quantiser pass. gu [rows, 2H] (gate | up), H a multiple of 128.
+// 73984 rows, H = 1408, no bf16 copy: 199 us -> 194 us (the exponential and the gate's division bound it).
 __global__ void __launch_bounds__(256) swiglu_quant_kernel(const bf16* __restrict__ gu,
                                                            bf16* __restrict__ h, int M, int H,
                                                            uint8_t* __restrict__ q,
@@ -382,47 +448,35 @@ __global__ void __launch_bounds__(256) swiglu_quant_kernel(const bf16* __restric
                                                            const int* __restrict__ rows_dev) {
   const int lane = threadIdx.x & 31;
   const int m_eff = rows_dev != nullptr ? min(M, *rows_dev) : M;
-  const long warps = (static_cast<long>(gridDim.x) * blockDim.x) >> 5;
-  for (long row = (static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; row < m_eff;
-       row += warps) {
-    const bf16* src = gu + static_cast<size_t>(row) * 2 * H;
-    for (int c0 = 0; c0 < H; c0 += 512) {
-      const int c = c0 + lane * 16;
-      const bool active = c < H;
-      float f[16];
-      if (active) {
-        float g[16], u[16];
-        unpack8(*reinterpret_cast<const bf16x8*>(src + c), g);
-        unpack8(*reinterpret_cast<const bf16x8*>(src + c + 8), g + 8);
-        unpack8(*reinterpret_cast<const bf16x8*>(src + H + c), u);
-        unpack8(*reinterpret_cast<const bf16x8*>(src + H + c + 8), u + 8);
+  int row0, c;
+  if (!warp_tile(QR_SWI, M, H, row0, c, lane) || row0 >= m_eff) return;
+  bf16x8 v[QR_SWI], up[QR_SWI];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const float s = 1.f / (1.f + __expf(-g[j]));
-          // quantise what the bf16 copy holds, so both forms of h agree
-          f[j] = bf16_to_f32(f32_to_bf16(g[j] * s * u[j]));
-        }
-        if (h != nullptr) {                  // callers that keep only the e4m3 rows pass null
-          bf16* dst = h + static_cast<size_t>(row) * H + c;
-          *reinterpret_cast<bf16x8*>(dst) = pack8(f);
-          *reinterpret_cast<bf16x8*>(dst + 8) = pack8(f + 8);
-        }
-      } else {
-#pragma unroll
-        for (int j = 0; j < 16; ++j) f[j] = 0.f;
-      }
-      float scale;
-      const uint4 pk = quant16(f, active, &scale);
-      if (active) {
-        *reinterpret_cast<uint4*>(q + static_cast<size_t>(row) * H + c) = pk;
-        if ((lane & 7) == 0) scales[static_cast<size_t>(c >> 7) * M + row] = scale;
-      }
-    }
+  for (int i = 0; i < QR_SWI; ++i) {
+    const bool in = row0 + i < m_eff && c < H;
+    const bf16* src = gu + static_cast<size_t>(row0 + i) * 2 * H + c;
+    v[i] = in ? *reinterpret_cast<const bf16x8*>(src) : zero8();
+    up[i] = in ? *reinterpret_cast<const bf16x8*>(src + H) : zero8();
   }
+#pragma unroll
+  for (int i = 0; i < QR_SWI; ++i) {
+    float g[8], u[8];
+    unpack8(v[i], g);
+    unpack8(up[i], u);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float s = 1.f / (1.f + __expf(-g[j]));
+      g[j] = g[j] * s * u[j];
+    }
+    v[i] = pack8(g);   // what the bf16 copy holds is what is quantised, so both forms of h agree
+    if (h != nullptr && row0 + i < m_eff && c < H)   // callers that keep only the e4m3 rows pass null
+      *reinterpret_cast<bf16x8*>(h + static_cast<size_t>(row0 + i) * H + c) = v[i];
+  }
+  quant_tile<QR_SWI>(v, row0, m_eff, M, c, H, lane, q, scales);
 }
 
-// y[row, :] = bf16(e4m3(q[row, :]) * scale of its 1 x 128 block); one warp per row, a lane
-// covers 16 consecutive elements (one 16-byte load, two 16-byte stores)
+// y[row, :] = bf16(e4m3(q[row, :]) * scale of its 1 x 128 block)
+// 73984 x 2048 and 73984 x 1408 together: 475 us -> 122 us; 5000 rows of each: 48 us -> 13 us.
 __global__ void __launch_bounds__(256) dequant_rows_kernel(const uint8_t* __restrict__ q,
                                                            const float* __restrict__ scales,
                                                            long ld_s, int M, int K,
@@ -430,110 +484,73 @@ __global__ void __launch_bounds__(256) dequant_rows_kernel(const uint8_t* __rest
                                                            const int* __restrict__ rows_dev) {
   const int lane = threadIdx.x & 31;
   const int m_eff = rows_dev != nullptr ? min(M, *rows_dev) : M;
-  const long warps = (static_cast<long>(gridDim.x) * blockDim.x) >> 5;
-  for (long row = (static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; row < m_eff;
-       row += warps) {
-    // four column groups (2048 elements of the row) per pass: their payload and scale loads are
-    // all issued before the first conversion, so a pass costs one memory latency, not four
-    for (int c0 = 0; c0 < K; c0 += 2048) {
-      uint4 raw[4];
-      float sc[4];
+  int row0, c;
+  if (!warp_tile(QR, M, K, row0, c, lane) || row0 >= m_eff || c >= K) return;   // no shuffles below
+  uint2 raw[QR];
+  float sc[QR];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int c = c0 + u * 512 + lane * 16;
-        if (c < K) {
-          raw[u] = *reinterpret_cast<const uint4*>(q + static_cast<size_t>(row) * K + c);
-          sc[u] = scales[static_cast<size_t>(c >> 7) * ld_s + row];
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int c = c0 + u * 512 + lane * 16;
-        if (c >= K) continue;
-        const float s = sc[u];
-        const uint32_t w4[4] = {raw[u].x, raw[u].y, raw[u].z, raw[u].w};
-        float f[16];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-#pragma unroll
-          for (int hh = 0; hh < 2; ++hh) {
-            const __half2_raw h2 = __nv_cvt_fp8x2_to_halfraw2(
-                static_cast<__nv_fp8x2_storage_t>((w4[j] >> (16 * hh)) & 0xffffu), __NV_E4M3);
-            const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&h2));
-            f[4 * j + 2 * hh] = v.x * s;
-            f[4 * j + 2 * hh + 1] = v.y * s;
-          }
-        }
-        bf16* dst = y + static_cast<size_t>(row) * K + c;
-        *reinterpret_cast<bf16x8*>(dst) = pack8(f);
-        *reinterpret_cast<bf16x8*>(dst + 8) = pack8(f + 8);
-      }
+  for (int i = 0; i < QR; ++i) {
+    if (row0 + i < m_eff) {
+      raw[i] = *reinterpret_cast<const uint2*>(q + static_cast<size_t>(row0 + i) * K + c);
+      sc[i] = scales[static_cast<size_t>(c >> 7) * ld_s + row0 + i];
     }
   }
+#pragma unroll
+  for (int i = 0; i < QR; ++i)
+    if (row0 + i < m_eff)
+      *reinterpret_cast<bf16x8*>(y + static_cast<size_t>(row0 + i) * K + c) = dequant8(raw[i], sc[i]);
 }
 
 // One CTA (256 threads) per 128 x 128 block of a [N, K] matrix (edges clipped).
 // q / scales may be null when only `deq` is wanted. deq (may be null): bf16 [N, K] image of the
 // quantised block, e4m3(w / scale) * scale: the operand the FP8 GEMM really multiplied, which is
 // what the backward of an FP8 linear differentiates against.
-__global__ void __launch_bounds__(256)
+// The block is read once and waits for the block-wide maximum as packed bf16 (32 registers a
+// thread, so that four CTAs share an SM and one's loads cover another's arithmetic).
+// 66 x (2816 x 2048 + 2048 x 1408), quantised and fake-quantised: 1372 us -> 674 us (610 at the copy rate).
+__global__ void __launch_bounds__(256, 4)
 quant_blocks_kernel(const bf16* __restrict__ w, long ld, int N, int K, uint8_t* __restrict__ q,
                     float* __restrict__ scales, bf16* __restrict__ deq) {
-  // The 128 x 128 block is read once: thread t keeps 16 consecutive elements of four rows
-  // (rows t / 8 + 32 i, columns 16 (t % 8) ..) in registers across the block-wide maximum.
   __shared__ float red[33];
   const int nb = blockIdx.y, kb = blockIdx.x;
-  const int r0 = nb * 128 + (threadIdx.x >> 3), c = kb * 128 + (threadIdx.x & 7) * 16;
+  const int r0 = nb * 128 + (threadIdx.x >> 4), c = kb * 128 + (threadIdx.x & 15) * 8;
   const bool vec_ok = (ld % 8) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0;
-  float v[4][16];
-  float amax = 0.f;
+  bf16x8 v[8];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int r = r0 + 32 * i;
-    if (r < N && c < K) {                      // K is a multiple of 128: the 16 columns are in range
+  for (int i = 0; i < 8; ++i) {
+    const int r = r0 + 16 * i;
+    v[i] = zero8();
+    if (r < N) {                               // K is a multiple of 128: the 8 columns are in range
       const bf16* src = w + static_cast<size_t>(r) * ld + c;
       if (vec_ok) {
-        unpack8(*reinterpret_cast<const bf16x8*>(src), v[i]);
-        unpack8(*reinterpret_cast<const bf16x8*>(src + 8), v[i] + 8);
+        v[i] = *reinterpret_cast<const bf16x8*>(src);
       } else {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) v[i][j] = __bfloat162float(src[j]);
+        for (int j = 0; j < 4; ++j) v[i].v[j] = __halves2bfloat162(src[2 * j], src[2 * j + 1]);
       }
-#pragma unroll
-      for (int j = 0; j < 16; ++j) amax = fmaxf(amax, fabsf(v[i][j]));
     }
   }
-  amax = block_max(amax, red);
-  const float scale = amax > 0.f ? amax / 448.f : 1.f;
+  bf16 m = amax8(v[0]);
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int r = r0 + 32 * i;
-    if (r >= N || c >= K) continue;
-    uint32_t pk[4];
+  for (int i = 1; i < 8; ++i) m = __hmax(m, amax8(v[i]));
+  const float scale = block_scale(block_max(bf16_to_f32(m), red));
+  const Quot quot(scale);
 #pragma unroll
-    for (int g = 0; g < 4; ++g)
-      pk[g] = to_e4m3x4(__fdiv_rn(v[i][4 * g], scale), __fdiv_rn(v[i][4 * g + 1], scale),
-                        __fdiv_rn(v[i][4 * g + 2], scale), __fdiv_rn(v[i][4 * g + 3], scale));
-    if (q != nullptr)
-      *reinterpret_cast<uint4*>(q + static_cast<size_t>(r) * K + c) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-    if (deq != nullptr) {
-      float f[16];
-#pragma unroll
-      for (int g = 0; g < 4; ++g)
-#pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-          const __half2_raw h2 = __nv_cvt_fp8x2_to_halfraw2(
-              static_cast<__nv_fp8x2_storage_t>((pk[g] >> (16 * hh)) & 0xffffu), __NV_E4M3);
-          const float2 t = __half22float2(*reinterpret_cast<const __half2*>(&h2));
-          f[4 * g + 2 * hh] = t.x * scale;
-          f[4 * g + 2 * hh + 1] = t.y * scale;
-        }
-      bf16* dst = deq + static_cast<size_t>(r) * K + c;
-      *reinterpret_cast<bf16x8*>(dst) = pack8(f);
-      *reinterpret_cast<bf16x8*>(dst + 8) = pack8(f + 8);
-    }
+  for (int i = 0; i < 8; ++i) {
+    const int r = r0 + 16 * i;
+    if (r >= N) continue;
+    const uint2 pk = quot(v[i]);
+    if (q != nullptr) *reinterpret_cast<uint2*>(q + static_cast<size_t>(r) * K + c) = pk;
+    if (deq != nullptr)
+      *reinterpret_cast<bf16x8*>(deq + static_cast<size_t>(r) * K + c) = dequant8(pk, scale);
   }
   if (threadIdx.x == 0 && scales != nullptr) scales[static_cast<size_t>(nb) * gridDim.x + kb] = scale;
+}
+
+// blocks of 8 warps that cover M rows, rows_per of them and 256 columns to a warp
+inline unsigned tile_grid(int rows_per, int M, int K) {
+  const long warps = static_cast<long>((M + rows_per - 1) / rows_per) * ((K + 255) / 256);
+  return static_cast<unsigned>((warps + 7) / 8);
 }
 
 }  // namespace f8
@@ -546,9 +563,7 @@ PB_API int pb_fp8_quant_rows(const void* x, long ld, int M, int K, void* q, floa
                              cudaStream_t st) {
   if (M <= 0 || K <= 0 || K % 128 != 0 || ld % 8 != 0 || (reinterpret_cast<uintptr_t>(x) & 15) != 0)
     return PB_BAD_ARG;
-  long blocks = (static_cast<long>(M) * 32 + 255) / 256;
-  // one warp per row, no grid-stride cap: measured 10 % faster than a persistent grid
-  f8::quant_rows_kernel<<<static_cast<unsigned>(blocks), 256, 0, st>>>(
+  f8::quant_rows_kernel<<<f8::tile_grid(f8::QR, M, K), 256, 0, st>>>(
       static_cast<const bf16*>(x), ld, M, K, static_cast<uint8_t*>(q), scales, nullptr);
   return static_cast<int>(cudaGetLastError());
 }
@@ -557,8 +572,7 @@ PB_API int pb_fp8_quant_rows_dyn(const void* x, long ld, int M, int K, void* q, 
                                  const int* rows_dev, cudaStream_t st) {
   if (M <= 0 || K <= 0 || K % 128 != 0 || ld % 8 != 0 || (reinterpret_cast<uintptr_t>(x) & 15) != 0)
     return PB_BAD_ARG;
-  long blocks = (static_cast<long>(M) * 32 + 255) / 256;
-  f8::quant_rows_kernel<<<static_cast<unsigned>(blocks), 256, 0, st>>>(
+  f8::quant_rows_kernel<<<f8::tile_grid(f8::QR, M, K), 256, 0, st>>>(
       static_cast<const bf16*>(x), ld, M, K, static_cast<uint8_t*>(q), scales, rows_dev);
   return static_cast<int>(cudaGetLastError());
 }
@@ -568,8 +582,7 @@ PB_API int pb_fp8_quant_rows_dyn(const void* x, long ld, int M, int K, void* q, 
 PB_API int pb_swiglu_quant(const void* gu, void* h, int M, int H, void* q, float* scales,
                            const int* rows_dev, cudaStream_t st) {
   if (M <= 0 || H <= 0 || H % 128 != 0) return PB_BAD_ARG;
-  long blocks = (static_cast<long>(M) * 32 + 255) / 256;
-  f8::swiglu_quant_kernel<<<static_cast<unsigned>(blocks), 256, 0, st>>>(
+  f8::swiglu_quant_kernel<<<f8::tile_grid(f8::QR_SWI, M, H), 256, 0, st>>>(
       static_cast<const bf16*>(gu), static_cast<bf16*>(h), M, H, static_cast<uint8_t*>(q), scales,
       rows_dev);
   return static_cast<int>(cudaGetLastError());
@@ -580,9 +593,7 @@ PB_API int pb_swiglu_quant(const void* gu, void* h, int M, int H, void* q, float
 PB_API int pb_fp8_dequant_rows(const void* q, const float* scales, long ld_s, int M, int K, void* y,
                                const int* rows_dev, cudaStream_t st) {
   if (M <= 0 || K <= 0 || K % 128 != 0 || ld_s < M) return PB_BAD_ARG;
-  long blocks = (static_cast<long>(M) * 32 + 255) / 256;
-  if (blocks > 148 * 32) blocks = 148 * 32;
-  f8::dequant_rows_kernel<<<static_cast<unsigned>(blocks), 256, 0, st>>>(
+  f8::dequant_rows_kernel<<<f8::tile_grid(f8::QR, M, K), 256, 0, st>>>(
       static_cast<const uint8_t*>(q), scales, ld_s, M, K, static_cast<bf16*>(y), rows_dev);
   return static_cast<int>(cudaGetLastError());
 }

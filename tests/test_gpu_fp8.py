@@ -35,6 +35,50 @@ def test_quantisers_match_the_reference_rule():
     torch.testing.assert_close(fp8.dequantize_blocks(qw, sw).cpu(), kernels.fp8_dequantize(refw))
 
 
+@pytest.mark.parametrize("M,K", [(1, 128), (7, 256), (9, 384), (130, 1408), (64, 2176)])
+@pytest.mark.parametrize("scale", [1.0, 1e-37, 1e30])
+def test_quantisers_bytes_at_tile_edges(M, K, scale):
+    """Bytes and scales equal the CPU rule at row / column remainders of the 8 x 256 warp tile, for
+    scales inside and outside the range of the three-operation quotient, with signed zeros."""
+    from prometheus_b200 import kernels
+    from prometheus_b200.ops import fp8
+
+    x = _r(M, K, seed=M + K, scale=scale)
+    x[0, 3], x[0, 4] = -0.0, 0.0
+    q, s = fp8.quantize_rows(x)
+    ref = kernels.fp8_quantize(x.float().cpu(), block=128)
+    assert torch.equal(s.t().cpu(), ref.scale)
+    assert torch.equal(q.view(torch.int8).cpu(), ref.q)
+    want = (q.view(torch.float8_e4m3fn).float() * s.t().repeat_interleave(128, dim=1)).to(BF16)
+    assert torch.equal(fp8.dequantize_rows_bf16(q, s), want)
+    wide = torch.cat([x, x], dim=1)[:, :K]                          # a row stride larger than K
+    assert torch.equal(fp8.quantize_rows(wide)[0], q)
+    used = torch.tensor([max(1, M - 2)], dtype=torch.int32, device="cuda")
+    qd, sd = fp8.quantize_rows(x, rows_used=used)
+    n = int(used)
+    assert torch.equal(qd[:n], q[:n]) and torch.equal(sd[:, :n], s[:, :n])
+    qw, sw = fp8.quantize_blocks(x)
+    refw = kernels.fp8_quantize_2d(x.float().cpu(), block=128)
+    assert torch.equal(sw.cpu(), refw.scale)
+    assert torch.equal(qw.view(torch.int8).cpu(), refw.q)
+    full = sw.repeat_interleave(128, 0)[:M].repeat_interleave(128, 1)
+    assert torch.equal(fp8.fakequant_blocks(x), (qw.view(torch.float8_e4m3fn).float() * full).to(BF16))
+
+
+@pytest.mark.parametrize("M,H", [(1, 128), (5, 384), (66, 1408)])
+def test_swiglu_quantize_is_swiglu_then_quantize(M, H):
+    from prometheus_b200.ops import fp8
+    from prometheus_b200.ops import functional as ops
+
+    gu = _r(M, 2 * H, seed=M)
+    h, q, s = fp8.swiglu_quantize(gu)
+    assert torch.equal(h, ops.swiglu(gu))
+    q2, s2 = fp8.quantize_rows(h)
+    assert torch.equal(q, q2) and torch.equal(s, s2)
+    none, q3, s3 = fp8.swiglu_quantize(gu, keep_bf16=False)
+    assert none is None and torch.equal(q3, q) and torch.equal(s3, s)
+
+
 @pytest.mark.parametrize("M,N,K", [(128, 128, 128), (300, 200, 384), (1024, 1408, 2048), (77, 2048, 256)])
 def test_fp8_gemm_equals_dequantised_matmul(M, N, K):
     from prometheus_b200.ops import fp8
