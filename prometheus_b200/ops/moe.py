@@ -107,16 +107,14 @@ def grouped_gemm(a: Tensor, w: Tensor, pl: Placement, *, b_mn: bool = False,
 
 def grouped_wgrad(a: Tensor, b: Tensor, pl: Placement, out: Tensor, accumulate: bool) -> Tensor:
     """out[e] (+)= A[rows_e]^T @ B[rows_e]; a [rows, M], b [rows, N], out [E, M, N] fp32 or bf16.
-    Experts without rows keep their previous contents (zero them first when not accumulating)."""
+    Experts without rows keep their previous contents when accumulating and get zeros otherwise."""
     from .functional import status_word
 
     R, M = a.shape
     N = b.shape[1]
     E = out.shape[0]
     f32 = out.dtype == torch.float32
-    if not accumulate:
-        out.zero_()
-    call("pb_gemm_bf16_grouped_wgrad", ptr(a), ptr(b), ptr(out), ptr(out), M, N, R, E, a.stride(0),
+    call("pb_gemm_bf16_grouped_wgrad", ptr(a), ptr(b), ptr(out), ptr(out) if accumulate else None, M, N, R, E, a.stride(0),
          b.stride(0), N, M * N, 1 if f32 else 0, 1 if f32 else 0, 1.0, ptr(pl.expert_off),
          ptr(pl.k_len), ptr(status_word(a.device)), 0, stream_ptr())
     return out

@@ -88,6 +88,36 @@ def test_grouped_gemms_match_per_expert_products():
     assert tot[4] == 0
 
 
+@pytest.mark.parametrize("M,N", [(128, 320), (256, 256), (384, 264), (640, 520)])
+@pytest.mark.parametrize("dtype", [BF16, torch.float32])
+def test_grouped_wgrad_single_and_pair_kernels(M, N, dtype):
+    """Grouped weight gradient with an empty first, middle and last group and tile remainders in M and
+    N, with and without accumulation, on the CTA-pair kernel and on the single-CTA one."""
+    from prometheus_b200.ops import moe
+    from prometheus_b200.ops._lib import call
+
+    E, T = 5, 500
+    ids = (1 + 2 * torch.randint(0, 2, (T, 1), device="cuda", dtype=torch.int32)).contiguous()   # groups 1 and 3
+    pl = moe.place(ids, E)
+    a, b = moe.permute(_r(T, M, seed=1), pl), moe.permute(_r(T, N, seed=2), pl)
+    off, tot = pl.expert_off.cpu().tolist(), pl.totals.cpu().tolist()
+    for variant in (0, 8):
+        try:
+            call("pb_gemm_set_variant", variant)
+            fresh = moe.grouped_wgrad(a, b, pl, torch.full((E, M, N), float("nan"), dtype=dtype, device="cuda"), False)
+            acc = moe.grouped_wgrad(a, b, pl, torch.full((E, M, N), 0.5, dtype=dtype, device="cuda"), True)
+        finally:
+            call("pb_gemm_set_variant", 0)
+        for e in range(E):
+            seg = slice(off[e], off[e] + tot[e])
+            ref = a[seg].float().t() @ b[seg].float()
+            if tot[e]:
+                _close(fresh[e], ref, 2e-2)
+                _close(acc[e], 0.5 + ref, 2e-2)
+            else:
+                assert (fresh[e] == 0).all() and (acc[e] == 0.5).all()
+
+
 @pytest.mark.parametrize("n_shared", [0, 2])
 def test_moe_ffn_matches_fp32_reference(n_shared):
     from prometheus_b200.ops import functional as ops
