@@ -660,6 +660,22 @@ __global__ void __launch_bounds__(512) softcap_ce_kernel(bf16* __restrict__ logi
   }
 }
 
+// out[i] = bf16(x[i] * g[0]): the unembedding gradient leaves its fp32 accumulator scaled by the
+// upstream gradient (a device scalar) in one pass. 131072 x 2048: an fp32 product and a conversion
+// as two library passes 976 us -> 223 us (1.6 GB).
+__global__ void __launch_bounds__(256) scale_cast_kernel(const float* __restrict__ x, const float* __restrict__ g,
+                                                         bf16* __restrict__ out, long n) {
+  const float s = *g;
+  const long i = (blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x) * 8;
+  if (i + 8 <= n) {
+    const float4 a = *reinterpret_cast<const float4*>(x + i), b = *reinterpret_cast<const float4*>(x + i + 4);
+    const float f[8] = {a.x * s, a.y * s, a.z * s, a.w * s, b.x * s, b.y * s, b.z * s, b.w * s};
+    *reinterpret_cast<bf16x8*>(out + i) = pack8(f);
+  } else {
+    for (long j = i; j < n; ++j) out[j] = f32_to_bf16(x[j] * s);
+  }
+}
+
 // out[i] = sigmoid(x[i]) (bf16 -> bf16), dx = dy * s * (1 - s)
 __global__ void sigmoid_fwd_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, long n) {
   for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < n;
@@ -893,6 +909,14 @@ PB_API int pb_softcap_ce(void* logits, const void* targets, const void* wt, void
       static_cast<bf16*>(logits), static_cast<const int*>(targets),
       static_cast<const float*>(wt), static_cast<float*>(loss_rows),
       static_cast<float*>(lse_rows), V, cap, write_grad);
+  return cudaGetLastError();
+}
+
+// x fp32 [n], g fp32 [1], out bf16 [n]; x and out 16-byte aligned.
+PB_API int pb_scale_cast(const void* x, const void* g, void* out, long n, cudaStream_t st) {
+  if (n <= 0 || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15)) return PB_BAD_ARG;
+  scale_cast_kernel<<<static_cast<unsigned>((n + 2047) / 2048), 256, 0, st>>>(
+      static_cast<const float*>(x), static_cast<const float*>(g), static_cast<bf16*>(out), n);
   return cudaGetLastError();
 }
 

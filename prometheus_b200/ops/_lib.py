@@ -35,6 +35,7 @@ _SIGS = {
     "pb_l2norm_bwd": [P, P, P, L, I, P],
     "pb_softcap_ce": [P, P, P, P, P, L, I, F, I, P],
     "pb_sigmoid": [P, P, L, P],
+    "pb_scale_cast": [P, P, P, L, P],
     "pb_sumsq_nparts": [L],
     "pb_sumsq_f32": [P, L, P, P, I, P],
     "pb_sumsq_bf16": [P, L, P, P, I, P],

@@ -446,7 +446,7 @@ class _SoftcapCeFn(torch.autograd.Function):
         mg = getattr(U, "main_grad", None)
         dU = None
         if need_U and mg is None:
-            dU = torch.zeros((V, d), dtype=torch.float32, device=dev)
+            dU = (torch.empty if rows else torch.zeros)((V, d), dtype=torch.float32, device=dev)
         acc = mg if mg is not None else dU
         for r0 in range(0, rows, chunk_rows):
             r1 = min(rows, r0 + chunk_rows)
@@ -456,8 +456,8 @@ class _SoftcapCeFn(torch.autograd.Function):
                  ptr(loss_rows[r0:r1]), None, r1 - r0, V, float(cap), write_grad, stream_ptr())
             if need_h:
                 gemm(logits, U, b_mn=True, out=dh[r0:r1])
-            if need_U:
-                gemm(logits, hc, a_mn=True, b_mn=True, out=acc, d=acc, beta=1.0)
+            if need_U:          # the first chunk of a fresh accumulator writes it: no fill, no read
+                gemm(logits, hc, a_mn=True, b_mn=True, out=acc, d=acc if mg is not None or r0 else None, beta=1.0)
             del logits
         ctx.save_for_backward(dh, dU)
         ctx.U_ref = U
@@ -471,7 +471,14 @@ class _SoftcapCeFn(torch.autograd.Function):
         gh = (dh * g.to(dh.dtype)) if dh is not None else None
         gU = None
         if dU is not None:
-            gU = (dU * g).to(ctx.U_ref.dtype)
+            # one pass for a plain first-order backward; a batched or differentiated upstream
+            # gradient goes through tensor operations
+            if (g.is_cuda and g.dtype == torch.float32 and ctx.U_ref.dtype == BF16 and dU.numel()
+                    and not torch.is_grad_enabled() and not torch._C._functorch.is_functorch_wrapped_tensor(g)):
+                gU = torch.empty(dU.shape, dtype=BF16, device=dU.device)
+                call("pb_scale_cast", ptr(dU), ptr(g), ptr(gU), dU.numel(), stream_ptr())
+            else:
+                gU = (dU * g).to(ctx.U_ref.dtype)
         return gh, gU, None, None, None, None
 
 

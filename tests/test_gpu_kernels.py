@@ -279,6 +279,35 @@ def test_softcap_ce_fused(cap):
     _close(U.grad, Ur.grad, 5e-2)
 
 
+@pytest.mark.parametrize("n", [1, 7, 8, 2047, 2056, 100003])
+def test_scale_cast(n):
+    from prometheus_b200.ops._lib import call, ptr, stream_ptr
+
+    x = _r(n, seed=n, dtype=torch.float32)
+    g = torch.full((1,), 0.37, device="cuda")
+    out = torch.empty(n, dtype=BF16, device="cuda")
+    call("pb_scale_cast", ptr(x), ptr(g), ptr(out), n, stream_ptr())
+    assert torch.equal(out, (x * g).to(BF16))
+
+
+def test_softcap_ce_fresh_gradient_chunks():
+    """A unembedding gradient that is not accumulated: one chunk, several, and a non-unit upstream
+    gradient, against the accumulating form's buffer (fp32 sums of the same products)."""
+    from prometheus_b200.ops import functional as ops
+
+    rows, d, V, cap = 130, 128, 1032, 30.0
+    h, U = _r(rows, d, seed=3), _r(V, d, seed=4, scale=0.1)
+    tgt = torch.randint(0, V, (rows,), device="cuda", dtype=torch.int32)
+    wt = torch.full((rows,), 1.0 / rows, device="cuda")
+    for chunk in (64, 4096):
+        Ug = U.clone().requires_grad_(True)
+        (gU,) = torch.autograd.grad(2.5 * ops.softcap_cross_entropy(h, Ug, tgt, wt, cap, chunk_rows=chunk), (Ug,))
+        Um = U.clone().requires_grad_(True)
+        Um.main_grad = torch.zeros(V, d, device="cuda")
+        ops.softcap_cross_entropy(h, Um, tgt, wt, cap, chunk_rows=chunk)
+        assert torch.equal(gU, (Um.main_grad * 2.5).to(BF16))
+
+
 def test_optimizer_kernels():
     from prometheus_b200 import train
     from prometheus_b200.ops import _lib
