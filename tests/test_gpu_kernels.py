@@ -431,6 +431,31 @@ def test_delta_rule_segmented_walk_equals_single_pass(B, S, H, seg):
     _close(cut[6], s0r.grad, 6e-2)
 
 
+@pytest.mark.parametrize("n_seq,n_seg", [(1, 1), (3, 8)])
+@pytest.mark.parametrize("reverse", [0, 1])
+def test_delta_compose(n_seq, n_seg, reverse):
+    """The fold of the segments' maps against 64 bits: 128 fp32 products a step, n_seg steps."""
+    from prometheus_b200.ops._lib import call, ptr, stream_ptr
+
+    p = _r(n_seq, n_seg, 128, 128, seed=1, scale=0.08, dtype=torch.float32)
+    r = _r(n_seq, n_seg, 128, 128, seed=2, dtype=torch.float32)
+    s0 = _r(n_seq, 128, 128, seed=3, dtype=torch.float32)
+    s_in, s_fin, p_tot = torch.empty_like(r), torch.empty_like(s0), torch.empty_like(s0)
+    for start in (s0, None):
+        call("pb_delta_compose", ptr(p), ptr(r), ptr(start), ptr(s_in), ptr(s_fin), None if reverse else ptr(p_tot),
+             n_seq, n_seg, reverse, stream_ptr())
+        cur = torch.zeros_like(s0).double() if start is None else start.double()
+        tot = torch.eye(128, device="cuda").double().expand(n_seq, 128, 128)
+        for j in reversed(range(n_seg)) if reverse else range(n_seg):
+            assert (s_in[:, j].double() - cur).norm() <= 1e-5 * (cur.norm() + 1e-6)
+            m = p[:, j].double()
+            cur = (m.transpose(1, 2) if reverse else m) @ cur + r[:, j].double()
+            tot = m @ tot
+        assert (s_fin.double() - cur).norm() <= 1e-5 * cur.norm()
+        if not reverse:
+            assert (p_tot.double() - tot).norm() <= 1e-5 * tot.norm()
+
+
 def test_delta_prep_bwd_kernel_matches_fp32_oracle():
     """The fused chunk-local backward against the same algebra in batched fp32 PyTorch."""
     from prometheus_b200.ops import delta as dl
