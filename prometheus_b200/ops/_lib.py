@@ -56,6 +56,7 @@ _SIGS = {
     "pb_delta_scan_bwd_seg": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, P, P],
     "pb_delta_scan_summary_fwd": [P, P, P, P, P, I, I, I, I, I, P, P],
     "pb_delta_scan_summary_bwd": [P, P, P, P, P, P, I, I, I, I, I, P, P],
+    "pb_delta_chunk_products": [P, P, P, P, P, P, P, P, P, I, I, I, I, P, P],
     "pb_delta_compose": [P, P, P, P, P, P, I, I, I, P],
     "pb_latent_gather": [P, P, I, I, I, I, I, P],
     "pb_latent_scatter": [P, P, I, I, I, I, I, P],

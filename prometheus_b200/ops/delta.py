@@ -192,7 +192,8 @@ class _DeltaFusedFn(torch.autograd.Function):
     """Delta rule, head dim 128, chunk 64, sequence a multiple of 64, on three kernels: the
     chunk-local WY operands (``pb_delta_prep_fwd``), the forward state walk and the backward
     state walk. q, k, v are read in place from their ``[B, S, H, 128]`` layout and the output
-    is written in that layout. The chunk-local part of the backward is batched tcgen05 GEMMs.
+    is written in that layout. The chunk-local part of the backward is
+    one kernel of batched products (``pb_delta_chunk_products``) and ``pb_delta_prep_bwd``.
 
     The walk is affine in the state, ``S_out = P S_in + R`` per run of chunks. When the batch
     has too few sequences to fill the GPU (``scan_segments`` > 1), or when the sequence is
@@ -261,7 +262,7 @@ class _DeltaFusedFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, d_out, d_sfin):
         from ._lib import call, ptr, stream_ptr
-        from .functional import gemm, status_word
+        from .functional import status_word
 
         q, k, v, beta, w, m, ap, t, u, sb, p_map = ctx.saved_tensors
         b, s, h, d = q.shape
@@ -292,11 +293,10 @@ class _DeltaFusedFn(torch.autograd.Function):
                  bh, seg, 1, stream_ptr())
             call("pb_delta_scan_bwd_seg", ptr(w), ptr(q), ptr(k), ptr(m), ptr(d_out), ptr(ndu),
                  ptr(dsb), ptr(g_in), None, bh, n, seg, h, h * d, status, stream_ptr())
-        doc = _to_chunks(d_out, n)
-        d_w = gemm(ndu, sb)                                   # dW = -dU S^T
-        d_m = gemm(doc, u)                                    # dM = dO U^T (masked in the kernel)
-        d_qs = gemm(doc, sb)                                  # walk's dQ = dO S^T
-        d_ks = gemm(u, dsb)                                   # walk's dK = U dS'^T
+        # dW = -dU S^T, the walk's dQ = dO S^T and dK = U dS'^T, dM = dO U^T (masked in the kernel)
+        d_w, d_qs, d_ks, d_m = (torch.empty_like(u), torch.empty_like(u), torch.empty_like(u), torch.empty_like(m))
+        call("pb_delta_chunk_products", ptr(ndu), ptr(d_out), ptr(u), ptr(sb), ptr(dsb), ptr(d_w), ptr(d_qs),
+             ptr(d_ks), ptr(d_m), b, s, h, h * d, status, stream_ptr())
         d_q, d_k, d_v = torch.empty_like(q), torch.empty_like(q), torch.empty_like(q)
         d_beta = torch.empty_like(beta)
         call("pb_delta_prep_bwd", ptr(q), ptr(k), ptr(v), ptr(beta),

@@ -431,6 +431,30 @@ def test_delta_rule_segmented_walk_equals_single_pass(B, S, H, seg):
     _close(cut[6], s0r.grad, 6e-2)
 
 
+@pytest.mark.parametrize("B,S,H", [(1, 64, 1), (2, 100, 3), (5, 4096, 2)])
+def test_delta_chunk_products(B, S, H):
+    """The four products against batched fp32, with fewer and with more chunks than CTAs."""
+    from prometheus_b200.ops import delta as dl
+    from prometheus_b200.ops import functional as ops
+    from prometheus_b200.ops._lib import call, ptr, stream_ptr
+
+    n = -(-S // 64)
+    G = B * H * n
+    ndu, u = _r(G, 64, 128, seed=1), _r(G, 64, 128, seed=2)
+    sb, dsb = _r(G, 128, 128, seed=3, scale=0.2), _r(G, 128, 128, seed=4, scale=0.2)
+    d_out = _r(B, S, H, 128, seed=5)
+    d_w, d_q, d_k = (torch.full_like(u, float("nan")) for _ in range(3))
+    d_m = torch.full((G, 64, 64), float("nan"), dtype=BF16, device="cuda")
+    call("pb_delta_chunk_products", ptr(ndu), ptr(d_out), ptr(u), ptr(sb), ptr(dsb), ptr(d_w), ptr(d_q), ptr(d_k),
+         ptr(d_m), B, S, H, H * 128, ptr(ops.status_word("cuda")), stream_ptr())
+    ops.check_status("cuda")
+    doc = dl._to_chunks(torch.nn.functional.pad(d_out, (0, 0, 0, 0, 0, n * 64 - S)), n).float()
+    _close(d_w, ndu.float() @ sb.float().transpose(1, 2), 1e-2)
+    _close(d_q, doc @ sb.float().transpose(1, 2), 1e-2)
+    _close(d_k, u.float() @ dsb.float().transpose(1, 2), 1e-2)
+    _close(d_m, doc @ u.float().transpose(1, 2), 1e-2)
+
+
 @pytest.mark.parametrize("n_seq,n_seg", [(1, 1), (3, 8)])
 @pytest.mark.parametrize("reverse", [0, 1])
 def test_delta_compose(n_seq, n_seg, reverse):
