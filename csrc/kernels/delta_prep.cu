@@ -11,9 +11,14 @@
 // accumulators in tensor memory; the unit-lower-triangular inverse is an fp32 forward
 // substitution with one column per thread (operand rows broadcast from shared memory as
 // 16-byte loads); A' goes back to shared memory as a 128-byte-swizzled bf16 operand for
-// the two products W and U^; every result leaves by a TMA store. Two CTAs of 64 threads
-// share an SM (256 tensor-memory columns each), so one chunk's substitution overlaps the
-// other's loads, products and stores.
+// the two products W and U^; every result leaves by a TMA store. A chunk is one long chain of
+// waits in two warps, so what counts is how many chunks an SM has in flight: three CTAs of 64
+// threads (75 KB and 128 tensor-memory columns each: U^ takes W's columns once W is in
+// registers). With two CTAs and columns of its own for U^, 4096 chunks took 165 us, with three
+// 141 us.
+//
+// Sequences need not be a multiple of 64 tokens: the token tensors are mapped per batch entry, so the
+// rows the last chunk lacks load as zeros and are clipped from the stores; their beta counts as 0.
 //
 // Reference semantics: kernels/__init__.py:357-376 of the reference (per-token delta-rule
 // recurrence); the chunked WY algebra and this kernel are this library's own.
@@ -30,14 +35,19 @@ int make_tmap_3d(CUtensorMap* tm, const void* base, int elem_bytes, uint64_t inn
 namespace dprep {
 
 constexpr int C = 64, D = 128;
-constexpr int KT = 0, QT = 16384, VT = 32768, AF = 49152, AP = 65536, BARS = 73728;
-constexpr int SMEM_BYTES = 100 * 1024;  // also keeps residency at two CTAs per SM
-constexpr int TMEM_COLS = 256;
+// A 64-row tile that serves as a 128-row A operand is read 8 KB past its end (A', the second halves of
+// K and Q); what follows each of them is inside the allocation, so the fp32 image of A, which no
+// product reads, comes last.
+constexpr int AP = 0, KT = 8192, QT = 24576, VT = 40960, AF = 57344, BARS = 73728;
+static_assert(AP + 16384 <= BARS && KT + 24576 <= BARS && QT + 24576 <= BARS, "A operands stay in bounds");
+constexpr int SMEM_BYTES = BARS + 256 + 1024;   // three CTAs per SM
+constexpr int FWD_CTAS = 3, FWD_COLS = 128;
+constexpr int TMEM_COLS = 256;   // backward
 
 struct Params {
   int n_chunks;   // chunks per sequence
   int heads;
-  int seq_len;    // tokens per sequence (multiple of 64)
+  int seq_len;    // tokens per sequence
   int total;      // batch * heads * n_chunks
   const void* beta;  // [batch, seq, heads]
   int beta_f32;
@@ -66,7 +76,7 @@ __device__ __forceinline__ void row_to_tile(uint32_t taddr, uint8_t* tile, int r
   }
 }
 
-__global__ void __launch_bounds__(64, 2)
+__global__ void __launch_bounds__(64, FWD_CTAS)
 delta_prep_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmQ,
                       const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmW,
                       const __grid_constant__ CUtensorMap tmU, const __grid_constant__ CUtensorMap tmM,
@@ -79,17 +89,18 @@ delta_prep_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   uint64_t* full = bars;
   uint64_t* mma1 = bars + 1;
   uint64_t* mma2 = bars + 2;
+  uint64_t* mma3 = bars + 3;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4);
   float4* af4 = reinterpret_cast<float4*>(smem + AF);
 
   const int r = threadIdx.x, warp = r >> 5;
   if (r == 0) {
-    mbar_init(full, 1); mbar_init(mma1, 1); mbar_init(mma2, 1);
+    mbar_init(full, 1); mbar_init(mma1, 1); mbar_init(mma2, 1); mbar_init(mma3, 1);
     fence_barrier_init();
     tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmV);
   }
   if (warp == 0) {
-    tmem_alloc(tmem_slot, TMEM_COLS);
+    tmem_alloc(tmem_slot, FWD_COLS);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -106,21 +117,24 @@ delta_prep_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   for (int g = blockIdx.x; g < p.total; g += gridDim.x, ph ^= 1) {
     const int seq = g / p.n_chunks, n = g - seq * p.n_chunks;
     const int b = seq / p.heads, h = seq - b * p.heads;
-    const int row0 = b * p.seq_len + n * C;   // token row of the projection outputs
+    const int t0 = n * C;                     // first token of the chunk
     const int x0 = h * D;
     if (r == 0) {
       tma_store_wait_read<0>();  // earlier stores have drained the tiles about to be refilled
       mbar_arrive_expect_tx(full, 3 * 16384);
-      tma_load_3d(smem + KT, &tmK, full, x0, row0, 0);
-      tma_load_3d(smem + KT + 8192, &tmK, full, x0 + 64, row0, 0);
-      tma_load_3d(smem + QT, &tmQ, full, x0, row0, 0);
-      tma_load_3d(smem + QT + 8192, &tmQ, full, x0 + 64, row0, 0);
-      tma_load_3d(smem + VT, &tmV, full, x0, row0, 0);
-      tma_load_3d(smem + VT + 8192, &tmV, full, x0 + 64, row0, 0);
+      tma_load_3d(smem + KT, &tmK, full, x0, t0, b);
+      tma_load_3d(smem + KT + 8192, &tmK, full, x0 + 64, t0, b);
+      tma_load_3d(smem + QT, &tmQ, full, x0, t0, b);
+      tma_load_3d(smem + QT + 8192, &tmQ, full, x0 + 64, t0, b);
+      tma_load_3d(smem + VT, &tmV, full, x0, t0, b);
+      tma_load_3d(smem + VT + 8192, &tmV, full, x0 + 64, t0, b);
     }
-    const size_t bidx = (static_cast<size_t>(row0) + r) * p.heads + h;
-    const float beta = p.beta_f32 ? static_cast<const float*>(p.beta)[bidx]
-                                  : bf16_to_f32(static_cast<const bf16*>(p.beta)[bidx]);
+    float beta = 0.f;
+    if (t0 + r < p.seq_len) {
+      const size_t bidx = (static_cast<size_t>(b) * p.seq_len + t0 + r) * p.heads + h;
+      beta = p.beta_f32 ? static_cast<const float*>(p.beta)[bidx]
+                        : bf16_to_f32(static_cast<const bf16*>(p.beta)[bidx]);
+    }
     bool ok = true;
     if (r == 0) {
       ok = mbar_wait(full, ph, p.status);
@@ -197,10 +211,6 @@ delta_prep_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
       for (int j = 0; j < 4; ++j)       // W = A' K -> columns [0, 128)
         umma_f16(tmem, make_sdesc_sw128(ap + j * 32, 16, 1024),
                  make_sdesc_sw128(kt + j * 2048, 8192, 1024), id_kn, j > 0);
-#pragma unroll
-      for (int j = 0; j < 4; ++j)       // U^ = A' V -> columns [128, 256)
-        umma_f16(tmem + 128, make_sdesc_sw128(ap + j * 32, 16, 1024),
-                 make_sdesc_sw128(vt + j * 2048, 8192, 1024), id_kn, j > 0);
       umma_commit(mma2);
       tma_store_3d(&tmM, smem + QT, 0, g * C, 0);
       tma_store_3d(&tmT, smem + QT + 8192, 0, g * C, 0);
@@ -210,17 +220,33 @@ delta_prep_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     ok = mbar_wait_spin(mma2, ph, p.status);
     if (!__syncthreads_and(ok)) break;
     tc_fence_after();
-    // W -> K tile, U^ -> V tile (both products have finished reading them), then out
+    // W -> K tile (the product has finished reading it)
     row_to_tile(lane_addr + 0, smem + KT, r, 63);
     row_to_tile(lane_addr + 64, smem + KT + 8192, r, 63);
-    row_to_tile(lane_addr + 128, smem + VT, r, 63);
-    row_to_tile(lane_addr + 192, smem + VT + 8192, r, 63);
     fence_proxy_async_smem();
     tc_fence_before();
     __syncthreads();
     if (r == 0) {
+      tc_fence_after();
+#pragma unroll
+      for (int j = 0; j < 4; ++j)       // U^ = A' V -> the same columns
+        umma_f16(tmem, make_sdesc_sw128(ap + j * 32, 16, 1024),
+                 make_sdesc_sw128(vt + j * 2048, 8192, 1024), id_kn, j > 0);
+      umma_commit(mma3);
       tma_store_3d(&tmW, smem + KT, 0, g * C, 0);
       tma_store_3d(&tmW, smem + KT + 8192, 64, g * C, 0);
+      tma_store_commit();
+    }
+    ok = mbar_wait_spin(mma3, ph, p.status);
+    if (!__syncthreads_and(ok)) break;
+    tc_fence_after();
+    // U^ -> V tile
+    row_to_tile(lane_addr + 0, smem + VT, r, 63);
+    row_to_tile(lane_addr + 64, smem + VT + 8192, r, 63);
+    fence_proxy_async_smem();
+    tc_fence_before();
+    __syncthreads();
+    if (r == 0) {
       tma_store_3d(&tmU, smem + VT, 0, g * C, 0);
       tma_store_3d(&tmU, smem + VT + 8192, 64, g * C, 0);
       tma_store_commit();
@@ -235,7 +261,7 @@ delta_prep_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   }
   if (warp == 0) {
     tc_fence_after();
-    tmem_dealloc(tmem, TMEM_COLS);
+    tmem_dealloc(tmem, FWD_COLS);
   }
 }
 
@@ -356,7 +382,7 @@ delta_prep_bwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   for (int g = blockIdx.x; g < p.total; g += gridDim.x, ph ^= 1) {
     const int seq = g / p.n_chunks, n = g - seq * p.n_chunks;
     const int b = seq / p.heads, h = seq - b * p.heads;
-    const int row0 = b * p.seq_len + n * C;
+    const int t0 = n * C;
     const int x0 = h * D;
     const int crow = g * C;
     if (r == 0) {
@@ -366,17 +392,20 @@ delta_prep_bwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
       tma_load_3d(smem + DW + 8192, &tmDW, full, 64, crow, 0);
       tma_load_3d(smem + NDU, &tmNDU, full, 0, crow, 0);
       tma_load_3d(smem + NDU + 8192, &tmNDU, full, 64, crow, 0);
-      tma_load_3d(smem + KTB, &tmK, full, x0, row0, 0);
-      tma_load_3d(smem + KTB + 8192, &tmK, full, x0 + 64, row0, 0);
-      tma_load_3d(smem + VQ, &tmV, full, x0, row0, 0);
-      tma_load_3d(smem + VQ + 8192, &tmV, full, x0 + 64, row0, 0);
+      tma_load_3d(smem + KTB, &tmK, full, x0, t0, b);
+      tma_load_3d(smem + KTB + 8192, &tmK, full, x0 + 64, t0, b);
+      tma_load_3d(smem + VQ, &tmV, full, x0, t0, b);
+      tma_load_3d(smem + VQ + 8192, &tmV, full, x0 + 64, t0, b);
       tma_load_3d(smem + APB, &tmAP, full, 0, crow, 0);
       tma_load_3d(smem + TT, &tmT, full, 0, crow, 0);
       tma_load_3d(smem + DM, &tmDM, full, 0, crow, 0);
     }
-    const size_t bidx = (static_cast<size_t>(row0) + r) * p.heads + h;
-    const float beta = p.beta_f32 ? static_cast<const float*>(p.beta)[bidx]
-                                  : bf16_to_f32(static_cast<const bf16*>(p.beta)[bidx]);
+    const bool valid = t0 + r < p.seq_len;
+    const size_t bidx = (static_cast<size_t>(b) * p.seq_len + t0 + r) * p.heads + h;
+    float beta = 0.f;
+    if (valid)
+      beta = p.beta_f32 ? static_cast<const float*>(p.beta)[bidx]
+                        : bf16_to_f32(static_cast<const bf16*>(p.beta)[bidx]);
     bool ok = true;
     // ---- pass 1: dA' parts and dV ----
     if (r == 0) {
@@ -397,8 +426,8 @@ delta_prep_bwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     tc_fence_after();
     if (r == 0) {   // V is consumed: bring Q into its place
       mbar_arrive_expect_tx(fullq, 16384);
-      tma_load_3d(smem + VQ, &tmQ, fullq, x0, row0, 0);
-      tma_load_3d(smem + VQ + 8192, &tmQ, fullq, x0 + 64, row0, 0);
+      tma_load_3d(smem + VQ, &tmQ, fullq, x0, t0, b);
+      tma_load_3d(smem + VQ + 8192, &tmQ, fullq, x0 + 64, t0, b);
     }
     // dV = -(A'^T (-dU)) -> staged over the -dU tile
     row128_to_tiles(lane_addr + 128, smem + NDU, r, -1.f, nullptr);
@@ -434,8 +463,8 @@ delta_prep_bwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     // ---- pass 2: X = dA' A'^T, Y = dA'^T T (diagonal = dbeta part), dK = A'^T dW ----
     if (r == 0) {
       tc_fence_after();
-      tma_store_3d(&tmDV, smem + NDU, x0, row0, 0);
-      tma_store_3d(&tmDV, smem + NDU + 8192, x0 + 64, row0, 0);
+      tma_store_3d(&tmDV, smem + NDU, x0, t0, b);
+      tma_store_3d(&tmDV, smem + NDU + 8192, x0 + 64, t0, b);
       tma_store_commit();
 #pragma unroll
       for (int j = 0; j < 4; ++j) umma_f16(tmem + 0, k64(tmp, j), k64(ap, j), id_kk64, j > 0);
@@ -492,8 +521,10 @@ delta_prep_bwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
         st_swz(smem + TMP, r, (c >> 3) + i, pack8(o));
       }
     }
-    if (p.beta_f32) static_cast<float*>(p.dbeta)[bidx] = dbeta;
-    else static_cast<bf16*>(p.dbeta)[bidx] = f32_to_bf16(dbeta);
+    if (valid) {
+      if (p.beta_f32) static_cast<float*>(p.dbeta)[bidx] = dbeta;
+      else static_cast<bf16*>(p.dbeta)[bidx] = f32_to_bf16(dbeta);
+    }
     fence_proxy_async_smem();
     tc_fence_before();
     __syncthreads();
@@ -526,10 +557,10 @@ delta_prep_bwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     tc_fence_before();
     __syncthreads();
     if (r == 0) {
-      tma_store_3d(&tmDQ, smem + DW, x0, row0, 0);
-      tma_store_3d(&tmDQ, smem + DW + 8192, x0 + 64, row0, 0);
-      tma_store_3d(&tmDK, smem + NDU, x0, row0, 0);
-      tma_store_3d(&tmDK, smem + NDU + 8192, x0 + 64, row0, 0);
+      tma_store_3d(&tmDQ, smem + DW, x0, t0, b);
+      tma_store_3d(&tmDQ, smem + DW + 8192, x0 + 64, t0, b);
+      tma_store_3d(&tmDK, smem + NDU, x0, t0, b);
+      tma_store_3d(&tmDK, smem + NDU + 8192, x0 + 64, t0, b);
       tma_store_commit();
     }
   }
@@ -551,15 +582,16 @@ delta_prep_bwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
 
 using namespace pb;
 
-// q, k, v: bf16 [batch * seq_len, ld] row-major with head h at columns [128 h, 128 h + 128)
+// q, k, v: bf16 [batch, seq_len, ld] row-major with head h at columns [128 h, 128 h + 128)
 // (ld >= heads * 128, a multiple of 8); beta: [batch, seq_len, heads], fp32 or bf16.
-// Outputs, chunk g = (b * heads + h) * n_chunks + n: W, U^ [g][64][128]; M, A', T [g][64][64].
+// Outputs, chunk g = (b * heads + h) * n_chunks + n, n_chunks = ceil(seq_len / 64): W, U^ [g][64][128];
+// M, A', T [g][64][64].
 PB_API int pb_delta_prep_fwd(const void* q, const void* k, const void* v, const void* beta,
                              int beta_f32, void* W, void* Uhat, void* M, void* Ap, void* T,
                              int batch, int seq_len, int heads, int ld, int* status,
                              int max_ctas, cudaStream_t st) {
   using namespace dprep;
-  if (batch <= 0 || heads <= 0 || seq_len <= 0 || seq_len % C != 0 || ld < heads * D || ld % 8)
+  if (batch <= 0 || heads <= 0 || seq_len <= 0 || ld < heads * D || ld % 8)
     return PB_BAD_ARG;
   static pb::DeviceOnce attr_once;   // per device: the attribute belongs to the current GPU
   if (attr_once.need()) {
@@ -569,16 +601,16 @@ PB_API int pb_delta_prep_fwd(const void* q, const void* k, const void* v, const 
     attr_once.done();
   }
   Params p;
-  p.n_chunks = seq_len / C; p.heads = heads; p.seq_len = seq_len;
+  p.n_chunks = (seq_len + C - 1) / C; p.heads = heads; p.seq_len = seq_len;
   p.total = batch * heads * p.n_chunks;
   p.beta = beta; p.beta_f32 = beta_f32; p.status = status;
-  const uint64_t tok = static_cast<uint64_t>(batch) * seq_len;
+  const uint64_t bstr = static_cast<uint64_t>(seq_len) * ld;   // batch stride of the token tensors
   const uint64_t rows = static_cast<uint64_t>(p.total) * C;
   CUtensorMap tK, tQ, tV, tW, tU, tM, tA, tT;
   int r = 0;
-  r |= make_tmap_3d(&tK, k, 2, static_cast<uint64_t>(heads) * D, tok, 1, ld, 0, 64, C);
-  r |= make_tmap_3d(&tQ, q, 2, static_cast<uint64_t>(heads) * D, tok, 1, ld, 0, 64, C);
-  r |= make_tmap_3d(&tV, v, 2, static_cast<uint64_t>(heads) * D, tok, 1, ld, 0, 64, C);
+  r |= make_tmap_3d(&tK, k, 2, static_cast<uint64_t>(heads) * D, seq_len, batch, ld, bstr, 64, C);
+  r |= make_tmap_3d(&tQ, q, 2, static_cast<uint64_t>(heads) * D, seq_len, batch, ld, bstr, 64, C);
+  r |= make_tmap_3d(&tV, v, 2, static_cast<uint64_t>(heads) * D, seq_len, batch, ld, bstr, 64, C);
   r |= make_tmap_3d(&tW, W, 2, D, rows, 1, D, 0, 64, C);
   r |= make_tmap_3d(&tU, Uhat, 2, D, rows, 1, D, 0, 64, C);
   r |= make_tmap_3d(&tM, M, 2, C, rows, 1, C, 0, 64, C);
@@ -588,7 +620,7 @@ PB_API int pb_delta_prep_fwd(const void* q, const void* k, const void* v, const 
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  int grid = 2 * sms;
+  int grid = FWD_CTAS * sms;
   if (max_ctas > 0 && max_ctas < grid) grid = max_ctas;
   if (grid > p.total) grid = p.total;
   delta_prep_fwd_kernel<<<grid, 64, SMEM_BYTES, st>>>(tK, tQ, tV, tW, tU, tM, tA, tT, p);
@@ -605,7 +637,7 @@ PB_API int pb_delta_prep_bwd(const void* q, const void* k, const void* v, const 
                              int batch, int seq_len, int heads, int ld, int* status,
                              int max_ctas, cudaStream_t st) {
   using namespace dprep;
-  if (batch <= 0 || heads <= 0 || seq_len <= 0 || seq_len % C != 0 || ld < heads * D || ld % 8)
+  if (batch <= 0 || heads <= 0 || seq_len <= 0 || ld < heads * D || ld % 8)
     return PB_BAD_ARG;
   static pb::DeviceOnce attr_once;   // per device: the attribute belongs to the current GPU
   if (attr_once.need()) {
@@ -616,28 +648,28 @@ PB_API int pb_delta_prep_bwd(const void* q, const void* k, const void* v, const 
     attr_once.done();
   }
   BwdParams p;
-  p.n_chunks = seq_len / C; p.heads = heads; p.seq_len = seq_len;
+  p.n_chunks = (seq_len + C - 1) / C; p.heads = heads; p.seq_len = seq_len;
   p.total = batch * heads * p.n_chunks;
   p.beta = beta; p.beta_f32 = beta_f32;
   p.dq_add = static_cast<const bf16*>(dq_add);
   p.dk_add = static_cast<const bf16*>(dk_add);
   p.dbeta = dbeta; p.status = status;
-  const uint64_t tok = static_cast<uint64_t>(batch) * seq_len;
+  const uint64_t bstr = static_cast<uint64_t>(seq_len) * ld;   // batch stride of the token tensors
   const uint64_t rows = static_cast<uint64_t>(p.total) * C;
   const uint64_t hd = static_cast<uint64_t>(heads) * D;
   CUtensorMap tK, tQ, tV, tDW, tNDU, tDM, tA, tT, tDQ, tDK, tDV;
   int r = 0;
-  r |= make_tmap_3d(&tK, k, 2, hd, tok, 1, ld, 0, 64, C);
-  r |= make_tmap_3d(&tQ, q, 2, hd, tok, 1, ld, 0, 64, C);
-  r |= make_tmap_3d(&tV, v, 2, hd, tok, 1, ld, 0, 64, C);
+  r |= make_tmap_3d(&tK, k, 2, hd, seq_len, batch, ld, bstr, 64, C);
+  r |= make_tmap_3d(&tQ, q, 2, hd, seq_len, batch, ld, bstr, 64, C);
+  r |= make_tmap_3d(&tV, v, 2, hd, seq_len, batch, ld, bstr, 64, C);
   r |= make_tmap_3d(&tDW, dW, 2, D, rows, 1, D, 0, 64, C);
   r |= make_tmap_3d(&tNDU, ndU, 2, D, rows, 1, D, 0, 64, C);
   r |= make_tmap_3d(&tDM, dM, 2, C, rows, 1, C, 0, 64, C);
   r |= make_tmap_3d(&tA, Ap, 2, C, rows, 1, C, 0, 64, C);
   r |= make_tmap_3d(&tT, T, 2, C, rows, 1, C, 0, 64, C);
-  r |= make_tmap_3d(&tDQ, dq, 2, hd, tok, 1, ld, 0, 64, C);
-  r |= make_tmap_3d(&tDK, dk, 2, hd, tok, 1, ld, 0, 64, C);
-  r |= make_tmap_3d(&tDV, dv, 2, hd, tok, 1, ld, 0, 64, C);
+  r |= make_tmap_3d(&tDQ, dq, 2, hd, seq_len, batch, ld, bstr, 64, C);
+  r |= make_tmap_3d(&tDK, dk, 2, hd, seq_len, batch, ld, bstr, 64, C);
+  r |= make_tmap_3d(&tDV, dv, 2, hd, seq_len, batch, ld, bstr, 64, C);
   if (r != 0) return 1000 + r;
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);

@@ -50,12 +50,12 @@ _SIGS = {
     "pb_transpose_bf16": [P, P, I, I, I, P],
     "pb_wait_flag_probe": [P, I, L, P, P],
     "pb_set_flag": [P, I, P],
-    "pb_delta_scan_fwd": [P, P, P, P, P, P, P, P, P, P, I, I, I, I, P, P],
-    "pb_delta_scan_bwd": [P, P, P, P, P, P, P, P, P, I, I, I, I, P, P],
-    "pb_delta_scan_fwd_seg": [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, P, P],
-    "pb_delta_scan_bwd_seg": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, P, P],
-    "pb_delta_scan_summary_fwd": [P, P, P, P, P, I, I, I, I, I, P, P],
-    "pb_delta_scan_summary_bwd": [P, P, P, P, P, P, I, I, I, I, I, P, P],
+    "pb_delta_scan_fwd": [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, P, P],
+    "pb_delta_scan_bwd": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, P, P],
+    "pb_delta_scan_fwd_seg": [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, P, P],
+    "pb_delta_scan_bwd_seg": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, P, P],
+    "pb_delta_scan_summary_fwd": [P, P, P, P, P, I, I, I, I, I, I, P, P],
+    "pb_delta_scan_summary_bwd": [P, P, P, P, P, P, I, I, I, I, I, I, P, P],
     "pb_delta_chunk_products": [P, P, P, P, P, P, P, P, P, I, I, I, I, P, P],
     "pb_delta_compose": [P, P, P, P, P, P, I, I, I, P],
     "pb_latent_gather": [P, P, I, I, I, I, I, P],

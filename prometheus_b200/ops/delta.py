@@ -188,12 +188,20 @@ def scan_segments(n_seq: int, n_chunks: int, ctas: int = 148) -> int:
     return best
 
 
+def _tma_ready(x: Tensor) -> Tensor:
+    """Contiguous and 16-byte aligned: what the kernels' tensor maps need."""
+    x = x.contiguous()
+    return x if x.data_ptr() % 16 == 0 else x.clone()
+
+
 class _DeltaFusedFn(torch.autograd.Function):
-    """Delta rule, head dim 128, chunk 64, sequence a multiple of 64, on three kernels: the
+    """Delta rule, head dim 128, chunk 64, any sequence length, on three kernels: the
     chunk-local WY operands (``pb_delta_prep_fwd``), the forward state walk and the backward
     state walk. q, k, v are read in place from their ``[B, S, H, 128]`` layout and the output
-    is written in that layout. The chunk-local part of the backward is
+    is written in that layout; the rows a last partial chunk lacks read as zeros with beta = 0,
+    which leaves the state untouched, and are not written. The chunk-local part of the backward is
     one kernel of batched products (``pb_delta_chunk_products``) and ``pb_delta_prep_bwd``.
+    ``keep``: something will run backward, so the walk's U and bf16 states are stored.
 
     The walk is affine in the state, ``S_out = P S_in + R`` per run of chunks. When the batch
     has too few sequences to fill the GPU (``scan_segments`` > 1), or when the sequence is
@@ -204,16 +212,16 @@ class _DeltaFusedFn(torch.autograd.Function):
     length instead of one full-length pass. The backward does the same with ``P^T``."""
 
     @staticmethod
-    def forward(ctx, q, k, v, beta, s0, cp=None, n_seg=None):
+    def forward(ctx, q, k, v, beta, s0, cp=None, n_seg=None, keep=True):
         from ._lib import call, ptr, stream_ptr
         from .functional import status_word
 
         b, s, h, d = q.shape
-        n = s // 64
+        n = -(-s // 64)
         g = b * h * n
         bh = b * h
         dev = q.device
-        q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
+        q, k, v = _tma_ready(q), _tma_ready(k), _tma_ready(v)
         beta = beta.contiguous()
         bf = torch.bfloat16
         w = torch.empty((g, 64, 128), dtype=bf, device=dev)
@@ -226,21 +234,21 @@ class _DeltaFusedFn(torch.autograd.Function):
              1 if beta.dtype == torch.float32 else 0, ptr(w), ptr(uhat), ptr(m), ptr(ap), ptr(t),
              b, s, h, h * d, status, 0, stream_ptr())
         out = torch.empty_like(q)
-        u = torch.empty_like(w)
-        sb = torch.empty((g, 128, 128), dtype=bf, device=dev)
+        u = torch.empty_like(w) if keep else None
+        sb = torch.empty((g, 128, 128), dtype=bf, device=dev) if keep else None
         sfin = torch.empty((bh, 128, 128), dtype=torch.float32, device=dev)
         s0c = None if s0 is None else s0.reshape(bh, d, d).float().contiguous()
         seg = int(n_seg) if n_seg else scan_segments(bh, n)
         p_map = None
         if seg == 1 and cp is None:
             call("pb_delta_scan_fwd", ptr(w), ptr(uhat), ptr(q), ptr(k), ptr(m), ptr(out), ptr(u),
-                 ptr(sb), ptr(s0c), ptr(sfin), bh, n, h, h * d, status, stream_ptr())
+                 ptr(sb), ptr(s0c), ptr(sfin), bh, n, h, s, h * d, status, stream_ptr())
         else:
             f32 = dict(dtype=torch.float32, device=dev)
             r_map = torch.empty((bh * seg, 128, 128), **f32)
             p_map = torch.empty_like(r_map)
             call("pb_delta_scan_summary_fwd", ptr(w), ptr(uhat), ptr(k), ptr(r_map), ptr(p_map),
-                 bh, n, seg, h, h * d, status, stream_ptr())
+                 bh, n, seg, h, s, h * d, status, stream_ptr())
             if cp is not None:
                 # this rank's whole slice as one map, exchanged; what comes back is the state
                 # entering the slice
@@ -253,8 +261,9 @@ class _DeltaFusedFn(torch.autograd.Function):
             call("pb_delta_compose", ptr(p_map), ptr(r_map), ptr(s0c), ptr(s_in), ptr(sfin), None,
                  bh, seg, 0, stream_ptr())
             call("pb_delta_scan_fwd_seg", ptr(w), ptr(uhat), ptr(q), ptr(k), ptr(m), ptr(out), ptr(u),
-                 ptr(sb), ptr(s_in), None, bh, n, seg, h, h * d, status, stream_ptr())
-        ctx.save_for_backward(q, k, v, beta, w, m, ap, t, u, sb, p_map)
+                 ptr(sb), ptr(s_in), None, bh, n, seg, h, s, h * d, status, stream_ptr())
+        if keep:
+            ctx.save_for_backward(q, k, v, beta, w, m, ap, t, u, sb, p_map)
         ctx.has_s0 = s0 is not None
         ctx.seg, ctx.cp = seg, cp
         return out, sfin.reshape(b, h, d, d)
@@ -266,11 +275,11 @@ class _DeltaFusedFn(torch.autograd.Function):
 
         q, k, v, beta, w, m, ap, t, u, sb, p_map = ctx.saved_tensors
         b, s, h, d = q.shape
-        n = s // 64
+        n = -(-s // 64)
         bh = b * h
         dev = q.device
         seg, cp = ctx.seg, ctx.cp
-        d_out = d_out.contiguous()
+        d_out = _tma_ready(d_out)
         ndu = torch.empty_like(u)          # the kernel writes -dU
         dsb = torch.empty_like(sb)
         ds0 = torch.empty((bh, 128, 128), dtype=torch.float32, device=dev)
@@ -278,11 +287,11 @@ class _DeltaFusedFn(torch.autograd.Function):
         status = ptr(status_word(dev))
         if p_map is None:
             call("pb_delta_scan_bwd", ptr(w), ptr(q), ptr(k), ptr(m), ptr(d_out), ptr(ndu), ptr(dsb),
-                 ptr(dfin), ptr(ds0), bh, n, h, h * d, status, stream_ptr())
+                 ptr(dfin), ptr(ds0), bh, n, h, s, h * d, status, stream_ptr())
         else:
             g_map = torch.empty_like(p_map)
             call("pb_delta_scan_summary_bwd", ptr(w), ptr(q), ptr(k), ptr(m), ptr(d_out), ptr(g_map),
-                 bh, n, seg, h, h * d, status, stream_ptr())
+                 bh, n, seg, h, s, h * d, status, stream_ptr())
             if cp is not None:
                 g_tot = torch.empty((bh, 128, 128), dtype=torch.float32, device=dev)
                 call("pb_delta_compose", ptr(p_map), ptr(g_map), None, None, ptr(g_tot), None,
@@ -292,7 +301,7 @@ class _DeltaFusedFn(torch.autograd.Function):
             call("pb_delta_compose", ptr(p_map), ptr(g_map), ptr(dfin), ptr(g_in), ptr(ds0), None,
                  bh, seg, 1, stream_ptr())
             call("pb_delta_scan_bwd_seg", ptr(w), ptr(q), ptr(k), ptr(m), ptr(d_out), ptr(ndu),
-                 ptr(dsb), ptr(g_in), None, bh, n, seg, h, h * d, status, stream_ptr())
+                 ptr(dsb), ptr(g_in), None, bh, n, seg, h, s, h * d, status, stream_ptr())
         # dW = -dU S^T, the walk's dQ = dO S^T and dK = U dS'^T, dM = dO U^T (masked in the kernel)
         d_w, d_qs, d_ks, d_m = (torch.empty_like(u), torch.empty_like(u), torch.empty_like(u), torch.empty_like(m))
         call("pb_delta_chunk_products", ptr(ndu), ptr(d_out), ptr(u), ptr(sb), ptr(dsb), ptr(d_w), ptr(d_qs),
@@ -303,7 +312,7 @@ class _DeltaFusedFn(torch.autograd.Function):
              1 if beta.dtype == torch.float32 else 0, ptr(ap), ptr(t), ptr(d_w), ptr(ndu), ptr(d_m),
              ptr(d_qs), ptr(d_ks), ptr(d_q), ptr(d_k), ptr(d_v), ptr(d_beta), b, s, h, h * d,
              status, 0, stream_ptr())
-        return (d_q, d_k, d_v, d_beta, (ds0.reshape(b, h, d, d) if ctx.has_s0 else None), None, None)
+        return (d_q, d_k, d_v, d_beta, (ds0.reshape(b, h, d, d) if ctx.has_s0 else None), None, None, None)
 
 
 def delta_prep_backward_ref(q, k, v, beta, ap, t, d_w, ndu, d_m, d_qs, d_ks):
@@ -333,20 +342,12 @@ def delta_prep_backward_ref(q, k, v, beta, ap, t, d_w, ndu, d_m, d_qs, d_ks):
 
 def delta_rule_fused(q: Tensor, k: Tensor, v: Tensor, beta: Tensor, state: Tensor | None,
                      cp=None, n_seg: int | None = None):
-    """bf16, head dim 128, chunk 64 (sequences are zero-padded to a multiple of 64: padded
-    tokens have beta = 0 and k = 0, so they leave the state untouched). ``cp``: a
+    """bf16, head dim 128, chunk 64, any sequence length. ``cp``: a
     ``parallel.cp.DeltaCpContext`` when the sequence is split over ranks (``state`` is then
     ignored: the incoming state is what the earlier ranks hand over). ``n_seg`` overrides the
     number of segments per sequence (default: ``scan_segments``)."""
-    s = q.shape[1]
-    pad = (-s) % 64
-    if pad:
-        q = torch.nn.functional.pad(q, (0, 0, 0, 0, 0, pad))
-        k = torch.nn.functional.pad(k, (0, 0, 0, 0, 0, pad))
-        v = torch.nn.functional.pad(v, (0, 0, 0, 0, 0, pad))
-        beta = torch.nn.functional.pad(beta, (0, 0, 0, pad))
-    out, sfin = _DeltaFusedFn.apply(q, k, v, beta, state, cp, n_seg)
-    return (out[:, :s] if pad else out), sfin
+    keep = torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (q, k, v, beta, state))
+    return _DeltaFusedFn.apply(q, k, v, beta, state, cp, n_seg, keep)
 
 
 class UnsupportedGeometry(ValueError):

@@ -431,6 +431,45 @@ def test_delta_rule_segmented_walk_equals_single_pass(B, S, H, seg):
     _close(cut[6], s0r.grad, 6e-2)
 
 
+@pytest.mark.parametrize("B,S,H,seg", [(2, 1, 1, 1), (3, 63, 2, 1), (2, 65, 2, 1), (2, 1000, 2, 4), (1, 250, 1, 2)])
+def test_delta_rule_ragged_equals_explicit_padding(B, S, H, seg):
+    """A length that is not a multiple of the chunk, read in place, gives the bits of the same call
+    on zero-padded tensors (batch entries follow one another without a gap, so a row too many
+    would be the next entry's), without grad as with it, and from a misaligned base."""
+    from prometheus_b200.ops import functional as ops
+    from prometheus_b200.ops.delta import delta_rule_fused
+
+    D = 128
+    q = torch.nn.functional.normalize(_r(B, S, H, D, seed=1).float(), dim=-1).to(BF16)
+    k = torch.nn.functional.normalize(_r(B, S, H, D, seed=2).float(), dim=-1).to(BF16)
+    v = _r(B, S, H, D, seed=3)
+    beta = torch.sigmoid(_r(B, S, H, seed=4).float()).to(BF16)
+    s0 = _r(B, H, D, D, seed=5, scale=0.05, dtype=torch.float32)
+    go, gs = _r(B, S, H, D, seed=6), _r(B, H, D, D, seed=7, scale=0.1, dtype=torch.float32)
+    pad = (-S) % 64
+
+    def run(ts, g):
+        leaves = [t.clone().requires_grad_(True) for t in ts]
+        s0l = s0.clone().requires_grad_(True)
+        out, st = delta_rule_fused(*leaves, s0l, n_seg=seg)
+        grads = torch.autograd.grad([out, st], leaves + [s0l], [g, gs])
+        ops.check_status("cuda")
+        return [out.detach(), st.detach(), *grads]
+
+    def padded(t):
+        return torch.cat([t, t.new_zeros(B, pad, *t.shape[2:])], dim=1)
+
+    got = run((q, k, v, beta), go)
+    want = run([padded(t) for t in (q, k, v, beta)], padded(go))
+    for name, a, b in zip(("out", "state", "dq", "dk", "dv", "dbeta", "ds0"), got, want):
+        assert torch.equal(a, b if name in ("state", "ds0") else b[:, :S]), name
+    with torch.no_grad():
+        out, st = delta_rule_fused(q, k, v, beta, s0, n_seg=seg)
+        assert torch.equal(out, got[0]) and torch.equal(st, got[1])
+        off = torch.empty(q.numel() + 1, dtype=BF16, device="cuda")[1:].view(q.shape).copy_(q)
+        assert torch.equal(delta_rule_fused(off, k, v, beta, s0, n_seg=seg)[0], out)
+
+
 @pytest.mark.parametrize("B,S,H", [(1, 64, 1), (2, 100, 3), (5, 4096, 2)])
 def test_delta_chunk_products(B, S, H):
     """The four products against batched fp32, with fewer and with more chunks than CTAs."""
