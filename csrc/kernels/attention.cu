@@ -17,7 +17,10 @@
 //
 // warps 0-3: one tensor-memory lane (= row) per thread; warp 4: MMA issue; warp 5: TMA producer.
 // All tensors are token-major: Q/O/dO/dQ [batch * seq, ldq] with head h at columns 128 h,
-// K/V/dK/dV [batch * seq, ldkv] with KV head g at columns 128 g. seq must be a multiple of 256 (forward) / 128 (backward).
+// K/V/dK/dV [batch * seq, ldkv] with KV head g at columns 128 g. Any seq: the tensor maps are per batch entry,
+// so the rows a last tile lacks read as zeros (no real query sees a key after itself, and a zero
+// query with zero dO adds nothing) and are clipped from the stores. 3 x 1000 x 16/4 forward: 84 us with
+// padded copies of q, k, v and a cut of the result, 36 us in place.
 //
 // Reference semantics: model/__init__.py gqa/mla attention (softmax(q k^T / sqrt(d)) v with a
 // causal mask) of the reference; the tiling is this library's own.
@@ -119,7 +122,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const int h = blockIdx.y, b = blockIdx.z;
   const int g = h / (p.heads / p.kv_heads);
   const int gb = cb + p.q_off / 256;   // position of this CTA's rows among all keys
-  const int row0 = b * p.seq + cb * 256;
+  const int row0 = cb * 256;           // first query row within the batch entry
   const int nj1 = 4 * gb + 4;     // 64-key blocks seen by tile 1; tile 0 sees nj1 - 2
 
   if (threadIdx.x == 0) {
@@ -145,20 +148,20 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     if (lane == 0) {
       mbar_arrive_expect_tx(q_full, 65536);
       for (int t = 0; t < 2; ++t) {
-        tma_load_3d(smem + Q_OFF + t * 32768, &tmQ, q_full, h * D, row0 + t * 128, 0);
-        tma_load_3d(smem + Q_OFF + t * 32768 + 16384, &tmQ, q_full, h * D + 64, row0 + t * 128, 0);
+        tma_load_3d(smem + Q_OFF + t * 32768, &tmQ, q_full, h * D, row0 + t * 128, b);
+        tma_load_3d(smem + Q_OFF + t * 32768 + 16384, &tmQ, q_full, h * D + 64, row0 + t * 128, b);
       }
       for (int j = 0; j < nj1; ++j) {
         const int s = j % KV_STAGES;
         const uint32_t ph = (j / KV_STAGES) & 1;
-        const int krow = b * p.seq_kv + j * 64;
+        const int krow = j * 64;
         if (!mbar_wait(&kv_empty[s], ph ^ 1, p.status)) break;
         mbar_arrive_expect_tx(&kv_full[s], KV_STAGE);
         uint8_t* st = smem + KV_OFF + s * KV_STAGE;
-        tma_load_3d(st, &tmK, &kv_full[s], g * D, krow, 0);
-        tma_load_3d(st + 8192, &tmK, &kv_full[s], g * D + 64, krow, 0);
-        tma_load_3d(st + 16384, &tmV, &kv_full[s], g * D, krow, 0);
-        tma_load_3d(st + 16384 + 8192, &tmV, &kv_full[s], g * D + 64, krow, 0);
+        tma_load_3d(st, &tmK, &kv_full[s], g * D, krow, b);
+        tma_load_3d(st + 8192, &tmK, &kv_full[s], g * D + 64, krow, b);
+        tma_load_3d(st + 16384, &tmV, &kv_full[s], g * D, krow, b);
+        tma_load_3d(st + 16384 + 8192, &tmV, &kv_full[s], g * D + 64, krow, b);
       }
     }
   } else if (warp >= 8) {
@@ -316,14 +319,17 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           st_swz(obuf + (col >> 6) * 16384, r, (col & 63) >> 3, pack_bf16x8(f));
         }
       }
-      const size_t vi = (static_cast<size_t>(b) * p.heads + h) * p.seq + cb * 256 + t * 128 + r;
-      p.lse2[vi] = m_used + log2f(l);
-      if (p.rowmax != nullptr) p.rowmax[vi] = m_true * 0.6931471805599453f;
+      const int qrow = row0 + t * 128 + r;
+      if (qrow < p.seq) {
+        const size_t vi = (static_cast<size_t>(b) * p.heads + h) * p.seq + qrow;
+        p.lse2[vi] = m_used + log2f(l);
+        if (p.rowmax != nullptr) p.rowmax[vi] = m_true * 0.6931471805599453f;
+      }
       fence_proxy_async_smem();
       sync_group();
-      if (r == 0) {
-        tma_store_3d(&tmO, obuf, h * D, row0 + t * 128, 0);
-        tma_store_3d(&tmO, obuf + 16384, h * D + 64, row0 + t * 128, 0);
+      if (r == 0 && row0 + t * 128 < p.seq) {
+        tma_store_3d(&tmO, obuf, h * D, row0 + t * 128, b);
+        tma_store_3d(&tmO, obuf + 16384, h * D + 64, row0 + t * 128, b);
         tma_store_commit();
         tma_store_wait<0>();
       }
@@ -399,10 +405,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
   const int gblk = DKV ? blk : blk + p.q_off / 128;
   const int q_off64 = p.q_off / 64;
   const int t_first = DKV ? max(0, 2 * blk - q_off64) : 0;
-  const int t_count = DKV ? max(0, p.seq / 64 - t_first) : 2 * gblk + 2;
+  const int t_count = DKV ? max(0, (p.seq + 63) / 64 - t_first) : 2 * gblk + 2;
   const int n_it = DKV ? group * t_count : t_count;
-  const int row0 = b * (DKV ? p.seq_kv : p.seq) + blk * 128;
-  const int t_seq = DKV ? p.seq : p.seq_kv;        // rows per batch entry of the streamed tensors
+  const int row0 = blk * 128;                      // within the batch entry
 
   if (threadIdx.x == 0) {
     mbar_init(r_full, 1);
@@ -433,24 +438,24 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
       // would wait for the loads to land first.
       if (n_it > 0) {
         mbar_arrive_expect_tx(r_full, 65536);
-        tma_load_3d(smem + RA_OFF, &tmRA, r_full, rx, row0, 0);
-        tma_load_3d(smem + RA_OFF + 16384, &tmRA, r_full, rx + 64, row0, 0);
-        tma_load_3d(smem + RB_OFF, &tmRB, r_full, rx, row0, 0);
-        tma_load_3d(smem + RB_OFF + 16384, &tmRB, r_full, rx + 64, row0, 0);
+        tma_load_3d(smem + RA_OFF, &tmRA, r_full, rx, row0, b);
+        tma_load_3d(smem + RA_OFF + 16384, &tmRA, r_full, rx + 64, row0, b);
+        tma_load_3d(smem + RB_OFF, &tmRB, r_full, rx, row0, b);
+        tma_load_3d(smem + RB_OFF + 16384, &tmRB, r_full, rx + 64, row0, b);
       }
       for (int it = 0; it < n_it; ++it) {
         const int s = it & 1;
         const uint32_t ph = (it >> 1) & 1;
         const int t = t_first + (DKV ? it % t_count : it);
         const int tx = (DKV ? g * group + it / t_count : g) * D;
-        const int trow = b * t_seq + t * 64;
+        const int trow = t * 64;
         if (!mbar_wait(&t_empty[s], ph ^ 1, p.status)) break;
         mbar_arrive_expect_tx(&t_full[s], 32768);
         uint8_t* st = smem + ST_OFF + s * 32768;
-        tma_load_3d(st, &tmT1, &t_full[s], tx, trow, 0);
-        tma_load_3d(st + 8192, &tmT1, &t_full[s], tx + 64, trow, 0);
-        tma_load_3d(st + 16384, &tmT2, &t_full[s], tx, trow, 0);
-        tma_load_3d(st + 16384 + 8192, &tmT2, &t_full[s], tx + 64, trow, 0);
+        tma_load_3d(st, &tmT1, &t_full[s], tx, trow, b);
+        tma_load_3d(st + 8192, &tmT1, &t_full[s], tx + 64, trow, b);
+        tma_load_3d(st + 16384, &tmT2, &t_full[s], tx, trow, b);
+        tma_load_3d(st + 16384 + 8192, &tmT2, &t_full[s], tx + 64, trow, b);
       }
     }
   } else if (warp == 8 || warp == 9) {
@@ -522,20 +527,20 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
     };
     const int pos = gblk * 128 + r;   // global query position (dQ) or key position (dKV) of this row
     float row_lse = 0.f, row_delta = 0.f;
-    if (!DKV) {
+    if (!DKV && blk * 128 + r < p.seq) {
       const size_t vi = (static_cast<size_t>(b) * p.heads + hy) * p.seq + blk * 128 + r;
       row_lse = p.lse2[vi];
       row_delta = p.delta[vi];
     }
     // dKV: per-column log-sum-exp and delta of the streamed query tile, prefetched one
     // iteration ahead by threads 0..63 (lse) and 64..127 (delta).
-    auto vec_src = [&](int it) -> const float* {
-      const int t = t_first + it % t_count;
+    auto vec_value = [&](int it) -> float {
+      const int q = (t_first + it % t_count) * 64 + (r & 63);
       const int h = g * group + it / t_count;
       const float* base = (r < 64) ? p.lse2 : p.delta;
-      return base + (static_cast<size_t>(b) * p.heads + h) * p.seq + t * 64 + (r & 63);
+      return q < p.seq ? base[(static_cast<size_t>(b) * p.heads + h) * p.seq + q] : 0.f;
     };
-    float vec_next = (DKV && wg < n_it) ? *vec_src(wg) : 0.f;
+    float vec_next = (DKV && wg < n_it) ? vec_value(wg) : 0.f;
     bool ok = true;
     for (int it = wg; it < n_it && ok; it += 2) {
       const int s = wg;
@@ -545,7 +550,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
       if (DKV) {
         sync_group();        // the group's readers of the previous tile are done
         vec[r] = vec_next;   // [0,64) lse2, [64,128) delta
-        if (it + 2 < n_it) vec_next = *vec_src(it + 2);
+        if (it + 2 < n_it) vec_next = vec_value(it + 2);
         sync_group();
       }
       if (!wait_all(&x_done[s], ph, p.status)) { ok = false; break; }
@@ -626,10 +631,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
         const int ox = (DKV ? g : hy) * D;
         if (DKV) {
           const CUtensorMap* tm = wg == 0 ? &tmO1 : &tmO2;
-          tma_store_3d(tm, stage, ox, row0, 0);
-          tma_store_3d(tm, stage + 16384, ox + 64, row0, 0);
+          tma_store_3d(tm, stage, ox, row0, b);
+          tma_store_3d(tm, stage + 16384, ox + 64, row0, b);
         } else {
-          tma_store_3d(&tmO1, stage + wg * 16384, ox + wg * 64, row0, 0);
+          tma_store_3d(&tmO1, stage + wg * 16384, ox + wg * 64, row0, b);
         }
         tma_store_commit();
         tma_store_wait<0>();
@@ -675,8 +680,13 @@ __global__ void attn_delta_kernel(const bf16* __restrict__ o, const bf16* __rest
 }
 }  // namespace bwd
 
+// map of a token-major tensor [batch, seq, ld], 64-column boxes of box_rows rows of one batch entry
+static int tok_map(CUtensorMap* tm, const void* base, uint64_t inner, int seq, int batch, int ld, int box_rows) {
+  return make_tmap_3d(tm, base, 2, inner, seq, batch, ld, static_cast<uint64_t>(seq) * ld, 64, box_rows);
+}
+
 static bool bad_geometry(int batch, int seq, int heads, int kv_heads, int ldq, int ldkv) {
-  return batch <= 0 || seq <= 0 || seq % 128 != 0 || heads <= 0 || kv_heads <= 0 ||
+  return batch <= 0 || seq <= 0 || heads <= 0 || kv_heads <= 0 ||
          heads % kv_heads != 0 || ldq < heads * D || ldkv < kv_heads * D || ldq % 8 != 0 ||
          ldkv % 8 != 0;
 }
@@ -690,8 +700,7 @@ using namespace pb;
 // at columns [128 h, 128 h + 128); k/v: [batch * seq_kv, ldkv] with KV head g likewise.
 // Query row i of a batch entry sits at global position q_off + i and sees keys 0 .. q_off + i
 // (q_off = 0 and seq_kv = seq is ordinary causal attention; a context-parallel rank passes its
-// slice of the queries, the gathered keys and its offset). seq, q_off multiples of 256;
-// seq_kv >= q_off + seq, a multiple of 128.
+// slice of the queries, the gathered keys and its offset). q_off a multiple of 256, seq_kv >= q_off + seq.
 // lse2: fp32 [batch, heads, seq], log2 of the softmax denominator plus the applied maximum.
 // rowmax (optional): fp32 [batch, heads, seq], the largest scaled logit of each row.
 PB_API int pb_attn_fwd_cp(const void* q, const void* k, const void* v, void* out, void* lse2,
@@ -700,8 +709,7 @@ PB_API int pb_attn_fwd_cp(const void* q, const void* k, const void* v, void* out
                           cudaStream_t st) {
   using namespace attn;
   if (bad_geometry(batch, seq, heads, kv_heads, ldq, ldkv) || ldo < heads * D || ldo % 8 != 0 ||
-      seq % 256 != 0 || !(scale > 0.f) || q_off < 0 || q_off % 256 != 0 || seq_kv % 128 != 0 ||
-      seq_kv < q_off + seq)
+      !(scale > 0.f) || q_off < 0 || q_off % 256 != 0 || seq_kv < q_off + seq)
     return PB_BAD_ARG;
   static pb::DeviceOnce attr_once;   // per device: the attribute belongs to the current GPU
   if (attr_once.need()) {
@@ -710,13 +718,12 @@ PB_API int pb_attn_fwd_cp(const void* q, const void* k, const void* v, void* out
     if (e != cudaSuccess) return static_cast<int>(e);
     attr_once.done();
   }
-  const uint64_t rows = static_cast<uint64_t>(batch) * seq, krows = static_cast<uint64_t>(batch) * seq_kv;
   CUtensorMap tQ, tK, tV, tO;
   int r = 0;
-  r |= make_tmap_3d(&tQ, q, 2, static_cast<uint64_t>(heads) * D, rows, 1, ldq, 0, 64, 128);
-  r |= make_tmap_3d(&tK, k, 2, static_cast<uint64_t>(kv_heads) * D, krows, 1, ldkv, 0, 64, 64);
-  r |= make_tmap_3d(&tV, v, 2, static_cast<uint64_t>(kv_heads) * D, krows, 1, ldkv, 0, 64, 64);
-  r |= make_tmap_3d(&tO, out, 2, static_cast<uint64_t>(heads) * D, rows, 1, ldo, 0, 64, 128);
+  r |= tok_map(&tQ, q, static_cast<uint64_t>(heads) * D, seq, batch, ldq, 128);
+  r |= tok_map(&tK, k, static_cast<uint64_t>(kv_heads) * D, seq_kv, batch, ldkv, 64);
+  r |= tok_map(&tV, v, static_cast<uint64_t>(kv_heads) * D, seq_kv, batch, ldkv, 64);
+  r |= tok_map(&tO, out, static_cast<uint64_t>(heads) * D, seq, batch, ldo, 128);
   if (r != 0) return 1000 + r;
   fwd::Params p;
   p.seq = seq; p.heads = heads; p.kv_heads = kv_heads;
@@ -725,7 +732,7 @@ PB_API int pb_attn_fwd_cp(const void* q, const void* k, const void* v, void* out
   p.lse2 = static_cast<float*>(lse2);
   p.rowmax = static_cast<float*>(rowmax);
   p.status = status;
-  fwd::attn_fwd_kernel<<<dim3(seq / 256, heads, batch), 352, fwd::SMEM, st>>>(tQ, tK, tV, tO, p);
+  fwd::attn_fwd_kernel<<<dim3((seq + 255) / 256, heads, batch), 352, fwd::SMEM, st>>>(tQ, tK, tV, tO, p);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -746,7 +753,7 @@ PB_API int pb_attn_bwd_cp(const void* q, const void* k, const void* v, const voi
                           cudaStream_t st) {
   using namespace attn;
   if (bad_geometry(batch, seq, heads, kv_heads, ldq, ldkv) || ldo < heads * D || ldo % 8 != 0 ||
-      !(scale > 0.f) || q_off < 0 || q_off % 128 != 0 || seq_kv % 128 != 0 || seq_kv < q_off + seq)
+      !(scale > 0.f) || q_off < 0 || q_off % 128 != 0 || seq_kv < q_off + seq)
     return PB_BAD_ARG;
   static pb::DeviceOnce attr_once;   // per device: the attribute belongs to the current GPU
   if (attr_once.need()) {
@@ -758,7 +765,7 @@ PB_API int pb_attn_bwd_cp(const void* q, const void* k, const void* v, const voi
     if (e != cudaSuccess) return static_cast<int>(e);
     attr_once.done();
   }
-  const uint64_t rows = static_cast<uint64_t>(batch) * seq, krows = static_cast<uint64_t>(batch) * seq_kv;
+  const uint64_t rows = static_cast<uint64_t>(batch) * seq;
   const uint64_t qi = static_cast<uint64_t>(heads) * D, ki = static_cast<uint64_t>(kv_heads) * D;
   {
     const long long warps = static_cast<long long>(rows) * heads;
@@ -778,27 +785,27 @@ PB_API int pb_attn_bwd_cp(const void* q, const void* k, const void* v, const voi
   {
     // dQ: resident Q, dO (128-row boxes); streamed K, V (64-row boxes)
     CUtensorMap tQ, tDO, tK, tV, tDQ;
-    r |= make_tmap_3d(&tQ, q, 2, qi, rows, 1, ldq, 0, 64, 128);
-    r |= make_tmap_3d(&tDO, dout, 2, qi, rows, 1, ldo, 0, 64, 128);
-    r |= make_tmap_3d(&tK, k, 2, ki, krows, 1, ldkv, 0, 64, 64);
-    r |= make_tmap_3d(&tV, v, 2, ki, krows, 1, ldkv, 0, 64, 64);
-    r |= make_tmap_3d(&tDQ, dq, 2, qi, rows, 1, ldq, 0, 64, 128);
+    r |= tok_map(&tQ, q, qi, seq, batch, ldq, 128);
+    r |= tok_map(&tDO, dout, qi, seq, batch, ldo, 128);
+    r |= tok_map(&tK, k, ki, seq_kv, batch, ldkv, 64);
+    r |= tok_map(&tV, v, ki, seq_kv, batch, ldkv, 64);
+    r |= tok_map(&tDQ, dq, qi, seq, batch, ldq, 128);
     if (r != 0) return 1000 + r;
-    p.n_blk = seq / 128;
+    p.n_blk = (seq + 127) / 128;
     bwd::attn_bwd_kernel<false><<<dim3(p.n_blk, heads, batch), 384, bwd::SMEM, st>>>(
         tQ, tDO, tK, tV, tDQ, tDQ, p);
   }
   {
     // dK, dV: resident K, V (every key block of the gathered keys); streamed local Q, dO
     CUtensorMap tK, tV, tQ, tDO, tDK, tDV;
-    r |= make_tmap_3d(&tK, k, 2, ki, krows, 1, ldkv, 0, 64, 128);
-    r |= make_tmap_3d(&tV, v, 2, ki, krows, 1, ldkv, 0, 64, 128);
-    r |= make_tmap_3d(&tQ, q, 2, qi, rows, 1, ldq, 0, 64, 64);
-    r |= make_tmap_3d(&tDO, dout, 2, qi, rows, 1, ldo, 0, 64, 64);
-    r |= make_tmap_3d(&tDK, dk, 2, ki, krows, 1, ldkv, 0, 64, 128);
-    r |= make_tmap_3d(&tDV, dv, 2, ki, krows, 1, ldkv, 0, 64, 128);
+    r |= tok_map(&tK, k, ki, seq_kv, batch, ldkv, 128);
+    r |= tok_map(&tV, v, ki, seq_kv, batch, ldkv, 128);
+    r |= tok_map(&tQ, q, qi, seq, batch, ldq, 64);
+    r |= tok_map(&tDO, dout, qi, seq, batch, ldo, 64);
+    r |= tok_map(&tDK, dk, ki, seq_kv, batch, ldkv, 128);
+    r |= tok_map(&tDV, dv, ki, seq_kv, batch, ldkv, 128);
     if (r != 0) return 2000 + r;
-    p.n_blk = seq_kv / 128;
+    p.n_blk = (seq_kv + 127) / 128;
     bwd::attn_bwd_kernel<true><<<dim3(p.n_blk, kv_heads, batch), 384, bwd::SMEM, st>>>(
         tK, tV, tQ, tDO, tDK, tDV, p);
   }

@@ -3,7 +3,7 @@
 On a GPU with head dim 128 this runs the package's own tcgen05 kernels
 (``csrc/kernels/attention.cu``): a flash-style forward with the scores and the output
 accumulator in tensor memory, and a two-kernel deterministic backward (dQ; dK/dV). q, k, v
-are read in place from their ``(B, S, H, 128)`` layout. Other geometries and the CPU use the
+are read in place from their ``(B, S, H, 128)`` layout, at any ``S``. Other geometries and the CPU use the
 plain fp32 formula, which is also the oracle of the tests
 (reference: model/__init__.py softmax attention with a causal mask, scale 1/sqrt(d)).
 """
@@ -13,6 +13,8 @@ import math
 
 import torch
 from torch import Tensor
+
+from .delta import _tma_ready
 
 
 def causal_gqa_ref(q: Tensor, k: Tensor, v: Tensor, scale: float | None = None) -> Tensor:
@@ -37,7 +39,7 @@ class _AttnFn(torch.autograd.Function):
 
         b, s, hq, d = q.shape
         hkv = k.shape[2]
-        q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
+        q, k, v = _tma_ready(q), _tma_ready(k), _tma_ready(v)
         out = torch.empty_like(q)
         lse2 = torch.empty((b, hq, s), dtype=torch.float32, device=q.device)
         rowmax = torch.empty_like(lse2) if want_max else None
@@ -58,7 +60,7 @@ class _AttnFn(torch.autograd.Function):
         q, k, v, out, lse2 = ctx.saved_tensors
         b, s, hq, d = q.shape
         hkv = k.shape[2]
-        d_out = d_out.contiguous()
+        d_out = _tma_ready(d_out)
         dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
         delta = torch.empty_like(lse2)
         call("pb_attn_bwd", ptr(q), ptr(k), ptr(v), ptr(out), ptr(d_out), ptr(lse2), ptr(delta),
@@ -161,12 +163,5 @@ def causal_gqa(q: Tensor, k: Tensor, v: Tensor, scale: float | None = None,
         s = q.shape[1]
         mask = torch.ones(s, s, dtype=torch.bool, device=q.device).tril()
         return out, logits.masked_fill(~mask, float("-inf")).amax(dim=-1)
-    s = q.shape[1]
-    pad = (-s) % 256
-    if pad:   # padded keys come after every real query, so the causal mask hides them
-        q, k, v = (torch.nn.functional.pad(t, (0, 0, 0, 0, 0, pad)) for t in (q, k, v))
     out, rowmax = _AttnFn.apply(q, k, v, scale, return_max_logit)
-    if pad:
-        out = out[:, :s]
-        rowmax = None if rowmax is None else rowmax[..., :s]
     return (out, rowmax) if return_max_logit else out

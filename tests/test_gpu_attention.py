@@ -114,3 +114,32 @@ def test_offset_attention_equals_a_slice_of_the_full_sequence(q_off, s_loc, s_kv
         assert dk[:, unseen:].abs().max() == 0 and dv[:, unseen:].abs().max() == 0
     with pytest.raises(ValueError):
         attention.causal_gqa_offset(ql, kl, vl, q_off + 128)
+
+
+@pytest.mark.parametrize("B,S,hq,hkv", [(2, 1, 2, 1), (3, 63, 4, 2), (2, 129, 2, 2), (2, 300, 4, 1), (2, 1000, 4, 2)])
+def test_ragged_lengths_equal_explicit_padding(B, S, hq, hkv):
+    """A length that is not a multiple of a tile, read in place, gives the bits of the same call on
+    tensors padded to whole tiles (batch entries follow one another without a gap, so a row too
+    many would be the next entry's), and from a misaligned base."""
+    from prometheus_b200.ops import attention
+    from prometheus_b200.ops import functional as ops
+
+    g = torch.Generator(device="cuda").manual_seed(S)
+    q, go = (torch.randn(B, S, hq, 128, generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    k, v = (torch.randn(B, S, hkv, 128, generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+
+    def run(ts, gout):
+        leaves = [t.clone().requires_grad_(True) for t in ts]
+        out, top = attention.causal_gqa(*leaves, return_max_logit=True)
+        grads = torch.autograd.grad(out, leaves, gout)
+        ops.check_status("cuda")
+        return [out.detach(), top.transpose(1, 2), *grads]
+
+    def padded(t):
+        return torch.nn.functional.pad(t, (0, 0, 0, 0, 0, (-S) % 256))
+
+    got, want = run((q, k, v), go), run([padded(t) for t in (q, k, v)], padded(go))
+    for name, a, b in zip(("out", "max", "dq", "dk", "dv"), got, want):
+        assert torch.equal(a, b[:, :S]), name
+    off = torch.empty(q.numel() + 1, dtype=torch.bfloat16, device="cuda")[1:].view(q.shape).copy_(q)
+    assert torch.equal(attention.causal_gqa(off, k, v), got[0])
