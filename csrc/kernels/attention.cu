@@ -72,11 +72,23 @@ __device__ __forceinline__ bf16x8 pack_bf16x8(const float* f) {
   for (int j = 0; j < 4; ++j) pk.v[j] = __floats2bfloat162_rn(f[2 * j], f[2 * j + 1]);
   return pk;
 }
+__device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
 __device__ __forceinline__ void sync_rows() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 // Warp-uniform bounded wait: the row warps run warp-collective tensor-memory loads, so either
 // every lane goes on or none does.
 __device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, int* status) {
   return __all_sync(0xffffffffu, mbar_wait_spin(bar, parity, status));
+}
+
+// Registers of a tensor-memory load are valid after the wait: no use of them may move above this.
+__device__ __forceinline__ void tie32(uint32_t (&v)[32]) {
+#pragma unroll
+  for (int i = 0; i < 32; i += 8)
+    asm volatile("" : "+r"(v[i]), "+r"(v[i + 1]), "+r"(v[i + 2]), "+r"(v[i + 3]), "+r"(v[i + 4]), "+r"(v[i + 5]),
+                      "+r"(v[i + 6]), "+r"(v[i + 7]));
 }
 
 // ------------------------------------------------------------------------------ forward
@@ -351,13 +363,19 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 
 // ----------------------------------------------------------------------------- backward
 namespace bwd {
-constexpr int STAGES = 3;
+constexpr int STAGES = 4;
 constexpr int RA_OFF = 0, RB_OFF = 32768, ST_OFF = 65536;       // stages: T1 16 KB + T2 16 KB
-constexpr int DS_OFF = ST_OFF + STAGES * 32768, PT_OFF = DS_OFF + 2 * 16384;
-constexpr int VEC_OFF = PT_OFF + 2 * 16384, BARS = VEC_OFF + 2 * 512;
+constexpr int VEC_OFF = ST_OFF + STAGES * 32768, BARS = VEC_OFF + 2 * 512;
 constexpr int SMEM = BARS + 256 + 1024;
 static_assert(SMEM <= 227 * 1024, "one CTA's shared memory");
-constexpr uint32_t COL_X1 = 0, COL_X2 = 128, COL_ACC1 = 256, COL_ACC2 = 384, TMEM_COLS = 512;
+// tensor memory: score buffers of 128 columns (X1 at 0, X2 at 64; P^T and dS take the first 32 columns
+// of each as packed bf16 operands), then the accumulators. dQ has one accumulator and so room for
+// a third score buffer.
+template <bool DKV> struct Cols {
+  static constexpr int BUFS = DKV ? 2 : 3;
+  static constexpr uint32_t ACC1 = BUFS * 128, ACC2 = 384;
+};
+constexpr uint32_t COL_X2 = 64, TMEM_COLS = 512;
 
 struct Params {
   int seq, heads, kv_heads, n_blk;  // seq: query rows per batch entry; n_blk: 128-row blocks of the grid
@@ -370,16 +388,20 @@ struct Params {
 
 // DKV = false: resident Q, dO (one head); streams K, V tiles; output dQ.
 // DKV = true : resident K, V (one KV head); streams Q, dO tiles of the group; outputs dK, dV.
-// Two warpgroups (warps 0-3, 4-7) take the streamed tiles alternately, each with its own score
-// buffers in tensor memory and its own dS / P^T operand buffers, and accumulate into the same
+// Two warpgroups (warps 0-3, 4-7) take the streamed tiles alternately and accumulate into the same
 // gradient accumulators.  MMA issue is spread over three warps because one thread cannot issue
 // 20+ small MMAs per tile fast enough: warp 8 the first score product, warp 9 the second,
 // warp 10 the gradient accumulations; warp 11: TMA producer.
-// A tile's stage is held until its gradient product is done, so with a stage per warpgroup every
-// tile waited for the next load in full; the third stage keeps one load ahead. The softmax scale is
-// applied to the finished dQ / dK accumulator instead of to every dS, and the streamed rows'
-// log-sum-exp and delta are read from shared memory four at a time (its bandwidth is what the
-// 128 x 64 products' operands need). 4 x 4096 x 16/4: dQ 618 -> 471 us, dK and dV 917 -> 721 us.
+//
+// Bound by shared-memory bandwidth: a 128 x 64 score product reads 6 KB of operands per 16-deep
+// step, half as much again as the tensor core can use. So what can be kept off shared memory is:
+// P^T and dS go back to tensor memory as bf16 over the scores they were made from and are the
+// gradient products' A operand there (64 KB less per tile than operand tiles written to and read from
+// shared memory), which also makes room for four stages of streamed tiles: a tile's stage is held
+// until its gradient product is done, and with fewer every tile waits for a load. The softmax
+// scale is applied to the finished dQ / dK accumulator instead of to every dS.
+// 4 x 4096 x 16/4: dQ 618 -> 398 us, dK and dV 917 -> 689 us (two stages and operand tiles; three
+// stages: 471 and 721 us).
 template <bool DKV>
 __global__ void __launch_bounds__(384, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant__ CUtensorMap tmRB,
@@ -392,13 +414,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + BARS);
   uint64_t* r_full = bars;
   uint64_t* t_full = bars + 1;    // [STAGES]
-  uint64_t* t_empty = bars + 4;   // [STAGES]
-  uint64_t* x_done = bars + 7;    // [2]
-  uint64_t* x_free = bars + 9;    // [2]
-  uint64_t* pd_ready = bars + 11; // [2]
-  uint64_t* pd_free = bars + 13;  // [2]
-  uint64_t* acc_done = bars + 15;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
+  uint64_t* t_empty = bars + 5;   // [STAGES]
+  uint64_t* x_done = bars + 9;    // [BUFS] scores of a buffer
+  uint64_t* x_free = bars + 12;   // [BUFS] its gradient products
+  uint64_t* pd_ready = bars + 15; // [BUFS] its P^T and dS
+  uint64_t* acc_done = bars + 18;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 20);
+  constexpr int BUFS = Cols<DKV>::BUFS;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int group = p.heads / p.kv_heads;
@@ -419,9 +441,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
   if (threadIdx.x == 0) {
     mbar_init(r_full, 1);
     for (int i = 0; i < STAGES; ++i) { mbar_init(&t_full[i], 1); mbar_init(&t_empty[i], 1); }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&x_done[i], 2); mbar_init(&x_free[i], 4);    // two issuing threads; one arrival per row warp
-      mbar_init(&pd_ready[i], 4); mbar_init(&pd_free[i], 1);
+    for (int i = 0; i < BUFS; ++i) {
+      mbar_init(&x_done[i], 2); mbar_init(&x_free[i], 1);    // two issuing threads
+      mbar_init(&pd_ready[i], 4);                            // one arrival per row warp
     }
     mbar_init(acc_done, 1);
     fence_barrier_init();
@@ -473,15 +495,15 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
       constexpr uint32_t HI = sdesc_hi_sw128(1024);
       const uint32_t r_lo = sdesc_lo(smem_u32(smem + (which == 0 ? RA_OFF : RB_OFF)), 16);
       const uint32_t st0 = smem_u32(smem + ST_OFF + which * 16384);
-      const uint32_t col = which == 0 ? COL_X1 : COL_X2;
+      const uint32_t col = which == 0 ? 0 : COL_X2;
       bool ok = n_it == 0 || mbar_wait_spin(r_full, 0, p.status);
       for (int it = 0; it < n_it && ok; ++it) {
-        const int s = it & 1, ts = it % STAGES;
+        const int s = it % BUFS, ts = it % STAGES;
         if (!mbar_wait_spin(&t_full[ts], (it / STAGES) & 1, p.status)) break;
-        if (!mbar_wait_spin(&x_free[s], ((it >> 1) & 1) ^ 1, p.status)) break;
+        if (!mbar_wait_spin(&x_free[s], ((it / BUFS) & 1) ^ 1, p.status)) break;
         tc_fence_after();
         const uint32_t t_lo = sdesc_lo(st0 + ts * 32768, 16);
-        const uint32_t d = tmem + col + s * 64;
+        const uint32_t d = tmem + col + s * 128;
 #pragma unroll
         for (int jj = 0; jj < 8; ++jj)
           umma_f16_words(d, r_lo + (((jj >> 2) * 16384 + (jj & 3) * 32) >> 4), HI,
@@ -492,35 +514,32 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
   } else if (warp == 10) {
     // gradient accumulations, all from this one thread so that they stay ordered
     if (lane == 0) {
-      const uint32_t id_acc = make_idesc(1, 1, 128, 128, 0, 1);  // A K-major, B MN-major
-      constexpr uint32_t HI = sdesc_hi_sw128(1024);
+      const uint32_t id_acc = make_idesc(1, 1, 128, 128, 0, 1);  // A from tensor memory, B MN-major
+      constexpr uint64_t HI = static_cast<uint64_t>(sdesc_hi_sw128(1024)) << 32;
       const uint32_t st0 = smem_u32(smem + ST_OFF);
-      const uint32_t ds_lo0 = sdesc_lo(smem_u32(smem + DS_OFF), 16);
-      const uint32_t pt_lo0 = sdesc_lo(smem_u32(smem + PT_OFF), 16);
       int it = 0;
       for (; it < n_it; ++it) {
-        const int s = it & 1;
-        const uint32_t ph = (it >> 1) & 1;
-        if (!mbar_wait_spin(&pd_ready[s], ph, p.status)) break;
+        const int s = it % BUFS, ts = it % STAGES;
+        if (!mbar_wait_spin(&pd_ready[s], (it / BUFS) & 1, p.status)) break;
         tc_fence_after();
-        // the streamed tiles again, now as MN-major B operands (64-wide chunks 8 KB apart)
-        const int ts = it % STAGES;
+        // the streamed tiles again, now as MN-major B operands (64-wide chunks 8 KB apart); 16
+        // values of a bf16 operand row are eight tensor-memory columns
         const uint32_t t1_mn = sdesc_lo(st0 + ts * 32768, 8192), t2_mn = t1_mn + (16384 >> 4);
-        const uint32_t ds_lo = ds_lo0 + ((s * 16384) >> 4), pt_lo = pt_lo0 + ((s * 16384) >> 4);
+        const uint32_t xb = tmem + s * 128;
 #pragma unroll
         for (int jj = 0; jj < 4; ++jj)
-          umma_f16_words(tmem + COL_ACC1, ds_lo + ((jj * 32) >> 4), HI, t1_mn + ((jj * 2048) >> 4),
-                         HI, id_acc, (it > 0) || (jj > 0));
+          umma_f16_ts(tmem + Cols<DKV>::ACC1, xb + COL_X2 + jj * 8, HI | (t1_mn + ((jj * 2048) >> 4)), id_acc,
+                      (it > 0) || (jj > 0));
         if (DKV) {
 #pragma unroll
           for (int jj = 0; jj < 4; ++jj)
-            umma_f16_words(tmem + COL_ACC2, pt_lo + ((jj * 32) >> 4), HI,
-                           t2_mn + ((jj * 2048) >> 4), HI, id_acc, (it > 0) || (jj > 0));
+            umma_f16_ts(tmem + Cols<DKV>::ACC2, xb + jj * 8, HI | (t2_mn + ((jj * 2048) >> 4)), id_acc,
+                        (it > 0) || (jj > 0));
         }
         // the score products of this tile finished before the row warps could signal pd_ready,
-        // so the completion of these MMAs releases the whole stage
+        // so the completion of these MMAs releases the whole stage and the score buffer
         umma_commit(&t_empty[ts]);
-        umma_commit(&pd_free[s]);
+        umma_commit(&x_free[s]);
       }
       if (it == n_it) umma_commit(acc_done);
     }
@@ -550,73 +569,82 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
     float vec_next = (DKV && wg < n_it) ? vec_value(wg) : 0.f;
     bool ok = true;
     for (int it = wg; it < n_it && ok; it += 2) {
-      const int s = wg;
-      const uint32_t ph = (it >> 1) & 1;
+      const int s = it % BUFS;
       const int t = t_first + (DKV ? it % t_count : it);
-      float* vec = reinterpret_cast<float*>(smem + VEC_OFF + s * 512);
+      float* vec = reinterpret_cast<float*>(smem + VEC_OFF + wg * 512);
       if (DKV) {
         sync_group();        // the group's readers of the previous tile are done
         vec[r] = vec_next;   // [0,64) lse2, [64,128) delta
         if (it + 2 < n_it) vec_next = vec_value(it + 2);
         sync_group();
       }
-      if (!wait_all(&x_done[s], ph, p.status)) { ok = false; break; }
-      if (!wait_all(&pd_free[s], ph ^ 1, p.status)) { ok = false; break; }
+      if (!wait_all(&x_done[s], (it / BUFS) & 1, p.status)) { ok = false; break; }
       tc_fence_after();
       // mask: dQ rows are queries, columns keys (key > query is masked);
       //       dKV rows are keys, columns queries (query < key is masked)
       const int tg = DKV ? t + q_off64 : t;     // global index of the streamed tile
       const bool edge = DKV ? (tg * 64 < gblk * 128 + 127) : (tg * 64 + 63 > gblk * 128);
-      uint8_t* dsb = smem + DS_OFF + s * 16384;
-      uint8_t* ptb = smem + PT_OFF + s * 16384;
-      auto tile_rows = [&](auto EDGE) {
-#pragma unroll 1
-        for (int c = 0; c < 64; c += 32) {
-          uint32_t x1[32], x2[32];
-          tmem_ld_32x32b_x32(lane_addr + COL_X1 + s * 64 + c, x1);
-          tmem_ld_32x32b_x32(lane_addr + COL_X2 + s * 64 + c, x2);
-          tmem_ld_wait();
+      const uint32_t xb = lane_addr + s * 128;
+      uint32_t pk_p[32], pk_d[32];               // the row's P and dS, two bf16 to a register
+      auto half = [&](auto EDGE, const int c, const uint32_t (&x1)[32], const uint32_t (&x2)[32]) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            float pf[8], df[8], lv[8], dv[8];
-            if (DKV) {
-              const float4* l4 = reinterpret_cast<const float4*>(vec + c + 8 * i);
-              const float4* d4 = reinterpret_cast<const float4*>(vec + 64 + c + 8 * i);
-              const float4 a = l4[0], b4 = l4[1], e = d4[0], f = d4[1];
-              lv[0] = a.x; lv[1] = a.y; lv[2] = a.z; lv[3] = a.w;
-              lv[4] = b4.x; lv[5] = b4.y; lv[6] = b4.z; lv[7] = b4.w;
-              dv[0] = e.x; dv[1] = e.y; dv[2] = e.z; dv[3] = e.w;
-              dv[4] = f.x; dv[5] = f.y; dv[6] = f.z; dv[7] = f.w;
-            }
+        for (int i = 0; i < 4; ++i) {
+          float pf[8], df[8], lv[8], dv[8];
+          if (DKV) {
+            const float4* l4 = reinterpret_cast<const float4*>(vec + c + 8 * i);
+            const float4* d4 = reinterpret_cast<const float4*>(vec + 64 + c + 8 * i);
+            const float4 a = l4[0], b4 = l4[1], e = d4[0], f = d4[1];
+            lv[0] = a.x; lv[1] = a.y; lv[2] = a.z; lv[3] = a.w;
+            lv[4] = b4.x; lv[5] = b4.y; lv[6] = b4.z; lv[7] = b4.w;
+            dv[0] = e.x; dv[1] = e.y; dv[2] = e.z; dv[3] = e.w;
+            dv[4] = f.x; dv[5] = f.y; dv[6] = f.z; dv[7] = f.w;
+          }
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-              const int col = c + 8 * i + k;
-              const float lse = DKV ? lv[k] : row_lse;
-              const float dl = DKV ? dv[k] : row_delta;
-              float pr = ex2(fmaf(__uint_as_float(x1[8 * i + k]), p.scale_log2, -lse));
-              if (decltype(EDGE)::value) {
-                const int other = tg * 64 + col;
-                const bool masked = DKV ? (other < pos) : (other > pos);
-                if (masked) pr = 0.f;
-              }
-              pf[k] = pr;
-              df[k] = pr * (__uint_as_float(x2[8 * i + k]) - dl);   // the scale waits for the epilogue
+          for (int k = 0; k < 8; ++k) {
+            const int col = c + 8 * i + k;
+            const float lse = DKV ? lv[k] : row_lse;
+            const float dl = DKV ? dv[k] : row_delta;
+            float pr = ex2(fmaf(__uint_as_float(x1[8 * i + k]), p.scale_log2, -lse));
+            if (decltype(EDGE)::value) {
+              const int other = tg * 64 + col;
+              const bool masked = DKV ? (other < pos) : (other > pos);
+              if (masked) pr = 0.f;
             }
-            const int c16 = (c >> 3) + i;
-            st_swz(dsb, r, c16, pack_bf16x8(df));
-            if (DKV) st_swz(ptb, r, c16, pack_bf16x8(pf));
+            pf[k] = pr;
+            df[k] = pr * (__uint_as_float(x2[8 * i + k]) - dl);   // the scale waits for the epilogue
+          }
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const int at = (c >> 1) + 4 * i + k;
+            pk_d[at] = pack_bf16x2(df[2 * k], df[2 * k + 1]);
+            if (DKV) pk_p[at] = pack_bf16x2(pf[2 * k], pf[2 * k + 1]);
           }
         }
       };
+      auto tile_rows = [&](auto EDGE) {
+        // the second half's scores arrive while the first half is worked on
+        uint32_t a1[32], a2[32], b1[32], b2[32];
+        tmem_ld_32x32b_x32(xb, a1);
+        tmem_ld_32x32b_x32(xb + COL_X2, a2);
+        tmem_ld_wait();
+        tie32(a1);
+        tie32(a2);
+        tmem_ld_32x32b_x32(xb + 32, b1);
+        tmem_ld_32x32b_x32(xb + COL_X2 + 32, b2);
+        half(EDGE, 0, a1, a2);
+        tmem_ld_wait();
+        tie32(b1);
+        tie32(b2);
+        half(EDGE, 32, b1, b2);
+      };
       if (edge) tile_rows(std::true_type{});
       else tile_rows(std::false_type{});
+      tmem_st_32x32b_x32(xb + COL_X2, pk_d);
+      if (DKV) tmem_st_32x32b_x32(xb, pk_p);
+      tmem_st_wait();
       tc_fence_before();
-      fence_proxy_async_smem();
       __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(&x_free[s]);
-        mbar_arrive(&pd_ready[s]);
-      }
+      if (lane == 0) mbar_arrive(&pd_ready[s]);
     }
     // every row thread gets here (no early exit above), so the group barriers below are safe
     if (wait_all(acc_done, 0, p.status) && ok) {
@@ -624,7 +652,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
       // resident tiles are no longer read: reuse them as the staging for the TMA stores.
       // dKV: group 0 drains dK, group 1 drains dV.  dQ: each group drains 64 columns.
       uint8_t* stage = smem + ((DKV && wg == 1) ? RB_OFF : RA_OFF);
-      const uint32_t col0 = (DKV && wg == 1) ? COL_ACC2 : COL_ACC1;
+      const uint32_t col0 = (DKV && wg == 1) ? Cols<DKV>::ACC2 : Cols<DKV>::ACC1;
       const float out_scale = DKV && wg == 1 ? 1.f : p.scale;
       const int c_lo = DKV ? 0 : wg * 64, c_hi = DKV ? D : wg * 64 + 64;
 #pragma unroll 1
