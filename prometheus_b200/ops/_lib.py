@@ -142,7 +142,10 @@ def load():
 
 
 def stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """Handle of the current stream of the current device: the two raw queries behind
+    ``torch.cuda.current_stream()`` without the Stream object it builds (3.3 us -> 0.2 us, on every
+    launch)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def ptr(t) -> int | None:
@@ -156,11 +159,14 @@ def ptr(t) -> int | None:
 _LAUNCHES = {"pb_rmsnorm_bwd": 2, "pb_sumsq_f32": 2, "pb_sumsq_bf16": 2, "pb_muon_prepare": 3,
              "pb_muon_prepare_batched": 3}
 launch_count = 0
+_bound: dict = {}       # name -> function of the loaded library
 
 
 def call(name: str, *args) -> None:
     global launch_count
-    fn = getattr(load(), name)
+    fn = _bound.get(name)
+    if fn is None:
+        fn = _bound[name] = getattr(load(), name)
     rc = fn(*args)
     launch_count += _LAUNCHES.get(name, 1)
     if rc != 0:

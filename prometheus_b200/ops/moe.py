@@ -56,12 +56,12 @@ def place(ids: Tensor, n_experts: int) -> Placement:
     dev = ids.device
     rows = (n_pairs + n_experts * 127 + 127) // 128 * 128
     nblocks = _lib.query("pb_moe_sort_nblocks", n_pairs, k)
-    i32 = dict(dtype=torch.int32, device=dev)
-    scratch = torch.empty(nblocks * n_experts, **i32)
-    pl = Placement(row_of=torch.empty(n_pairs, **i32), expert_off=torch.empty(n_experts + 1, **i32),
-                   totals=torch.empty(n_experts, **i32), k_len=torch.empty(n_experts, **i32),
-                   mblk_group=torch.empty(rows // 128, **i32), rows=rows, n_experts=n_experts,
-                   top_k=k)
+    # one allocation, six views
+    row_of, expert_off, totals, k_len, mblk_group, scratch = torch.empty(
+        n_pairs + 3 * n_experts + 1 + rows // 128 + nblocks * n_experts, dtype=torch.int32, device=dev).split(
+        [n_pairs, n_experts + 1, n_experts, n_experts, rows // 128, nblocks * n_experts])
+    pl = Placement(row_of=row_of, expert_off=expert_off, totals=totals, k_len=k_len, mblk_group=mblk_group,
+                   rows=rows, n_experts=n_experts, top_k=k)
     call("pb_moe_sort", ptr(ids), n_pairs, k, n_experts, ptr(scratch), ptr(pl.row_of),
          ptr(pl.expert_off), ptr(pl.totals), ptr(pl.k_len), ptr(pl.mblk_group), rows // 128,
          stream_ptr())
@@ -134,6 +134,7 @@ class _MoeFfnFn(torch.autograd.Function):
     def forward(ctx, x, router_w, router_bias, w_gu_p, w_down_p, top_k, n_shared, shapes, fp8=False):
         from .functional import gemm
 
+        ctx.set_materialize_grads(False)   # the scores' and logits' gradients are often absent
         w_gu = w_gu_p.view(shapes[0]) if shapes is not None else w_gu_p
         w_down = w_down_p.view(shapes[1]) if shapes is not None else w_down_p
         T, d = x.shape
@@ -208,7 +209,7 @@ class _MoeFfnFn(torch.autograd.Function):
         h = two_h // 2
         k = pl.top_k                       # routed + shared slots
         k_r = ctx.top_k
-        d_out = d_out.contiguous()
+        d_out = torch.zeros_like(x) if d_out is None else d_out.contiguous()
         dgates = torch.empty((T, k), dtype=torch.float32, device=x.device)
         call("pb_moe_combine_bwd", ptr(y), ptr(d_out), ptr(pl.row_of), T * k, k, d, ptr(dgates),
              stream_ptr())

@@ -80,6 +80,41 @@ def test_gemm_batched_epilogue_variants():
     ops.check_status("cuda")
 
 
+def test_gemm_2d_forms_equal_the_batched_form():
+    """The two-matrix path against the same product as a batch of one: layouts, strided operands and
+    destinations, accumulation, and a thread whose first CUDA call is a product."""
+    import threading
+
+    from prometheus_b200.ops import functional as ops
+
+    base = _r(200, 520, seed=1)
+    for a_mn, b_mn in ((False, False), (False, True), (True, False), (True, True)):
+        a = _r(264, 208, seed=2) if a_mn else base[:, 8:272]            # a row stride of 520
+        a = a[:, :200] if a_mn else a
+        b = _r(264, 328, seed=3) if b_mn else _r(328, 264, seed=3)
+        kw = dict(a_mn=a_mn, b_mn=b_mn)
+        want = ops.gemm(a[None], b[None], **kw)[0]
+        assert torch.equal(ops.gemm(a, b, **kw), want)
+        d = _r(200, 328, seed=4, dtype=torch.float32)
+        acc, acc3 = d.clone(), d.clone()[None]
+        ops.gemm(a, b, out=acc, d=acc, beta=1.0, **kw)
+        ops.gemm(a[None], b[None], out=acc3, d=acc3, beta=1.0, **kw)
+        assert torch.equal(acc, acc3[0])
+        wide = torch.zeros(200, 336, dtype=BF16, device="cuda")
+        ops.gemm(a, b, out=wide[:, :328], **kw)
+        assert torch.equal(wide[:, :328], want) and (wide[:, 328:] == 0).all()
+        assert torch.equal(ops.gemm(a, b, out=torch.empty(1, 200, 328, dtype=BF16, device="cuda"), **kw), want)
+        assert torch.equal(ops.gemm(a, b.t().contiguous().t(), **kw), want)      # not row-major: copied
+        got = []
+        out = torch.empty_like(want)
+        torch.cuda.synchronize()
+        th = threading.Thread(target=lambda: got.append(ops.gemm(a, b, out=out, **kw)))
+        th.start()
+        th.join()
+        torch.cuda.synchronize()
+        assert got and torch.equal(got[0], want)
+
+
 def test_gemm_limited_grid_and_many_tiles():
     from prometheus_b200.ops import functional as ops
 
