@@ -382,37 +382,43 @@ __global__ void rope_kernel(bf16* __restrict__ x, const int* __restrict__ pos, l
 // ---------------------------------------------------------------------------
 // rows_dev (may be null): device-side row count; rows beyond it are left untouched. Buffers
 // sized for a worst case (expert-parallel receive buffers) then cost only what is in use.
-__global__ void swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict__ out, long rows,
-                                  int H, const int* __restrict__ rows_dev) {
+// Index is 32-bit wherever rows * H / 8 fits (the launch decides): finding a vector's row by a 64-bit
+// division cost as much as the arithmetic on its eight elements.
+// 16384 x 5632: forward 121 -> 116 us, backward 162 -> 147 us (floors 85 and 141).
+template <typename Index>
+__global__ void __launch_bounds__(256) swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict__ out,
+                                                         long rows, int H, const int* __restrict__ rows_dev) {
   if (rows_dev != nullptr) rows = min(rows, static_cast<long>(*rows_dev));
-  const int vph = H >> 3;
-  const long total = rows * vph;
-  for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<long>(gridDim.x) * blockDim.x) {
-    const long r = i / vph;
-    const int c = static_cast<int>(i % vph) * 8;
+  const Index vph = static_cast<Index>(H >> 3);
+  const Index total = static_cast<Index>(rows) * vph;
+  for (Index i = blockIdx.x * static_cast<Index>(blockDim.x) + threadIdx.x; i < total;
+       i += static_cast<Index>(gridDim.x) * blockDim.x) {
+    const Index r = i / vph;
+    const long c = static_cast<long>(i - r * vph) * 8;
+    const bf16* src = gu + static_cast<long>(r) * 2 * H + c;
     float g[8], u[8], o[8];
-    unpack8(*reinterpret_cast<const bf16x8*>(gu + r * 2 * H + c), g);
-    unpack8(*reinterpret_cast<const bf16x8*>(gu + r * 2 * H + H + c), u);
+    unpack8(*reinterpret_cast<const bf16x8*>(src), g);
+    unpack8(*reinterpret_cast<const bf16x8*>(src + H), u);
 #pragma unroll
     for (int j = 0; j < 8; ++j) o[j] = g[j] * sigmoidf_(g[j]) * u[j];
-    *reinterpret_cast<bf16x8*>(out + r * H + c) = pack8(o);
+    *reinterpret_cast<bf16x8*>(out + static_cast<long>(r) * H + c) = pack8(o);
   }
 }
-__global__ void swiglu_bwd_kernel(const bf16* __restrict__ dout, const bf16* __restrict__ gu,
-                                  bf16* __restrict__ dgu, long rows, int H,
-                                  const int* __restrict__ rows_dev) {
+template <typename Index>
+__global__ void __launch_bounds__(256) swiglu_bwd_kernel(const bf16* __restrict__ dout, const bf16* __restrict__ gu,
+                                                         bf16* __restrict__ dgu, long rows, int H,
+                                                         const int* __restrict__ rows_dev) {
   if (rows_dev != nullptr) rows = min(rows, static_cast<long>(*rows_dev));
-  const int vph = H >> 3;
-  const long total = rows * vph;
-  for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<long>(gridDim.x) * blockDim.x) {
-    const long r = i / vph;
-    const int c = static_cast<int>(i % vph) * 8;
+  const Index vph = static_cast<Index>(H >> 3);
+  const Index total = static_cast<Index>(rows) * vph;
+  for (Index i = blockIdx.x * static_cast<Index>(blockDim.x) + threadIdx.x; i < total;
+       i += static_cast<Index>(gridDim.x) * blockDim.x) {
+    const Index r = i / vph;
+    const long c = static_cast<long>(i - r * vph) * 8, at = static_cast<long>(r) * 2 * H + c;
     float g[8], u[8], d[8], dg[8], du[8];
-    unpack8(*reinterpret_cast<const bf16x8*>(gu + r * 2 * H + c), g);
-    unpack8(*reinterpret_cast<const bf16x8*>(gu + r * 2 * H + H + c), u);
-    unpack8(*reinterpret_cast<const bf16x8*>(dout + r * H + c), d);
+    unpack8(*reinterpret_cast<const bf16x8*>(gu + at), g);
+    unpack8(*reinterpret_cast<const bf16x8*>(gu + at + H), u);
+    unpack8(*reinterpret_cast<const bf16x8*>(dout + static_cast<long>(r) * H + c), d);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const float s = sigmoidf_(g[j]);
@@ -420,8 +426,8 @@ __global__ void swiglu_bwd_kernel(const bf16* __restrict__ dout, const bf16* __r
       du[j] = d[j] * silu;
       dg[j] = d[j] * u[j] * (s + silu * (1.f - s));
     }
-    *reinterpret_cast<bf16x8*>(dgu + r * 2 * H + c) = pack8(dg);
-    *reinterpret_cast<bf16x8*>(dgu + r * 2 * H + H + c) = pack8(du);
+    *reinterpret_cast<bf16x8*>(dgu + at) = pack8(dg);
+    *reinterpret_cast<bf16x8*>(dgu + at + H) = pack8(du);
   }
 }
 
@@ -814,27 +820,38 @@ PB_API int pb_rope(void* x, const void* pos, long tokens, int heads, int D, int 
   return cudaGetLastError();
 }
 
+static int swiglu_fwd_launch(const void* gu, void* out, long rows, int H, const int* rows_dev, cudaStream_t st) {
+  const bf16* g_ = static_cast<const bf16*>(gu);
+  bf16* o_ = static_cast<bf16*>(out);
+  const int grid = grid_for(rows * (H / 8), 256);
+  // a grid stride past the end must not wrap either
+  if (rows * (H / 8) < (1L << 31)) swiglu_fwd_kernel<uint32_t><<<grid, 256, 0, st>>>(g_, o_, rows, H, rows_dev);
+  else swiglu_fwd_kernel<uint64_t><<<grid, 256, 0, st>>>(g_, o_, rows, H, rows_dev);
+  return cudaGetLastError();
+}
+static int swiglu_bwd_launch(const void* dout, const void* gu, void* dgu, long rows, int H, const int* rows_dev,
+                             cudaStream_t st) {
+  const bf16 *d_ = static_cast<const bf16*>(dout), *g_ = static_cast<const bf16*>(gu);
+  bf16* o_ = static_cast<bf16*>(dgu);
+  const int grid = grid_for(rows * (H / 8), 256);
+  if (rows * (H / 8) < (1L << 31)) swiglu_bwd_kernel<uint32_t><<<grid, 256, 0, st>>>(d_, g_, o_, rows, H, rows_dev);
+  else swiglu_bwd_kernel<uint64_t><<<grid, 256, 0, st>>>(d_, g_, o_, rows, H, rows_dev);
+  return cudaGetLastError();
+}
 PB_API int pb_swiglu_fwd(const void* gu, void* out, long rows, int H, cudaStream_t st) {
   if (H % 8 != 0) return PB_BAD_ARG;
-  swiglu_fwd_kernel<<<grid_for(rows * (H / 8), 256), 256, 0, st>>>(
-      static_cast<const bf16*>(gu), static_cast<bf16*>(out), rows, H, nullptr);
-  return cudaGetLastError();
+  return swiglu_fwd_launch(gu, out, rows, H, nullptr, st);
 }
 // The same over the first min(rows, *rows_dev) rows (rows_dev: a device int).
 PB_API int pb_swiglu_fwd_dyn(const void* gu, void* out, long rows, int H, const int* rows_dev,
                              cudaStream_t st) {
   if (H % 8 != 0) return PB_BAD_ARG;
-  swiglu_fwd_kernel<<<grid_for(rows * (H / 8), 256), 256, 0, st>>>(
-      static_cast<const bf16*>(gu), static_cast<bf16*>(out), rows, H, rows_dev);
-  return cudaGetLastError();
+  return swiglu_fwd_launch(gu, out, rows, H, rows_dev, st);
 }
 PB_API int pb_swiglu_bwd_dyn(const void* dout, const void* gu, void* dgu, long rows, int H,
                              const int* rows_dev, cudaStream_t st) {
   if (H % 8 != 0) return PB_BAD_ARG;
-  swiglu_bwd_kernel<<<grid_for(rows * (H / 8), 256), 256, 0, st>>>(
-      static_cast<const bf16*>(dout), static_cast<const bf16*>(gu), static_cast<bf16*>(dgu), rows,
-      H, rows_dev);
-  return cudaGetLastError();
+  return swiglu_bwd_launch(dout, gu, dgu, rows, H, rows_dev, st);
 }
 
 // dst[0 : n) = src[0 : n) rows of row_bytes each, n = min(max_rows, *rows_dev): a copy of the
@@ -865,10 +882,7 @@ PB_API int pb_copy_rows_dyn(const void* src, void* dst, long row_bytes, long max
 PB_API int pb_swiglu_bwd(const void* dout, const void* gu, void* dgu, long rows, int H,
                          cudaStream_t st) {
   if (H % 8 != 0) return PB_BAD_ARG;
-  swiglu_bwd_kernel<<<grid_for(rows * (H / 8), 256), 256, 0, st>>>(
-      static_cast<const bf16*>(dout), static_cast<const bf16*>(gu), static_cast<bf16*>(dgu), rows,
-      H, nullptr);
-  return cudaGetLastError();
+  return swiglu_bwd_launch(dout, gu, dgu, rows, H, nullptr, st);
 }
 
 PB_API int pb_l2norm_fwd(void* x, void* inv_norm, long nvec, int D, float eps, cudaStream_t st) {
