@@ -85,6 +85,7 @@ _SIGS = {
     "pb_moe_sort_nblocks": [I, I],
     "pb_moe_sort": [P, I, I, I, P, P, P, P, P, P, I, P],
     "pb_moe_permute": [P, P, P, I, I, I, L, P, P, P, I, P],
+    "pb_moe_permute_q": [P, P, P, I, I, I, P, P, L, P, P, I, P],
     "pb_moe_combine": [P, P, P, P, I, I, I, P, L, P],
     "pb_debug_bounds_enabled": [],
     "pb_moe_zero_pad": [P, I, P, P, I, P],

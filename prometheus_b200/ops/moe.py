@@ -77,6 +77,21 @@ def permute(x: Tensor, pl: Placement, scale: Tensor | None = None) -> Tensor:
     return out
 
 
+def permute_quantized(x: Tensor, pl: Placement):
+    """``fp8.quantize_rows(permute(x, pl))`` with each token quantised once: ``(q [rows, d] e4m3 bytes,
+    scales [d / 128, rows])``, padding rows zero with scale 1. Rows past the last expert's segment are
+    not written."""
+    from . import fp8 as F8
+
+    T, d = x.shape
+    q, s = F8.quantize_rows(x)
+    out = torch.empty((pl.rows, d), dtype=torch.uint8, device=x.device)
+    scales = torch.empty((d // 128, pl.rows), dtype=torch.float32, device=x.device)
+    call("pb_moe_permute_q", ptr(q), ptr(s), ptr(pl.row_of), T, pl.top_k, d, ptr(out), ptr(scales), pl.rows,
+         ptr(pl.expert_off), ptr(pl.totals), pl.n_experts, stream_ptr())
+    return out, scales
+
+
 def combine(y: Tensor, pl: Placement, gates: Tensor | None, T: int, add: Tensor | None = None) -> Tensor:
     d = y.shape[1]
     out = torch.empty((T, d), dtype=BF16, device=y.device)
@@ -151,7 +166,6 @@ class _MoeFfnFn(torch.autograd.Function):
         else:
             ids, gates = ids_r, gates_r
         pl = place(ids, E)
-        xp = permute(x, pl)
         empty = x.new_empty(0)
         # FP8 products keep their quantised inputs (e4m3 + scales) for the backward, which
         # differentiates the product that was really computed: g w^ and g^T x^
@@ -160,11 +174,12 @@ class _MoeFfnFn(torch.autograd.Function):
         if q_gu:
             from . import fp8 as F8
 
-            xq, sx = F8.quantize_rows(xp)
+            xq, sx = permute_quantized(x, pl)
             wq, sw = F8.quantize_blocks(w_gu.contiguous())
             gu = F8.gemm_fp8(xq, sx, wq, sw, mblk_group=pl.mblk_group)
             x_saved = (xq, sx)
         else:
+            xp = permute(x, pl)
             gu = grouped_gemm(xp, w_gu, pl)
             x_saved = (xp, empty)
         if q_dn:

@@ -88,6 +88,37 @@ def test_grouped_gemms_match_per_expert_products():
     assert tot[4] == 0
 
 
+@pytest.mark.parametrize("T,k,E,d", [(1, 1, 1, 128), (300, 2, 5, 384), (130, 7, 16, 2176)])
+def test_token_movement_kernels(T, k, E, d):
+    """Permute (plain, scaled, quantised) and combine (gated, summed, with an addend) against index
+    arithmetic in fp32, at column counts that leave remainders of their steps and with empty experts."""
+    from prometheus_b200.ops import fp8, moe
+
+    g = torch.Generator(device="cuda").manual_seed(T)
+    ids = torch.stack([torch.randperm(E, generator=g, device="cuda")[:k] for _ in range(T)]).to(torch.int32).contiguous()
+    if E > 4:
+        ids[ids == 3] = 0                                    # expert 3 gets nothing
+    pl = moe.place(ids, E)
+    row = pl.row_of.view(T, k).long()
+    x = _r(T, d, seed=1)
+    sc = _r(T * k, seed=2, dtype=torch.float32)
+    want = torch.zeros(pl.rows, d, device="cuda")
+    want[row] = x.float()[:, None].expand(T, k, d)
+    end = int(pl.expert_off[-1])
+    xp = moe.permute(x, pl)
+    assert torch.equal(xp[:end].float(), want[:end])
+    scaled = moe.permute(x, pl, scale=sc)
+    assert torch.equal(scaled[row], (x.float()[:, None] * sc.view(T, k, 1)).to(BF16))
+    q, s = moe.permute_quantized(x, pl)
+    q2, s2 = fp8.quantize_rows(xp)
+    assert torch.equal(q[:end], q2[:end]) and torch.equal(s[:, :end], s2[:, :end])
+    y = _r(pl.rows, d, seed=3)
+    gates, add = torch.rand(T, k, device="cuda"), _r(T, d, seed=4)
+    ref = (gates[..., None] * y.float()[row]).sum(1)
+    _close(moe.combine(y, pl, gates, T), ref, 1e-2)
+    _close(moe.combine(y, pl, None, T, add=add), y.float()[row].sum(1) + add.float(), 1e-2)
+
+
 @pytest.mark.parametrize("M,N", [(128, 320), (256, 256), (384, 264), (640, 520)])
 @pytest.mark.parametrize("dtype", [BF16, torch.float32])
 def test_grouped_wgrad_single_and_pair_kernels(M, N, dtype):
