@@ -130,8 +130,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 26);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int cb = static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x);  // long rows first
-  const int h = blockIdx.y, b = blockIdx.z;
+  // blocks start in index order, so the row block is the slowest index: the longest rows of all heads and
+  // batch entries first, the shortest fill the gaps at the end
+  const int cb = static_cast<int>(gridDim.z) - 1 - static_cast<int>(blockIdx.z);
+  const int h = blockIdx.x, b = blockIdx.y;
   const int g = h / (p.heads / p.kv_heads);
   const int gb = cb + p.q_off / 256;   // position of this CTA's rows among all keys
   const int row0 = cb * 256;           // first query row within the batch entry
@@ -424,10 +426,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int group = p.heads / p.kv_heads;
-  const int b = blockIdx.z;
-  // dQ: heavy blocks are the late query blocks; dKV: the early key blocks.
-  const int blk = DKV ? static_cast<int>(blockIdx.x) : p.n_blk - 1 - static_cast<int>(blockIdx.x);
-  const int hy = blockIdx.y;                       // query head (dQ) or KV head (dKV)
+  const int b = blockIdx.y;
+  // dQ: heavy blocks are the late query blocks; dKV: the early key blocks. Heavy blocks of all heads and
+  // batch entries come first, as in the forward.
+  const int blk = DKV ? static_cast<int>(blockIdx.z) : p.n_blk - 1 - static_cast<int>(blockIdx.z);
+  const int hy = blockIdx.x;                       // query head (dQ) or KV head (dKV)
   const int g = DKV ? hy : hy / group;
   // dQ: blk is a local query block, streamed tiles are global key tiles 0 .. diagonal.
   // dKV: blk is a global key block, streamed tiles are the local query tiles at or after it.
@@ -777,7 +780,7 @@ PB_API int pb_attn_fwd_cp(const void* q, const void* k, const void* v, void* out
   p.lse2 = static_cast<float*>(lse2);
   p.rowmax = static_cast<float*>(rowmax);
   p.status = status;
-  fwd::attn_fwd_kernel<<<dim3((seq + 255) / 256, heads, batch), 352, fwd::SMEM, st>>>(tQ, tK, tV, tO, p);
+  fwd::attn_fwd_kernel<<<dim3(heads, batch, (seq + 255) / 256), 352, fwd::SMEM, st>>>(tQ, tK, tV, tO, p);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -837,7 +840,7 @@ PB_API int pb_attn_bwd_cp(const void* q, const void* k, const void* v, const voi
     r |= tok_map(&tDQ, dq, qi, seq, batch, ldq, 128);
     if (r != 0) return 1000 + r;
     p.n_blk = (seq + 127) / 128;
-    bwd::attn_bwd_kernel<false><<<dim3(p.n_blk, heads, batch), 384, bwd::SMEM, st>>>(
+    bwd::attn_bwd_kernel<false><<<dim3(heads, batch, p.n_blk), 384, bwd::SMEM, st>>>(
         tQ, tDO, tK, tV, tDQ, tDQ, p);
   }
   {
@@ -851,7 +854,7 @@ PB_API int pb_attn_bwd_cp(const void* q, const void* k, const void* v, const voi
     r |= tok_map(&tDV, dv, ki, seq_kv, batch, ldkv, 128);
     if (r != 0) return 2000 + r;
     p.n_blk = (seq_kv + 127) / 128;
-    bwd::attn_bwd_kernel<true><<<dim3(p.n_blk, kv_heads, batch), 384, bwd::SMEM, st>>>(
+    bwd::attn_bwd_kernel<true><<<dim3(kv_heads, batch, p.n_blk), 384, bwd::SMEM, st>>>(
         tK, tV, tQ, tDO, tDK, tDV, p);
   }
   return static_cast<int>(cudaGetLastError());
