@@ -402,7 +402,7 @@ struct Params {
 // shared memory), which also makes room for four stages of streamed tiles: a tile's stage is held
 // until its gradient product is done, and with fewer every tile waits for a load. The softmax
 // scale is applied to the finished dQ / dK accumulator instead of to every dS.
-// 4 x 4096 x 16/4: dQ 618 -> 398 us, dK and dV 917 -> 689 us (two stages and operand tiles; three
+// 4 x 4096 x 16/4: dQ 618 -> 386 us, dK and dV 917 -> 555 us (two stages and operand tiles; three
 // stages: 471 and 721 us).
 template <bool DKV>
 __global__ void __launch_bounds__(384, 1)
