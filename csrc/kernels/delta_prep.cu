@@ -12,10 +12,10 @@
 // substitution with one column per thread (operand rows broadcast from shared memory as
 // 16-byte loads); A' goes back to shared memory as a 128-byte-swizzled bf16 operand for
 // the two products W and U^; every result leaves by a TMA store. A chunk is one long chain of
-// waits in two warps, so what counts is how many chunks an SM has in flight: three CTAs of 64
-// threads (75 KB and 128 tensor-memory columns each: U^ takes W's columns once W is in
-// registers). With two CTAs and columns of its own for U^, 4096 chunks took 165 us, with three
-// 141 us.
+// waits in two warps, so what counts is how many chunks an SM has in flight: four CTAs of 64
+// threads, 49 KB and 128 tensor-memory columns each. V takes the place of the fp32 A once the
+// substitution has read it, A' that of M once M is stored, and U^ W's columns once W is in registers.
+// 4096 chunks: two CTAs with room for everything 165 us, three 141 us, four 129 us.
 //
 // Sequences need not be a multiple of 64 tokens: the token tensors are mapped per batch entry, so the
 // rows the last chunk lacks load as zeros and are clipped from the stores; their beta counts as 0.
@@ -36,12 +36,11 @@ namespace dprep {
 
 constexpr int C = 64, D = 128;
 // A 64-row tile that serves as a 128-row A operand is read 8 KB past its end (A', the second halves of
-// K and Q); what follows each of them is inside the allocation, so the fp32 image of A, which no
-// product reads, comes last.
-constexpr int AP = 0, KT = 8192, QT = 24576, VT = 40960, AF = 57344, BARS = 73728;
-static_assert(AP + 16384 <= BARS && KT + 24576 <= BARS && QT + 24576 <= BARS, "A operands stay in bounds");
-constexpr int SMEM_BYTES = BARS + 256 + 1024;   // three CTAs per SM
-constexpr int FWD_CTAS = 3, FWD_COLS = 128;
+// K and Q); what follows each of them is inside the allocation.
+constexpr int KT = 0, QT = 16384, VA = 32768, BARS = 49152;   // Q, then M | T, then A' | T; A (fp32), then V
+static_assert(KT + 24576 <= BARS && QT + 24576 <= BARS, "A operands stay in bounds");
+constexpr int SMEM_BYTES = BARS + 256 + 1024;   // four CTAs per SM
+constexpr int FWD_CTAS = 4, FWD_COLS = 128;
 constexpr int TMEM_COLS = 256;   // backward
 
 struct Params {
@@ -90,12 +89,13 @@ delta_prep_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   uint64_t* mma1 = bars + 1;
   uint64_t* mma2 = bars + 2;
   uint64_t* mma3 = bars + 3;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4);
-  float4* af4 = reinterpret_cast<float4*>(smem + AF);
+  uint64_t* fullv = bars + 4;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 5);
+  float4* af4 = reinterpret_cast<float4*>(smem + VA);
 
   const int r = threadIdx.x, warp = r >> 5;
   if (r == 0) {
-    mbar_init(full, 1); mbar_init(mma1, 1); mbar_init(mma2, 1); mbar_init(mma3, 1);
+    mbar_init(full, 1); mbar_init(mma1, 1); mbar_init(mma2, 1); mbar_init(mma3, 1); mbar_init(fullv, 1);
     fence_barrier_init();
     tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmV);
   }
@@ -110,8 +110,8 @@ delta_prep_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   const uint32_t lane_addr = tmem + (static_cast<uint32_t>(warp * 32) << 16);
   const uint32_t id_kk64 = make_idesc(1, 1, 128, 64, 0, 0);    // A, B K-major, N = 64
   const uint32_t id_kn = make_idesc(1, 1, 128, 128, 0, 1);     // A K-major, B MN-major
-  const uint32_t kt = smem_u32(smem + KT), qt = smem_u32(smem + QT), vt = smem_u32(smem + VT);
-  const uint32_t ap = smem_u32(smem + AP);
+  const uint32_t kt = smem_u32(smem + KT), qt = smem_u32(smem + QT), vt = smem_u32(smem + VA);
+  const uint32_t ap = qt;
 
   uint32_t ph = 0;
   for (int g = blockIdx.x; g < p.total; g += gridDim.x, ph ^= 1) {
@@ -121,13 +121,11 @@ delta_prep_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     const int x0 = h * D;
     if (r == 0) {
       tma_store_wait_read<0>();  // earlier stores have drained the tiles about to be refilled
-      mbar_arrive_expect_tx(full, 3 * 16384);
+      mbar_arrive_expect_tx(full, 2 * 16384);
       tma_load_3d(smem + KT, &tmK, full, x0, t0, b);
       tma_load_3d(smem + KT + 8192, &tmK, full, x0 + 64, t0, b);
       tma_load_3d(smem + QT, &tmQ, full, x0, t0, b);
       tma_load_3d(smem + QT + 8192, &tmQ, full, x0 + 64, t0, b);
-      tma_load_3d(smem + VT, &tmV, full, x0, t0, b);
-      tma_load_3d(smem + VT + 8192, &tmV, full, x0 + 64, t0, b);
     }
     float beta = 0.f;
     if (t0 + r < p.seq_len) {
@@ -173,7 +171,12 @@ delta_prep_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     }
     // M = tril(Q K^T) -> the Q tile's first half (the products that read Q are complete)
     row_to_tile(lane_addr + 64, smem + QT, r, r);
+    fence_proxy_async_smem();
     __syncthreads();
+    if (r == 0) {
+      tma_store_3d(&tmM, smem + QT, 0, g * C, 0);
+      tma_store_commit();
+    }
 
     // column r of T = (I + A)^-1 by forward substitution
     float t[64];
@@ -190,10 +193,19 @@ delta_prep_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
       }
       t[i] = (a0 + a1) + (a2 + a3);
     }
-    // T -> the Q tile's second half, A' = T diag(beta) -> operand tile (element (i, r) each)
+    // A has been read and M has left: V comes into A's place, A' goes into M's
+    if (r == 0) tma_store_wait_read<0>();
+    fence_proxy_async_smem();
+    __syncthreads();
+    if (r == 0) {
+      mbar_arrive_expect_tx(fullv, 16384);
+      tma_load_3d(smem + VA, &tmV, fullv, x0, t0, b);
+      tma_load_3d(smem + VA + 8192, &tmV, fullv, x0 + 64, t0, b);
+    }
+    // T -> the Q tile's second half, A' = T diag(beta) -> its first (element (i, r) each)
     {
       uint8_t* tt = smem + QT + 8192;
-      uint8_t* at = smem + AP;
+      uint8_t* at = smem + QT;
       const int sub = (r & 7) * 2, c16 = r >> 3;
 #pragma unroll
       for (int i = 0; i < 64; ++i) {
@@ -212,9 +224,8 @@ delta_prep_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
         umma_f16(tmem, make_sdesc_sw128(ap + j * 32, 16, 1024),
                  make_sdesc_sw128(kt + j * 2048, 8192, 1024), id_kn, j > 0);
       umma_commit(mma2);
-      tma_store_3d(&tmM, smem + QT, 0, g * C, 0);
       tma_store_3d(&tmT, smem + QT + 8192, 0, g * C, 0);
-      tma_store_3d(&tmAP, smem + AP, 0, g * C, 0);
+      tma_store_3d(&tmAP, smem + QT, 0, g * C, 0);
       tma_store_commit();
     }
     ok = mbar_wait_spin(mma2, ph, p.status);
@@ -226,7 +237,7 @@ delta_prep_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     fence_proxy_async_smem();
     tc_fence_before();
     __syncthreads();
-    if (r == 0) {
+    if (r == 0 && (ok = mbar_wait_spin(fullv, ph, p.status))) {
       tc_fence_after();
 #pragma unroll
       for (int j = 0; j < 4; ++j)       // U^ = A' V -> the same columns
@@ -237,18 +248,18 @@ delta_prep_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
       tma_store_3d(&tmW, smem + KT + 8192, 64, g * C, 0);
       tma_store_commit();
     }
-    ok = mbar_wait_spin(mma3, ph, p.status);
+    ok = mbar_wait_spin(mma3, ph, p.status) && ok;
     if (!__syncthreads_and(ok)) break;
     tc_fence_after();
     // U^ -> V tile
-    row_to_tile(lane_addr + 0, smem + VT, r, 63);
-    row_to_tile(lane_addr + 64, smem + VT + 8192, r, 63);
+    row_to_tile(lane_addr + 0, smem + VA, r, 63);
+    row_to_tile(lane_addr + 64, smem + VA + 8192, r, 63);
     fence_proxy_async_smem();
     tc_fence_before();
     __syncthreads();
     if (r == 0) {
-      tma_store_3d(&tmU, smem + VT, 0, g * C, 0);
-      tma_store_3d(&tmU, smem + VT + 8192, 64, g * C, 0);
+      tma_store_3d(&tmU, smem + VA, 0, g * C, 0);
+      tma_store_3d(&tmU, smem + VA + 8192, 64, g * C, 0);
       tma_store_commit();
     }
   }
