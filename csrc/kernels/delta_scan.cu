@@ -23,6 +23,11 @@
 // before the state image is ready. 64 sequences of 64 chunks, forward 230 us -> 144 us (3.6 -> 2.3 us a
 // chunk), backward 133 -> 117 us, against four row warps that did all of it in order.
 //
+// The columns of the state never mix (U, O and dU have the same columns), so when the sequences or
+// segments take at most half of the SMs, two CTAs walk each of them with 64 columns: the conversions
+// and products between two waits are half as long. 64 sequences: 144 -> 115 us forward, 109 -> 103 us
+// backward. With more CTAs than SMs it would be two waves of a chain that is not half as long.
+//
 // warps 0-7: tensor-memory <-> registers <-> shared/global (lane = state row or token)
 // warp 8   : MMA issue (one lane)          warp 9: TMA producer (one lane)
 //
@@ -37,6 +42,7 @@ namespace pb {
 int make_tmap_3d(CUtensorMap* tm, const void* base, int elem_bytes, uint64_t inner,
                  uint64_t outer, uint64_t batch, uint64_t ld_elems, uint64_t batch_stride_elems,
                  uint32_t box_inner, uint32_t box_outer);
+int num_sms();
 
 namespace dscan {
 
@@ -79,12 +85,8 @@ struct Smem {
   static constexpr int TOTAL = BARS + 256 + 1024;
 };
 
-// 16-byte store of 8 bf16 into a [rows][64 n] 128B-swizzled MN-major operand chunk.
-__device__ __forceinline__ void st_swz(uint8_t* chunk_base, int krow, int c16, const bf16x8& v) {
-  *reinterpret_cast<bf16x8*>(chunk_base + krow * 128 + ((c16 ^ (krow & 7)) << 4)) = v;
-}
-
-template <bool BWD>
+// NC: state columns of a CTA, 128 or 64 (then two CTAs per segment, not in summary mode)
+template <bool BWD, int NC>
 __global__ void __launch_bounds__(THREADS, 1)
 delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmQ,
                   const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmM,
@@ -110,14 +112,17 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_units = p.n_seq * p.n_seg;
-  const int half = static_cast<int>(blockIdx.x) / n_units;      // 1: the identity-start CTA
+  constexpr int HALVES = NC / 64;       // 64-column operand chunks
+  constexpr int WC = NC / 2;            // columns of a row warp
+  const int half = static_cast<int>(blockIdx.x) / n_units;      // 1: the identity-start CTA, or the upper columns
   const int unit = static_cast<int>(blockIdx.x) % n_units;      // seq * n_seg + seg
+  const int col0 = NC == 64 ? half * 64 : 0;                    // this CTA's first state column
   const int seq = unit / p.n_seg;
   const int N = p.n_chunks / p.n_seg;                           // chunks this CTA walks
   const int n0 = (unit % p.n_seg) * N;                          // its first chunk
   const int NT = p.n_chunks;
   const bool sum = p.summary != 0;
-  const bool lin = sum && half == 1;                            // linear part only: U^ = 0
+  const bool lin = NC == 128 && sum && half == 1;                            // linear part only: U^ = 0
   const bool store_ux = !sum && p.store_ux != 0;
   const bool tokmaj = p.heads > 0;
   // token tensors: batch entry, first row and first column of this sequence
@@ -150,7 +155,7 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
       // a forward summary needs neither Q nor M (no output product), its linear half no U^
       const bool need_qm = BWD || !sum;
       const bool need_fifth = BWD || !lin;
-      const uint32_t stage_tx = 32768u + (need_qm ? 24576u : 0u) + (need_fifth ? 16384u : 0u);
+      const uint32_t stage_tx = 32768u + (need_qm ? 24576u : 0u) + (need_fifth ? HALVES * 8192u : 0u);
       for (int it = 0; it < N; ++it) {
         const int n = n0 + (BWD ? (N - 1 - it) : it);
         const int s = it & 1;
@@ -170,19 +175,21 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
           tma_load_3d(st + TILE_M, &tmM, &full[s], 0, row, 0);
         }
         if (BWD) {
-          tma_load_3d(st + TILE_DO, &tmDO, &full[s], tx, trow, tb);
-          tma_load_3d(st + TILE_DO + 8192, &tmDO, &full[s], tx + 64, trow, tb);
+#pragma unroll
+          for (int hf = 0; hf < HALVES; ++hf)
+            tma_load_3d(st + TILE_DO + hf * 8192, &tmDO, &full[s], tx + col0 + hf * 64, trow, tb);
         } else if (need_fifth) {
-          tma_load_3d(st + TILE_DO, &tmDO, &full[s], 0, row, 0);
-          tma_load_3d(st + TILE_DO + 8192, &tmDO, &full[s], 64, row, 0);
+#pragma unroll
+          for (int hf = 0; hf < HALVES; ++hf)
+            tma_load_3d(st + TILE_DO + hf * 8192, &tmDO, &full[s], col0 + hf * 64, row, 0);
         }
       }
     }
   } else if (warp == 8) {
     // -------------------------------- MMA issuer --------------------------------
     if (lane == 0) {
-      const uint32_t id_kn = make_idesc(1, 1, 128, 128, 0, 1);  // A K-major, B MN-major
-      const uint32_t id_nn = make_idesc(1, 1, 128, 128, 1, 1);  // A MN-major, B MN-major
+      const uint32_t id_kn = make_idesc(1, 1, 128, NC, 0, 1);  // A K-major, B MN-major
+      const uint32_t id_nn = make_idesc(1, 1, 128, NC, 1, 1);  // A MN-major, B MN-major
       const uint32_t xb_a = smem_u32(xb), ub_a = smem_u32(ub);
       for (int it = 0; it < N; ++it) {
         const int s = it & 1;
@@ -256,7 +263,7 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     // the bf16 state image is stored from the very tile the MMAs read, U / -dU from the
     // operand tile, O from a staging tile. Thread 0 issues and tracks the stores.
     const int r = (warp & 3) * 32 + lane;  // tensor-memory lane = state row (or token row < 64)
-    const int ch = warp >> 2, c0 = ch * 64;   // this warp's half of the columns
+    const int ch = warp >> 2, c0 = ch * WC;   // this warp's half of the CTA's columns
     const bool tok_warp = (warp & 3) < 2;     // warps whose lanes are token rows
     const uint32_t lane_addr = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + c0;
     auto sync_rows = [] { asm volatile("bar.sync 1, 256;" ::: "memory"); };
@@ -267,26 +274,31 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
       __syncwarp();
       if (lane == 0) mbar_arrive(bar);
     };
-    // 64 accumulator columns at `col` of this lane
-    auto load64 = [&](uint32_t col, uint32_t (&v)[64]) {
-      tmem_ld_32x32b_x32(lane_addr + col, v);
-      tmem_ld_32x32b_x32(lane_addr + col + 32, v + 32);
+    // this warp's accumulator columns from `col` of this lane
+    auto load_cols = [&](uint32_t col, uint32_t (&v)[WC]) {
+#pragma unroll
+      for (int c = 0; c < WC; c += 32) tmem_ld_32x32b_x32(lane_addr + col + c, v + c);
       tmem_ld_wait();
     };
-    auto put64 = [&](uint8_t* tile, const uint32_t (&v)[64]) {   // -> bf16 swizzled 64-column chunk
+    // 16-byte piece i of this warp's columns in an operand image of `rows` rows per 64-column chunk
+    auto piece = [&](uint8_t* tile, int rows, int i) -> uint8_t* {
+      const int cc = c0 + 8 * i;
+      return tile + (cc >> 6) * rows * 128 + r * 128 + ((((cc & 63) >> 3) ^ (r & 7)) << 4);
+    };
+    auto put_cols = [&](uint8_t* tile, int rows, const uint32_t (&v)[WC]) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
+      for (int i = 0; i < WC / 8; ++i) {
         bf16x8 pk;
 #pragma unroll
         for (int j = 0; j < 4; ++j)
           pk.v[j] = __floats2bfloat162_rn(__uint_as_float(v[8 * i + 2 * j]), __uint_as_float(v[8 * i + 2 * j + 1]));
-        st_swz(tile, r, i, pk);
+        *reinterpret_cast<bf16x8*>(piece(tile, rows, i)) = pk;
       }
     };
     {
-      const float* x0 = (p.x_init && !sum) ? p.x_init + (static_cast<size_t>(unit) * D + r) * D + c0 : nullptr;
+      const float* x0 = (p.x_init && !sum) ? p.x_init + (static_cast<size_t>(unit) * D + r) * D + col0 + c0 : nullptr;
 #pragma unroll 1
-      for (int c = 0; c < 64; c += 32) {
+      for (int c = 0; c < WC; c += 32) {
         uint32_t v[32];
 #pragma unroll
         for (int i = 0; i < 32; ++i)
@@ -311,9 +323,9 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
       }
       // bf16 image of the state entering this chunk
       {
-        uint32_t v[64];
-        load64(COL_X, v);
-        put64(xb + ch * 16384, v);
+        uint32_t v[WC];
+        load_cols(COL_X, v);
+        put_cols(xb, D, v);
       }
       arrive(x_ready);
       if (!BWD && !sum && it > 0) {
@@ -321,9 +333,9 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
         if (!mbar_wait_spin(o_done, cph ^ 1, p.status)) { ok = false; break; }
         tc_fence_after();
         if (tok_warp) {
-          uint32_t v[64];
-          load64(COL_O + (cph ^ 1) * 128, v);
-          put64(ob + ch * 8192, v);
+          uint32_t v[WC];
+          load_cols(COL_O + (cph ^ 1) * 128, v);
+          put_cols(ob, C, v);
           fence_proxy_async_smem();
         }
       }
@@ -332,12 +344,12 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
         if (r == 0 && ch == 0) {
           if (!BWD && it > 0) {
             const int prow = tok0 + (n - 1) * C;
-            tma_store_3d(&tmO, ob, tx, prow, tb);
-            tma_store_3d(&tmO, ob + 8192, tx + 64, prow, tb);
+#pragma unroll
+            for (int hf = 0; hf < HALVES; ++hf) tma_store_3d(&tmO, ob + hf * 8192, tx + col0 + hf * 64, prow, tb);
           }
           if (store_ux) {
-            tma_store_3d(&tmXB, xb, 0, g * D, 0);
-            tma_store_3d(&tmXB, xb + 16384, 64, g * D, 0);
+#pragma unroll
+            for (int hf = 0; hf < HALVES; ++hf) tma_store_3d(&tmXB, xb + hf * 16384, col0 + hf * 64, g * D, 0);
           }
           tma_store_commit();
         }
@@ -345,31 +357,31 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
       if (!mbar_wait_spin(y_done, cph, p.status)) { ok = false; break; }
       tc_fence_after();
       if (tok_warp) {
-        uint32_t v[64];
-        load64(COL_Y, v);
-        const uint8_t* uh = smem + (it & 1) * S::STAGE + TILE_DO + ch * 8192 + r * 128;
+        uint32_t v[WC];
+        load_cols(COL_Y, v);
+        uint8_t* uh = smem + (it & 1) * S::STAGE + TILE_DO;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < WC / 8; ++i) {
           float y[8];
 #pragma unroll
           for (int j = 0; j < 8; ++j) y[j] = __uint_as_float(v[8 * i + j]);
           if (!BWD && !lin) {
             float uhv[8];
-            unpack8(*reinterpret_cast<const bf16x8*>(uh + ((i ^ (r & 7)) << 4)), uhv);
+            unpack8(*reinterpret_cast<const bf16x8*>(piece(uh, C, i)), uhv);
 #pragma unroll
             for (int j = 0; j < 8; ++j) y[j] = uhv[j] - y[j];  // U = U^ - W S
           } else {
 #pragma unroll
             for (int j = 0; j < 8; ++j) y[j] = -y[j];          // operand (and output) is -dU
           }
-          st_swz(ub + ch * 8192, r, i, pack8(y));
+          *reinterpret_cast<bf16x8*>(piece(ub, C, i)) = pack8(y);
         }
         arrive(u_ready);
         if (store_ux) {
           sync_tok();
           if (r == 0 && ch == 0) {
-            tma_store_3d(&tmU, ub, 0, g * C, 0);
-            tma_store_3d(&tmU, ub + 8192, 64, g * C, 0);
+#pragma unroll
+            for (int hf = 0; hf < HALVES; ++hf) tma_store_3d(&tmU, ub + hf * 8192, col0 + hf * 64, g * C, 0);
             tma_store_commit();
           }
         }
@@ -383,26 +395,26 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
         if (r == 0 && ch == 0) tma_store_wait_read<0>();
         sync_rows();
         if (tok_warp) {
-          uint32_t v[64];
-          load64(COL_O + ((N - 1) & 1) * 128, v);
-          put64(ob + ch * 8192, v);
+          uint32_t v[WC];
+          load_cols(COL_O + ((N - 1) & 1) * 128, v);
+          put_cols(ob, C, v);
           fence_proxy_async_smem();
         }
         sync_rows();
         if (r == 0 && ch == 0) {
           const int prow = tok0 + (n0 + N - 1) * C;
-          tma_store_3d(&tmO, ob, tx, prow, tb);
-          tma_store_3d(&tmO, ob + 8192, tx + 64, prow, tb);
+#pragma unroll
+          for (int hf = 0; hf < HALVES; ++hf) tma_store_3d(&tmO, ob + hf * 8192, tx + col0 + hf * 64, prow, tb);
           tma_store_commit();
         }
       }
       float* fin = lin ? p.p_final : p.x_final;
       if (fin != nullptr) {
-        float* xf = fin + (static_cast<size_t>(unit) * D + r) * D + c0;
-        uint32_t v[64];
-        load64(COL_X, v);
+        float* xf = fin + (static_cast<size_t>(unit) * D + r) * D + col0 + c0;
+        uint32_t v[WC];
+        load_cols(COL_X, v);
 #pragma unroll
-        for (int i = 0; i < 16; ++i)
+        for (int i = 0; i < WC / 4; ++i)
           reinterpret_cast<float4*>(xf)[i] =
               make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]),
                           __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3]));
@@ -423,17 +435,25 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
   }
 }
 
-template <bool BWD>
-int launch(const void* W, const void* Q, const void* K, const void* M, const void* fifth,
-           void* xb_out, void* u_out, void* o_out, int seq_len, int ld, const Params& p, cudaStream_t st) {
+template <bool BWD, int NC>
+int launch_cols(const CUtensorMap& tW, const CUtensorMap& tQ, const CUtensorMap& tK, const CUtensorMap& tM,
+                const CUtensorMap& tD, const CUtensorMap& tXB, const CUtensorMap& tU, const CUtensorMap& tO,
+                const Params& p, int ctas, cudaStream_t st) {
   static pb::DeviceOnce attr_once;   // per device: the attribute belongs to the current GPU
   if (attr_once.need()) {
-    cudaError_t e = cudaFuncSetAttribute(delta_scan_kernel<BWD>,
+    cudaError_t e = cudaFuncSetAttribute(delta_scan_kernel<BWD, NC>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          Smem<BWD>::TOTAL);
     if (e != cudaSuccess) return static_cast<int>(e);
     attr_once.done();
   }
+  delta_scan_kernel<BWD, NC><<<ctas, THREADS, Smem<BWD>::TOTAL, st>>>(tW, tQ, tK, tM, tD, tXB, tU, tO, p);
+  return static_cast<int>(cudaGetLastError());
+}
+
+template <bool BWD>
+int launch(const void* W, const void* Q, const void* K, const void* M, const void* fifth,
+           void* xb_out, void* u_out, void* o_out, int seq_len, int ld, const Params& p, cudaStream_t st) {
   const uint64_t G = static_cast<uint64_t>(p.n_seq) * p.n_chunks;
   const uint64_t rows = G * C;
   CUtensorMap tW, tQ, tK, tM, tD, tXB, tU, tO;
@@ -458,9 +478,10 @@ int launch(const void* W, const void* Q, const void* K, const void* M, const voi
   if (BWD) tO = tU;
   else r |= tok_map(&tO, o_out);
   if (r != 0) return 1000 + r;
-  const int ctas = p.n_seq * p.n_seg * ((p.summary && !BWD) ? 2 : 1);
-  delta_scan_kernel<BWD><<<ctas, THREADS, Smem<BWD>::TOTAL, st>>>(tW, tQ, tK, tM, tD, tXB, tU, tO, p);
-  return static_cast<int>(cudaGetLastError());
+  const int units = p.n_seq * p.n_seg;
+  if (!p.summary && 2 * units <= num_sms())
+    return launch_cols<BWD, 64>(tW, tQ, tK, tM, tD, tXB, tU, tO, p, 2 * units, st);
+  return launch_cols<BWD, 128>(tW, tQ, tK, tM, tD, tXB, tU, tO, p, units * ((p.summary && !BWD) ? 2 : 1), st);
 }
 
 }  // namespace dscan

@@ -505,6 +505,34 @@ def test_delta_rule_ragged_equals_explicit_padding(B, S, H, seg):
         assert torch.equal(delta_rule_fused(off, k, v, beta, s0, n_seg=seg)[0], out)
 
 
+@pytest.mark.parametrize("S,seg", [(130, 1), (512, 2)])
+def test_delta_walk_column_split_equals_whole_state(S, seg):
+    """More CTAs than half the GPU walk the state in one piece, fewer in two halves of its columns: a
+    batch of 96 sequences against its entries one by one, with state and gradients."""
+    from prometheus_b200.ops import functional as ops
+    from prometheus_b200.ops.delta import delta_rule_fused
+
+    B, H, D = 6, 16, 128
+    q = torch.nn.functional.normalize(_r(B, S, H, D, seed=1).float(), dim=-1).to(BF16)
+    k = torch.nn.functional.normalize(_r(B, S, H, D, seed=2).float(), dim=-1).to(BF16)
+    v, go = _r(B, S, H, D, seed=3), _r(B, S, H, D, seed=6)
+    beta = torch.sigmoid(_r(B, S, H, seed=4).float()).to(BF16)
+    s0 = _r(B, H, D, D, seed=5, scale=0.05, dtype=torch.float32)
+    gs = _r(B, H, D, D, seed=7, scale=0.1, dtype=torch.float32)
+
+    def run(sl):
+        leaves = [t[sl].clone().requires_grad_(True) for t in (q, k, v, beta, s0)]
+        out = delta_rule_fused(*leaves, n_seg=seg)
+        grads = torch.autograd.grad(out, leaves, (go[sl], gs[sl]))
+        ops.check_status("cuda")
+        return [t.detach() for t in (*out, *grads)]
+
+    whole = run(slice(0, B))
+    for i in range(B):
+        for name, a, b in zip(("out", "state", "dq", "dk", "dv", "dbeta", "ds0"), run(slice(i, i + 1)), whole):
+            assert torch.equal(a[0], b[i]), (name, i)
+
+
 @pytest.mark.parametrize("B,S,H", [(1, 64, 1), (2, 100, 3), (5, 4096, 2)])
 def test_delta_chunk_products(B, S, H):
     """The four products against batched fp32, with fewer and with more chunks than CTAs."""
