@@ -50,6 +50,7 @@ struct Params {
   int total;      // batch * heads * n_chunks
   const void* beta;  // [batch, seq, heads]
   int beta_f32;
+  int store_ta;   // 0: A' and T are not wanted (nothing will run backward)
   int* status;
 };
 
@@ -208,10 +209,12 @@ delta_prep_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
       uint8_t* at = smem + QT;
       const int sub = (r & 7) * 2, c16 = r >> 3;
 #pragma unroll
-      for (int i = 0; i < 64; ++i) {
-        const int off = i * 128 + ((c16 ^ (i & 7)) << 4) + sub;
-        *reinterpret_cast<bf16*>(tt + off) = f32_to_bf16(t[i]);
-        *reinterpret_cast<bf16*>(at + off) = f32_to_bf16(t[i] * beta);
+      for (int i = 0; i < 64; ++i)
+        *reinterpret_cast<bf16*>(at + i * 128 + ((c16 ^ (i & 7)) << 4) + sub) = f32_to_bf16(t[i] * beta);
+      if (p.store_ta) {
+#pragma unroll
+        for (int i = 0; i < 64; ++i)
+          *reinterpret_cast<bf16*>(tt + i * 128 + ((c16 ^ (i & 7)) << 4) + sub) = f32_to_bf16(t[i]);
       }
     }
     fence_proxy_async_smem();
@@ -224,9 +227,11 @@ delta_prep_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
         umma_f16(tmem, make_sdesc_sw128(ap + j * 32, 16, 1024),
                  make_sdesc_sw128(kt + j * 2048, 8192, 1024), id_kn, j > 0);
       umma_commit(mma2);
-      tma_store_3d(&tmT, smem + QT + 8192, 0, g * C, 0);
-      tma_store_3d(&tmAP, smem + QT, 0, g * C, 0);
-      tma_store_commit();
+      if (p.store_ta) {
+        tma_store_3d(&tmT, smem + QT + 8192, 0, g * C, 0);
+        tma_store_3d(&tmAP, smem + QT, 0, g * C, 0);
+        tma_store_commit();
+      }
     }
     ok = mbar_wait_spin(mma2, ph, p.status);
     if (!__syncthreads_and(ok)) break;
@@ -611,7 +616,7 @@ using namespace pb;
 // q, k, v: bf16 [batch, seq_len, ld] row-major with head h at columns [128 h, 128 h + 128)
 // (ld >= heads * 128, a multiple of 8); beta: [batch, seq_len, heads], fp32 or bf16.
 // Outputs, chunk g = (b * heads + h) * n_chunks + n, n_chunks = ceil(seq_len / 64): W, U^ [g][64][128];
-// M, A', T [g][64][64].
+// M, A', T [g][64][64]. A' and T may both be null when nothing will run backward.
 PB_API int pb_delta_prep_fwd(const void* q, const void* k, const void* v, const void* beta,
                              int beta_f32, void* W, void* Uhat, void* M, void* Ap, void* T,
                              int batch, int seq_len, int heads, int ld, int* status,
@@ -630,6 +635,8 @@ PB_API int pb_delta_prep_fwd(const void* q, const void* k, const void* v, const 
   p.n_chunks = (seq_len + C - 1) / C; p.heads = heads; p.seq_len = seq_len;
   p.total = batch * heads * p.n_chunks;
   p.beta = beta; p.beta_f32 = beta_f32; p.status = status;
+  p.store_ta = Ap != nullptr;
+  if (p.store_ta != (T != nullptr)) return PB_BAD_ARG;
   const uint64_t bstr = static_cast<uint64_t>(seq_len) * ld;   // batch stride of the token tensors
   const uint64_t rows = static_cast<uint64_t>(p.total) * C;
   CUtensorMap tK, tQ, tV, tW, tU, tM, tA, tT;
@@ -640,8 +647,11 @@ PB_API int pb_delta_prep_fwd(const void* q, const void* k, const void* v, const 
   r |= make_tmap_3d(&tW, W, 2, D, rows, 1, D, 0, 64, C);
   r |= make_tmap_3d(&tU, Uhat, 2, D, rows, 1, D, 0, 64, C);
   r |= make_tmap_3d(&tM, M, 2, C, rows, 1, C, 0, 64, C);
-  r |= make_tmap_3d(&tA, Ap, 2, C, rows, 1, C, 0, 64, C);
-  r |= make_tmap_3d(&tT, T, 2, C, rows, 1, C, 0, 64, C);
+  tA = tT = tM;
+  if (p.store_ta) {
+    r |= make_tmap_3d(&tA, Ap, 2, C, rows, 1, C, 0, 64, C);
+    r |= make_tmap_3d(&tT, T, 2, C, rows, 1, C, 0, 64, C);
+  }
   if (r != 0) return 1000 + r;
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);

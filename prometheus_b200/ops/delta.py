@@ -201,7 +201,7 @@ class _DeltaFusedFn(torch.autograd.Function):
     is written in that layout; the rows a last partial chunk lacks read as zeros with beta = 0,
     which leaves the state untouched, and are not written. The chunk-local part of the backward is
     one kernel of batched products (``pb_delta_chunk_products``) and ``pb_delta_prep_bwd``.
-    ``keep``: something will run backward, so the walk's U and bf16 states are stored.
+    ``keep``: something will run backward, so A', T, the walk's U and the bf16 states are stored.
 
     The walk is affine in the state, ``S_out = P S_in + R`` per run of chunks. When the batch
     has too few sequences to fill the GPU (``scan_segments`` > 1), or when the sequence is
@@ -228,8 +228,8 @@ class _DeltaFusedFn(torch.autograd.Function):
         w = torch.empty((g, 64, 128), dtype=bf, device=dev)
         uhat = torch.empty_like(w)
         m = torch.empty((g, 64, 64), dtype=bf, device=dev)
-        ap = torch.empty_like(m)
-        t = torch.empty_like(m)
+        ap = torch.empty_like(m) if keep else None
+        t = torch.empty_like(m) if keep else None
         status = ptr(status_word(dev))
         call("pb_delta_prep_fwd", ptr(q), ptr(k), ptr(v), ptr(beta),
              1 if beta.dtype == torch.float32 else 0, ptr(w), ptr(uhat), ptr(m), ptr(ap), ptr(t),
