@@ -121,23 +121,12 @@ __global__ void count_kernel(const int* __restrict__ ids, int n_pairs, int pairs
     block_counts[static_cast<size_t>(blockIdx.x) * E + e] = hist[e];
 }
 
-// One block. Turns block_counts into exclusive per-block bases, and writes
+// Segment starts from the experts' totals (one block; tot and off in shared memory):
 //   expert_off[e] (128-aligned segment starts, expert_off[E] = rows in use), totals[e],
 //   k_len[e] = padded segment length, mblk_group[m] for m < max_mblk (-1 beyond the data).
-__global__ void scan_kernel(int* __restrict__ block_counts, int nblocks, int E,
-                            int* __restrict__ expert_off, int* __restrict__ totals,
-                            int* __restrict__ k_len, int* __restrict__ mblk_group, int max_mblk) {
-  __shared__ int tot[MAX_E];
-  __shared__ int off[MAX_E + 1];
-  for (int e = threadIdx.x; e < E; e += blockDim.x) {
-    int run = 0;
-    for (int b = 0; b < nblocks; ++b) {
-      const int c = block_counts[static_cast<size_t>(b) * E + e];
-      block_counts[static_cast<size_t>(b) * E + e] = run;
-      run += c;
-    }
-    tot[e] = run;
-  }
+__device__ __forceinline__ void write_segments(const int* tot, int* off, int E, int* __restrict__ expert_off,
+                                               int* __restrict__ totals, int* __restrict__ k_len,
+                                               int* __restrict__ mblk_group, int max_mblk) {
   __syncthreads();
   if (threadIdx.x == 0) {
     int run = 0;
@@ -170,17 +159,27 @@ __global__ void scan_kernel(int* __restrict__ block_counts, int nblocks, int E,
   }
 }
 
-// One warp per block of pairs walks them in order; row_of[i] = expert_off + block base + rank.
-__global__ void place_kernel(const int* __restrict__ ids, int n_pairs, int pairs_per_block, int E,
-                             const int* __restrict__ block_base, const int* __restrict__ expert_off,
-                             int* __restrict__ row_of) {
-  __shared__ int run[MAX_E];
-  const int lane = threadIdx.x;
-  for (int e = lane; e < E; e += 32)
-    run[e] = expert_off[e] + block_base[static_cast<size_t>(blockIdx.x) * E + e];
-  __syncwarp();
-  const int lo = blockIdx.x * pairs_per_block;
-  const int hi = min(lo + pairs_per_block, n_pairs);
+// One block. Turns block_counts into exclusive per-block bases and writes the segments.
+__global__ void scan_kernel(int* __restrict__ block_counts, int nblocks, int E,
+                            int* __restrict__ expert_off, int* __restrict__ totals,
+                            int* __restrict__ k_len, int* __restrict__ mblk_group, int max_mblk) {
+  __shared__ int tot[MAX_E];
+  __shared__ int off[MAX_E + 1];
+  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+    int run = 0;
+    for (int b = 0; b < nblocks; ++b) {
+      const int c = block_counts[static_cast<size_t>(b) * E + e];
+      block_counts[static_cast<size_t>(b) * E + e] = run;
+      run += c;
+    }
+    tot[e] = run;
+  }
+  write_segments(tot, off, E, expert_off, totals, k_len, mblk_group, max_mblk);
+}
+
+// One warp walks the pairs [lo, hi) in order; run[e] is the next row of expert e for them.
+__device__ __forceinline__ void place_pairs(const int* __restrict__ ids, int lo, int hi, int* run,
+                                            int* __restrict__ row_of, int lane) {
   for (int base = lo; base < hi; base += 32) {
     const int i = base + lane;
     const bool on = i < hi;
@@ -198,12 +197,97 @@ __global__ void place_kernel(const int* __restrict__ ids, int n_pairs, int pairs
   }
 }
 
+// One warp per block of pairs; row_of[i] = expert_off + block base + rank.
+__global__ void place_kernel(const int* __restrict__ ids, int n_pairs, int pairs_per_block, int E,
+                             const int* __restrict__ block_base, const int* __restrict__ expert_off,
+                             int* __restrict__ row_of) {
+  __shared__ int run[MAX_E];
+  const int lane = threadIdx.x;
+  for (int e = lane; e < E; e += 32)
+    run[e] = expert_off[e] + block_base[static_cast<size_t>(blockIdx.x) * E + e];
+  __syncwarp();
+  const int lo = blockIdx.x * pairs_per_block;
+  place_pairs(ids, lo, min(lo + pairs_per_block, n_pairs), run, row_of, lane);
+}
+
+// The whole sort in one block, each warp an eighth of the pairs: three launches less two for inputs whose
+// kernels are shorter than a launch. Same placement (stable in the pair index).
+// 1024 pairs, 8 experts: 10 us in three kernels -> 3.1 us in one; SORT_MAX pairs are where its walk takes as long
+// as the three together.
+constexpr int SORT_WARPS = 8, SORT_MAX = 4096;
+__global__ void __launch_bounds__(SORT_WARPS * 32) sort_small_kernel(const int* __restrict__ ids, int n_pairs, int E,
+                                                                     int* __restrict__ row_of,
+                                                                     int* __restrict__ expert_off,
+                                                                     int* __restrict__ totals,
+                                                                     int* __restrict__ k_len,
+                                                                     int* __restrict__ mblk_group, int max_mblk) {
+  __shared__ int run[SORT_WARPS][MAX_E];
+  __shared__ int tot[MAX_E];
+  __shared__ int off[MAX_E + 1];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int e = lane; e < E; e += 32) run[warp][e] = 0;
+  __syncwarp();
+  const int per = ((n_pairs + SORT_WARPS - 1) / SORT_WARPS + 31) / 32 * 32;
+  const int lo = min(warp * per, n_pairs), hi = min(lo + per, n_pairs);
+  for (int i = lo + lane; i < hi; i += 32) atomicAdd(&run[warp][ids[i]], 1);
+  __syncthreads();
+  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+    int sum = 0;
+#pragma unroll
+    for (int w = 0; w < SORT_WARPS; ++w) {
+      const int c = run[w][e];
+      run[w][e] = sum;
+      sum += c;
+    }
+    tot[e] = sum;
+  }
+  write_segments(tot, off, E, expert_off, totals, k_len, mblk_group, max_mblk);   // synchronises first
+  for (int e = lane; e < E; e += 32) run[warp][e] += off[e];
+  __syncwarp();
+  place_pairs(ids, lo, hi, run[warp], row_of, lane);
+}
+
+constexpr int PAD_SPLIT = 8;   // blocks per expert that clear its padding rows
+// zero rows [expert_off[e] + totals[e], expert_off[e + 1]), part of `parts` blocks
+__device__ __forceinline__ void zero_pad_rows(bf16* __restrict__ buf, int d, int e, int part, int parts,
+                                              const int* __restrict__ expert_off, const int* __restrict__ totals) {
+  const int lo = expert_off[e] + totals[e], hi = expert_off[e + 1];
+  const size_t n8 = static_cast<size_t>(hi - lo) * d / 8;
+  bf16x8 z;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) z.v[j] = __floats2bfloat162_rn(0.f, 0.f);
+  bf16x8* p = reinterpret_cast<bf16x8*>(buf + static_cast<size_t>(lo) * d);
+  for (size_t i = part * blockDim.x + threadIdx.x; i < n8; i += static_cast<size_t>(parts) * blockDim.x) p[i] = z;
+}
+__global__ void __launch_bounds__(256) zero_pad_kernel(bf16* __restrict__ buf, int d, const int* __restrict__ expert_off,
+                                                       const int* __restrict__ totals) {
+  zero_pad_rows(buf, d, blockIdx.x, blockIdx.y, gridDim.y, expert_off, totals);
+}
+// the same rows of a quantised buffer: zero bytes, scale 1 (what the row quantiser makes of zeros)
+__device__ __forceinline__ void zero_pad_q_rows(uint8_t* __restrict__ q, float* __restrict__ scales, int K, long rows,
+                                                int e, int part, const int* __restrict__ expert_off,
+                                                const int* __restrict__ totals) {
+  const int lo = expert_off[e] + totals[e], n = expert_off[e + 1] - lo;
+  const size_t first = part * blockDim.x + threadIdx.x, step = static_cast<size_t>(PAD_SPLIT) * blockDim.x;
+  uint4* p = reinterpret_cast<uint4*>(q + static_cast<size_t>(lo) * K);
+  for (size_t i = first; i < static_cast<size_t>(n) * K / 16; i += step) p[i] = make_uint4(0u, 0u, 0u, 0u);
+  for (size_t i = first; i < static_cast<size_t>(n) * (K / 128); i += step)
+    scales[(i / n) * rows + lo + i % n] = 1.f;
+}
+
 // dst[row_of[t, s]] = scale * src[t]; one warp per pair, up to 2048 columns in flight. d % 8 == 0.
 // 65536 pairs x 2048: 92 -> 80 us (with the loads of one 256-column step at a time the warp waited
 // once per step).
 __global__ void __launch_bounds__(256) permute_kernel(const bf16* __restrict__ src, const int* __restrict__ row_of,
                                                       const float* __restrict__ scale, int n_pairs, int k, int d,
-                                                      long ld_src, bf16* __restrict__ dst, long dst_rows) {
+                                                      long ld_src, bf16* __restrict__ dst, long dst_rows,
+                                                      int pair_blocks, const int* __restrict__ expert_off,
+                                                      const int* __restrict__ totals) {
+  if (static_cast<int>(blockIdx.x) >= pair_blocks) {   // the blocks after the pairs' clear the padding rows
+    const int i = blockIdx.x - pair_blocks;
+    zero_pad_rows(dst, d, i / PAD_SPLIT, i % PAD_SPLIT, PAD_SPLIT, expert_off, totals);
+    return;
+  }
   const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (w >= n_pairs) return;
   const bf16* s = src + static_cast<size_t>(w / k) * ld_src;
@@ -237,7 +321,14 @@ __global__ void __launch_bounds__(256) permute_kernel(const bf16* __restrict__ s
 __global__ void __launch_bounds__(256) permute_q_kernel(const uint8_t* __restrict__ q, const float* __restrict__ scales,
                                                         const int* __restrict__ row_of, int n_pairs, int k, int K,
                                                         int T, uint8_t* __restrict__ dq,
-                                                        float* __restrict__ dscales, long dst_rows) {
+                                                        float* __restrict__ dscales, long dst_rows, int pair_blocks,
+                                                        const int* __restrict__ expert_off,
+                                                        const int* __restrict__ totals) {
+  if (static_cast<int>(blockIdx.x) >= pair_blocks) {
+    const int i = blockIdx.x - pair_blocks;
+    zero_pad_q_rows(dq, dscales, K, dst_rows, i / PAD_SPLIT, i % PAD_SPLIT, expert_off, totals);
+    return;
+  }
   const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (w >= n_pairs) return;
   const int t = w / k;
@@ -257,32 +348,6 @@ __global__ void __launch_bounds__(256) permute_q_kernel(const uint8_t* __restric
   for (int kb = lane; kb < K / 128; kb += 32)
     dscales[static_cast<size_t>(kb) * dst_rows + row] = scales[static_cast<size_t>(kb) * T + t];
 }
-
-// zero rows [expert_off[e] + totals[e], expert_off[e + 1]); gridDim.y blocks per expert
-__global__ void __launch_bounds__(256) zero_pad_kernel(bf16* __restrict__ buf, int d, const int* __restrict__ expert_off,
-                                                       const int* __restrict__ totals) {
-  const int e = blockIdx.x;
-  const int lo = expert_off[e] + totals[e], hi = expert_off[e + 1];
-  const size_t n8 = static_cast<size_t>(hi - lo) * d / 8;
-  bf16x8 z;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) z.v[j] = __floats2bfloat162_rn(0.f, 0.f);
-  bf16x8* p = reinterpret_cast<bf16x8*>(buf + static_cast<size_t>(lo) * d);
-  for (size_t i = blockIdx.y * blockDim.x + threadIdx.x; i < n8; i += static_cast<size_t>(gridDim.y) * blockDim.x) p[i] = z;
-}
-// the same rows of a quantised buffer: zero bytes, scale 1 (what the row quantiser makes of zeros)
-__global__ void __launch_bounds__(256) zero_pad_q_kernel(uint8_t* __restrict__ q, float* __restrict__ scales, int K,
-                                                         long rows, const int* __restrict__ expert_off,
-                                                         const int* __restrict__ totals) {
-  const int e = blockIdx.x;
-  const int lo = expert_off[e] + totals[e], n = expert_off[e + 1] - lo;
-  const size_t first = blockIdx.y * blockDim.x + threadIdx.x, step = static_cast<size_t>(gridDim.y) * blockDim.x;
-  uint4* p = reinterpret_cast<uint4*>(q + static_cast<size_t>(lo) * K);
-  for (size_t i = first; i < static_cast<size_t>(n) * K / 16; i += step) p[i] = make_uint4(0u, 0u, 0u, 0u);
-  for (size_t i = first; i < static_cast<size_t>(n) * (K / 128); i += step)
-    scales[(i / n) * rows + lo + i % n] = 1.f;
-}
-constexpr int PAD_SPLIT = 8;
 
 // out[t] = sum_s gate[t, s] * y[row_of[t, s]] (+ add[t]); fp32 accumulate, slots in order. One warp
 // per token and 512 columns, the rows of four slots in flight.
@@ -388,6 +453,11 @@ PB_API int pb_moe_sort(const int* ids, int n_pairs, int k, int E, int* scratch, 
                        int* expert_off, int* totals, int* k_len, int* mblk_group, int max_mblk,
                        cudaStream_t st) {
   if (n_pairs <= 0 || E <= 0 || E > moe::MAX_E || k <= 0) return PB_BAD_ARG;
+  if (n_pairs <= moe::SORT_MAX) {
+    moe::sort_small_kernel<<<1, moe::SORT_WARPS * 32, 0, st>>>(ids, n_pairs, E, row_of, expert_off, totals, k_len,
+                                                               mblk_group, max_mblk);
+    return static_cast<int>(cudaGetLastError());
+  }
   const int per = moe::TOK_PER_BLOCK * k;
   const int nblocks = (n_pairs + per - 1) / per;
   moe::count_kernel<<<nblocks, 256, 0, st>>>(ids, n_pairs, per, E, scratch);
@@ -403,11 +473,11 @@ PB_API int pb_moe_permute(const void* src, const int* row_of, const float* scale
   if (n_pairs <= 0 || d % 8 != 0) return PB_BAD_ARG;
   // rows of dst: the worst case the placement sizes its buffers for
   const long dst_rows = (static_cast<long>(n_pairs) + static_cast<long>(E > 0 ? E : 1) * 127 + 127) / 128 * 128;
-  moe::permute_kernel<<<warps_grid(n_pairs, 256), 256, 0, st>>>(
-      static_cast<const bf16*>(src), row_of, scale, n_pairs, k, d, ld_src, static_cast<bf16*>(dst),
-      dst_rows);
-  if (expert_off != nullptr)
-    moe::zero_pad_kernel<<<dim3(E, moe::PAD_SPLIT), 256, 0, st>>>(static_cast<bf16*>(dst), d, expert_off, totals);
+  const int pair_blocks = warps_grid(n_pairs, 256);
+  const int pad_blocks = expert_off != nullptr ? E * moe::PAD_SPLIT : 0;
+  moe::permute_kernel<<<pair_blocks + pad_blocks, 256, 0, st>>>(static_cast<const bf16*>(src), row_of, scale, n_pairs, k,
+                                                                d, ld_src, static_cast<bf16*>(dst), dst_rows,
+                                                                pair_blocks, expert_off, totals);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -418,10 +488,10 @@ PB_API int pb_moe_permute_q(const void* q, const float* scales, const int* row_o
                             cudaStream_t st) {
   if (T <= 0 || k <= 0 || K <= 0 || K % 128 != 0 || E <= 0) return PB_BAD_ARG;
   const int n_pairs = T * k;
-  moe::permute_q_kernel<<<warps_grid(n_pairs, 256), 256, 0, st>>>(static_cast<const uint8_t*>(q), scales, row_of, n_pairs,
-                                                                  k, K, T, static_cast<uint8_t*>(dq), dscales, rows);
-  moe::zero_pad_q_kernel<<<dim3(E, moe::PAD_SPLIT), 256, 0, st>>>(static_cast<uint8_t*>(dq), dscales, K, rows,
-                                                                  expert_off, totals);
+  const int pair_blocks = warps_grid(n_pairs, 256);
+  moe::permute_q_kernel<<<pair_blocks + E * moe::PAD_SPLIT, 256, 0, st>>>(
+      static_cast<const uint8_t*>(q), scales, row_of, n_pairs, k, K, T, static_cast<uint8_t*>(dq), dscales, rows,
+      pair_blocks, expert_off, totals);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -88,6 +88,35 @@ def test_grouped_gemms_match_per_expert_products():
     assert tot[4] == 0
 
 
+@pytest.mark.parametrize("T,k,E", [(1, 1, 1), (33, 1, 3), (512, 2, 8), (1024, 4, 64), (1366, 3, 512), (2048, 2, 5)])
+def test_placement_one_and_three_kernels(T, k, E):
+    """Rows of the pairs grouped by expert against a stable sort, on both sides of the size up to which one
+    kernel does it."""
+    from prometheus_b200.ops import moe
+
+    g = torch.Generator(device="cuda").manual_seed(T)
+    ids = torch.randint(0, E, (T, k), generator=g, device="cuda", dtype=torch.int32)
+    if E > 3:
+        ids[ids == 2] = 0                                    # an empty expert
+    pl = moe.place(ids, E)
+    flat = ids.reshape(-1).long()
+    tot = torch.bincount(flat, minlength=E)
+    off = torch.cat([torch.zeros(1, dtype=torch.long, device="cuda"), ((tot + 127) // 128 * 128).cumsum(0)])
+    order = torch.argsort(flat, stable=True)
+    start = tot.cumsum(0) - tot
+    row = torch.empty_like(flat)
+    row[order] = off[flat[order]] + torch.arange(T * k, device="cuda") - start[flat[order]]
+    assert torch.equal(pl.row_of.long(), row)
+    assert torch.equal(pl.expert_off.long(), off) and torch.equal(pl.totals.long(), tot)
+    assert torch.equal(pl.k_len.long(), off[1:] - off[:-1])
+    blocks = torch.arange(pl.rows // 128, device="cuda") * 128
+    want = torch.where(blocks < off[-1], torch.searchsorted(off[:-1].contiguous(), blocks, right=True) - 1, -1)
+    got = pl.mblk_group.long()
+    used = blocks < off[-1]
+    # empty experts share their start with the next one: any expert with rows there is the last of them
+    assert torch.equal(got[~used], want[~used]) and torch.equal(got[used], want[used])
+
+
 @pytest.mark.parametrize("T,k,E,d", [(1, 1, 1, 128), (300, 2, 5, 384), (130, 7, 16, 2176)])
 def test_token_movement_kernels(T, k, E, d):
     """Permute (plain, scaled, quantised) and combine (gated, summed, with an addend) against index
