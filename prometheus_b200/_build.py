@@ -1,6 +1,6 @@
 """In-tree build of the native libraries.
 
-Two shared objects are produced next to the package (never installed into
+Three shared objects are produced next to the package (never installed into
 site-packages, so a process that loads them shows the in-tree path):
 
 * ``prometheus_b200/_lib/libpb200_kernels.so`` — every ``csrc/kernels/*.cu`` and
@@ -8,11 +8,13 @@ site-packages, so a process that loads them shows the in-tree path):
   export a plain C ABI (raw device pointers + a stream handle) and are bound
   with ``ctypes``; nothing in them depends on the PyTorch headers, so a file
   compiles in seconds.
+* ``prometheus_b200/_lib/_pb200_call*.so`` — typed callers for those symbols' signatures,
+  generated from their declarations in ``ops/_lib.py``: what a launch from Python goes through.
 * ``prometheus_b200/_lib/_pb200_native*.so`` — the C++17 systems code under
   ``csrc/native`` (checkpoint store, data loader, controller, observability,
   harness) bound with pybind11.
 
-``python -m prometheus_b200._build`` builds both; ``build_all()`` is what
+``python -m prometheus_b200._build`` builds all; ``build_all()`` is what
 ``__graft_entry__.build()`` calls. Objects are rebuilt only when their source
 (or a shared header) is newer.
 """
@@ -168,7 +170,103 @@ def build_native(verbose: bool = False, force: bool = False, sanitize: str = "")
     return out
 
 
+CALL_CPP_HEAD = r"""// Generated from the signatures of prometheus_b200/ops/_lib.py: one typed caller per distinct signature.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+#include <cstring>
+namespace {
+bool get(PyObject* o, void*& v) {
+  if (o == Py_None) { v = nullptr; return true; }
+  if (!PyLong_Check(o)) { PyErr_SetString(PyExc_TypeError, "a device pointer is an int or None"); return false; }
+  v = reinterpret_cast<void*>(PyLong_AsUnsignedLongLongMask(o));
+  return !PyErr_Occurred();
+}
+bool get(PyObject* o, long& v) { v = static_cast<long>(PyLong_AsLongLong(o)); return !(v == -1 && PyErr_Occurred()); }
+bool get(PyObject* o, int& v) { long l; if (!get(o, l)) return false; v = static_cast<int>(l); return true; }
+bool get(PyObject* o, float& v) {
+  const double d = PyFloat_AsDouble(o);
+  v = static_cast<float>(d);
+  return !(d == -1.0 && PyErr_Occurred());
+}
+template <typename... A> struct Caller {
+  template <size_t... I>
+  static PyObject* run(PyObject* self, PyObject* const* a, std::index_sequence<I...>) {
+    std::tuple<A...> v;
+    if (!(get(a[I], std::get<I>(v)) && ...)) return nullptr;
+    const auto fn = reinterpret_cast<int (*)(A...)>(PyCapsule_GetPointer(self, nullptr));
+    int rc;
+    Py_BEGIN_ALLOW_THREADS   // as a foreign call does: a full launch queue must not hold up other threads
+    rc = fn(std::get<I>(v)...);
+    Py_END_ALLOW_THREADS
+    return PyLong_FromLong(rc);
+  }
+  static PyObject* call(PyObject* self, PyObject* const* a, Py_ssize_t n) {
+    if (n != static_cast<Py_ssize_t>(sizeof...(A))) {
+      PyErr_Format(PyExc_TypeError, "%zd arguments, %zd expected", n, static_cast<Py_ssize_t>(sizeof...(A)));
+      return nullptr;
+    }
+    return run(self, a, std::index_sequence_for<A...>{});
+  }
+};
+struct Entry { const char* sig; PyMethodDef def; };
+"""
+
+CALL_CPP_TAIL = r"""
+// bind(address, signature): a callable for the exported function at that address, or None
+PyObject* bind(PyObject*, PyObject* args) {
+  unsigned long long addr;
+  const char* sig;
+  if (!PyArg_ParseTuple(args, "Ks", &addr, &sig)) return nullptr;
+  for (Entry& e : entries)
+    if (std::strcmp(e.sig, sig) == 0) {
+      PyObject* cap = PyCapsule_New(reinterpret_cast<void*>(addr), nullptr, nullptr);
+      if (cap == nullptr) return nullptr;
+      PyObject* f = PyCFunction_New(&e.def, cap);
+      Py_DECREF(cap);
+      return f;
+    }
+  Py_RETURN_NONE;
+}
+PyMethodDef methods[] = {{"bind", bind, METH_VARARGS, nullptr}, {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_pb200_call", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+}  // namespace
+PyMODINIT_FUNC PyInit__pb200_call() { return PyModule_Create(&module); }
+"""
+
+
+def call_lib_path() -> Path:
+    return LIB_DIR / f"_pb200_call{sysconfig.get_config_var('EXT_SUFFIX') or '.so'}"
+
+
+def build_call(verbose: bool = False, force: bool = False) -> Path:
+    """The launch path's binding: typed callers for the signatures declared in ``ops/_lib.py`` (read
+    from its source, nothing is imported). Converting the 27 arguments of a matrix product through
+    ctypes took as long as launching it."""
+    import ast
+
+    src = Path(__file__).resolve().parent / "ops" / "_lib.py"
+    tree = ast.parse(src.read_text())
+    table = next(n.value for n in tree.body if isinstance(n, ast.Assign) and getattr(n.targets[0], "id", "") == "_SIGS")
+    sigs = sorted({"".join(e.id for e in v.elts) for v in table.values})
+    types = {"P": "void*", "I": "int", "L": "long", "F": "float"}
+    rows = ",\n".join(f'    {{"{s}", {{"{s or "none"}", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>('
+                      f'Caller<{", ".join(types[c] for c in s)}>::call)), METH_FASTCALL, nullptr}}}}' for s in sigs)
+    head = CALL_CPP_HEAD.replace("#include <cstring>", "#include <cstring>\n#include <tuple>\n#include <utility>")
+    text = head + "Entry entries[] = {\n" + rows + "};\n" + CALL_CPP_TAIL
+    LIB_DIR.mkdir(parents=True, exist_ok=True)
+    OBJ_DIR.mkdir(parents=True, exist_ok=True)
+    cpp, out = OBJ_DIR / "pb200_call.cpp", call_lib_path()
+    if force or not cpp.exists() or cpp.read_text() != text or _newer([cpp], out):
+        cpp.write_text(text)
+        tmp = out.with_name(out.name + ".tmp")
+        _run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-Wall",
+              "-I", sysconfig.get_paths()["include"], cpp, "-o", tmp], verbose)
+        os.replace(tmp, out)
+    return out
+
+
 def build_all(verbose: bool = False, force: bool = False) -> None:
+    build_call(verbose, force)
     build_kernels(verbose, force)
     build_kernels(verbose, force, debug_bounds=True)     # the self-checking variant rides along
     build_native(verbose, force)

@@ -1,0 +1,35 @@
+"""The typed callers behind ``ops._lib.call`` (host only: no kernel is launched)."""
+import ctypes
+
+import pytest
+
+from prometheus_b200.ops import _lib
+
+pytestmark = pytest.mark.skipif(not (_lib.available() and _lib._CALL_PATH.exists()), reason="libraries not built")
+
+
+def test_plain_symbols_get_a_typed_caller_and_host_array_ones_do_not():
+    lib = _lib.load()
+    for name in _lib._SIGS:
+        if hasattr(lib, name):
+            assert (_lib._bind(name) is not getattr(lib, name)) == (name in _lib._PLAIN), name
+    assert "pb_cp_push" not in _lib._PLAIN and "pb_gemm_bf16_ag" not in _lib._PLAIN
+    _lib._bound.clear()
+
+
+@pytest.mark.parametrize("args", [(1, 128), (300, 2048), (1 << 20, 4096), (True, 8)])
+def test_values_agree_with_the_foreign_call(args):
+    fn = _lib._bind("pb_rmsnorm_bwd_nparts")
+    assert fn(*args) == _lib.query("pb_rmsnorm_bwd_nparts", *args)
+    assert _lib._bind("pb_sumsq_nparts")(args[0] << 20) == _lib.query("pb_sumsq_nparts", args[0] << 20)
+
+
+def test_argument_checks_and_status_codes():
+    fn = _lib._bind("pb_sigmoid")
+    with pytest.raises(TypeError):
+        fn(1, 2)
+    for bad in (("x", None, 1, 0), (1.5, None, 1, 0), (None, None, "n", 0), (ctypes.c_void_p(1), None, 1, 0)):
+        with pytest.raises(TypeError):
+            fn(*bad)
+    with pytest.raises(RuntimeError, match="pb_scale_cast failed"):      # refused by the host check
+        _lib.call("pb_scale_cast", None, None, None, 0, None)
