@@ -384,7 +384,7 @@ struct Params {
   int seq_kv, q_off;                // key rows per batch entry; global position of query row 0
   float scale_log2, scale;
   const float* lse2;    // [batch, heads, seq]
-  const float* delta;   // [batch, heads, seq]  rowsum(dO * O)
+  float* delta;         // [batch, heads, seq]  rowsum(dO * O): written by the dQ kernel, read by the other
   int* status;
 };
 
@@ -402,14 +402,15 @@ struct Params {
 // shared memory), which also makes room for four stages of streamed tiles: a tile's stage is held
 // until its gradient product is done, and with fewer every tile waits for a load. The softmax
 // scale is applied to the finished dQ / dK accumulator instead of to every dS.
-// 4 x 4096 x 16/4: dQ 618 -> 386 us, dK and dV 917 -> 555 us (two stages and operand tiles; three
+// 4 x 4096 x 16/4: dQ 618 -> 406 us with delta (45 us as a kernel of its own),
+// dK and dV 917 -> 550 us (two stages and operand tiles; three
 // stages: 471 and 721 us).
 template <bool DKV>
 __global__ void __launch_bounds__(384, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant__ CUtensorMap tmRB,
                 const __grid_constant__ CUtensorMap tmT1, const __grid_constant__ CUtensorMap tmT2,
                 const __grid_constant__ CUtensorMap tmO1, const __grid_constant__ CUtensorMap tmO2,
-                const Params p) {
+                const __grid_constant__ CUtensorMap tmFO, const Params p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -421,7 +422,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
   uint64_t* x_free = bars + 12;   // [BUFS] its gradient products
   uint64_t* pd_ready = bars + 15; // [BUFS] its P^T and dS
   uint64_t* acc_done = bars + 18;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 20);
+  uint64_t* o_full = bars + 19;   // dQ: the forward's output tile, in the last stage until the row warps
+  uint64_t* o_read = bars + 20;   //     have taken delta from it
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 22);
+  constexpr int O_STAGE = STAGES - 1;
   constexpr int BUFS = Cols<DKV>::BUFS;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -449,6 +453,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
       mbar_init(&pd_ready[i], 4);                            // one arrival per row warp
     }
     mbar_init(acc_done, 1);
+    mbar_init(o_full, 1); mbar_init(o_read, 8);
     fence_barrier_init();
     tma_prefetch_desc(&tmRA); tma_prefetch_desc(&tmRB);
     tma_prefetch_desc(&tmT1); tma_prefetch_desc(&tmT2);
@@ -475,6 +480,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
         tma_load_3d(smem + RB_OFF, &tmRB, r_full, rx, row0, b);
         tma_load_3d(smem + RB_OFF + 16384, &tmRB, r_full, rx + 64, row0, b);
       }
+      if (!DKV) {
+        mbar_arrive_expect_tx(o_full, 32768);
+        tma_load_3d(smem + ST_OFF + O_STAGE * 32768, &tmFO, o_full, rx, row0, b);
+        tma_load_3d(smem + ST_OFF + O_STAGE * 32768 + 16384, &tmFO, o_full, rx + 64, row0, b);
+      }
       for (int it = 0; it < n_it; ++it) {
         const int s = it % STAGES;
         const uint32_t ph = (it / STAGES) & 1;
@@ -482,6 +492,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
         const int tx = (DKV ? g * group + it / t_count : g) * D;
         const int trow = t * 64;
         if (!mbar_wait(&t_empty[s], ph ^ 1, p.status)) break;
+        if (!DKV && it == O_STAGE && !mbar_wait(o_read, 0, p.status)) break;
         mbar_arrive_expect_tx(&t_full[s], 32768);
         uint8_t* st = smem + ST_OFF + s * 32768;
         tma_load_3d(st, &tmT1, &t_full[s], tx, trow, b);
@@ -556,10 +567,31 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
     };
     const int pos = gblk * 128 + r;   // global query position (dQ) or key position (dKV) of this row
     float row_lse = 0.f, row_delta = 0.f;
-    if (!DKV && blk * 128 + r < p.seq) {
+    bool ok = true;
+    if (!DKV) {
       const size_t vi = (static_cast<size_t>(b) * p.heads + hy) * p.seq + blk * 128 + r;
-      row_lse = p.lse2[vi];
-      row_delta = p.delta[vi];
+      const bool in = blk * 128 + r < p.seq;
+      if (in) row_lse = p.lse2[vi];
+      // delta of the row from the resident dO and the forward's output: a kernel of its own read both
+      // again (268 MB, 45 us at 4 x 4096 x 16). Both groups need it, one stores it.
+      ok = wait_all(r_full, 0, p.status) && wait_all(o_full, 0, p.status);
+      if (ok) {
+        float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+        for (int i = 0; i < 16; ++i) {
+          const int off = (i >> 3) * 16384 + r * 128 + (((i & 7) ^ (r & 7)) << 4);
+          float x[8], y[8];
+          unpack8(*reinterpret_cast<const bf16x8*>(smem + RB_OFF + off), x);
+          unpack8(*reinterpret_cast<const bf16x8*>(smem + ST_OFF + O_STAGE * 32768 + off), y);
+#pragma unroll
+          for (int k = 0; k < 8; ++k) sum[k & 3] = fmaf(x[k], y[k], sum[k & 3]);
+        }
+        row_delta = (sum[0] + sum[1]) + (sum[2] + sum[3]);
+        if (in && wg == 0) p.delta[vi] = row_delta;
+      }
+      fence_proxy_async_smem();   // the producer's next load goes over what was read here
+      __syncwarp();
+      if (lane == 0) mbar_arrive(o_read);
     }
     // dKV: per-column log-sum-exp and delta of the streamed query tile, prefetched one
     // iteration ahead by threads 0..63 (lse) and 64..127 (delta).
@@ -570,7 +602,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
       return q < p.seq ? base[(static_cast<size_t>(b) * p.heads + h) * p.seq + q] : 0.f;
     };
     float vec_next = (DKV && wg < n_it) ? vec_value(wg) : 0.f;
-    bool ok = true;
     for (int it = wg; it < n_it && ok; it += 2) {
       const int s = it % BUFS;
       const int t = t_first + (DKV ? it % t_count : it);
@@ -701,31 +732,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
     tmem_dealloc(tmem, TMEM_COLS);
   }
 }
-
-// delta[b, h, s] = sum_d dO * O  (one warp per row)
-__global__ void attn_delta_kernel(const bf16* __restrict__ o, const bf16* __restrict__ dout,
-                                  float* __restrict__ delta, int rows, int seq, int heads, int ldo,
-                                  int lddo) {
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (w >= rows * heads) return;
-  const int tok = w / heads, h = w % heads;
-  const bf16* po = o + static_cast<size_t>(tok) * ldo + h * D + lane * 4;
-  const bf16* pd = dout + static_cast<size_t>(tok) * lddo + h * D + lane * 4;
-  const uint2 a = *reinterpret_cast<const uint2*>(po), d = *reinterpret_cast<const uint2*>(pd);
-  const __nv_bfloat162* a2 = reinterpret_cast<const __nv_bfloat162*>(&a);
-  const __nv_bfloat162* d2 = reinterpret_cast<const __nv_bfloat162*>(&d);
-  float acc = 0.f;
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const float2 x = __bfloat1622float2(a2[i]), y = __bfloat1622float2(d2[i]);
-    acc += x.x * y.x + x.y * y.y;
-  }
-  acc = warp_sum(acc);
-  if (lane == 0) {
-    const int bb = tok / seq, s = tok % seq;
-    delta[(static_cast<size_t>(bb) * heads + h) * seq + s] = acc;
-  }
-}
 }  // namespace bwd
 
 // map of a token-major tensor [batch, seq, ld], 64-column boxes of box_rows rows of one batch entry
@@ -813,26 +819,19 @@ PB_API int pb_attn_bwd_cp(const void* q, const void* k, const void* v, const voi
     if (e != cudaSuccess) return static_cast<int>(e);
     attr_once.done();
   }
-  const uint64_t rows = static_cast<uint64_t>(batch) * seq;
   const uint64_t qi = static_cast<uint64_t>(heads) * D, ki = static_cast<uint64_t>(kv_heads) * D;
-  {
-    const long long warps = static_cast<long long>(rows) * heads;
-    const int blocks = static_cast<int>((warps * 32 + 255) / 256);
-    bwd::attn_delta_kernel<<<blocks, 256, 0, st>>>(
-        static_cast<const bf16*>(out), static_cast<const bf16*>(dout), static_cast<float*>(delta),
-        static_cast<int>(rows), seq, heads, ldo, ldo);
-  }
   bwd::Params p;
   p.seq = seq; p.heads = heads; p.kv_heads = kv_heads;
   p.seq_kv = seq_kv; p.q_off = q_off;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;
   p.lse2 = static_cast<const float*>(lse2);
-  p.delta = static_cast<const float*>(delta);
+  p.delta = static_cast<float*>(delta);
   p.status = status;
   int r = 0;
   {
     // dQ: resident Q, dO (128-row boxes); streamed K, V (64-row boxes)
-    CUtensorMap tQ, tDO, tK, tV, tDQ;
+    CUtensorMap tQ, tDO, tK, tV, tDQ, tO;
+    r |= tok_map(&tO, out, qi, seq, batch, ldo, 128);
     r |= tok_map(&tQ, q, qi, seq, batch, ldq, 128);
     r |= tok_map(&tDO, dout, qi, seq, batch, ldo, 128);
     r |= tok_map(&tK, k, ki, seq_kv, batch, ldkv, 64);
@@ -841,7 +840,7 @@ PB_API int pb_attn_bwd_cp(const void* q, const void* k, const void* v, const voi
     if (r != 0) return 1000 + r;
     p.n_blk = (seq + 127) / 128;
     bwd::attn_bwd_kernel<false><<<dim3(heads, batch, p.n_blk), 384, bwd::SMEM, st>>>(
-        tQ, tDO, tK, tV, tDQ, tDQ, p);
+        tQ, tDO, tK, tV, tDQ, tDQ, tO, p);
   }
   {
     // dK, dV: resident K, V (every key block of the gathered keys); streamed local Q, dO
@@ -855,7 +854,7 @@ PB_API int pb_attn_bwd_cp(const void* q, const void* k, const void* v, const voi
     if (r != 0) return 2000 + r;
     p.n_blk = (seq_kv + 127) / 128;
     bwd::attn_bwd_kernel<true><<<dim3(kv_heads, batch, p.n_blk), 384, bwd::SMEM, st>>>(
-        tK, tV, tQ, tDO, tDK, tDV, p);
+        tK, tV, tQ, tDO, tDK, tDV, tK, p);
   }
   return static_cast<int>(cudaGetLastError());
 }
