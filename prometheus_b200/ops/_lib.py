@@ -39,6 +39,9 @@ _SIGS = {
     "pb_l2norm_fwd": [P, P, L, I, F, P],
     "pb_l2norm_bwd": [P, P, P, L, I, P],
     "pb_softcap_ce": [P, P, P, P, P, L, I, F, I, P],
+    "pb_softcap_ce_sums": [P, P, P, P, P, L, I, F, I, P],
+    "pb_gemm_softcap_ok": [I, I, I],
+    "pb_gemm_softcap_logits": [P, P, P, I, I, I, L, L, L, F, P, P, P, P],
     "pb_sigmoid": [P, P, L, P],
     "pb_scale_cast": [P, P, P, L, P],
     "pb_sumsq_nparts": [L],
@@ -162,7 +165,7 @@ def ptr(t) -> int | None:
 
 
 # kernels launched by one call of each entry point (for launch accounting)
-_LAUNCHES = {"pb_rmsnorm_bwd": 2, "pb_sumsq_f32": 2, "pb_sumsq_bf16": 2, "pb_muon_prepare": 3,
+_LAUNCHES = {"pb_rmsnorm_bwd": 2, "pb_sumsq_f32": 2, "pb_sumsq_bf16": 2, "pb_muon_prepare": 3, "pb_gemm_softcap_logits": 2,
              "pb_muon_prepare_batched": 3}
 launch_count = 0
 _bound: dict = {}       # name -> callable of the loaded library's function

@@ -471,7 +471,9 @@ def l2norm_(x: Tensor, head_dim: int, eps: float = 1e-6) -> Tensor:
 class _SoftcapCeFn(torch.autograd.Function):
     """loss = sum_rows wt[row] * CE(softcap(h @ U^T), target). Rows are processed in chunks:
     logits chunk (bf16) -> fused CE kernel rewrites it as d(loss)/d(logits) -> dh and dU
-    GEMMs, so full-vocabulary fp32 logits never exist and the backward is free."""
+    GEMMs, so full-vocabulary fp32 logits never exist and the backward is free. Under a cap, and where
+    the product's kernel takes it (``pb_gemm_softcap_ok``), its epilogue adds up each row's
+    exponentials, so the CE kernel reads the logits once instead of twice."""
 
     @staticmethod
     def forward(ctx, h, U, targets, wt, cap, chunk_rows):
@@ -490,9 +492,20 @@ class _SoftcapCeFn(torch.autograd.Function):
         for r0 in range(0, rows, chunk_rows):
             r1 = min(rows, r0 + chunk_rows)
             hc = h[r0:r1]
-            logits = gemm(hc, U)
-            call("pb_softcap_ce", ptr(logits), ptr(targets[r0:r1]), ptr(wt[r0:r1]),
-                 ptr(loss_rows[r0:r1]), None, r1 - r0, V, float(cap), write_grad, stream_ptr())
+            n = r1 - r0
+            if cap > 0 and hc.dtype == U.dtype == BF16 and hc.is_contiguous() and U.is_contiguous() and \
+                    (hc.data_ptr() | U.data_ptr()) % 16 == 0 and _lib.query("pb_gemm_softcap_ok", n, V, d):
+                logits = torch.empty((n, V), dtype=BF16, device=dev)
+                sums = torch.empty(n, dtype=torch.float32, device=dev)
+                part = torch.empty(2 * ((V + 255) // 256) * n, dtype=torch.float32, device=dev)
+                call("pb_gemm_softcap_logits", ptr(hc), ptr(U), ptr(logits), n, V, d, d, d, V, float(cap), ptr(part),
+                     ptr(sums), status_word(dev).data_ptr(), stream_ptr())
+                call("pb_softcap_ce_sums", ptr(logits), ptr(targets[r0:r1]), ptr(wt[r0:r1]), ptr(loss_rows[r0:r1]),
+                     ptr(sums), n, V, float(cap), write_grad, stream_ptr())
+            else:
+                logits = gemm(hc, U)
+                call("pb_softcap_ce", ptr(logits), ptr(targets[r0:r1]), ptr(wt[r0:r1]),
+                     ptr(loss_rows[r0:r1]), None, n, V, float(cap), write_grad, stream_ptr())
             if need_h:
                 gemm(logits, U, b_mn=True, out=dh[r0:r1])
             if need_U:          # the first chunk of a fresh accumulator writes it: no fill, no read

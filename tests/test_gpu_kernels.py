@@ -325,6 +325,43 @@ def test_scale_cast(n):
     assert torch.equal(out, (x * g).to(BF16))
 
 
+@pytest.mark.parametrize("rows,d,V", [(256, 1024, 136), (200, 2048, 1000), (512, 1544, 4104)])
+@pytest.mark.parametrize("scale", [0.5, 20.0])
+def test_softcap_sums_from_the_logits_product(rows, d, V, scale):
+    """The row sums that the product's epilogue adds up against 64 bits over the stored logits (tanh of the
+    special-function unit, 2^-11 of a capped logit's slope: up to cap 2^-11 in the exponent), and loss and
+    gradients against the two-sweep kernel."""
+    from prometheus_b200.ops import functional as ops
+    from prometheus_b200.ops._lib import call, ptr, query, stream_ptr
+
+    cap = 30.0
+    h, U = _r(rows, d, seed=1), _r(V, d, seed=2, scale=scale / math.sqrt(d))
+    assert query("pb_gemm_softcap_ok", rows, V, d) == 1 and query("pb_gemm_softcap_ok", rows, V, 512) == 0
+    lg = torch.empty(rows, V, dtype=BF16, device="cuda")
+    sums = torch.empty(rows, device="cuda")
+    part = torch.full((2 * ((V + 255) // 256) * rows,), float("nan"), device="cuda")
+    call("pb_gemm_softcap_logits", ptr(h), ptr(U), ptr(lg), rows, V, d, d, d, V, cap, ptr(part), ptr(sums),
+         ptr(ops.status_word("cuda")), stream_ptr())
+    assert torch.equal(lg, ops.gemm(h, U))
+    want = torch.exp(cap * torch.tanh(lg.double() / cap) - cap).sum(1)
+    assert ((sums.double() - want).abs() <= cap * 2.0 ** -10 * want).all()
+    tgt = torch.randint(0, V, (rows,), device="cuda", dtype=torch.int32)
+    wt = (torch.arange(rows, device="cuda") % 5 != 0).float() / rows
+
+    def run(variant):
+        call("pb_gemm_set_variant", variant)       # 8: no CTA pairs, so the two-sweep kernel
+        try:
+            hg, Ug = h.clone().requires_grad_(True), U.clone().requires_grad_(True)
+            loss = ops.softcap_cross_entropy(hg, Ug, tgt, wt, cap)
+            return (loss.detach(), *torch.autograd.grad(loss, (hg, Ug)))
+        finally:
+            call("pb_gemm_set_variant", 0)
+
+    for a, b in zip(run(0), run(8)):
+        assert (a.float() - b.float()).norm() <= 5e-3 * b.float().norm()
+    ops.check_status("cuda")
+
+
 def test_softcap_ce_fresh_gradient_chunks():
     """A unembedding gradient that is not accumulated: one chunk, several, and a non-unit upstream
     gradient, against the accumulating form's buffer (fp32 sums of the same products)."""
