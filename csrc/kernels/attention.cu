@@ -403,7 +403,7 @@ struct Params {
 // until its gradient product is done, and with fewer every tile waits for a load. The softmax
 // scale is applied to the finished dQ / dK accumulator instead of to every dS.
 // 4 x 4096 x 16/4: dQ 618 -> 406 us with delta (45 us as a kernel of its own),
-// dK and dV 917 -> 550 us (two stages and operand tiles; three
+// dK and dV 917 -> 536 us (two stages and operand tiles; three
 // stages: 471 and 721 us).
 template <bool DKV>
 __global__ void __launch_bounds__(384, 1)
@@ -595,21 +595,33 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
     }
     // dKV: per-column log-sum-exp and delta of the streamed query tile, prefetched one
     // iteration ahead by threads 0..63 (lse) and 64..127 (delta).
-    auto vec_value = [&](int it) -> float {
-      const int q = (t_first + it % t_count) * 64 + (r & 63);
-      const int h = g * group + it / t_count;
-      const float* base = (r < 64) ? p.lse2 : p.delta;
-      return q < p.seq ? base[(static_cast<size_t>(b) * p.heads + h) * p.seq + q] : 0.f;
+    // (head of the group, tile) of an iteration, stepped by the two iterations between a group's tiles
+    // (a division by the tile count twice an iteration was a sixth of the instructions)
+    struct Step { int h, t; };
+    auto advance = [&](Step& s) {
+      s.t += 2;
+      while (s.t >= t_count) { s.t -= t_count; ++s.h; }
     };
-    float vec_next = (DKV && wg < n_it) ? vec_value(wg) : 0.f;
+    auto vec_value = [&](const Step& s) -> float {
+      const int q = (t_first + s.t) * 64 + (r & 63);
+      const float* base = (r < 64) ? p.lse2 : p.delta;
+      return q < p.seq ? base[(static_cast<size_t>(b) * p.heads + g * group + s.h) * p.seq + q] : 0.f;
+    };
+    Step cur = {0, wg};
+    float vec_next = 0.f;
+    if (DKV && wg < n_it) {
+      if (cur.t >= t_count) cur = {wg / t_count, wg % t_count};
+      vec_next = vec_value(cur);
+    }
     for (int it = wg; it < n_it && ok; it += 2) {
       const int s = it % BUFS;
-      const int t = t_first + (DKV ? it % t_count : it);
+      const int t = t_first + (DKV ? cur.t : it);
       float* vec = reinterpret_cast<float*>(smem + VEC_OFF + wg * 512);
       if (DKV) {
         sync_group();        // the group's readers of the previous tile are done
         vec[r] = vec_next;   // [0,64) lse2, [64,128) delta
-        if (it + 2 < n_it) vec_next = vec_value(it + 2);
+        advance(cur);   // t above is this iteration's
+        if (it + 2 < n_it) vec_next = vec_value(cur);
         sync_group();
       }
       if (!wait_all(&x_done[s], (it / BUFS) & 1, p.status)) { ok = false; break; }
