@@ -301,6 +301,10 @@ namespace bwd {
 constexpr int DW = 0, NDU = 16384, KTB = 32768, VQ = 49152, APB = 65536, TT = 73728, DM = 81920,
               TMP = 90112, BARSB = 98304;
 constexpr int SMEM_BWD = 108 * 1024;
+// Two warps cover the 64 rows (a warp reads the tensor-memory lanes of its quarter); warps 4 and 5 read the
+// same lanes and take the other half of the columns, warps 2 and 3 only keep step. The conversions between two
+// products are most of the chain, so halving them paid: 4096 chunks 162 -> 150 us.
+constexpr int THREADS_BWD = 192;
 }  // namespace bwd
 
 struct BwdParams {
@@ -320,11 +324,11 @@ __device__ __forceinline__ void ld_row32(uint32_t taddr, float* f) {
   for (int i = 0; i < 32; ++i) f[i] = __uint_as_float(v[i]);
 }
 
-// 128 accumulator columns of row `row`, times `sign`, -> two swizzled [64][64] bf16 tiles 8 KB apart;
+// Accumulator columns [c0, c0 + 64) of row `row`, times `sign`, -> two swizzled [64][64] bf16 tiles 8 KB apart;
 // with `add` the tiles' present values are added first (each cell is this thread's alone)
-__device__ __forceinline__ void row128_to_tiles(uint32_t taddr, uint8_t* tiles, int row, float sign, bool add) {
+__device__ __forceinline__ void row64_to_tile(uint32_t taddr, uint8_t* tiles, int row, int c0, float sign, bool add) {
 #pragma unroll 1
-  for (int c = 0; c < 128; c += 32) {
+  for (int c = c0; c < c0 + 64; c += 32) {
     float f[32];
     ld_row32(taddr + c, f);
 #pragma unroll
@@ -346,7 +350,7 @@ __device__ __forceinline__ void row128_to_tiles(uint32_t taddr, uint8_t* tiles, 
   }
 }
 
-__global__ void __launch_bounds__(64, 2)
+__global__ void __launch_bounds__(bwd::THREADS_BWD, 2)
 delta_prep_bwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmQ,
                       const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDW,
                       const __grid_constant__ CUtensorMap tmNDU, const __grid_constant__ CUtensorMap tmDM,
@@ -365,8 +369,13 @@ delta_prep_bwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   uint64_t* fulla = bars + 6;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
 
-  const int r = threadIdx.x, warp = r >> 5;
-  if (r == 0) {
+  __shared__ float dbeta_part[C];
+  const int warp = threadIdx.x >> 5;
+  const bool lead = threadIdx.x == 0;
+  const bool active = (warp & 3) < 2;
+  const int half = warp >> 2;                                   // which half of the columns
+  const int r = (warp & 1) * 32 + (threadIdx.x & 31);           // row of the active warps
+  if (lead) {
     mbar_init(full, 1); mbar_init(fullq, 1); mbar_init(fulla, 1);
     for (int i = 0; i < 4; ++i) mbar_init(&mma[i], 1);
     fence_barrier_init();
@@ -382,7 +391,8 @@ delta_prep_bwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t lane_addr = tmem + (static_cast<uint32_t>(warp * 32) << 16);
+  const uint32_t lane_addr = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+  const int c32 = half * 32, c64 = half * 64;
   const uint32_t id_kk64 = make_idesc(1, 1, 128, 64, 0, 0);
   const uint32_t id_mm64 = make_idesc(1, 1, 128, 64, 1, 1);
   const uint32_t id_kn = make_idesc(1, 1, 128, 128, 0, 1);
@@ -404,7 +414,7 @@ delta_prep_bwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     const int t0 = n * C;
     const int x0 = h * D;
     const int crow = g * C;
-    if (r == 0) {
+    if (lead) {
       tma_store_wait_read<0>();
       mbar_arrive_expect_tx(full, 4 * 16384 + 3 * 8192);
       tma_load_3d(smem + DW, &tmDW, full, 0, crow, 0);
@@ -419,7 +429,7 @@ delta_prep_bwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
       tma_load_3d(smem + TT, &tmT, full, 0, crow, 0);
       tma_load_3d(smem + DM, &tmDM, full, 0, crow, 0);
     }
-    const bool valid = t0 + r < p.seq_len;
+    const bool valid = active && t0 + r < p.seq_len;
     const size_t bidx = (static_cast<size_t>(b) * p.seq_len + t0 + r) * p.heads + h;
     float beta = 0.f;
     if (valid)
@@ -427,7 +437,7 @@ delta_prep_bwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
                         : bf16_to_f32(static_cast<const bf16*>(p.beta)[bidx]);
     bool ok = true;
     // ---- pass 1: dA' parts and dV ----
-    if (r == 0) {
+    if (lead) {
       ok = mbar_wait(full, ph, p.status);
       if (ok) {
         tc_fence_after();
@@ -443,44 +453,46 @@ delta_prep_bwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     ok = mbar_wait_spin(&mma[0], ph, p.status) && ok;
     if (!__syncthreads_and(ok)) break;
     tc_fence_after();
-    if (r == 0) {   // V is consumed: bring Q into its place
+    if (lead) {   // V is consumed: bring Q into its place
       mbar_arrive_expect_tx(fullq, 16384);
       tma_load_3d(smem + VQ, &tmQ, fullq, x0, t0, b);
       tma_load_3d(smem + VQ + 8192, &tmQ, fullq, x0 + 64, t0, b);
     }
-    // dV = -(A'^T (-dU)) -> staged over the -dU tile
-    row128_to_tiles(lane_addr + 128, smem + NDU, r, -1.f, false);
-    // dA' = dW K^T - (-dU) V^T -> operand tile
-#pragma unroll 1
-    for (int c = 0; c < 64; c += 32) {
-      float a[32], s[32];
-      ld_row32(lane_addr + c, a);
-      ld_row32(lane_addr + 64 + c, s);
+    if (active) {
+      // dV = -(A'^T (-dU)) -> staged over the -dU tile
+      row64_to_tile(lane_addr + 128, smem + NDU, r, c64, -1.f, false);
+      // dA' = dW K^T - (-dU) V^T -> operand tile
+      {
+        float a[32], s[32];
+        ld_row32(lane_addr + c32, a);
+        ld_row32(lane_addr + 64 + c32, s);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          float o[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) o[j] = a[8 * i + j] - s[8 * i + j];
+          st_swz(smem + TMP, r, (c32 >> 3) + i, pack8(o));
+        }
+      }
+      // tril(dM) in place (row r keeps columns <= r)
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        float o[8];
+        const int c16 = (c32 >> 3) + i;
+        bf16x8* cell = reinterpret_cast<bf16x8*>(smem + DM + r * 128 + ((c16 ^ (r & 7)) << 4));
+        if (8 * c16 + 7 > r) {
+          float f[8];
+          unpack8(*cell, f);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = a[8 * i + j] - s[8 * i + j];
-        st_swz(smem + TMP, r, (c >> 3) + i, pack8(o));
-      }
-    }
-    // tril(dM) in place (row r keeps columns <= r)
-#pragma unroll
-    for (int c16 = 0; c16 < 8; ++c16) {
-      bf16x8* cell = reinterpret_cast<bf16x8*>(smem + DM + r * 128 + ((c16 ^ (r & 7)) << 4));
-      if (8 * c16 + 7 > r) {
-        float f[8];
-        unpack8(*cell, f);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) if (8 * c16 + j > r) f[j] = 0.f;
-        *cell = pack8(f);
+          for (int j = 0; j < 8; ++j) if (8 * c16 + j > r) f[j] = 0.f;
+          *cell = pack8(f);
+        }
       }
     }
     fence_proxy_async_smem();
     tc_fence_before();
     __syncthreads();
     // ---- pass 2: X = dA' A'^T, Y = dA'^T T (diagonal = dbeta part), dK = A'^T dW ----
-    if (r == 0) {
+    if (lead) {
       tc_fence_after();
       tma_store_3d(&tmDV, smem + NDU, x0, t0, b);
       tma_store_3d(&tmDV, smem + NDU + 8192, x0 + 64, t0, b);
@@ -496,7 +508,7 @@ delta_prep_bwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     ok = mbar_wait_spin(&mma[1], ph, p.status);
     if (!__syncthreads_and(ok)) break;
     tc_fence_after();
-    if (r == 0 && (p.has_dq || p.has_dk)) {
+    if (lead && (p.has_dq || p.has_dk)) {
       // dW and dV's staging are done with: the walk's dQ and dK arrive in the tiles that dq and dk will
       // leave from, while the next two passes run
       tma_store_wait_read<0>();
@@ -511,21 +523,20 @@ delta_prep_bwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
       }
     }
     float dbeta = 0.f;
-#pragma unroll 1
-    for (int c = 0; c < 64; c += 32) {
+    if (active) {
       float x[32], y[32];
-      ld_row32(lane_addr + c, x);
-      ld_row32(lane_addr + 64 + c, y);
+      ld_row32(lane_addr + c32, x);
+      ld_row32(lane_addr + 64 + c32, y);
 #pragma unroll
-      for (int i = 0; i < 32; ++i) if (c + i == r) dbeta = y[i];
+      for (int i = 0; i < 32; ++i) if (c32 + i == r) dbeta = y[i];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) st_swz(smem + TMP, r, (c >> 3) + i, pack8(x + 8 * i));
+      for (int i = 0; i < 4; ++i) st_swz(smem + TMP, r, (c32 >> 3) + i, pack8(x + 8 * i));
     }
     fence_proxy_async_smem();
     tc_fence_before();
     __syncthreads();
     // ---- pass 3: -dA = T^T X, G = K K^T ----
-    if (r == 0) {
+    if (lead) {
       tc_fence_after();
 #pragma unroll
       for (int j = 0; j < 4; ++j) umma_f16(tmem + 0, mn(tt, j), mn(tmp, j), id_mm64, j > 0);
@@ -536,33 +547,34 @@ delta_prep_bwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     ok = mbar_wait_spin(&mma[2], ph, p.status);
     if (!__syncthreads_and(ok)) break;
     tc_fence_after();
-#pragma unroll 1
-    for (int c = 0; c < 64; c += 32) {
+    if (active) {
       float na[32], gk[32];
-      ld_row32(lane_addr + c, na);
-      ld_row32(lane_addr + 64 + c, gk);
+      ld_row32(lane_addr + c32, na);
+      ld_row32(lane_addr + 64 + c32, gk);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         float o[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          const bool low = c + 8 * i + j < r;
+          const bool low = c32 + 8 * i + j < r;
           const float da = low ? -na[8 * i + j] : 0.f;
           dbeta = fmaf(da, low ? gk[8 * i + j] : 0.f, dbeta);
           o[j] = beta * da;
         }
-        st_swz(smem + TMP, r, (c >> 3) + i, pack8(o));
+        st_swz(smem + TMP, r, (c32 >> 3) + i, pack8(o));
       }
-    }
-    if (valid) {
-      if (p.beta_f32) static_cast<float*>(p.dbeta)[bidx] = dbeta;
-      else static_cast<bf16*>(p.dbeta)[bidx] = f32_to_bf16(dbeta);
+      if (half == 1) dbeta_part[r] = dbeta;
     }
     fence_proxy_async_smem();
     tc_fence_before();
     __syncthreads();
+    if (valid && half == 0) {
+      dbeta += dbeta_part[r];
+      if (p.beta_f32) static_cast<float*>(p.dbeta)[bidx] = dbeta;
+      else static_cast<bf16*>(p.dbeta)[bidx] = f32_to_bf16(dbeta);
+    }
     // ---- pass 4: dK += dG K + dG^T K + tril(dM)^T Q ; dQ = tril(dM) K ----
-    if (r == 0) {
+    if (lead) {
       ok = mbar_wait(fullq, ph, p.status);
       if (ok) {
         tc_fence_after();
@@ -582,12 +594,14 @@ delta_prep_bwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     ok = mbar_wait_spin(&mma[3], ph, p.status) && ok;
     if (!__syncthreads_and(ok)) break;
     tc_fence_after();
-    row128_to_tiles(lane_addr + 0, smem + DW, r, 1.f, p.has_dq != 0);
-    row128_to_tiles(lane_addr + 128, smem + NDU, r, 1.f, p.has_dk != 0);
+    if (active) {
+      row64_to_tile(lane_addr + 0, smem + DW, r, c64, 1.f, p.has_dq != 0);
+      row64_to_tile(lane_addr + 128, smem + NDU, r, c64, 1.f, p.has_dk != 0);
+    }
     fence_proxy_async_smem();
     tc_fence_before();
     __syncthreads();
-    if (r == 0) {
+    if (lead) {
       tma_store_3d(&tmDQ, smem + DW, x0, t0, b);
       tma_store_3d(&tmDQ, smem + DW + 8192, x0 + 64, t0, b);
       tma_store_3d(&tmDK, smem + NDU, x0, t0, b);
@@ -595,7 +609,7 @@ delta_prep_bwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
       tma_store_commit();
     }
   }
-  if (r == 0) tma_store_wait<0>();
+  if (lead) tma_store_wait<0>();
   tc_fence_before();
   __syncthreads();
   if (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != PB_OK) {
@@ -715,7 +729,7 @@ PB_API int pb_delta_prep_bwd(const void* q, const void* k, const void* v, const 
   int grid = 2 * sms;
   if (max_ctas > 0 && max_ctas < grid) grid = max_ctas;
   if (grid > p.total) grid = p.total;
-  delta_prep_bwd_kernel<<<grid, 64, bwd::SMEM_BWD, st>>>(tK, tQ, tV, tDW, tNDU, tDM, tA, tT, tDQ,
+  delta_prep_bwd_kernel<<<grid, bwd::THREADS_BWD, bwd::SMEM_BWD, st>>>(tK, tQ, tV, tDW, tNDU, tDM, tA, tT, tDQ,
                                                            tDK, tDV, tAQ, tAK, p);
   return static_cast<int>(cudaGetLastError());
 }
