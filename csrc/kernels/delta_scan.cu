@@ -28,8 +28,16 @@
 // and products between two waits are half as long. 64 sequences: 144 -> 115 us forward, 109 -> 103 us
 // backward. With more CTAs than SMs it would be two waves of a chain that is not half as long.
 //
+// A forward summary walks every segment twice, once per map, over the same W and K. When the two CTAs a
+// segment that takes are more than the SMs, one CTA does both, as two independent chains whose conversions
+// and products fall into each other's waits: one wave and half of the operand reads. 16 sequences x 8
+// segments x 32 chunks: 104 us -> 87 us. (One chain of 256 columns: 120 us, its conversions and products
+// take turns.) With a CTA for each map on SMs of their own a chain is the shorter, so up to half of the
+// SMs it stays so. The initial state of that walk is read 16 bytes at a time: 79 us -> 73 us.
+//
 // warps 0-7: tensor-memory <-> registers <-> shared/global (lane = state row or token)
 // warp 8   : MMA issue (one lane)          warp 9: TMA producer (one lane)
+// (two chains: 0-15 rows, 16 and 17 MMA issue, 18 TMA)
 //
 // Reference semantics: kernels/__init__.py:357-376 (per-token recurrence, post-update
 // read) of the reference; the chunked algebra is this library's own.
@@ -48,12 +56,8 @@ namespace dscan {
 
 constexpr int C = 64;    // tokens per chunk
 constexpr int D = 128;   // head dim (keys and values)
-constexpr int TILE_W = 0, TILE_Q = 16384, TILE_K = 32768, TILE_M = 49152, TILE_DO = 57344;
-constexpr int STAGE_BYTES = 57344 + 16384;  // W, Q, K (16 KB each), M (8 KB), U^ or dO (16 KB)
-constexpr int XB_BYTES = 32768, UB_BYTES = 16384, OB_BYTES = 16384;
 constexpr int TMEM_COLS = 512;
-constexpr uint32_t COL_X = 0, COL_Y = 128, COL_O = 256;   // COL_O: two buffers of 128
-constexpr int THREADS = 320;
+constexpr uint32_t COL_X = 0;
 
 struct Params {
   int n_chunks;        // chunks per sequence
@@ -61,10 +65,11 @@ struct Params {
   int n_seg;           // segments per sequence: CTA (seq, seg) walks n_chunks / n_seg chunks from
                        //   x_init[seq * n_seg + seg] and leaves x_final[seq * n_seg + seg]
   int summary;         // 1: only the segment's affine map is wanted. Nothing but x_final is
-                       //   written, the output products are skipped. Forward launches two CTAs
-                       //   per segment: CTA half 0 starts from zero (x_final <- R, the state the
-                       //   segment adds), half 1 from the identity with U^ = 0 (p_final <- P, the
-                       //   linear part). Backward launches half 0 only (its linear part is P^T).
+                       //   written, the output products are skipped. Forward walks twice per
+                       //   segment, in two CTAs (NC 128) or as the two chains of one (NC 256): from
+                       //   zero (x_final <- R, the state the segment adds), and from the identity
+                       //   with U^ = 0 (p_final <- P, the linear part). Backward only the first
+                       //   (its linear part is P^T).
   float* p_final;      // [n_seq * n_seg, 128, 128], summary forward only
   int heads;           // > 0: Q, K, O and dO live in [batch, seq_len, ld] (head h at columns 128 h)
                        //      instead of the per-chunk layout; rows past seq_len in the last chunk
@@ -75,45 +80,64 @@ struct Params {
   int* status;
 };
 
-template <bool BWD>
-struct Smem {
-  static constexpr int STAGE = STAGE_BYTES;
+// NC: state columns of a CTA. 128, or 64 (then two CTAs per segment, not in summary mode), or 256: both
+// maps of a forward summary as two chains of 128 columns (0: R, 1: P), each with its own row warps, MMA
+// warp and barriers, over the same W and K tiles; no Q, M and output staging.
+template <int NC>
+struct Shape {
+  static constexpr bool BOTH = NC == 256;
+  static constexpr int CHAINS = BOTH ? 2 : 1;
+  static constexpr int CC = NC / CHAINS;                    // columns of a chain, and of each of its
+  static constexpr int WC = CC / 2;                         //   eight row warps
+  static constexpr int ROW_WARPS = 8 * CHAINS;
+  static constexpr int THREADS = (ROW_WARPS + CHAINS + 1) * 32;
+  static constexpr uint32_t COL_Y = BOTH ? 256 : 128, COL_O = 256;   // COL_O: two buffers of 128
+  // a stage: W, Q, K (16 KB each), M (8 KB), U^ or dO (16 KB). W's second half is followed by at
+  // least 8 KB of the stage: as a 128-row A operand its upper rows are read from there.
+  static constexpr int TILE_W = 0, TILE_Q = 16384, TILE_K = BOTH ? 16384 : 32768, TILE_M = 49152,
+                       TILE_DO = BOTH ? 32768 : 57344, STAGE = TILE_DO + 16384;
   static constexpr int XB = 2 * STAGE;
-  static constexpr int UB = XB + XB_BYTES;
-  static constexpr int OB = UB + UB_BYTES;
-  static constexpr int BARS = OB + OB_BYTES;
+  static constexpr int UB = XB + (BOTH ? 65536 : 32768);
+  static constexpr int OB = UB + (BOTH ? 32768 : 16384);
+  static constexpr int BARS = OB + (BOTH ? 0 : 16384);
   static constexpr int TOTAL = BARS + 256 + 1024;
+  static_assert(TOTAL <= 227 * 1024, "shared memory of a CTA");
 };
 
-// NC: state columns of a CTA, 128 or 64 (then two CTAs per segment, not in summary mode)
 template <bool BWD, int NC>
-__global__ void __launch_bounds__(THREADS, 1)
+__global__ void __launch_bounds__(Shape<NC>::THREADS, 1)
 delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmQ,
                   const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmM,
                   const __grid_constant__ CUtensorMap tmDO, const __grid_constant__ CUtensorMap tmXB,
                   const __grid_constant__ CUtensorMap tmU, const __grid_constant__ CUtensorMap tmO,
                   const Params p) {
-  using S = Smem<BWD>;
+  using S = Shape<NC>;
+  static_assert(!(BWD && S::BOTH), "both maps at once: forward summary only");
+  constexpr int TILE_W = S::TILE_W, TILE_Q = S::TILE_Q, TILE_K = S::TILE_K, TILE_M = S::TILE_M, TILE_DO = S::TILE_DO;
+  constexpr uint32_t COL_Y = S::COL_Y, COL_O = S::COL_O;
+  constexpr int MMA_WARP = S::ROW_WARPS, TMA_WARP = MMA_WARP + S::CHAINS;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  uint8_t* xb = smem + S::XB;
-  uint8_t* ub = smem + S::UB;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int chain = !S::BOTH ? 0 : (warp < MMA_WARP ? warp >> 3 : warp == MMA_WARP + 1);
+  uint8_t* xb = smem + S::XB + chain * 32768;
+  uint8_t* ub = smem + S::UB + chain * 16384;
   uint8_t* ob = smem + S::OB;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::BARS);
   uint64_t* full = bars;          // [2]
   uint64_t* empty = bars + 2;     // [2]
-  uint64_t* x_ready = bars + 4;
-  uint64_t* y_done = bars + 5;
-  uint64_t* u_ready = bars + 6;
-  uint64_t* x_done = bars + 7;    // the state update of a chunk
-  uint64_t* o_done = bars + 8;    // its output product (forward)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
+  uint64_t* chain_bars = bars + 4 + 5 * chain;
+  uint64_t* x_ready = chain_bars;
+  uint64_t* y_done = chain_bars + 1;
+  uint64_t* u_ready = chain_bars + 2;
+  uint64_t* x_done = chain_bars + 3;    // the state update of a chunk
+  uint64_t* o_done = chain_bars + 4;    // its output product (forward)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4 + 5 * S::CHAINS);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_units = p.n_seq * p.n_seg;
-  constexpr int HALVES = NC / 64;       // 64-column operand chunks
-  constexpr int WC = NC / 2;            // columns of a row warp
+  constexpr int HALVES = NC == 64 ? 1 : 2;   // 64-column chunks of U^, dO and the outputs
+  constexpr int WC = S::WC;                  // columns of a row warp
   const int half = static_cast<int>(blockIdx.x) / n_units;      // 1: the identity-start CTA, or the upper columns
   const int unit = static_cast<int>(blockIdx.x) % n_units;      // seq * n_seg + seg
   const int col0 = NC == 64 ? half * 64 : 0;                    // this CTA's first state column
@@ -121,8 +145,9 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
   const int N = p.n_chunks / p.n_seg;                           // chunks this CTA walks
   const int n0 = (unit % p.n_seg) * N;                          // its first chunk
   const int NT = p.n_chunks;
-  const bool sum = p.summary != 0;
-  const bool lin = NC == 128 && sum && half == 1;                            // linear part only: U^ = 0
+  const bool sum = S::BOTH || p.summary != 0;
+  // linear part (U^ = 0): the second chain, or the identity-start CTA
+  const bool lin = S::BOTH ? chain == 1 : NC == 128 && sum && half == 1;
   const bool store_ux = !sum && p.store_ux != 0;
   const bool tokmaj = p.heads > 0;
   // token tensors: batch entry, first row and first column of this sequence
@@ -132,29 +157,33 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
 
   if (threadIdx.x == 0) {
     mbar_init(&full[0], 1); mbar_init(&full[1], 1);
-    mbar_init(&empty[0], 1); mbar_init(&empty[1], 1);
-    mbar_init(x_ready, 8); mbar_init(u_ready, 4);   // one arrival per warp that takes part
-    mbar_init(y_done, 1); mbar_init(x_done, 1); mbar_init(o_done, 1);
+    mbar_init(&empty[0], S::CHAINS); mbar_init(&empty[1], S::CHAINS);
+#pragma unroll
+    for (int c = 0; c < S::CHAINS; ++c) {
+      uint64_t* b = bars + 4 + 5 * c;
+      mbar_init(b, 8); mbar_init(b + 2, 4);   // x_ready, u_ready: one arrival per warp that takes part
+      mbar_init(b + 1, 1); mbar_init(b + 3, 1); mbar_init(b + 4, 1);
+    }
     fence_barrier_init();
     tma_prefetch_desc(&tmW); tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK);
     tma_prefetch_desc(&tmM);
     tma_prefetch_desc(&tmDO);
   }
-  if (warp == 8) {
+  if (warp == MMA_WARP) {
     tmem_alloc(tmem_slot, TMEM_COLS);
     tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = *tmem_slot + chain * 128;
 
-  if (warp == 9) {
+  if (warp == TMA_WARP) {
     // ------------------------------- TMA producer -------------------------------
     if (lane == 0) {
       // a forward summary needs neither Q nor M (no output product), its linear half no U^
       const bool need_qm = BWD || !sum;
-      const bool need_fifth = BWD || !lin;
+      const bool need_fifth = BWD || S::BOTH || !lin;
       const uint32_t stage_tx = 32768u + (need_qm ? 24576u : 0u) + (need_fifth ? HALVES * 8192u : 0u);
       for (int it = 0; it < N; ++it) {
         const int n = n0 + (BWD ? (N - 1 - it) : it);
@@ -185,11 +214,11 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
         }
       }
     }
-  } else if (warp == 8) {
+  } else if (warp >= MMA_WARP) {
     // -------------------------------- MMA issuer --------------------------------
     if (lane == 0) {
-      const uint32_t id_kn = make_idesc(1, 1, 128, NC, 0, 1);  // A K-major, B MN-major
-      const uint32_t id_nn = make_idesc(1, 1, 128, NC, 1, 1);  // A MN-major, B MN-major
+      const uint32_t id_kn = make_idesc(1, 1, 128, S::CC, 0, 1);  // A K-major, B MN-major
+      const uint32_t id_nn = make_idesc(1, 1, 128, S::CC, 1, 1);  // A MN-major, B MN-major
       const uint32_t xb_a = smem_u32(xb), ub_a = smem_u32(ub);
       for (int it = 0; it < N; ++it) {
         const int s = it & 1;
@@ -263,7 +292,8 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     // the bf16 state image is stored from the very tile the MMAs read, U / -dU from the
     // operand tile, O from a staging tile. Thread 0 issues and tracks the stores.
     const int r = (warp & 3) * 32 + lane;  // tensor-memory lane = state row (or token row < 64)
-    const int ch = warp >> 2, c0 = ch * WC;   // this warp's half of the CTA's columns
+    const int ch = (warp >> 2) & 1, c0 = ch * WC;   // this warp's half of the chain's columns
+    const int g0 = col0 + c0;                 // its first column in the state or map
     const bool tok_warp = (warp & 3) < 2;     // warps whose lanes are token rows
     const uint32_t lane_addr = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + c0;
     auto sync_rows = [] { asm volatile("bar.sync 1, 256;" ::: "memory"); };
@@ -288,21 +318,38 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     auto put_cols = [&](uint8_t* tile, int rows, const uint32_t (&v)[WC]) {
 #pragma unroll
       for (int i = 0; i < WC / 8; ++i) {
-        bf16x8 pk;
+        uint32_t pk[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          pk.v[j] = __floats2bfloat162_rn(__uint_as_float(v[8 * i + 2 * j]), __uint_as_float(v[8 * i + 2 * j + 1]));
-        *reinterpret_cast<bf16x8*>(piece(tile, rows, i)) = pk;
+        for (int j = 0; j < 4; ++j) {
+          const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(v[8 * i + 2 * j]), __uint_as_float(v[8 * i + 2 * j + 1]));
+          pk[j] = *reinterpret_cast<const uint32_t*>(&h);
+        }
+        // one 16-byte store: as four of 4 bytes, which the compiler may make of a struct, each is a
+        // four-way bank conflict
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(smem_u32(piece(tile, rows, i))), "r"(pk[0]),
+                     "r"(pk[1]), "r"(pk[2]), "r"(pk[3]) : "memory");
       }
     };
     {
-      const float* x0 = (p.x_init && !sum) ? p.x_init + (static_cast<size_t>(unit) * D + r) * D + col0 + c0 : nullptr;
+      const float* x0 = (p.x_init && !sum) ? p.x_init + (static_cast<size_t>(unit) * D + r) * D + g0 : nullptr;
+      const bool wide = (reinterpret_cast<uintptr_t>(x0) & 15) == 0;   // a caller's state may lie at any float
 #pragma unroll 1
       for (int c = 0; c < WC; c += 32) {
         uint32_t v[32];
+        if (wide) {
 #pragma unroll
-        for (int i = 0; i < 32; ++i)
-          v[i] = x0 ? __float_as_uint(x0[c + i]) : ((lin && c0 + c + i == r) ? __float_as_uint(1.f) : 0u);
+          for (int i = 0; i < 32; i += 4) {
+            const uint4 w = x0 ? *reinterpret_cast<const uint4*>(x0 + c + i) : make_uint4(0u, 0u, 0u, 0u);
+            v[i] = w.x; v[i + 1] = w.y; v[i + 2] = w.z; v[i + 3] = w.w;
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(x0[c + i]);
+        }
+        if (lin) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] = g0 + c + i == r ? __float_as_uint(1.f) : 0u;
+        }
         tmem_st_32x32b_x32(lane_addr + COL_X + c, v);
       }
       tmem_st_wait();
@@ -354,9 +401,9 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
           tma_store_commit();
         }
       }
-      if (!mbar_wait_spin(y_done, cph, p.status)) { ok = false; break; }
-      tc_fence_after();
       if (tok_warp) {
+        if (!mbar_wait_spin(y_done, cph, p.status)) { ok = false; break; }
+        tc_fence_after();
         uint32_t v[WC];
         load_cols(COL_Y, v);
         uint8_t* uh = smem + (it & 1) * S::STAGE + TILE_DO;
@@ -410,7 +457,7 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
       }
       float* fin = lin ? p.p_final : p.x_final;
       if (fin != nullptr) {
-        float* xf = fin + (static_cast<size_t>(unit) * D + r) * D + col0 + c0;
+        float* xf = fin + (static_cast<size_t>(unit) * D + r) * D + g0;
         uint32_t v[WC];
         load_cols(COL_X, v);
 #pragma unroll
@@ -429,7 +476,7 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     for (int i = 0; i < 2000; ++i) __nanosleep(1000);  // let copies in flight land
     __syncthreads();
   }
-  if (warp == 8) {
+  if (warp == MMA_WARP) {
     tc_fence_after();
     tmem_dealloc(tmem, TMEM_COLS);
   }
@@ -443,11 +490,11 @@ int launch_cols(const CUtensorMap& tW, const CUtensorMap& tQ, const CUtensorMap&
   if (attr_once.need()) {
     cudaError_t e = cudaFuncSetAttribute(delta_scan_kernel<BWD, NC>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         Smem<BWD>::TOTAL);
+                                         Shape<NC>::TOTAL);
     if (e != cudaSuccess) return static_cast<int>(e);
     attr_once.done();
   }
-  delta_scan_kernel<BWD, NC><<<ctas, THREADS, Smem<BWD>::TOTAL, st>>>(tW, tQ, tK, tM, tD, tXB, tU, tO, p);
+  delta_scan_kernel<BWD, NC><<<ctas, Shape<NC>::THREADS, Shape<NC>::TOTAL, st>>>(tW, tQ, tK, tM, tD, tXB, tU, tO, p);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -481,6 +528,11 @@ int launch(const void* W, const void* Q, const void* K, const void* M, const voi
   const int units = p.n_seq * p.n_seg;
   if (!p.summary && 2 * units <= num_sms())
     return launch_cols<BWD, 64>(tW, tQ, tK, tM, tD, tXB, tU, tO, p, 2 * units, st);
+  if constexpr (!BWD) {
+    // both maps in one CTA where a CTA for each would be a second wave
+    if (p.summary && 2 * units > num_sms())
+      return launch_cols<false, 256>(tW, tQ, tK, tM, tD, tXB, tU, tO, p, units, st);
+  }
   return launch_cols<BWD, 128>(tW, tQ, tK, tM, tD, tXB, tU, tO, p, units * ((p.summary && !BWD) ? 2 : 1), st);
 }
 
@@ -541,8 +593,8 @@ PB_API int pb_delta_scan_fwd_seg(const void* W, const void* Uhat, const void* Q,
 }
 
 // Affine map of every segment, S_out = P S_in + R, without outputs: r_out, p_out fp32
-// [n_seq * n_seg, 128, 128]. Two CTAs per segment (one per map), three products per chunk
-// instead of six, no stores but the two maps.
+// [n_seq * n_seg, 128, 128]. Three products per chunk and map instead of six, no stores but the
+// two maps.
 PB_API int pb_delta_scan_summary_fwd(const void* W, const void* Uhat, const void* K, void* r_out,
                                      void* p_out, int n_seq, int n_chunks, int n_seg, int heads,
                                      int seq_len, int ld, int* status, cudaStream_t st) {

@@ -165,7 +165,7 @@ def _from_chunks(x: Tensor, b: int, h: int, n: int) -> Tensor:
 def scan_segments(n_seq: int, n_chunks: int, ctas: int = 148) -> int:
     """Segments per sequence for the state walk, chosen by a cost model in units of one chunk
     step of one CTA wave. The single-pass walk costs ``waves(n_seq) * n_chunks``. With ``seg``
-    segments the summary launch has two CTAs per segment and does about 0.6 of a chunk step
+    segments the summary launch does two maps per segment, each about 0.6 of a chunk step
     per chunk (three of the six products, no stores), the segmented walk one step per chunk,
     and the two extra launches plus the fold about 24 steps of start-up (tensor-memory
     allocation, first loads, state load / store: measured at about ten chunk steps per launch):
@@ -173,7 +173,10 @@ def scan_segments(n_seq: int, n_chunks: int, ctas: int = 148) -> int:
         waves(2 n_seq seg) * 0.6 n_chunks / seg  +  waves(n_seq seg) * n_chunks / seg  +  24
 
     The smallest power of two (at least four chunks per segment) that beats the single pass
-    by a fifth is taken; 1 means the plain single-pass walk."""
+    by a fifth is taken; 1 means the plain single-pass walk. Measured, forward us at 1 / 4 / 8 / 16
+    segments (the rule's choice in parentheses): 16 sequences x 256 chunks 492 / 359 / 316 / 404
+    (8), 16 x 128 252 / 201 / 193 / 241 (8), 16 x 64 134 / 123 / 127 / 176 (4), 8 x 256 431 / 300 /
+    216 / 223 (16), 32 x 128 314 / 319 / 419 / 471 (4), 32 x 64 163 / 194 / 241 / 334 (1)."""
     def waves(c):
         return -(-c // ctas)
 
@@ -206,7 +209,7 @@ class _DeltaFusedFn(torch.autograd.Function):
     The walk is affine in the state, ``S_out = P S_in + R`` per run of chunks. When the batch
     has too few sequences to fill the GPU (``scan_segments`` > 1), or when the sequence is
     split over the ranks of a context-parallel group (``cp``), each segment's ``(P, R)`` comes
-    from a summary walk without outputs (two CTAs per segment), a small sequential kernel folds
+    from a summary walk without outputs, a small sequential kernel folds
     them into the state entering every segment -- with the cross-rank hand-off in the middle
     under ``cp`` -- and one segmented walk produces the outputs: two passes of 1 / n_seg the
     length instead of one full-length pass. The backward does the same with ``P^T``."""

@@ -594,6 +594,63 @@ def test_delta_chunk_products(B, S, H):
     _close(d_m, doc @ u.float().transpose(1, 2), 1e-2)
 
 
+@pytest.mark.parametrize("n_seq,n_chunks,n_seg,cut", [(37, 6, 2, 0), (75, 3, 1, 0), (75, 1, 1, 0), (40, 8, 4, 0), (80, 4, 2, 27)])
+def test_delta_summary_maps(n_seq, n_chunks, n_seg, cut):
+    """The affine map of every segment against 64 bits, on both sides of the line where one CTA computes
+    both maps (more than 74 segments on 148 SMs), and with a last chunk of 64 - ``cut`` tokens in place
+    (16 heads). The images of the state and of U are bf16: each chunk adds at most 2^-9 of the state
+    twice, and 2^-9 sqrt(2) of at most four chunks stays under 2e-2."""
+    from prometheus_b200.ops import functional as ops
+    from prometheus_b200.ops._lib import call, ptr, stream_ptr
+
+    heads, s = (16, n_chunks * 64 - cut) if cut else (0, n_chunks * 64)
+    rows = n_seq * n_chunks * 64
+    w, uh = (_r(rows, 128, seed=i, scale=128 ** -0.5) for i in (1, 2))
+    if heads:
+        k = _r(n_seq // heads, s, heads * 128, seed=3, scale=128 ** -0.5)
+        kc = torch.nn.functional.pad(k, (0, 0, 0, cut)).reshape(n_seq // heads, n_chunks * 64, heads, 128).transpose(1, 2)
+    else:
+        k = kc = _r(rows, 128, seed=3, scale=128 ** -0.5)
+    r, p = (torch.full((n_seq * n_seg, 128, 128), float("nan"), device="cuda") for _ in range(2))
+    call("pb_delta_scan_summary_fwd", ptr(w), ptr(uh), ptr(k), ptr(r), ptr(p), n_seq, n_chunks, n_seg, heads, s,
+         heads * 128, ptr(ops.status_word(torch.device("cuda"))), stream_ptr())
+    torch.cuda.synchronize()
+    ops.check_status("cuda")
+    per = n_chunks // n_seg
+    wd, ud, kd = (t.reshape(n_seq * n_seg, per, 64, 128).double() for t in (w, uh, kc))
+    rd = torch.zeros_like(r, dtype=torch.float64)
+    pd = torch.eye(128, device="cuda").double().expand_as(rd)
+    for c in range(per):
+        kt = kd[:, c].transpose(1, 2)
+        rd = rd + kt @ (ud[:, c] - wd[:, c] @ rd)
+        pd = pd - kt @ (wd[:, c] @ pd)
+    for got, ref in ((r, rd), (p, pd)):
+        err = (got.double() - ref).flatten(1).norm(dim=1) / ref.flatten(1).norm(dim=1)
+        assert err.max() <= 2e-2, err.max()
+
+
+@pytest.mark.parametrize("H", [4, 80])          # 64- and 128-column walks
+def test_delta_initial_state_at_any_float(H):
+    """An initial state and a final-state gradient whose storage starts 4 bytes off a 16-byte boundary
+    give what aligned ones give, bit for bit (the wide reads are not taken)."""
+    from prometheus_b200.ops.delta import delta_rule_fused
+
+    q, k, v = (_r(1, 128, H, 128, seed=i, scale=0.08) for i in (1, 2, 3))
+    beta = torch.sigmoid(_r(1, 128, H, seed=4, dtype=torch.float32))
+    flat = _r(2 * H * 128 * 128 + 1, seed=5, scale=0.05, dtype=torch.float32)
+    n = H * 128 * 128
+
+    def run(s0, gs):
+        leaf = s0.requires_grad_(True)
+        out, st = delta_rule_fused(q, k, v, beta, leaf, n_seg=1)
+        return out, st, torch.autograd.grad([out, st], leaf, [v, gs])[0]
+
+    off = [flat[1 + i * n:1 + (i + 1) * n].view(1, H, 128, 128).detach() for i in (0, 1)]
+    assert all(x.data_ptr() % 16 == 4 for x in off)
+    for a, b in zip(run(*off), run(*(x.clone() for x in off))):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("n_seq,n_seg", [(1, 1), (3, 8)])
 @pytest.mark.parametrize("reverse", [0, 1])
 def test_delta_compose(n_seq, n_seg, reverse):
