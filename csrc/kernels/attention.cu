@@ -76,7 +76,28 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<const uint32_t*>(&v);
 }
-__device__ __forceinline__ void sync_rows() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+// Two fp32 operations in one instruction, each rounded as the scalar one.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 pa, pb, pc;\n\tmov.b64 pa, {%2, %3};\n\tmov.b64 pb, {%4, %5};\n\tmov.b64 pc, {%6, %7};\n\t"
+      "fma.rn.f32x2 pa, pa, pb, pc;\n\tmov.b64 {%0, %1}, pa;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 pa, pb;\n\tmov.b64 pa, {%2, %3};\n\tmov.b64 pb, {%4, %5};\n\t"
+      "add.rn.f32x2 pa, pa, pb;\n\tmov.b64 {%0, %1}, pa;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 pa, pb;\n\tmov.b64 pa, {%2, %3};\n\tmov.b64 pb, {%4, %5};\n\t"
+      "mul.rn.f32x2 pa, pa, pb;\n\tmov.b64 {%0, %1}, pa;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
 // Warp-uniform bounded wait: the row warps run warp-collective tensor-memory loads, so either
 // every lane goes on or none does.
 __device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, int* status) {
@@ -400,11 +421,12 @@ struct Params {
 // P^T and dS go back to tensor memory as bf16 over the scores they were made from and are the
 // gradient products' A operand there (64 KB less per tile than operand tiles written to and read from
 // shared memory), which also makes room for four stages of streamed tiles: a tile's stage is held
-// until its gradient product is done, and with fewer every tile waits for a load. The softmax
-// scale is applied to the finished dQ / dK accumulator instead of to every dS.
-// 4 x 4096 x 16/4: dQ 618 -> 406 us with delta (45 us as a kernel of its own),
-// dK and dV 917 -> 536 us (two stages and operand tiles; three
-// stages: 471 and 721 us).
+// until its gradient product is done, and with fewer every tile waits for a load. dS is rounded to
+// bf16 once, with the softmax scale in it: P (dP - delta) scale costs two multiplications an element, so
+// the rows' arithmetic is packed two elements to an instruction (as scalar operations the backward
+// of 4 x 4096 x 16/4 takes 35 us longer).
+// 4 x 4096 x 16/4: dQ 396 us with delta (618 with two stages and operand tiles, and 45 more for delta as a
+// kernel of its own; 471 with three stages), dK and dV 535 us (917; 721).
 template <bool DKV>
 __global__ void __launch_bounds__(384, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant__ CUtensorMap tmRB,
@@ -576,24 +598,30 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
       // again (268 MB, 45 us at 4 x 4096 x 16). Both groups need it, one stores it.
       ok = wait_all(r_full, 0, p.status) && wait_all(o_full, 0, p.status);
       if (ok) {
-        float sum[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4
-        for (int i = 0; i < 16; ++i) {
+        // Columns are added as a warp with four of them to a lane adds its lanes up (halves, quarters, ..):
+        // dS, and with it the gradients' bf16 roundings, depend on the sum's last bit.
+        auto lanes = [&](const int i) -> float2 {   // 16-byte piece i: two lanes' partial sums
           const int off = (i >> 3) * 16384 + r * 128 + (((i & 7) ^ (r & 7)) << 4);
           float x[8], y[8];
           unpack8(*reinterpret_cast<const bf16x8*>(smem + RB_OFF + off), x);
           unpack8(*reinterpret_cast<const bf16x8*>(smem + ST_OFF + O_STAGE * 32768 + off), y);
+          float t[4];   // products of bf16 values are exact
 #pragma unroll
-          for (int k = 0; k < 8; ++k) sum[k & 3] = fmaf(x[k], y[k], sum[k & 3]);
-        }
-        row_delta = (sum[0] + sum[1]) + (sum[2] + sum[3]);
+          for (int e = 0; e < 4; ++e) t[e] = fmaf(x[2 * e], y[2 * e], x[2 * e + 1] * y[2 * e + 1]);
+          return add2(make_float2(t[0], t[2]), make_float2(t[1], t[3]));
+        };
+        auto half_sum = [&](const int i) { return add2(lanes(i), lanes(i + 8)); };
+        auto quarter_sum = [&](const int i) { return add2(half_sum(i), half_sum(i + 4)); };
+        const float2 even = add2(quarter_sum(0), quarter_sum(2)), odd = add2(quarter_sum(1), quarter_sum(3));
+        const float2 sum = add2(even, odd);
+        row_delta = __fadd_rn(sum.x, sum.y);
         if (in && wg == 0) p.delta[vi] = row_delta;
       }
       fence_proxy_async_smem();   // the producer's next load goes over what was read here
       __syncwarp();
       if (lane == 0) mbar_arrive(o_read);
     }
-    // dKV: per-column log-sum-exp and delta of the streamed query tile, prefetched one
+    // dKV: per-column log-sum-exp and delta of the streamed query tile (negated), prefetched one
     // iteration ahead by threads 0..63 (lse) and 64..127 (delta).
     // (head of the group, tile) of an iteration, stepped by the two iterations between a group's tiles
     // (a division by the tile count twice an iteration was a sixth of the instructions)
@@ -605,7 +633,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
     auto vec_value = [&](const Step& s) -> float {
       const int q = (t_first + s.t) * 64 + (r & 63);
       const float* base = (r < 64) ? p.lse2 : p.delta;
-      return q < p.seq ? base[(static_cast<size_t>(b) * p.heads + g * group + s.h) * p.seq + q] : 0.f;
+      return q < p.seq ? -base[(static_cast<size_t>(b) * p.heads + g * group + s.h) * p.seq + q] : 0.f;
     };
     Step cur = {0, wg};
     float vec_next = 0.f;
@@ -613,13 +641,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
       if (cur.t >= t_count) cur = {wg / t_count, wg % t_count};
       vec_next = vec_value(cur);
     }
+    const float2 log2_scale = make_float2(p.scale_log2, p.scale_log2), lin_scale = make_float2(p.scale, p.scale);
     for (int it = wg; it < n_it && ok; it += 2) {
       const int s = it % BUFS;
       const int t = t_first + (DKV ? cur.t : it);
       float* vec = reinterpret_cast<float*>(smem + VEC_OFF + wg * 512);
       if (DKV) {
         sync_group();        // the group's readers of the previous tile are done
-        vec[r] = vec_next;   // [0,64) lse2, [64,128) delta
+        vec[r] = vec_next;   // [0,64) -lse2, [64,128) -delta
         advance(cur);   // t above is this iteration's
         if (it + 2 < n_it) vec_next = vec_value(cur);
         sync_group();
@@ -635,35 +664,41 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
       auto half = [&](auto EDGE, const int c, const uint32_t (&x1)[32], const uint32_t (&x2)[32]) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          float pf[8], df[8], lv[8], dv[8];
+          float2 pf[4], df[4], nl[4], nd[4];
           if (DKV) {
-            const float4* l4 = reinterpret_cast<const float4*>(vec + c + 8 * i);
-            const float4* d4 = reinterpret_cast<const float4*>(vec + 64 + c + 8 * i);
-            const float4 a = l4[0], b4 = l4[1], e = d4[0], f = d4[1];
-            lv[0] = a.x; lv[1] = a.y; lv[2] = a.z; lv[3] = a.w;
-            lv[4] = b4.x; lv[5] = b4.y; lv[6] = b4.z; lv[7] = b4.w;
-            dv[0] = e.x; dv[1] = e.y; dv[2] = e.z; dv[3] = e.w;
-            dv[4] = f.x; dv[5] = f.y; dv[6] = f.z; dv[7] = f.w;
+#pragma unroll
+            for (int k = 0; k < 4; k += 2) {
+              const float4 l4 = *reinterpret_cast<const float4*>(vec + c + 8 * i + 2 * k);
+              const float4 d4 = *reinterpret_cast<const float4*>(vec + 64 + c + 8 * i + 2 * k);
+              nl[k] = make_float2(l4.x, l4.y); nl[k + 1] = make_float2(l4.z, l4.w);
+              nd[k] = make_float2(d4.x, d4.y); nd[k + 1] = make_float2(d4.z, d4.w);
+            }
+          } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              nl[k] = make_float2(-row_lse, -row_lse);
+              nd[k] = make_float2(-row_delta, -row_delta);
+            }
           }
 #pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            const int col = c + 8 * i + k;
-            const float lse = DKV ? lv[k] : row_lse;
-            const float dl = DKV ? dv[k] : row_delta;
-            float pr = ex2(fmaf(__uint_as_float(x1[8 * i + k]), p.scale_log2, -lse));
+          for (int k = 0; k < 4; ++k) {
+            const int at = 8 * i + 2 * k;
+            const float2 e = fma2(make_float2(__uint_as_float(x1[at]), __uint_as_float(x1[at + 1])), log2_scale, nl[k]);
+            float2 pr = make_float2(ex2(e.x), ex2(e.y));
             if (decltype(EDGE)::value) {
-              const int other = tg * 64 + col;
-              const bool masked = DKV ? (other < pos) : (other > pos);
-              if (masked) pr = 0.f;
+              const int other = tg * 64 + c + at;
+              if (DKV ? (other < pos) : (other > pos)) pr.x = 0.f;
+              if (DKV ? (other + 1 < pos) : (other + 1 > pos)) pr.y = 0.f;
             }
             pf[k] = pr;
-            df[k] = pr * (__uint_as_float(x2[8 * i + k]) - dl);   // the scale waits for the epilogue
+            const float2 dp = make_float2(__uint_as_float(x2[at]), __uint_as_float(x2[at + 1]));
+            df[k] = mul2(pr, mul2(add2(dp, nd[k]), lin_scale));   // the scale before the one rounding to bf16
           }
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
             const int at = (c >> 1) + 4 * i + k;
-            pk_d[at] = pack_bf16x2(df[2 * k], df[2 * k + 1]);
-            if (DKV) pk_p[at] = pack_bf16x2(pf[2 * k], pf[2 * k + 1]);
+            pk_d[at] = pack_bf16x2(df[k].x, df[k].y);
+            if (DKV) pk_p[at] = pack_bf16x2(pf[k].x, pf[k].y);
           }
         }
       };
@@ -699,7 +734,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
       // dKV: group 0 drains dK, group 1 drains dV.  dQ: each group drains 64 columns.
       uint8_t* stage = smem + ((DKV && wg == 1) ? RB_OFF : RA_OFF);
       const uint32_t col0 = (DKV && wg == 1) ? Cols<DKV>::ACC2 : Cols<DKV>::ACC1;
-      const float out_scale = DKV && wg == 1 ? 1.f : p.scale;
       const int c_lo = DKV ? 0 : wg * 64, c_hi = DKV ? D : wg * 64 + 64;
 #pragma unroll 1
       for (int c = c_lo; c < c_hi; c += 32) {
@@ -711,7 +745,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
           float f[8];
 #pragma unroll
           // a key block with no local query at or after it gets an all-zero gradient
-          for (int k = 0; k < 8; ++k) f[k] = n_it > 0 ? __uint_as_float(v[8 * i + k]) * out_scale : 0.f;
+          for (int k = 0; k < 8; ++k) f[k] = n_it > 0 ? __uint_as_float(v[8 * i + k]) : 0.f;
           const int col = c + 8 * i;
           st_swz(stage + (col >> 6) * 16384, r, (col & 63) >> 3, pack_bf16x8(f));
         }
