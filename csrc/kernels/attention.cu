@@ -98,10 +98,8 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
       : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
   return d;
 }
-// Warp-uniform bounded wait: the row warps run warp-collective tensor-memory loads, so either
-// every lane goes on or none does.
 __device__ __forceinline__ bool wait_all(uint64_t* bar, uint32_t parity, int* status) {
-  return __all_sync(0xffffffffu, mbar_wait_spin(bar, parity, status));
+  return mbar_wait_spin_warp(bar, parity, status);
 }
 
 // Registers of a tensor-memory load are valid after the wait: no use of them may move above this.
@@ -254,10 +252,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const int qpos = gb * 256 + t * 128 + r;     // global position (for the causal mask)
     const int q0 = gb * 256 + t * 128;
     const int nj = nj1 - (t == 0 ? 2 : 0);
-    auto sync_group = [&] {
-      if (t == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
-      else asm volatile("bar.sync 2, 128;" ::: "memory");
-    };
     float m_used = -INFINITY, m_true = -INFINITY, l = 0.f;
     bool ok = true;
     for (int j = 0; j < nj && ok; ++j) {
@@ -336,9 +330,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       if (r == 0) atomicAdd(&g_attn_prof[6], 1ull);
 #endif
     }
-    if (ok && wait_all(&o_done[t * 2 + ((nj - 1) & 1)], ((nj - 1) >> 1) & 1, p.status)) {
+    ok = ok && wait_all(&o_done[t * 2 + ((nj - 1) & 1)], ((nj - 1) >> 1) & 1, p.status);
+    uint8_t* obuf = smem + P_OFF + t * 32768;   // both P buffers of the tile, now idle
+    if (ok) {
       tc_fence_after();
-      uint8_t* obuf = smem + P_OFF + t * 32768;   // both P buffers of the tile, now idle
       const float inv = 1.f / l;
 #pragma unroll 1
       for (int c = 0; c < D; c += 32) {
@@ -361,13 +356,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         if (p.rowmax != nullptr) p.rowmax[vi] = m_true * 0.6931471805599453f;
       }
       fence_proxy_async_smem();
-      sync_group();
-      if (r == 0 && row0 + t * 128 < p.seq) {
-        tma_store_3d(&tmO, obuf, h * D, row0 + t * 128, b);
-        tma_store_3d(&tmO, obuf + 16384, h * D + 64, row0 + t * 128, b);
-        tma_store_commit();
-        tma_store_wait<0>();
-      }
+    }
+    // a warp whose wait ran out arrives too: the group stores its tile or leaves together
+    if (bar_sync_and(1 + t, 128, ok) && r == 0 && row0 + t * 128 < p.seq) {
+      tma_store_3d(&tmO, obuf, h * D, row0 + t * 128, b);
+      tma_store_3d(&tmO, obuf + 16384, h * D + 64, row0 + t * 128, b);
+      tma_store_commit();
+      tma_store_wait<0>();
     }
   }
 
@@ -642,18 +637,20 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
       vec_next = vec_value(cur);
     }
     const float2 log2_scale = make_float2(p.scale_log2, p.scale_log2), lin_scale = make_float2(p.scale, p.scale);
-    for (int it = wg; it < n_it && ok; it += 2) {
+    for (int it = wg; it < n_it && (DKV || ok); it += 2) {
       const int s = it % BUFS;
       const int t = t_first + (DKV ? cur.t : it);
       float* vec = reinterpret_cast<float*>(smem + VEC_OFF + wg * 512);
       if (DKV) {
-        sync_group();        // the group's readers of the previous tile are done
+        // the group's readers of the previous tile are done; who ran out of a wait takes the group along
+        ok = bar_sync_and(1 + wg, 128, ok);
+        if (!ok) break;
         vec[r] = vec_next;   // [0,64) -lse2, [64,128) -delta
         advance(cur);   // t above is this iteration's
         if (it + 2 < n_it) vec_next = vec_value(cur);
         sync_group();
       }
-      if (!wait_all(&x_done[s], (it / BUFS) & 1, p.status)) { ok = false; break; }
+      if (!wait_all(&x_done[s], (it / BUFS) & 1, p.status)) { ok = false; continue; }
       tc_fence_after();
       // mask: dQ rows are queries, columns keys (key > query is masked);
       //       dKV rows are keys, columns queries (query < key is masked)
@@ -727,12 +724,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
       __syncwarp();
       if (lane == 0) mbar_arrive(&pd_ready[s]);
     }
-    // every row thread gets here (no early exit above), so the group barriers below are safe
-    if (wait_all(acc_done, 0, p.status) && ok) {
+    // every row thread gets here (no early exit above), so the group barrier below is safe
+    ok = wait_all(acc_done, 0, p.status) && ok;
+    // resident tiles are no longer read: reuse them as the staging for the TMA stores.
+    // dKV: group 0 drains dK, group 1 drains dV.  dQ: each group drains 64 columns.
+    uint8_t* stage = smem + ((DKV && wg == 1) ? RB_OFF : RA_OFF);
+    if (ok) {
       tc_fence_after();
-      // resident tiles are no longer read: reuse them as the staging for the TMA stores.
-      // dKV: group 0 drains dK, group 1 drains dV.  dQ: each group drains 64 columns.
-      uint8_t* stage = smem + ((DKV && wg == 1) ? RB_OFF : RA_OFF);
       const uint32_t col0 = (DKV && wg == 1) ? Cols<DKV>::ACC2 : Cols<DKV>::ACC1;
       const int c_lo = DKV ? 0 : wg * 64, c_hi = DKV ? D : wg * 64 + 64;
 #pragma unroll 1
@@ -751,19 +749,18 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
         }
       }
       fence_proxy_async_smem();
-      sync_group();
-      if (r == 0) {
-        const int ox = (DKV ? g : hy) * D;
-        if (DKV) {
-          const CUtensorMap* tm = wg == 0 ? &tmO1 : &tmO2;
-          tma_store_3d(tm, stage, ox, row0, b);
-          tma_store_3d(tm, stage + 16384, ox + 64, row0, b);
-        } else {
-          tma_store_3d(&tmO1, stage + wg * 16384, ox + wg * 64, row0, b);
-        }
-        tma_store_commit();
-        tma_store_wait<0>();
+    }
+    if (bar_sync_and(1 + wg, 128, ok) && r == 0) {
+      const int ox = (DKV ? g : hy) * D;
+      if (DKV) {
+        const CUtensorMap* tm = wg == 0 ? &tmO1 : &tmO2;
+        tma_store_3d(tm, stage, ox, row0, b);
+        tma_store_3d(tm, stage + 16384, ox + 64, row0, b);
+      } else {
+        tma_store_3d(&tmO1, stage + wg * 16384, ox + wg * 64, row0, b);
       }
+      tma_store_commit();
+      tma_store_wait<0>();
     }
   }
 

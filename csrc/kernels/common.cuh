@@ -255,6 +255,29 @@ __device__ __forceinline__ bool mbar_wait_spin(uint64_t* bar, uint32_t parity, i
   return false;
 }
 
+// The two waits for a warp whose next instructions are collective (tensor-memory loads, barriers): every lane
+// goes on or none does. Lanes that gave up one by one would leave the others at a collective they never reach.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int* status) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, status));
+}
+__device__ __forceinline__ bool mbar_wait_spin_warp(uint64_t* bar, uint32_t parity, int* status) {
+  return __all_sync(0xffffffffu, mbar_wait_spin(bar, parity, status));
+}
+// bar.sync of named barrier `id` that also tells every thread whether `ok` holds in all of them: warps that share
+// a named barrier leave a loop together or not at all.
+__device__ __forceinline__ bool bar_sync_and(int id, int threads, bool ok) {
+  uint32_t all;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "bar.red.and.pred q, %2, %3, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(all)
+      : "r"(static_cast<uint32_t>(ok)), "r"(id), "r"(threads)
+      : "memory");
+  return all != 0;
+}
+
 // ---------------------------------------------------------------------------
 // TMA (tiled bulk tensor copies), no cluster multicast anywhere
 // ---------------------------------------------------------------------------

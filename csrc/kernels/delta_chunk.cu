@@ -132,11 +132,11 @@ delta_chunk_kernel(const __grid_constant__ CUtensorMap tmNDU, const __grid_const
     uint32_t it = 0;
     for (int g = blockIdx.x; g < p.total; g += gridDim.x, ++it) {
       const int s = it & 1;
-      if (!mbar_wait(acc_full, it & 1, p.status)) break;
+      const bool ok = mbar_wait_warp(acc_full, it & 1, p.status);
       tc_fence_after();
       uint8_t* out = smem + s * STAGE + stage_off;
 #pragma unroll 1
-      for (int c = 0; c < cols; c += 64) {
+      for (int c = 0; ok && c < cols; c += 64) {
         uint32_t v[64];
         tmem_ld_32x32b_x32(taddr + c, v);
         tmem_ld_32x32b_x32(taddr + c + 32, v + 32);
@@ -152,9 +152,9 @@ delta_chunk_kernel(const __grid_constant__ CUtensorMap tmNDU, const __grid_const
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(acc_free);
+      if (ok && lane == 0) mbar_arrive(acc_free);
       fence_proxy_async_smem();
-      asm volatile("bar.sync %0, 64;" ::"r"(1 + res) : "memory");   // both halves of the rows are staged
+      if (!bar_sync_and(1 + res, 64, ok)) break;   // both halves of the rows are staged
       if ((warp & 1) == 0 && lane == 0) {
         tma_store_3d(tm, out, 0, g * C, 0);
         if (cols == 128) tma_store_3d(tm, out + 8192, 64, g * C, 0);

@@ -296,8 +296,10 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     const int g0 = col0 + c0;                 // its first column in the state or map
     const bool tok_warp = (warp & 3) < 2;     // warps whose lanes are token rows
     const uint32_t lane_addr = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + c0;
-    auto sync_rows = [] { asm volatile("bar.sync 1, 256;" ::: "memory"); };
-    auto sync_tok = [] { asm volatile("bar.sync 2, 128;" ::: "memory"); };
+    // barriers of the row warps and of the token warps: true when nobody's wait ran out (a summary walk has
+    // neither, there every warp decides for itself)
+    auto sync_rows = [](bool ok) { return bar_sync_and(1, 256, ok); };
+    auto sync_tok = [](bool ok) { return bar_sync_and(2, 128, ok); };
     auto arrive = [&](uint64_t* bar) {   // the warp's shared-memory writes and tensor-memory reads are done
       fence_proxy_async_smem();
       tc_fence_before();
@@ -355,19 +357,20 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
       tmem_st_wait();
     }
     bool ok = true;
-    for (int it = 0; it < N && ok; ++it) {
+    for (int it = 0; it < N; ++it) {
       const int n = n0 + (BWD ? (N - 1 - it) : it);
       const uint32_t cph = it & 1;
       const int g = seq * NT + n;
       if (it > 0) {
-        if (!mbar_wait_spin(x_done, cph ^ 1, p.status)) { ok = false; break; }
+        ok = ok && mbar_wait_spin_warp(x_done, cph ^ 1, p.status);
         tc_fence_after();
       }
       // all earlier bulk stores have finished reading xb / ub / ob before they are rewritten
       if (!sum) {
         if (r == 0 && ch == 0) tma_store_wait_read<0>();
-        sync_rows();
+        ok = sync_rows(ok);
       }
+      if (!ok) break;
       // bf16 image of the state entering this chunk
       {
         uint32_t v[WC];
@@ -377,9 +380,9 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
       arrive(x_ready);
       if (!BWD && !sum && it > 0) {
         // rows of the previous chunk's output: tensor memory -> staging tile, while Y is computed
-        if (!mbar_wait_spin(o_done, cph ^ 1, p.status)) { ok = false; break; }
+        ok = mbar_wait_spin_warp(o_done, cph ^ 1, p.status);
         tc_fence_after();
-        if (tok_warp) {
+        if (ok && tok_warp) {
           uint32_t v[WC];
           load_cols(COL_O + (cph ^ 1) * 128, v);
           put_cols(ob, C, v);
@@ -387,7 +390,8 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
         }
       }
       if (!sum) {
-        sync_rows();
+        ok = sync_rows(ok);
+        if (!ok) break;
         if (r == 0 && ch == 0) {
           if (!BWD && it > 0) {
             const int prow = tok0 + (n - 1) * C;
@@ -401,8 +405,7 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
           tma_store_commit();
         }
       }
-      if (tok_warp) {
-        if (!mbar_wait_spin(y_done, cph, p.status)) { ok = false; break; }
+      if (tok_warp && (ok = mbar_wait_spin_warp(y_done, cph, p.status))) {
         tc_fence_after();
         uint32_t v[WC];
         load_cols(COL_Y, v);
@@ -424,30 +427,33 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
           *reinterpret_cast<bf16x8*>(piece(ub, C, i)) = pack8(y);
         }
         arrive(u_ready);
-        if (store_ux) {
-          sync_tok();
-          if (r == 0 && ch == 0) {
+      }
+      if (tok_warp && store_ux) {
+        ok = sync_tok(ok);   // the other row warps hear of it at the next sync_rows
+        if (ok && r == 0 && ch == 0) {
 #pragma unroll
-            for (int hf = 0; hf < HALVES; ++hf) tma_store_3d(&tmU, ub + hf * 8192, col0 + hf * 64, g * C, 0);
-            tma_store_commit();
-          }
+          for (int hf = 0; hf < HALVES; ++hf) tma_store_3d(&tmU, ub + hf * 8192, col0 + hf * 64, g * C, 0);
+          tma_store_commit();
         }
       }
     }
     // drain: last chunk's output rows and the final state
-    if (ok && N > 0 && mbar_wait_spin(x_done, (N - 1) & 1, p.status) &&
-        (BWD || sum || mbar_wait_spin(o_done, (N - 1) & 1, p.status))) {
+    ok = ok && N > 0 && mbar_wait_spin_warp(x_done, (N - 1) & 1, p.status) &&
+         (BWD || sum || mbar_wait_spin_warp(o_done, (N - 1) & 1, p.status));
+    if (!BWD && !sum) {
+      if (r == 0 && ch == 0) tma_store_wait_read<0>();
+      ok = sync_rows(ok);
+    }
+    if (ok) {
       tc_fence_after();
       if (!BWD && !sum) {
-        if (r == 0 && ch == 0) tma_store_wait_read<0>();
-        sync_rows();
         if (tok_warp) {
           uint32_t v[WC];
           load_cols(COL_O + ((N - 1) & 1) * 128, v);
           put_cols(ob, C, v);
           fence_proxy_async_smem();
         }
-        sync_rows();
+        sync_rows(true);
         if (r == 0 && ch == 0) {
           const int prow = tok0 + (n0 + N - 1) * C;
 #pragma unroll

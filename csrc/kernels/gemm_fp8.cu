@@ -227,7 +227,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       }
       for (int kb = 0; kb < (PROBE == 2 ? 1 : nkb); ++kb, ++it) {
         const int a = it & 1;
-        if (!mbar_wait(&tfull[a], (it >> 1) & 1, p.status)) { ok = false; break; }
+        if (!mbar_wait_warp(&tfull[a], (it >> 1) & 1, p.status)) { ok = false; break; }
         tc_fence_after();
         if (!have) scale_cur = __ldcg(sa_row + static_cast<size_t>(kb) * p.M) * sb[kb];
         const float scale = scale_cur;

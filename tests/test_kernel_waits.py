@@ -1,0 +1,62 @@
+"""How the kernels leave a bounded wait that ran out, read from their sources (no GPU).
+
+A wait is per thread. Where the next instructions are collective (tensor-memory loads, barriers), lanes that
+gave up one by one would leave the others at an instruction that never completes: a timeout that has to be
+reported would become a kernel that never returns. So a wait either belongs to a single thread, or it is one of
+the warp-uniform forms, or its result goes through ``__syncthreads_and`` before anybody acts on it; and a named
+barrier that follows a wait carries the result (``bar_sync_and``)."""
+import re
+from pathlib import Path
+
+import pytest
+
+SRC = Path(__file__).resolve().parent.parent / "csrc" / "kernels"
+FILES = ("attention.cu", "delta_chunk.cu", "delta_prep.cu", "delta_scan.cu", "gemm.cu", "gemm_fp8.cu")
+ONE_THREAD = re.compile(r"\blane == 0|\blead\b|\br == 0|threadIdx\.x == 0")
+
+
+def _text(name):
+    text = re.sub(r"//[^\n]*", lambda m: " " * len(m.group()), (SRC / name).read_text())
+    return re.sub(r"/\*.*?\*/", lambda m: " " * len(m.group()), text, flags=re.S)
+
+
+def per_thread_waits(text):
+    """(line, statement) of every per-lane wait that a whole warp may run and act on lane by lane."""
+    bad, heads, start = [], [], 0
+    call = re.compile(r"\bmbar_wait(_spin|_cluster)?\(")
+    for i, c in enumerate(text):
+        if c in "{};":
+            stmt = text[start:i]
+            if call.search(stmt) and not any(ONE_THREAD.search(h) for h in heads + [stmt]):
+                rest = text[i:i + 400]
+                stop = re.search(r"\bbreak\b|\breturn\b", rest)
+                agreed = rest.find("__syncthreads_and")
+                inline = c == "{" or "break" in stmt or "return" in stmt      # acted on in the same statement
+                if inline or agreed < 0 or (stop and stop.start() < agreed - 6):
+                    bad.append((text.count("\n", 0, i) + 1, " ".join(stmt.split())))
+            if c == "{":
+                heads.append(stmt)
+            elif c == "}" and heads:
+                heads.pop()
+            start = i + 1
+    return bad
+
+
+@pytest.mark.parametrize("name", FILES)
+def test_waits_before_collective_instructions_are_uniform(name):
+    assert per_thread_waits(_text(name)) == []
+
+
+def test_row_warps_that_share_a_named_barrier_leave_together():
+    scan, chunk, att = _text("delta_scan.cu"), _text("delta_chunk.cu"), _text("attention.cu")
+    assert "bar.sync" not in scan and "bar.sync" not in chunk
+    # attention: the only plain barriers left stand behind an agreed one, with no wait in between
+    for m in re.finditer(r"\bsync_group\(\);", att):
+        before = att[:m.start()]
+        assert before.rfind("bar_sync_and") > before.rfind("wait_all("), att.count("\n", 0, m.start()) + 1
+
+
+def test_the_reader_of_sources_sees_a_wait_that_splits_a_warp():
+    text = _text("gemm.cu")
+    assert "mbar_wait_warp(&tfull" in text
+    assert per_thread_waits(text.replace("mbar_wait_warp(&tfull", "mbar_wait(&tfull"))
