@@ -115,6 +115,44 @@ def test_gemm_2d_forms_equal_the_batched_form():
         assert got and torch.equal(got[0], want)
 
 
+@pytest.mark.parametrize("M,N", [(200, 328), (520, 264)])
+@pytest.mark.parametrize("c_f32", [False, True])
+@pytest.mark.parametrize("d_f32", [False, True])
+def test_gemm_c_and_d_at_any_base(M, N, c_f32, d_f32):
+    """A destination or D that starts at an odd element, or whose batch entries do, is written and read element
+    by element: the bits of the aligned call, and nothing next to the destination."""
+    from prometheus_b200.ops import functional as ops
+    from prometheus_b200.ops._lib import call
+
+    dts = {False: BF16, True: torch.float32}
+
+    def shifted(t, by=1):      # the same values, contiguous, `by` elements past a 16-byte boundary
+        buf = torch.full((t.numel() + 16,), 7.0, dtype=t.dtype, device="cuda")
+        return buf, buf[by:by + t.numel()].view(t.shape).copy_(t)
+
+    a, b = _r(2, M, 192, seed=1), _r(2, N, 192, seed=2)
+    d = _r(2, M, N, seed=3, dtype=dts[d_f32])
+    try:
+        for variant in (0, 8):         # CTA pairs where they apply, the single-CTA kernel
+            call("pb_gemm_set_variant", variant)
+            kw = dict(out_dtype=dts[c_f32], alpha=0.5, beta=-2.0)
+            want = ops.gemm(a, b, d=d, **kw)
+            for off_c, off_d in ((0, 1), (1, 0), (1, 1)):
+                buf, out = shifted(torch.zeros_like(want), off_c)
+                got = ops.gemm(a, b, out=out, d=shifted(d, off_d)[1], **kw)
+                assert torch.equal(got, want), (variant, off_c, off_d)
+                assert (buf[:off_c] == 7).all() and (buf[off_c + want.numel():] == 7).all()
+                buf, out = shifted(torch.zeros_like(want[0]), off_c)
+                got = ops.gemm(a[0], b[0], out=out, d=shifted(d[0], off_d)[1], **kw)
+                assert torch.equal(got, want[0]), (variant, off_c, off_d)
+            # aligned base, batch entries an odd number of elements apart
+            gap = torch.empty(2 * M * N + 1, dtype=d.dtype, device="cuda").as_strided((2, M, N), (M * N + 1, N, 1)).copy_(d)
+            assert torch.equal(ops.gemm(a, b, d=gap, **kw), want)
+    finally:
+        call("pb_gemm_set_variant", 0)
+    ops.check_status("cuda")
+
+
 def test_gemm_limited_grid_and_many_tiles():
     from prometheus_b200.ops import functional as ops
 
