@@ -26,6 +26,7 @@
 // causal mask) of the reference; the tiling is this library's own.
 #include <cuda.h>
 
+#include <climits>
 #include <type_traits>
 
 #include "common.cuh"
@@ -119,7 +120,7 @@ constexpr int SMEM = BARS + 512 + 1024;
 constexpr uint32_t COL_S = 0, COL_O = 256, TMEM_COLS = 512;   // S[tile][buf] 64 cols, O[tile] 128
 
 struct Params {
-  int seq, heads, kv_heads;   // seq: query rows per batch entry
+  int batch, seq, heads, kv_heads;   // seq: query rows per batch entry
   int seq_kv, q_off;          // key rows per batch entry; global position of query row 0
   float scale_log2;   // softmax scale * log2(e)
   float* lse2;        // [batch, heads, seq], log2 domain
@@ -150,9 +151,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // blocks start in index order, so the row block is the slowest index: the longest rows of all heads and
-  // batch entries first, the shortest fill the gaps at the end
-  const int cb = static_cast<int>(gridDim.z) - 1 - static_cast<int>(blockIdx.z);
-  const int h = blockIdx.x, b = blockIdx.y;
+  // batch entries first, the shortest fill the gaps at the end. One grid dimension for all three: the others end
+  // at 65535 blocks
+  const int per = p.heads * p.batch;
+  const int at = static_cast<int>(blockIdx.x % per);
+  const int cb = static_cast<int>(gridDim.x / per) - 1 - static_cast<int>(blockIdx.x / per);
+  const int b = at / p.heads, h = at - b * p.heads;
   const int g = h / (p.heads / p.kv_heads);
   const int gb = cb + p.q_off / 256;   // position of this CTA's rows among all keys
   const int row0 = cb * 256;           // first query row within the batch entry
@@ -396,7 +400,7 @@ template <bool DKV> struct Cols {
 constexpr uint32_t COL_X2 = 64, TMEM_COLS = 512;
 
 struct Params {
-  int seq, heads, kv_heads, n_blk;  // seq: query rows per batch entry; n_blk: 128-row blocks of the grid
+  int batch, seq, heads, kv_heads, n_blk;  // seq: query rows per batch entry; n_blk: 128-row blocks of the grid
   int seq_kv, q_off;                // key rows per batch entry; global position of query row 0
   float scale_log2, scale;
   const float* lse2;    // [batch, heads, seq]
@@ -447,11 +451,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int group = p.heads / p.kv_heads;
-  const int b = blockIdx.y;
   // dQ: heavy blocks are the late query blocks; dKV: the early key blocks. Heavy blocks of all heads and
-  // batch entries come first, as in the forward.
-  const int blk = DKV ? static_cast<int>(blockIdx.z) : p.n_blk - 1 - static_cast<int>(blockIdx.z);
-  const int hy = blockIdx.x;                       // query head (dQ) or KV head (dKV)
+  // batch entries come first, in one grid dimension, as in the forward.
+  const int rows_y = DKV ? p.kv_heads : p.heads, per = rows_y * p.batch;
+  const int blk0 = static_cast<int>(blockIdx.x / per), at = static_cast<int>(blockIdx.x % per);
+  const int blk = DKV ? blk0 : p.n_blk - 1 - blk0;
+  const int b = at / rows_y;
+  const int hy = at - b * rows_y;                  // query head (dQ) or KV head (dKV)
   const int g = DKV ? hy : hy / group;
   // dQ: blk is a local query block, streamed tiles are global key tiles 0 .. diagonal.
   // dKV: blk is a global key block, streamed tiles are the local query tiles at or after it.
@@ -782,6 +788,13 @@ static int tok_map(CUtensorMap* tm, const void* base, uint64_t inner, int seq, i
   return make_tmap_3d(tm, base, 2, inner, seq, batch, ld, static_cast<uint64_t>(seq) * ld, 64, box_rows);
 }
 
+// CTAs of a grid of row blocks x heads x batch entries; more than a grid dimension holds is refused (-1)
+static long grid_ctas(int rows, int block, int heads, int batch) {
+  const long per = static_cast<long>(heads) * batch;
+  const long blocks = (static_cast<long>(rows) + block - 1) / block;
+  return per > INT_MAX || blocks > INT_MAX / per ? -1 : blocks * per;
+}
+
 static bool bad_geometry(int batch, int seq, int heads, int kv_heads, int ldq, int ldkv) {
   return batch <= 0 || seq <= 0 || heads <= 0 || kv_heads <= 0 ||
          heads % kv_heads != 0 || ldq < heads * D || ldkv < kv_heads * D || ldq % 8 != 0 ||
@@ -808,6 +821,8 @@ PB_API int pb_attn_fwd_cp(const void* q, const void* k, const void* v, void* out
   if (bad_geometry(batch, seq, heads, kv_heads, ldq, ldkv) || ldo < heads * D || ldo % 8 != 0 ||
       !(scale > 0.f) || q_off < 0 || q_off % 256 != 0 || seq_kv < q_off + seq)
     return PB_BAD_ARG;
+  const long grid = grid_ctas(seq, 256, heads, batch);
+  if (grid < 0) return PB_BAD_ARG;
   static pb::DeviceOnce attr_once;   // per device: the attribute belongs to the current GPU
   if (attr_once.need()) {
     cudaError_t e = cudaFuncSetAttribute(fwd::attn_fwd_kernel,
@@ -823,13 +838,13 @@ PB_API int pb_attn_fwd_cp(const void* q, const void* k, const void* v, void* out
   r |= tok_map(&tO, out, static_cast<uint64_t>(heads) * D, seq, batch, ldo, 128);
   if (r != 0) return 1000 + r;
   fwd::Params p;
-  p.seq = seq; p.heads = heads; p.kv_heads = kv_heads;
+  p.batch = batch; p.seq = seq; p.heads = heads; p.kv_heads = kv_heads;
   p.seq_kv = seq_kv; p.q_off = q_off;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.lse2 = static_cast<float*>(lse2);
   p.rowmax = static_cast<float*>(rowmax);
   p.status = status;
-  fwd::attn_fwd_kernel<<<dim3(heads, batch, (seq + 255) / 256), 352, fwd::SMEM, st>>>(tQ, tK, tV, tO, p);
+  fwd::attn_fwd_kernel<<<static_cast<unsigned>(grid), 352, fwd::SMEM, st>>>(tQ, tK, tV, tO, p);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -852,6 +867,8 @@ PB_API int pb_attn_bwd_cp(const void* q, const void* k, const void* v, const voi
   if (bad_geometry(batch, seq, heads, kv_heads, ldq, ldkv) || ldo < heads * D || ldo % 8 != 0 ||
       !(scale > 0.f) || q_off < 0 || q_off % 128 != 0 || seq_kv < q_off + seq)
     return PB_BAD_ARG;
+  const long grid_q = grid_ctas(seq, 128, heads, batch), grid_kv = grid_ctas(seq_kv, 128, kv_heads, batch);
+  if (grid_q < 0 || grid_kv < 0) return PB_BAD_ARG;
   static pb::DeviceOnce attr_once;   // per device: the attribute belongs to the current GPU
   if (attr_once.need()) {
     cudaError_t e = cudaFuncSetAttribute(bwd::attn_bwd_kernel<false>,
@@ -864,7 +881,7 @@ PB_API int pb_attn_bwd_cp(const void* q, const void* k, const void* v, const voi
   }
   const uint64_t qi = static_cast<uint64_t>(heads) * D, ki = static_cast<uint64_t>(kv_heads) * D;
   bwd::Params p;
-  p.seq = seq; p.heads = heads; p.kv_heads = kv_heads;
+  p.batch = batch; p.seq = seq; p.heads = heads; p.kv_heads = kv_heads;
   p.seq_kv = seq_kv; p.q_off = q_off;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;
   p.lse2 = static_cast<const float*>(lse2);
@@ -882,7 +899,7 @@ PB_API int pb_attn_bwd_cp(const void* q, const void* k, const void* v, const voi
     r |= tok_map(&tDQ, dq, qi, seq, batch, ldq, 128);
     if (r != 0) return 1000 + r;
     p.n_blk = (seq + 127) / 128;
-    bwd::attn_bwd_kernel<false><<<dim3(heads, batch, p.n_blk), 384, bwd::SMEM, st>>>(
+    bwd::attn_bwd_kernel<false><<<static_cast<unsigned>(grid_q), 384, bwd::SMEM, st>>>(
         tQ, tDO, tK, tV, tDQ, tDQ, tO, p);
   }
   {
@@ -896,7 +913,7 @@ PB_API int pb_attn_bwd_cp(const void* q, const void* k, const void* v, const voi
     r |= tok_map(&tDV, dv, ki, seq_kv, batch, ldkv, 128);
     if (r != 0) return 2000 + r;
     p.n_blk = (seq_kv + 127) / 128;
-    bwd::attn_bwd_kernel<true><<<dim3(kv_heads, batch, p.n_blk), 384, bwd::SMEM, st>>>(
+    bwd::attn_bwd_kernel<true><<<static_cast<unsigned>(grid_kv), 384, bwd::SMEM, st>>>(
         tK, tV, tQ, tDO, tDK, tDV, tK, p);
   }
   return static_cast<int>(cudaGetLastError());

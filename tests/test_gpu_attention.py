@@ -172,3 +172,26 @@ def test_ds_is_rounded_once_with_the_scale_in_it():
                             ("dk1", dk[:, 1] / q[:, 1], ds[1])):
         assert torch.equal(got, got[..., :1].expand_as(got)), name
         assert (got[..., 0] != want.to(BF16)).float().mean() < 0.02, name
+
+
+def test_more_row_blocks_than_a_second_grid_dimension_holds():
+    """Gradients of 65537 key blocks (the y and z dimensions of a grid end at 65535): a short query slice against
+    8.4 M keys of which it sees the first 256."""
+    from prometheus_b200.ops import attention
+    from prometheus_b200.ops import functional as ops
+
+    s_kv = 65537 * 128
+    q, ks, vs = _rand(1, 256, 1, 1, 31)
+    k, v = (torch.zeros(1, s_kv, 1, 128, dtype=BF16, device="cuda") for _ in range(2))
+    k[:, :256], v[:, :256] = ks, vs
+    leaves = [t.requires_grad_() for t in (q, k, v)]
+    out = attention.causal_gqa_offset(*leaves, 0)
+    go = torch.randn_like(out)
+    dq, dk, dv = torch.autograd.grad(out, leaves, go)
+    ops.check_status("cuda")
+    small = [t.detach().clone().requires_grad_() for t in (q, ks, vs)]
+    want_out = attention.causal_gqa(*small)
+    want = torch.autograd.grad(want_out, small, go)
+    assert torch.equal(out, want_out) and torch.equal(dq, want[0])
+    assert torch.equal(dk[:, :256], want[1]) and torch.equal(dv[:, :256], want[2])
+    assert not dk[:, 256:].any() and not dv[:, 256:].any()
