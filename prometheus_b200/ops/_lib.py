@@ -193,7 +193,11 @@ def _bind(name: str):
 
 def call(name: str, *args) -> None:
     global launch_count
-    rc = (_bound.get(name) or _bind(name))(*args)
+    try:
+        rc = (_bound.get(name) or _bind(name))(*args)
+    except TypeError:
+        # an argument that the typed caller does not convert (a ctypes object, say): the foreign call decides
+        rc = getattr(load(), name)(*args)
     launch_count += _LAUNCHES.get(name, 1)
     if rc != 0:
         raise RuntimeError(f"{name} failed with code {rc}")

@@ -33,3 +33,19 @@ def test_argument_checks_and_status_codes():
             fn(*bad)
     with pytest.raises(RuntimeError, match="pb_scale_cast failed"):      # refused by the host check
         _lib.call("pb_scale_cast", None, None, None, 0, None)
+
+
+def test_call_takes_and_refuses_what_the_foreign_call_does():
+    """A symbol with host checks only on this path (n = 0 is refused before a pointer is looked at)."""
+    numpy = pytest.importorskip("numpy")
+    n0 = "pb_scale_cast failed with code"
+    for args in ((ctypes.c_void_p(16), None, None, 0, None), (None, ctypes.byref(ctypes.c_int(3)), None, 0, None),
+                 (None, None, None, ctypes.c_long(0), None), (None, None, None, 1 << 64, None), (16, 16, 16, False, 0),
+                 (None, None, None, numpy.int64(0), None)):
+        with pytest.raises(RuntimeError, match=n0):
+            _lib.call("pb_scale_cast", *args)
+    for args in ((1.5, None, None, 0, None), (None, None, None, "0", None), (None, None, None, 0.0, None)):
+        with pytest.raises((TypeError, ctypes.ArgumentError)):
+            _lib.call("pb_scale_cast", *args)
+        with pytest.raises((TypeError, ctypes.ArgumentError)):
+            getattr(_lib.load(), "pb_scale_cast")(*args)
