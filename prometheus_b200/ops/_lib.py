@@ -10,6 +10,7 @@ from __future__ import annotations
 import ctypes
 import importlib.util
 import sysconfig
+import warnings
 from ctypes import c_float, c_int, c_long, c_void_p
 from pathlib import Path
 
@@ -25,6 +26,7 @@ _lib = None
 # typed callers generated from the signatures below (prometheus_b200._build.build_call)
 _CALL_PATH = _LIB_PATH.parent / ("_pb200_call" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
 _binder = None
+_warned = False          # of a missing or stale one, once a process
 
 P, I, L, F = c_void_p, c_int, c_long, c_float
 
@@ -178,15 +180,23 @@ _PLAIN = frozenset(n for n in _SIGS if not n.startswith("pb_cp_") and n != "pb_g
 def _bind(name: str):
     """The typed caller of the launch binding for a plain symbol (pb_gemm_bf16: 8.2 -> 3.9 us a launch),
     the ctypes function for every other one."""
+    global _binder, _warned
     fn = getattr(load(), name)
-    if name in _PLAIN and _CALL_PATH.exists():
-        global _binder
-        if _binder is None:
+    if name in _PLAIN:
+        typed = None
+        if _binder is None and _CALL_PATH.exists():
             spec = importlib.util.spec_from_file_location("_pb200_call", _CALL_PATH)
             _binder = importlib.util.module_from_spec(spec)
             spec.loader.exec_module(_binder)
-        sig = "".join(_CODES.get(t, "?") for t in (fn.argtypes or ()))
-        fn = _binder.bind(ctypes.cast(fn, c_void_p).value, sig) or fn
+        if _binder is not None:
+            sig = "".join(_CODES.get(t, "?") for t in (fn.argtypes or ()))
+            typed = _binder.bind(ctypes.cast(fn, c_void_p).value, sig)
+        if typed is None and not _warned:
+            _warned = True
+            warnings.warn(f"{_CALL_PATH} is missing or older than the kernels' signatures ({name}): launches go through "
+                          "ctypes at twice the host time each; python -m prometheus_b200._build makes it",
+                          RuntimeWarning, stacklevel=3)
+        fn = typed or fn
     _bound[name] = fn
     return fn
 

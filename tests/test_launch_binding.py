@@ -49,3 +49,21 @@ def test_call_takes_and_refuses_what_the_foreign_call_does():
             _lib.call("pb_scale_cast", *args)
         with pytest.raises((TypeError, ctypes.ArgumentError)):
             getattr(_lib.load(), "pb_scale_cast")(*args)
+
+
+@pytest.mark.parametrize("stale", [False, True])
+def test_a_missing_or_stale_caller_module_is_reported_once(stale, monkeypatch, tmp_path):
+    """Launches still work, at twice the host time: that must not go unnoticed."""
+    import types
+    import warnings
+
+    monkeypatch.setattr(_lib, "_bound", {})
+    monkeypatch.setattr(_lib, "_warned", False, raising=False)
+    monkeypatch.setattr(_lib, "_CALL_PATH", tmp_path / "absent.so")
+    monkeypatch.setattr(_lib, "_binder", types.SimpleNamespace(bind=lambda address, sig: None) if stale else None)
+    with pytest.warns(RuntimeWarning, match="missing or older"):
+        fn = _lib._bind("pb_rmsnorm_bwd_nparts")
+    assert fn(300, 2048) == _lib.query("pb_rmsnorm_bwd_nparts", 300, 2048)
+    with warnings.catch_warnings():
+        warnings.simplefilter("error")
+        _lib._bind("pb_sigmoid")
