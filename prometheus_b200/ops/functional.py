@@ -523,9 +523,10 @@ class _SoftcapCeFn(torch.autograd.Function):
         gh = (dh * g.to(dh.dtype)) if dh is not None else None
         gU = None
         if dU is not None:
-            # one pass for a plain first-order backward; a batched or differentiated upstream
-            # gradient goes through tensor operations
+            # one pass for a plain first-order backward; a batched or differentiated upstream gradient goes
+            # through tensor operations, and so does an accumulator that saved-tensor hooks gave back in another form
             if (g.is_cuda and g.dtype == torch.float32 and ctx.U_ref.dtype == BF16 and dU.numel()
+                    and dU.dtype == torch.float32 and dU.device == g.device and dU.is_contiguous() and dU.data_ptr() % 16 == 0
                     and not torch.is_grad_enabled() and not torch._C._functorch.is_functorch_wrapped_tensor(g)):
                 gU = torch.empty(dU.shape, dtype=BF16, device=dU.device)
                 call("pb_scale_cast", ptr(dU), ptr(g), ptr(gU), dU.numel(), stream_ptr())

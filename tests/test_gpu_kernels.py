@@ -418,6 +418,41 @@ def test_softcap_ce_fresh_gradient_chunks():
         assert torch.equal(gU, (Um.main_grad * 2.5).to(BF16))
 
 
+@pytest.mark.parametrize("form", ["bf16", "transposed", "shifted"])
+def test_softcap_ce_accumulator_from_saved_tensor_hooks(form):
+    """Hooks may give the fp32 accumulator back as another type, with other strides or from a base that is
+    not 16-byte aligned; the scaled gradient is then that tensor's."""
+    from prometheus_b200.ops import functional as ops
+
+    rows, d, V, cap = 64, 128, 1032, 30.0
+    h, U = _r(rows, d, seed=3), _r(V, d, seed=4, scale=0.1)
+    tgt = torch.randint(0, V, (rows,), device="cuda", dtype=torch.int32)
+    wt = torch.full((rows,), 1.0 / rows, device="cuda")
+
+    def unpack(t):
+        if t.shape != (V, d) or t.dtype != torch.float32:
+            return t
+        if form == "bf16":
+            return t.to(BF16)
+        if form == "transposed":
+            return t.t().contiguous().t()
+        return torch.empty(V * d + 1, device="cuda")[1:].view(V, d).copy_(t)
+
+    def grad(hooked):
+        Ug = U.clone().requires_grad_(True)
+        if not hooked:
+            return torch.autograd.grad(2.5 * ops.softcap_cross_entropy(h, Ug, tgt, wt, cap), (Ug,))[0]
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t, unpack):
+            loss = 2.5 * ops.softcap_cross_entropy(h, Ug, tgt, wt, cap)
+        return torch.autograd.grad(loss, (Ug,))[0]
+
+    got, want = grad(True), grad(False)
+    if form == "bf16":       # one more rounding, of the accumulator: 2^-8 of each element
+        assert ((got.float() - want.float()).abs() <= 2.0 ** -7 * want.float().abs()).all()
+    else:
+        assert torch.equal(got, want)
+
+
 def test_optimizer_kernels():
     from prometheus_b200 import train
     from prometheus_b200.ops import _lib
