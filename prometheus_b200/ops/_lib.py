@@ -43,6 +43,7 @@ _SIGS = {
     "pb_softcap_ce": [P, P, P, P, P, L, I, F, I, P],
     "pb_softcap_ce_sums": [P, P, P, P, P, L, I, F, I, P],
     "pb_gemm_softcap_ok": [I, I, I],
+    "pb_gemm_softcap_pays": [I, I, I],
     "pb_gemm_softcap_logits": [P, P, P, I, I, I, L, L, L, F, P, P, P, P],
     "pb_sigmoid": [P, P, L, P],
     "pb_scale_cast": [P, P, P, L, P],

@@ -472,7 +472,7 @@ class _SoftcapCeFn(torch.autograd.Function):
     """loss = sum_rows wt[row] * CE(softcap(h @ U^T), target). Rows are processed in chunks:
     logits chunk (bf16) -> fused CE kernel rewrites it as d(loss)/d(logits) -> dh and dU
     GEMMs, so full-vocabulary fp32 logits never exist and the backward is free. Under a cap, and where
-    the product's kernel takes it (``pb_gemm_softcap_ok``), its epilogue adds up each row's
+    it is the faster way (``pb_gemm_softcap_pays``), the product's epilogue adds up each row's
     exponentials, so the CE kernel reads the logits once instead of twice."""
 
     @staticmethod
@@ -494,7 +494,7 @@ class _SoftcapCeFn(torch.autograd.Function):
             hc = h[r0:r1]
             n = r1 - r0
             if cap > 0 and hc.dtype == U.dtype == BF16 and hc.is_contiguous() and U.is_contiguous() and \
-                    (hc.data_ptr() | U.data_ptr()) % 16 == 0 and _lib.query("pb_gemm_softcap_ok", n, V, d):
+                    (hc.data_ptr() | U.data_ptr()) % 16 == 0 and _lib.query("pb_gemm_softcap_pays", n, V, d):
                 logits = torch.empty((n, V), dtype=BF16, device=dev)
                 sums = torch.empty(n, dtype=torch.float32, device=dev)
                 part = torch.empty(2 * ((V + 255) // 256) * n, dtype=torch.float32, device=dev)

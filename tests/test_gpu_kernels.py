@@ -400,6 +400,42 @@ def test_softcap_sums_from_the_logits_product(rows, d, V, scale):
     ops.check_status("cuda")
 
 
+@pytest.mark.parametrize("grad", [True, False])
+def test_softcap_sums_over_chunks_and_without_gradients(grad):
+    """The head with its row sums from the logits product against the two-sweep kernel: chunks of different row
+    counts (one with a last row block of 8), a ragged vocabulary, and a loss alone. The rule that chooses it
+    leaves products of few tiles to the two sweeps."""
+    from prometheus_b200.ops import functional as ops
+    from prometheus_b200.ops._lib import call, query
+
+    rows, d, V, cap, chunk = 2 * 768 + 520, 1024, 65544, 30.0, 768
+    for n in (768, 520):
+        assert query("pb_gemm_softcap_pays", n, V, d) == 1
+    for n, v in ((200, 8192), (256, 65544), (4096, 8192)):      # 32, 257 and 512 tiles
+        assert query("pb_gemm_softcap_ok", n, v, d) == 1 and query("pb_gemm_softcap_pays", n, v, d) == 0
+    assert query("pb_gemm_softcap_pays", 4096, 131072, 1016) == 0
+    h, U = _r(rows, d, seed=1), _r(V, d, seed=2, scale=2.0 / math.sqrt(d))
+    tgt = torch.randint(0, V, (rows,), device="cuda", dtype=torch.int32)
+    wt = (torch.arange(rows, device="cuda") % 5 != 0).float() / rows
+
+    def run(variant):
+        call("pb_gemm_set_variant", variant)       # 8: no CTA pairs, so the two-sweep kernel
+        try:
+            with torch.set_grad_enabled(grad):
+                hg, Ug = h.clone().requires_grad_(grad), U.clone().requires_grad_(grad)
+                loss = ops.softcap_cross_entropy(hg, Ug, tgt, wt, cap, chunk_rows=chunk)
+                return (loss.detach(), *(torch.autograd.grad(loss, (hg, Ug)) if grad else ()))
+        finally:
+            call("pb_gemm_set_variant", 0)
+
+    got, want = run(0), run(8)
+    # the same logits and exponentials, added up in another order in fp32
+    assert (got[0] - want[0]).abs() <= 1e-5 * want[0].abs()
+    for a, b in zip(got[1:], want[1:]):
+        assert (a.float() - b.float()).norm() <= 5e-3 * b.float().norm()
+    ops.check_status("cuda")
+
+
 def test_softcap_ce_fresh_gradient_chunks():
     """A unembedding gradient that is not accumulated: one chunk, several, and a non-unit upstream
     gradient, against the accumulating form's buffer (fp32 sums of the same products)."""
