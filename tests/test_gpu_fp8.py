@@ -203,3 +203,33 @@ def test_rmsnorm_emits_the_fp8_rows_the_gemm_reads(rows, d):
         outs.append((o, yl.grad, wp.grad))
     for a, b in zip(*outs):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("exponent", [0, -52, 68, -100, 120])
+def test_quotient_of_every_pair_of_significands(exponent):
+    """Bytes against the correctly rounded division for every significand of a block's largest magnitude (so of
+    the scale) times every significand, at every exponent distance up to where quotients round to zero, both signs.
+    At exponents -52 and 68 the scales lie on both sides of 2^-60 and 2^60, the bounds of the
+    three-operation quotient; at -100 and 120 the division is taken throughout."""
+    from prometheus_b200.ops import fp8
+
+    sig = 1.0 + torch.arange(128, dtype=torch.float64) / 128
+    top = sig * 2.0 ** exponent                                      # one row each
+    dist = torch.arange(0, 21)                                       # 448 / 2^-10 is 2^18.8
+    x = sig[None, :, None] * 2.0 ** (exponent - dist.double())[None, None, :]
+    x = x.reshape(1, -1).repeat(128, 1)
+    x = torch.minimum(x, top[:, None])                               # none above the row's largest
+    x = torch.cat([x, -x], 1)                                        # 5376 values, 127 to a block
+    x = torch.nn.functional.pad(x, (0, (-x.shape[1]) % 127)).view(128, -1, 127)
+    x = torch.cat([top[:, None, None].expand(-1, x.shape[1], 1), x], 2).reshape(128, -1)
+    xb = x.to(BF16)
+    assert torch.equal(xb.double(), x)                               # every value is a bf16
+    q, s = fp8.quantize_rows(xb.cuda())
+    scale = top.float() / 448.0
+    assert torch.equal(s.cpu(), scale[None].expand_as(s))
+    if exponent == -52:
+        assert (scale < 2.0 ** -60).any() and (scale > 2.0 ** -60).any()
+    if exponent == 68:
+        assert (scale < 2.0 ** 60).any() and (scale > 2.0 ** 60).any()
+    want = (xb.float() / scale[:, None]).to(torch.float8_e4m3fn)
+    assert torch.equal(q.cpu(), want.view(torch.uint8))

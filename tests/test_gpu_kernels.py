@@ -153,6 +153,35 @@ def test_gemm_c_and_d_at_any_base(M, N, c_f32, d_f32):
     ops.check_status("cuda")
 
 
+@pytest.mark.parametrize("M,N", [(200, 328), (456, 264), (520, 264)])     # column remainders 8, row remainders 8 and 72
+@pytest.mark.parametrize("c_f32", [False, True])
+@pytest.mark.parametrize("d_f32", [False, True])
+def test_gemm_d_at_remainders_against_fp32(M, N, c_f32, d_f32):
+    """alpha A B^T + beta D where a row's D is read partly in whole slabs ahead of the accumulator and partly by
+    column chunks: every combination of the types of C and D, a contiguous D and a column slice of a wider one, on
+    CTA pairs and on single CTAs, alone and batched."""
+    from prometheus_b200.ops import functional as ops
+    from prometheus_b200.ops._lib import call
+
+    dts = {False: BF16, True: torch.float32}
+    a, b = _r(2, M, 192, seed=1), _r(2, N, 192, seed=2)
+    wide = _r(2, M, N + 24, seed=3, dtype=dts[d_f32], scale=8.0)      # D as large as the product
+    kw = dict(out_dtype=dts[c_f32], alpha=0.5, beta=-2.0)
+    try:
+        for variant in (0, 8):
+            call("pb_gemm_set_variant", variant)
+            for d in (wide[:, :, 8:8 + N], wide[:, :, 8:8 + N].contiguous(), wide[:, :, 1:1 + N]):
+                want = ops.gemm_ref(a, b, d=d, alpha=0.5, beta=-2.0)
+                tol = 1e-5 if c_f32 else 2.0 ** -8      # fp32 sums of 192 products, one rounding of the result
+                for got, ref in ((ops.gemm(a, b, d=d, **kw), want), (ops.gemm(a[0], b[0], d=d[0], **kw), want[0])):
+                    assert got.dtype == dts[c_f32]
+                    err = (got.float() - ref).abs()
+                    assert (err <= tol * ref.abs() + 1e-3).all(), (variant, float(err.max()))
+    finally:
+        call("pb_gemm_set_variant", 0)
+    ops.check_status("cuda")
+
+
 def test_gemm_limited_grid_and_many_tiles():
     from prometheus_b200.ops import functional as ops
 
