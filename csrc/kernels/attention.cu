@@ -1,6 +1,6 @@
 // Causal softmax attention with grouped KV heads on tcgen05 (sm_100a), head dim 128.
 //
-// Forward (flash-style, one CTA per 128 query rows of one head):
+// Forward (flash-style, one CTA per 256 query rows of one head, two tiles of 128):
 //   S = Q K_j^T  (tensor memory, double-buffered)      P = exp2(S c - m)   (registers, one
 //   O += P V_j   (tensor memory)                                             query row per thread)
 // The running maximum is only raised when it would grow by more than 2^8 (the rescale of O is a
@@ -15,12 +15,13 @@
 // Every streamed tile is used twice from the same shared-memory image: as the K-major B operand
 // of the score product and as the MN-major B operand of the gradient product.
 //
-// warps 0-3: one tensor-memory lane (= row) per thread; warp 4: MMA issue; warp 5: TMA producer.
+// Forward: warps 0-3 and 4-7 the rows of the two tiles, one tensor-memory lane (= row) per thread; warps 8 and 9 MMA
+// issue, one tile each; warp 10 TMA producer. Backward: warps 0-7 rows, 8-10 MMA issue, 11 TMA producer.
 // All tensors are token-major: Q/O/dO/dQ [batch * seq, ldq] with head h at columns 128 h,
 // K/V/dK/dV [batch * seq, ldkv] with KV head g at columns 128 g. Any seq: the tensor maps are per batch entry,
 // so the rows a last tile lacks read as zeros (no real query sees a key after itself, and a zero
-// query with zero dO adds nothing) and are clipped from the stores. 3 x 1000 x 16/4 forward: 84 us with
-// padded copies of q, k, v and a cut of the result, 36 us in place.
+// query with zero dO adds nothing) and are clipped from the stores. 3 x 1000 x 16/4 forward: 24.6 us; with
+// padded copies of q, k, v and a cut of the result it took 48 us more.
 //
 // Reference semantics: model/__init__.py gqa/mla attention (softmax(q k^T / sqrt(d)) v with a
 // causal mask) of the reference; the tiling is this library's own.
@@ -424,8 +425,8 @@ struct Params {
 // bf16 once, with the softmax scale in it: P (dP - delta) scale costs two multiplications an element, so
 // the rows' arithmetic is packed two elements to an instruction (as scalar operations the backward
 // of 4 x 4096 x 16/4 takes 35 us longer).
-// 4 x 4096 x 16/4: dQ 396 us with delta (618 with two stages and operand tiles, and 45 more for delta as a
-// kernel of its own; 471 with three stages), dK and dV 535 us (917; 721).
+// 4 x 4096 x 16/4: dQ 391 us with delta (618 with two stages and operand tiles, and 45 more for delta as a
+// kernel of its own; 471 with three stages), dK and dV 521 us (917; 721).
 template <bool DKV>
 __global__ void __launch_bounds__(384, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant__ CUtensorMap tmRB,

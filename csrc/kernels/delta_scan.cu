@@ -7,9 +7,9 @@
 //   forward   Y = W S            U = U^ - Y          O = Q S + M U      S += K^T U
 //   backward  dU = M^T dO + K dS                     dS += Q^T dO - W^T dU
 //
-// One CTA owns one (batch, head) sequence. The state lives in tensor memory for the
-// whole walk (fp32, 128 lanes x 128 columns); every product is a tcgen05.mma with
-// M = 128, N = 128; the bf16 image of the state and of U that the MMAs consume as
+// A CTA walks one (batch, head) sequence, or one segment of it, with all 128 columns of the state or with 64. The
+// state lives in tensor memory for the whole walk (fp32, 128 lanes); every product is a tcgen05.mma with
+// M = 128, N = its columns; the bf16 image of the state and of U that the MMAs consume as
 // their B operand is rewritten in shared memory each chunk in the 128-byte-swizzled
 // layout TMA itself produces; Q/K/W/M and U^ (or dO) tiles arrive by TMA through a
 // two-stage ring, and every output leaves by a TMA store from shared memory. Tiles with 64 token rows are used as 128-row A operands: the upper 64
@@ -20,20 +20,22 @@
 // quarter, 64 columns each); the state update is issued before the output product and has its own
 // barrier; the output accumulator is double-buffered, so chunk n's output rows are staged while
 // chunk n + 1's Y product runs; the part of the backward's Y that does not need the state is issued
-// before the state image is ready. 64 sequences of 64 chunks, forward 230 us -> 144 us (3.6 -> 2.3 us a
-// chunk), backward 133 -> 117 us, against four row warps that did all of it in order.
+// before the state image is ready. 64 sequences of 64 chunks: forward 115 us (1.8 us a chunk), backward 102 us;
+// four row warps that did all of it in order, in one CTA a sequence, took 230 and 133 us.
 //
 // The columns of the state never mix (U, O and dU have the same columns), so when the sequences or
 // segments take at most half of the SMs, two CTAs walk each of them with 64 columns: the conversions
-// and products between two waits are half as long. 64 sequences: 144 -> 115 us forward, 109 -> 103 us
-// backward. With more CTAs than SMs it would be two waves of a chain that is not half as long.
+// and products between two waits are half as long. On both sides of the line, 64 chunks each: 74 sequences with
+// 64 columns a CTA 121 us forward and 108 us backward, 75 sequences with 128 columns 148 and 116 us. With more
+// CTAs than SMs it would be two waves of a chain that is not half as long.
 //
 // A forward summary walks every segment twice, once per map, over the same W and K. When the two CTAs a
 // segment that takes are more than the SMs, one CTA does both, as two independent chains whose conversions
 // and products fall into each other's waits: one wave and half of the operand reads. 16 sequences x 8
-// segments x 32 chunks: 104 us -> 87 us. (One chain of 256 columns: 120 us, its conversions and products
-// take turns.) With a CTA for each map on SMs of their own a chain is the shorter, so up to half of the
-// SMs it stays so. The initial state of that walk is read 16 bytes at a time: 79 us -> 73 us.
+// segments x 32 chunks: 90 us, against 104 us as two waves of a CTA for each map. (One chain of 256 columns:
+// 120 us, its conversions and products take turns.) With a CTA for each map on SMs of their own a chain is the
+// shorter, so up to half of the SMs it stays so: 72 segments of 32 chunks 65 us, 80 segments in a CTA each 92 us.
+// The initial state is read 16 bytes at a time: element by element the walk of those segments, 76 us, takes 6 us more.
 //
 // warps 0-7: tensor-memory <-> registers <-> shared/global (lane = state row or token)
 // warp 8   : MMA issue (one lane)          warp 9: TMA producer (one lane)
@@ -715,7 +717,7 @@ compose_kernel(const float* __restrict__ P, const float* __restrict__ R,
                              : *reinterpret_cast<const float4*>(R + j * mat + row * D + col0 + c0);
       a[h][0] = rv.x; a[h][1] = rv.y; a[h][2] = rv.z; a[h][3] = rv.w;
     }
-    if (step + 1 < n_seg) {   // its image was last read two steps ago
+    if (step + 1 < n_seg) {   // its image was read in the previous step, whose closing barrier orders those reads before
       fetch(step + 1);
       asm volatile("cp.async.wait_group 1;" ::: "memory");
     } else {

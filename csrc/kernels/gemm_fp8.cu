@@ -319,15 +319,14 @@ __device__ __forceinline__ uint32_t to_e4m3x4(float a, float b, float c, float d
 // loads are all in flight before the first use. What bounds them is memory once the arithmetic is
 // out of the way: a warp per row with one 512-column step at a time left one load latency per step
 // exposed, and a compiler division per element (about ten instructions) made the kernels
-// issue-bound. 73984 x 2048, 73984 x 1408 and the 66 x (2816 + 1408) x 2048 expert weights, before ->
-// after: see the figures at each kernel.
+// issue-bound.
 //
 // e4m3(x / scale) must round as the correctly rounded quotient does (a reciprocal multiply moves
 // some ties). Markstein (1990): with r = RN(1 / s) and q0 = RN(x r), the residual x - q0 s is exact in
 // one FMA and RN(q0 + r residual) is RN(x / s): three operations. The range check keeps every
 // quotient that does not round to zero clear of underflow and r clear of overflow; other scales
-// take the division. The sign of a zero quotient is the numerator's. All 128 x 128 pairs of bf16
-// significands at every exponent distance that matters give the quotient's bits.
+// take the division. The sign of a zero quotient is the numerator's. The tests compare the bytes of all
+// 128 x 128 pairs of bf16 significands, at every exponent distance that does not round to zero, with the division's.
 struct Quot {
   float s, r;
   bool fast;

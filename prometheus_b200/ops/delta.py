@@ -164,19 +164,22 @@ def _from_chunks(x: Tensor, b: int, h: int, n: int) -> Tensor:
 
 def scan_segments(n_seq: int, n_chunks: int, ctas: int = 148) -> int:
     """Segments per sequence for the state walk, chosen by a cost model in units of one chunk
-    step of one CTA wave. The single-pass walk costs ``waves(n_seq) * n_chunks``. With ``seg``
-    segments the summary launch does two maps per segment, each about 0.6 of a chunk step
-    per chunk (three of the six products, no stores), the segmented walk one step per chunk,
-    and the two extra launches plus the fold about 24 steps of start-up (tensor-memory
-    allocation, first loads, state load / store: measured at about ten chunk steps per launch):
+    step of one CTA wave, a CTA for each sequence, segment and map. The single-pass walk costs
+    ``waves(n_seq) * n_chunks``. With ``seg`` segments the summary launch does two maps per segment, each
+    about 0.6 of a chunk step per chunk (three of the six products, no stores), the segmented walk one step
+    per chunk, and the two extra launches plus the fold about 24 steps of start-up (tensor-memory
+    allocation, first loads, state load / store: about ten chunk steps per launch):
 
         waves(2 n_seq seg) * 0.6 n_chunks / seg  +  waves(n_seq seg) * n_chunks / seg  +  24
 
-    The smallest power of two (at least four chunks per segment) that beats the single pass
-    by a fifth is taken; 1 means the plain single-pass walk. Measured, forward us at 1 / 4 / 8 / 16
-    segments (the rule's choice in parentheses): 16 sequences x 256 chunks 492 / 359 / 316 / 404
-    (8), 16 x 128 252 / 201 / 193 / 241 (8), 16 x 64 134 / 123 / 127 / 176 (4), 8 x 256 431 / 300 /
-    216 / 223 (16), 32 x 128 314 / 319 / 419 / 471 (4), 32 x 64 163 / 194 / 241 / 334 (1)."""
+    The smallest power of two (at least four chunks per segment) whose estimate beats the single
+    pass's by a fifth is taken; 1 means the plain single-pass walk. The kernels differ from the model: walks
+    that take at most half of the SMs run as two CTAs each, and a summary whose CTAs do not fit runs both
+    maps in one (``csrc/kernels/delta_scan.cu``), so the choice is near the best and not always the best. Measured,
+    forward us at 1 / 4 / 8 / 16 segments (the rule's choice in parentheses): 16 sequences x 256 chunks
+    492 / 359 / 316 / 404 (8), 16 x 128 252 / 201 / 193 / 241 (8), 16 x 64 134 / 123 / 127 / 176 (4), 8 x 256
+    431 / 300 / 216 / 223 (16, 3 % slower than 8), 32 x 128 314 / 319 / 419 / 471 (4, 2 % slower than uncut),
+    32 x 64 163 / 194 / 241 / 334 (1). The backward, which uses the same segments, was not measured apart."""
     def waves(c):
         return -(-c // ctas)
 
