@@ -182,7 +182,12 @@ bool get(PyObject* o, void*& v) {
   return !PyErr_Occurred();
 }
 // integers as a foreign call takes them: anything with an index, cut to the width of the argument
-bool get(PyObject* o, long& v) { v = static_cast<long>(PyLong_AsUnsignedLongLongMask(o)); return !PyErr_Occurred(); }
+bool get(PyObject* o, long& v) {
+  int wide = 0;
+  v = PyLong_AsLongAndOverflow(o, &wide);
+  if (wide) v = static_cast<long>(PyLong_AsUnsignedLongLongMask(o));
+  return !(v == -1 && PyErr_Occurred());
+}
 bool get(PyObject* o, int& v) { long l; if (!get(o, l)) return false; v = static_cast<int>(l); return true; }
 bool get(PyObject* o, float& v) {
   const double d = PyFloat_AsDouble(o);
