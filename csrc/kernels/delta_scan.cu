@@ -26,16 +26,16 @@
 // The columns of the state never mix (U, O and dU have the same columns), so when the sequences or
 // segments take at most half of the SMs, two CTAs walk each of them with 64 columns: the conversions
 // and products between two waits are half as long. On both sides of the line, 64 chunks each: 74 sequences with
-// 64 columns a CTA 121 us forward and 108 us backward, 75 sequences with 128 columns 148 and 116 us. With more
+// 64 columns a CTA 122 us forward and 109 us backward, 75 sequences with 128 columns 143 and 115 us. With more
 // CTAs than SMs it would be two waves of a chain that is not half as long.
 //
 // A forward summary walks every segment twice, once per map, over the same W and K. When the two CTAs a
 // segment that takes are more than the SMs, one CTA does both, as two independent chains whose conversions
 // and products fall into each other's waits: one wave and half of the operand reads. 16 sequences x 8
-// segments x 32 chunks: 90 us, against 104 us as two waves of a CTA for each map. (One chain of 256 columns:
+// segments x 32 chunks: 86 us, against 104 us as two waves of a CTA for each map. (One chain of 256 columns:
 // 120 us, its conversions and products take turns.) With a CTA for each map on SMs of their own a chain is the
-// shorter, so up to half of the SMs it stays so: 72 segments of 32 chunks 65 us, 80 segments in a CTA each 92 us.
-// The initial state is read 16 bytes at a time: element by element the walk of those segments, 76 us, takes 6 us more.
+// shorter, so up to half of the SMs it stays so: 72 segments of 32 chunks 62 us, 80 segments in a CTA each 87 us.
+// The initial state is read 16 bytes at a time: element by element the walk of those segments, 70 us, takes 6 us more.
 //
 // warps 0-7: tensor-memory <-> registers <-> shared/global (lane = state row or token)
 // warp 8   : MMA issue (one lane)          warp 9: TMA producer (one lane)
@@ -298,10 +298,18 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     const int g0 = col0 + c0;                 // its first column in the state or map
     const bool tok_warp = (warp & 3) < 2;     // warps whose lanes are token rows
     const uint32_t lane_addr = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + c0;
-    // barriers of the row warps and of the token warps: true when nobody's wait ran out (a summary walk has
-    // neither, there every warp decides for itself)
-    auto sync_rows = [](bool ok) { return bar_sync_and(1, 256, ok); };
-    auto sync_tok = [](bool ok) { return bar_sync_and(2, 128, ok); };
+    auto sync_rows = [] { asm volatile("bar.sync 1, 256;" ::: "memory"); };
+    auto sync_tok = [] { asm volatile("bar.sync 2, 128;" ::: "memory"); };
+    // A lane whose wait ran out waits no more but stays in the loop to its end: whoever shares a barrier or a
+    // collective instruction with it finds it there, and what is computed and stored meanwhile is reported as
+    // invalid by the status word. 16 sequences x 8 segments x 32 chunks: 70.4 us, as with lanes that leave one by one
+    // (69.9); a vote after each wait 72.5 us, and barriers that carry the result as well 75.5 us.
+    bool ok = true;
+    auto wait = [&](uint64_t* bar, uint32_t parity) {
+      if (ok) ok = mbar_wait_spin(bar, parity, p.status);
+      __syncwarp();   // lanes leave the spin one by one
+      tc_fence_after();
+    };
     auto arrive = [&](uint64_t* bar) {   // the warp's shared-memory writes and tensor-memory reads are done
       fence_proxy_async_smem();
       tc_fence_before();
@@ -358,21 +366,16 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
       }
       tmem_st_wait();
     }
-    bool ok = true;
     for (int it = 0; it < N; ++it) {
       const int n = n0 + (BWD ? (N - 1 - it) : it);
       const uint32_t cph = it & 1;
       const int g = seq * NT + n;
-      if (it > 0) {
-        ok = ok && mbar_wait_spin_warp(x_done, cph ^ 1, p.status);
-        tc_fence_after();
-      }
+      if (it > 0) wait(x_done, cph ^ 1);
       // all earlier bulk stores have finished reading xb / ub / ob before they are rewritten
       if (!sum) {
         if (r == 0 && ch == 0) tma_store_wait_read<0>();
-        ok = sync_rows(ok);
+        sync_rows();
       }
-      if (!ok) break;
       // bf16 image of the state entering this chunk
       {
         uint32_t v[WC];
@@ -382,9 +385,8 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
       arrive(x_ready);
       if (!BWD && !sum && it > 0) {
         // rows of the previous chunk's output: tensor memory -> staging tile, while Y is computed
-        ok = mbar_wait_spin_warp(o_done, cph ^ 1, p.status);
-        tc_fence_after();
-        if (ok && tok_warp) {
+        wait(o_done, cph ^ 1);
+        if (tok_warp) {
           uint32_t v[WC];
           load_cols(COL_O + (cph ^ 1) * 128, v);
           put_cols(ob, C, v);
@@ -392,8 +394,7 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
         }
       }
       if (!sum) {
-        ok = sync_rows(ok);
-        if (!ok) break;
+        sync_rows();
         if (r == 0 && ch == 0) {
           if (!BWD && it > 0) {
             const int prow = tok0 + (n - 1) * C;
@@ -407,8 +408,8 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
           tma_store_commit();
         }
       }
-      if (tok_warp && (ok = mbar_wait_spin_warp(y_done, cph, p.status))) {
-        tc_fence_after();
+      if (tok_warp) {
+        wait(y_done, cph);
         uint32_t v[WC];
         load_cols(COL_Y, v);
         uint8_t* uh = smem + (it & 1) * S::STAGE + TILE_DO;
@@ -429,33 +430,30 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
           *reinterpret_cast<bf16x8*>(piece(ub, C, i)) = pack8(y);
         }
         arrive(u_ready);
-      }
-      if (tok_warp && store_ux) {
-        ok = sync_tok(ok);   // the other row warps hear of it at the next sync_rows
-        if (ok && r == 0 && ch == 0) {
+        if (store_ux) {
+          sync_tok();
+          if (r == 0 && ch == 0) {
 #pragma unroll
-          for (int hf = 0; hf < HALVES; ++hf) tma_store_3d(&tmU, ub + hf * 8192, col0 + hf * 64, g * C, 0);
-          tma_store_commit();
+            for (int hf = 0; hf < HALVES; ++hf) tma_store_3d(&tmU, ub + hf * 8192, col0 + hf * 64, g * C, 0);
+            tma_store_commit();
+          }
         }
       }
     }
     // drain: last chunk's output rows and the final state
-    ok = ok && N > 0 && mbar_wait_spin_warp(x_done, (N - 1) & 1, p.status) &&
-         (BWD || sum || mbar_wait_spin_warp(o_done, (N - 1) & 1, p.status));
-    if (!BWD && !sum) {
-      if (r == 0 && ch == 0) tma_store_wait_read<0>();
-      ok = sync_rows(ok);
-    }
-    if (ok) {
-      tc_fence_after();
+    if (N > 0) {
+      wait(x_done, (N - 1) & 1);
       if (!BWD && !sum) {
+        wait(o_done, (N - 1) & 1);
+        if (r == 0 && ch == 0) tma_store_wait_read<0>();
+        sync_rows();
         if (tok_warp) {
           uint32_t v[WC];
           load_cols(COL_O + ((N - 1) & 1) * 128, v);
           put_cols(ob, C, v);
           fence_proxy_async_smem();
         }
-        sync_rows(true);
+        sync_rows();
         if (r == 0 && ch == 0) {
           const int prow = tok0 + (n0 + N - 1) * C;
 #pragma unroll

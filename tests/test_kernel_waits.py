@@ -3,8 +3,8 @@
 A wait is per thread. Where the next instructions are collective (tensor-memory loads, barriers), lanes that
 gave up one by one would leave the others at an instruction that never completes: a timeout that has to be
 reported would become a kernel that never returns. So a wait either belongs to a single thread, or it is one of
-the warp-uniform forms, or its result goes through ``__syncthreads_and`` before anybody acts on it; and a named
-barrier that follows a wait carries the result (``bar_sync_and``)."""
+the warp-uniform forms, or its result goes through ``__syncthreads_and`` before anybody acts on it; and where a
+named barrier follows a wait, either the barrier carries the result (``bar_sync_and``) or nobody leaves the loop."""
 import re
 from pathlib import Path
 
@@ -32,7 +32,9 @@ def per_thread_waits(text):
                 stop = re.search(r"\bbreak\b|\breturn\b", rest)
                 agreed = rest.find("__syncthreads_and")
                 inline = c == "{" or "break" in stmt or "return" in stmt      # acted on in the same statement
-                if inline or agreed < 0 or (stop and stop.start() < agreed - 6):
+                if not inline and rest[1:].lstrip().startswith("__syncwarp();"):
+                    pass                                                      # kept, not acted on: see the walks below
+                elif inline or agreed < 0 or (stop and stop.start() < agreed - 6):
                     bad.append((text.count("\n", 0, i) + 1, " ".join(stmt.split())))
             if c == "{":
                 heads.append(stmt)
@@ -49,7 +51,12 @@ def test_waits_before_collective_instructions_are_uniform(name):
 
 def test_row_warps_that_share_a_named_barrier_leave_together():
     scan, chunk, att = _text("delta_scan.cu"), _text("delta_chunk.cu"), _text("attention.cu")
-    assert "bar.sync" not in scan and "bar.sync" not in chunk
+    assert "bar.sync" not in chunk
+    # the walks: row warps run their loop to its end whatever a wait returned, and skip no barrier over it
+    first = scan.rindex("for (int it = 0; it < N; ++it)")
+    rows = scan[first:scan.index("tma_store_wait<0>();", first)]
+    assert rows.count("sync_rows();") == 4 and not re.search(r"\b(break|continue|return|ok)\b|mbar_wait", rows)
+    assert len(re.findall(r"if \(ok\) ok = mbar_wait_spin\(bar, parity, p\.status\);\s+__syncwarp\(\);", scan[:first])) == 1
     # attention: the only plain barriers left stand behind an agreed one, with no wait in between
     for m in re.finditer(r"\bsync_group\(\);", att):
         before = att[:m.start()]
