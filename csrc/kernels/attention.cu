@@ -117,6 +117,13 @@ __device__ __forceinline__ void tie32(uint32_t (&v)[32]) {
                       "+r"(v[i + 6]), "+r"(v[i + 7]));
 }
 
+__device__ __forceinline__ void tie16(uint32_t (&v)[16]) {
+#pragma unroll
+  for (int i = 0; i < 16; i += 8)
+    asm volatile("" : "+r"(v[i]), "+r"(v[i + 1]), "+r"(v[i + 2]), "+r"(v[i + 3]), "+r"(v[i + 4]), "+r"(v[i + 5]),
+                      "+r"(v[i + 6]), "+r"(v[i + 7]));
+}
+
 // ------------------------------------------------------------------------------ forward
 namespace fwd {
 // shared memory: Q (two 128-row tiles, at the end the staging of O), five K/V stages of 64 keys
@@ -395,47 +402,52 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 
 // ----------------------------------------------------------------------------- backward
 namespace bwd {
-constexpr int STAGES = 4;
-constexpr int RA_OFF = 0, RB_OFF = 32768, ST_OFF = 65536;       // stages: T1 16 KB + T2 16 KB
-constexpr int VEC_OFF = ST_OFF + STAGES * 32768, BARS = VEC_OFF + 2 * 512;
+// Streamed tiles: T1 16 KB + T2 16 KB a stage. dQ copies its resident tiles into tensor memory and then
+// streams through their shared memory too (stages 4 and 5); dK / dV keeps them, and has 512 bytes a stage of
+// the streamed queries' log-sum-exp and delta.
+constexpr int RA_OFF = 0, RB_OFF = 32768, ST_OFF = 65536;
+template <bool DKV> struct Ring {
+  static constexpr int STAGES = DKV ? 4 : 6;
+  __device__ static int off(int s) { return s < 4 ? ST_OFF + s * 32768 : (s - 4) * 32768; }
+};
+constexpr int VEC_OFF = ST_OFF + 4 * 32768, BARS = VEC_OFF + 4 * 512;
 constexpr int SMEM = BARS + 256 + 1024;
 static_assert(SMEM <= 227 * 1024, "one CTA's shared memory");
-// tensor memory: score buffers of 128 columns (X1 at 0, X2 at 64; P^T and dS take the first 32 columns
-// of each as packed bf16 operands), then the accumulators. dQ has one accumulator and so room for
-// a third score buffer.
-template <bool DKV> struct Cols {
-  static constexpr int BUFS = DKV ? 2 : 3;
-  static constexpr uint32_t ACC1 = BUFS * 128, ACC2 = 384;
-};
-constexpr uint32_t COL_X2 = 64, TMEM_COLS = 512;
+// tensor memory: two score buffers of 128 columns (X1 at 0, X2 at 64), then the accumulators, and for dQ
+// its resident tiles. Row warpgroup g works on columns 32 g .. 32 g + 31 of X1 and X2 and puts what it makes of
+// them, packed bf16 operands (P^T over X1, dS over X2), over the first 16 of its own: no warp writes
+// what another still reads.
+constexpr uint32_t COL_X2 = 64, COL_ACC1 = 256, COL_ACC2 = 384, COL_R = 384, TMEM_COLS = 512;
 
 struct Params {
   int batch, seq, heads, kv_heads, n_blk;  // seq: query rows per batch entry; n_blk: 128-row blocks of the grid
   int seq_kv, q_off;                // key rows per batch entry; global position of query row 0
   float scale_log2, scale;
   const float* lse2;    // [batch, heads, seq]
-  float* delta;         // [batch, heads, seq]  rowsum(dO * O): written by the dQ kernel, read by the other
+  // [batch, heads, ceil(seq / 64), 32 pairs of rows, {-lse2, -lse2, -delta, -delta}], delta = rowsum(dO * O), zeros
+  // past seq: written by the dQ kernel, read by the other a tile (512 bytes) at a time
+  float* vec;
   int* status;
 };
 
 // DKV = false: resident Q, dO (one head); streams K, V tiles; output dQ.
 // DKV = true : resident K, V (one KV head); streams Q, dO tiles of the group; outputs dK, dV.
-// Two warpgroups (warps 0-3, 4-7) take the streamed tiles alternately and accumulate into the same
-// gradient accumulators.  MMA issue is spread over three warps because one thread cannot issue
+// Two warpgroups (warps 0-3, 4-7) share every streamed tile, half of its columns each: what a tile waits for is its
+// score products, the rows' work on them and its gradient products one after the other, with two tiles on the
+// way, and the rows' part of that chain halves.  MMA issue is spread over three warps because one thread cannot issue
 // 20+ small MMAs per tile fast enough: warp 8 the first score product, warp 9 the second,
 // warp 10 the gradient accumulations; warp 11: TMA producer.
 //
-// Bound by shared-memory bandwidth: a 128 x 64 score product reads 6 KB of operands per 16-deep
-// step, half as much again as the tensor core can use. So what can be kept off shared memory is:
-// P^T and dS go back to tensor memory as bf16 over the scores they were made from and are the
-// gradient products' A operand there (64 KB less per tile than operand tiles written to and read from
-// shared memory), which also makes room for four stages of streamed tiles: a tile's stage is held
-// until its gradient product is done, and with fewer every tile waits for a load. dS is rounded to
-// bf16 once, with the softmax scale in it: P (dP - delta) scale costs two multiplications an element, so
-// the rows' arithmetic is packed two elements to an instruction (as scalar operations the backward
-// of 4 x 4096 x 16/4 takes 35 us longer).
-// 4 x 4096 x 16/4: dQ 391 us with delta (618 with two stages and operand tiles, and 45 more for delta as a
-// kernel of its own; 471 with three stages), dK and dV 521 us (917; 721).
+// Shared-memory bandwidth is what the products compete for: a 128 x 64 score product with both operands there reads
+// 6 KB per 16-deep step, half as much again as the tensor core can use. So what can be kept off it is: P^T
+// and dS go back to tensor memory as bf16 and are the gradient products' A operand there; dQ's resident
+// tiles are A operands in tensor memory too (2 KB a step), and their shared memory holds two more stages of streamed
+// tiles, whose loads were late with four (dK / dV has no tensor memory left for its own). The streamed queries'
+// log-sum-exp and delta come with their tile, and a lane of the dK / dV rows reads 8 columns of them instead of 64.
+// dS is rounded to bf16 once, with the softmax scale in it: P (dP - delta) scale costs two multiplications an
+// element, so the rows' arithmetic is packed two elements to an instruction.
+// 4 x 4096 x 16/4, clocks a 128 x 64 tile: dQ 1157 -> 1081 (768 of them MMAs), dK and dV 1908 -> 1644 (1280);
+// together 909 -> 835 us, under the power cap 1045 -> 956.
 template <bool DKV>
 __global__ void __launch_bounds__(384, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant__ CUtensorMap tmRB,
@@ -448,16 +460,16 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + BARS);
   uint64_t* r_full = bars;
   uint64_t* t_full = bars + 1;    // [STAGES]
-  uint64_t* t_empty = bars + 5;   // [STAGES]
-  uint64_t* x_done = bars + 9;    // [BUFS] scores of a buffer
-  uint64_t* x_free = bars + 12;   // [BUFS] its gradient products
-  uint64_t* pd_ready = bars + 15; // [BUFS] its P^T and dS
-  uint64_t* acc_done = bars + 18;
-  uint64_t* o_full = bars + 19;   // dQ: the forward's output tile, in the last stage until the row warps
-  uint64_t* o_read = bars + 20;   //     have taken delta from it
+  uint64_t* t_empty = bars + 7;   // [STAGES]
+  uint64_t* x_done = bars + 13;   // [2] scores of a buffer
+  uint64_t* x_free = bars + 15;   // [2] its gradient products
+  uint64_t* pd_ready = bars + 17; // [2] its P^T and dS
+  uint64_t* acc_done = bars + 19;
+  uint64_t* o_full = bars + 20;   // dQ: the forward's output tile, in the last of the first four stages
+  uint64_t* r_read = bars + 21;   // dQ: delta is taken from it and the resident tiles are in tensor memory
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 22);
-  constexpr int O_STAGE = STAGES - 1;
-  constexpr int BUFS = Cols<DKV>::BUFS;
+  constexpr int STAGES = Ring<DKV>::STAGES, O_STAGE = 3;
+  auto stage = [&](int s) { return smem + Ring<DKV>::off(s); };
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int group = p.heads / p.kv_heads;
@@ -481,12 +493,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
   if (threadIdx.x == 0) {
     mbar_init(r_full, 1);
     for (int i = 0; i < STAGES; ++i) { mbar_init(&t_full[i], 1); mbar_init(&t_empty[i], 1); }
-    for (int i = 0; i < BUFS; ++i) {
+    for (int i = 0; i < 2; ++i) {
       mbar_init(&x_done[i], 2); mbar_init(&x_free[i], 1);    // two issuing threads
-      mbar_init(&pd_ready[i], 4);                            // one arrival per row warp
+      mbar_init(&pd_ready[i], 8);                            // one arrival per row warp
     }
     mbar_init(acc_done, 1);
-    mbar_init(o_full, 1); mbar_init(o_read, 8);
+    mbar_init(o_full, 1); mbar_init(r_read, 8);
     fence_barrier_init();
     tma_prefetch_desc(&tmRA); tma_prefetch_desc(&tmRB);
     tma_prefetch_desc(&tmT1); tma_prefetch_desc(&tmT2);
@@ -515,19 +527,22 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
       }
       if (!DKV) {
         mbar_arrive_expect_tx(o_full, 32768);
-        tma_load_3d(smem + ST_OFF + O_STAGE * 32768, &tmFO, o_full, rx, row0, b);
-        tma_load_3d(smem + ST_OFF + O_STAGE * 32768 + 16384, &tmFO, o_full, rx + 64, row0, b);
+        tma_load_3d(stage(O_STAGE), &tmFO, o_full, rx, row0, b);
+        tma_load_3d(stage(O_STAGE) + 16384, &tmFO, o_full, rx + 64, row0, b);
       }
       for (int it = 0; it < n_it; ++it) {
         const int s = it % STAGES;
         const uint32_t ph = (it / STAGES) & 1;
         const int t = t_first + (DKV ? it % t_count : it);
-        const int tx = (DKV ? g * group + it / t_count : g) * D;
+        const int th = DKV ? g * group + it / t_count : g, tx = th * D;
         const int trow = t * 64;
         if (!mbar_wait(&t_empty[s], ph ^ 1, p.status)) break;
-        if (!DKV && it == O_STAGE && !mbar_wait(o_read, 0, p.status)) break;
-        mbar_arrive_expect_tx(&t_full[s], 32768);
-        uint8_t* st = smem + ST_OFF + s * 32768;
+        if (!DKV && it == O_STAGE && !mbar_wait(r_read, 0, p.status)) break;
+        mbar_arrive_expect_tx(&t_full[s], DKV ? 32768 + 512 : 32768);
+        uint8_t* st = stage(s);
+        if (DKV)
+          bulk_load(smem + VEC_OFF + s * 512,
+                    p.vec + ((static_cast<size_t>(b) * p.heads + th) * ((p.seq + 63) / 64) + t) * 128, 512, &t_full[s]);
         tma_load_3d(st, &tmT1, &t_full[s], tx, trow, b);
         tma_load_3d(st + 8192, &tmT1, &t_full[s], tx + 64, trow, b);
         tma_load_3d(st + 16384, &tmT2, &t_full[s], tx, trow, b);
@@ -541,21 +556,28 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
       const uint32_t id_x = make_idesc(1, 1, 128, 64, 0, 0);     // A K-major, B K-major, N = 64
       constexpr uint32_t HI = sdesc_hi_sw128(1024);
       const uint32_t r_lo = sdesc_lo(smem_u32(smem + (which == 0 ? RA_OFF : RB_OFF)), 16);
-      const uint32_t st0 = smem_u32(smem + ST_OFF + which * 16384);
+      const uint32_t r_col = tmem + COL_R + which * 64;
       const uint32_t col = which == 0 ? 0 : COL_X2;
-      bool ok = n_it == 0 || mbar_wait_spin(r_full, 0, p.status);
+      bool ok = n_it == 0 || mbar_wait_spin(DKV ? r_full : r_read, 0, p.status);
+      int ts = 0;
+      uint32_t ph = 0;
       for (int it = 0; it < n_it && ok; ++it) {
-        const int s = it % BUFS, ts = it % STAGES;
-        if (!mbar_wait_spin(&t_full[ts], (it / STAGES) & 1, p.status)) break;
-        if (!mbar_wait_spin(&x_free[s], ((it / BUFS) & 1) ^ 1, p.status)) break;
+        const int s = it & 1;
+        if (!mbar_wait_spin(&t_full[ts], ph, p.status)) break;
+        if (!mbar_wait_spin(&x_free[s], ((it >> 1) & 1) ^ 1, p.status)) break;
         tc_fence_after();
-        const uint32_t t_lo = sdesc_lo(st0 + ts * 32768, 16);
+        const uint32_t t_lo = sdesc_lo(smem_u32(stage(ts)) + which * 16384, 16);
         const uint32_t d = tmem + col + s * 128;
 #pragma unroll
-        for (int jj = 0; jj < 8; ++jj)
-          umma_f16_words(d, r_lo + (((jj >> 2) * 16384 + (jj & 3) * 32) >> 4), HI,
-                         t_lo + (((jj >> 2) * 8192 + (jj & 3) * 32) >> 4), HI, id_x, jj > 0);
+        for (int jj = 0; jj < 8; ++jj) {
+          const uint32_t b_lo = t_lo + (((jj >> 2) * 8192 + (jj & 3) * 32) >> 4);
+          if (DKV)
+            umma_f16_words(d, r_lo + (((jj >> 2) * 16384 + (jj & 3) * 32) >> 4), HI, b_lo, HI, id_x, jj > 0);
+          else
+            umma_f16_ts(d, r_col + jj * 8, (static_cast<uint64_t>(HI) << 32) | b_lo, id_x, jj > 0);
+        }
         umma_commit(&x_done[s]);
+        if (++ts == STAGES) { ts = 0; ph ^= 1; }
       }
     }
   } else if (warp == 10) {
@@ -563,50 +585,46 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
     if (lane == 0) {
       const uint32_t id_acc = make_idesc(1, 1, 128, 128, 0, 1);  // A from tensor memory, B MN-major
       constexpr uint64_t HI = static_cast<uint64_t>(sdesc_hi_sw128(1024)) << 32;
-      const uint32_t st0 = smem_u32(smem + ST_OFF);
-      int it = 0;
+      int it = 0, ts = 0;
       for (; it < n_it; ++it) {
-        const int s = it % BUFS, ts = it % STAGES;
-        if (!mbar_wait_spin(&pd_ready[s], (it / BUFS) & 1, p.status)) break;
+        const int s = it & 1;
+        if (!mbar_wait_spin(&pd_ready[s], (it >> 1) & 1, p.status)) break;
         tc_fence_after();
         // the streamed tiles again, now as MN-major B operands (64-wide chunks 8 KB apart); 16
-        // values of a bf16 operand row are eight tensor-memory columns
-        const uint32_t t1_mn = sdesc_lo(st0 + ts * 32768, 8192), t2_mn = t1_mn + (16384 >> 4);
+        // values of a bf16 operand row are eight tensor-memory columns, 32 of them to a warpgroup's part
+        const uint32_t t1_mn = sdesc_lo(smem_u32(stage(ts)), 8192), t2_mn = t1_mn + (16384 >> 4);
         const uint32_t xb = tmem + s * 128;
+        auto a_col = [](const int jj) { return static_cast<uint32_t>((jj >> 1) * 32 + (jj & 1) * 8); };
 #pragma unroll
         for (int jj = 0; jj < 4; ++jj)
-          umma_f16_ts(tmem + Cols<DKV>::ACC1, xb + COL_X2 + jj * 8, HI | (t1_mn + ((jj * 2048) >> 4)), id_acc,
+          umma_f16_ts(tmem + COL_ACC1, xb + COL_X2 + a_col(jj), HI | (t1_mn + ((jj * 2048) >> 4)), id_acc,
                       (it > 0) || (jj > 0));
         if (DKV) {
 #pragma unroll
           for (int jj = 0; jj < 4; ++jj)
-            umma_f16_ts(tmem + Cols<DKV>::ACC2, xb + jj * 8, HI | (t2_mn + ((jj * 2048) >> 4)), id_acc,
+            umma_f16_ts(tmem + COL_ACC2, xb + a_col(jj), HI | (t2_mn + ((jj * 2048) >> 4)), id_acc,
                         (it > 0) || (jj > 0));
         }
         // the score products of this tile finished before the row warps could signal pd_ready,
         // so the completion of these MMAs releases the whole stage and the score buffer
         umma_commit(&t_empty[ts]);
         umma_commit(&x_free[s]);
+        if (++ts == STAGES) ts = 0;
       }
       if (it == n_it) umma_commit(acc_done);
     }
   } else {
-    const int wg = warp >> 2;          // warpgroup = score buffer = parity of its iterations
+    const int wg = warp >> 2;          // warpgroup = half of a tile's columns
     const int r = threadIdx.x & 127;
     const uint32_t lane_addr = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
-    auto sync_group = [&] {
-      if (wg == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
-      else asm volatile("bar.sync 2, 128;" ::: "memory");
-    };
-    const int pos = gblk * 128 + r;   // global query position (dQ) or key position (dKV) of this row
     float row_lse = 0.f, row_delta = 0.f;
     bool ok = true;
     if (!DKV) {
-      const size_t vi = (static_cast<size_t>(b) * p.heads + hy) * p.seq + blk * 128 + r;
-      const bool in = blk * 128 + r < p.seq;
-      if (in) row_lse = p.lse2[vi];
+      const int q = blk * 128 + r;
+      const size_t bh = static_cast<size_t>(b) * p.heads + hy;
+      if (q < p.seq) row_lse = p.lse2[bh * p.seq + q];
       // delta of the row from the resident dO and the forward's output: a kernel of its own read both
-      // again (268 MB, 45 us at 4 x 4096 x 16). Both groups need it, one stores it.
+      // again (268 MB, 45 us at 4 x 4096 x 16). Both groups need it.
       ok = wait_all(r_full, 0, p.status) && wait_all(o_full, 0, p.status);
       if (ok) {
         // Columns are added as a warp with four of them to a lane adds its lanes up (halves, quarters, ..):
@@ -615,7 +633,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
           const int off = (i >> 3) * 16384 + r * 128 + (((i & 7) ^ (r & 7)) << 4);
           float x[8], y[8];
           unpack8(*reinterpret_cast<const bf16x8*>(smem + RB_OFF + off), x);
-          unpack8(*reinterpret_cast<const bf16x8*>(smem + ST_OFF + O_STAGE * 32768 + off), y);
+          unpack8(*reinterpret_cast<const bf16x8*>(stage(O_STAGE) + off), y);
           float t[4];   // products of bf16 values are exact
 #pragma unroll
           for (int e = 0; e < 4; ++e) t[e] = fmaf(x[2 * e], y[2 * e], x[2 * e + 1] * y[2 * e + 1]);
@@ -626,128 +644,127 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
         const float2 even = add2(quarter_sum(0), quarter_sum(2)), odd = add2(quarter_sum(1), quarter_sum(3));
         const float2 sum = add2(even, odd);
         row_delta = __fadd_rn(sum.x, sum.y);
-        if (in && wg == 0) p.delta[vi] = row_delta;
+        if (q < (p.seq + 63) / 64 * 64) {   // rows past seq have zeros in all four
+          float* v = p.vec + (bh * ((p.seq + 63) / 64) + (q >> 6)) * 128 + ((q & 63) >> 1) * 4 + (q & 1);
+          if (wg == 0) v[0] = -row_lse;
+          else v[2] = -row_delta;
+        }
+        // group 0 puts Q, group 1 dO where the score products read them: a row is 64 columns of bf16 pairs
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          uint32_t w[32];
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            *reinterpret_cast<uint4*>(w + 4 * i) = *reinterpret_cast<const uint4*>(
+                smem + (wg == 0 ? RA_OFF : RB_OFF) + c * 16384 + r * 128 + ((i ^ (r & 7)) << 4));
+          tmem_st_32x32b_x32(lane_addr + COL_R + wg * 64 + c * 32, w);
+        }
+        tmem_st_wait();
       }
-      fence_proxy_async_smem();   // the producer's next load goes over what was read here
+      fence_proxy_async_smem();   // the producer's next loads go over what was read here
+      tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(o_read);
-    }
-    // dKV: per-column log-sum-exp and delta of the streamed query tile (negated), prefetched one
-    // iteration ahead by threads 0..63 (lse) and 64..127 (delta).
-    // (head of the group, tile) of an iteration, stepped by the two iterations between a group's tiles
-    // (a division by the tile count twice an iteration was a sixth of the instructions)
-    struct Step { int h, t; };
-    auto advance = [&](Step& s) {
-      s.t += 2;
-      while (s.t >= t_count) { s.t -= t_count; ++s.h; }
-    };
-    auto vec_value = [&](const Step& s) -> float {
-      const int q = (t_first + s.t) * 64 + (r & 63);
-      const float* base = (r < 64) ? p.lse2 : p.delta;
-      return q < p.seq ? -base[(static_cast<size_t>(b) * p.heads + g * group + s.h) * p.seq + q] : 0.f;
-    };
-    Step cur = {0, wg};
-    float vec_next = 0.f;
-    if (DKV && wg < n_it) {
-      if (cur.t >= t_count) cur = {wg / t_count, wg % t_count};
-      vec_next = vec_value(cur);
+      if (ok && lane == 0) mbar_arrive(r_read);
     }
     const float2 log2_scale = make_float2(p.scale_log2, p.scale_log2), lin_scale = make_float2(p.scale, p.scale);
-    for (int it = wg; it < n_it && (DKV || ok); it += 2) {
-      const int s = it % BUFS;
-      const int t = t_first + (DKV ? cur.t : it);
-      float* vec = reinterpret_cast<float*>(smem + VEC_OFF + wg * 512);
-      if (DKV) {
-        // the group's readers of the previous tile are done; who ran out of a wait takes the group along
-        ok = bar_sync_and(1 + wg, 128, ok);
-        if (!ok) break;
-        vec[r] = vec_next;   // [0,64) -lse2, [64,128) -delta
-        advance(cur);   // t above is this iteration's
-        if (it + 2 < n_it) vec_next = vec_value(cur);
-        sync_group();
-      }
-      if (!wait_all(&x_done[s], (it / BUFS) & 1, p.status)) { ok = false; continue; }
-      tc_fence_after();
+    // P and dS of two neighbouring columns of a row: nl, nd are the columns' (or the row's) -lse2 and -delta
+    auto grad2 = [&](const uint32_t xa, const uint32_t xc, const uint32_t da, const uint32_t dc, const float2 nl,
+                     const float2 nd, const bool mask_x, const bool mask_y, uint32_t& pk_p, uint32_t& pk_d) {
+      const float2 e = fma2(make_float2(__uint_as_float(xa), __uint_as_float(xc)), log2_scale, nl);
+      float2 pr = make_float2(ex2(e.x), ex2(e.y));
+      if (mask_x) pr.x = 0.f;
+      if (mask_y) pr.y = 0.f;
+      const float2 dp = make_float2(__uint_as_float(da), __uint_as_float(dc));
+      const float2 ds = mul2(pr, mul2(add2(dp, nd), lin_scale));   // the scale before the one rounding to bf16
+      pk_d = pack_bf16x2(ds.x, ds.y);
+      if (DKV) pk_p = pack_bf16x2(pr.x, pr.y);
+    };
+    int ts = 0, t = t_first;
+    uint32_t t_ph = 0;
+    for (int it = 0; it < n_it; ++it) {
+      const int s = it & 1;
       // mask: dQ rows are queries, columns keys (key > query is masked);
       //       dKV rows are keys, columns queries (query < key is masked)
       const int tg = DKV ? t + q_off64 : t;     // global index of the streamed tile
       const bool edge = DKV ? (tg * 64 < gblk * 128 + 127) : (tg * 64 + 63 > gblk * 128);
-      const uint32_t xb = lane_addr + s * 128;
-      uint32_t pk_p[32], pk_d[32];               // the row's P and dS, two bf16 to a register
-      auto half = [&](auto EDGE, const int c, const uint32_t (&x1)[32], const uint32_t (&x2)[32]) {
+      const uint32_t xb = lane_addr + s * 128 + wg * 32;
+      const int col0 = tg * 64 + wg * 32;
+      ok = ok && (!DKV || wait_all(&t_full[ts], t_ph, p.status)) && wait_all(&x_done[s], (it >> 1) & 1, p.status);
+      if (!ok) break;
+      tc_fence_after();
+      if constexpr (DKV) {
+        // Fragments of 16 rows x 8 columns: a lane has two neighbouring columns of eight, in rows lane / 4 and
+        // lane / 4 + 8, so it needs the log-sum-exp and delta of 8 of its group's 32 columns, not of all: a
+        // shared-memory read that all lanes share costs as much as one of 32 different words.
+        uint32_t x1[2][16], x2[2][16], pk_p[2][8], pk_d[2][8];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          float2 pf[4], df[4], nl[4], nd[4];
-          if (DKV) {
-#pragma unroll
-            for (int k = 0; k < 4; k += 2) {
-              const float4 l4 = *reinterpret_cast<const float4*>(vec + c + 8 * i + 2 * k);
-              const float4 d4 = *reinterpret_cast<const float4*>(vec + 64 + c + 8 * i + 2 * k);
-              nl[k] = make_float2(l4.x, l4.y); nl[k + 1] = make_float2(l4.z, l4.w);
-              nd[k] = make_float2(d4.x, d4.y); nd[k + 1] = make_float2(d4.z, d4.w);
-            }
-          } else {
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              nl[k] = make_float2(-row_lse, -row_lse);
-              nd[k] = make_float2(-row_delta, -row_delta);
-            }
-          }
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const int at = 8 * i + 2 * k;
-            const float2 e = fma2(make_float2(__uint_as_float(x1[at]), __uint_as_float(x1[at + 1])), log2_scale, nl[k]);
-            float2 pr = make_float2(ex2(e.x), ex2(e.y));
-            if (decltype(EDGE)::value) {
-              const int other = tg * 64 + c + at;
-              if (DKV ? (other < pos) : (other > pos)) pr.x = 0.f;
-              if (DKV ? (other + 1 < pos) : (other + 1 > pos)) pr.y = 0.f;
-            }
-            pf[k] = pr;
-            const float2 dp = make_float2(__uint_as_float(x2[at]), __uint_as_float(x2[at + 1]));
-            df[k] = mul2(pr, mul2(add2(dp, nd[k]), lin_scale));   // the scale before the one rounding to bf16
-          }
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const int at = (c >> 1) + 4 * i + k;
-            pk_d[at] = pack_bf16x2(df[k].x, df[k].y);
-            if (DKV) pk_p[at] = pack_bf16x2(pf[k].x, pf[k].y);
-          }
+        for (int h = 0; h < 2; ++h) {
+          tmem_ld_16x256b_x4(xb + (static_cast<uint32_t>(16 * h) << 16), x1[h]);
+          tmem_ld_16x256b_x4(xb + COL_X2 + (static_cast<uint32_t>(16 * h) << 16), x2[h]);
         }
-      };
-      auto tile_rows = [&](auto EDGE) {
-        // the second half's scores arrive while the first half is worked on
-        uint32_t a1[32], a2[32], b1[32], b2[32];
-        tmem_ld_32x32b_x32(xb, a1);
-        tmem_ld_32x32b_x32(xb + COL_X2, a2);
+        float4 v[4];   // -lse2 and -delta of the lane's columns
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          v[j] = *reinterpret_cast<const float4*>(smem + VEC_OFF + ts * 512 + (wg * 16 + j * 4 + (lane & 3)) * 16);
         tmem_ld_wait();
-        tie32(a1);
-        tie32(a2);
-        tmem_ld_32x32b_x32(xb + 32, b1);
-        tmem_ld_32x32b_x32(xb + COL_X2 + 32, b2);
-        half(EDGE, 0, a1, a2);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) { tie16(x1[h]); tie16(x2[h]); }
+        auto rows = [&](auto EDGE) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+              for (int u = 0; u < 2; ++u) {
+                const int at = 4 * j + 2 * u, pos = gblk * 128 + (warp & 3) * 32 + h * 16 + u * 8 + (lane >> 2);
+                const int q = col0 + 8 * j + 2 * (lane & 3);
+                grad2(x1[h][at], x1[h][at + 1], x2[h][at], x2[h][at + 1], make_float2(v[j].x, v[j].y),
+                      make_float2(v[j].z, v[j].w), decltype(EDGE)::value && q < pos,
+                      decltype(EDGE)::value && q + 1 < pos, pk_p[h][2 * j + u], pk_d[h][2 * j + u]);
+              }
+        };
+        if (edge) rows(std::true_type{});
+        else rows(std::false_type{});
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          tmem_st_16x128b_x4(xb + (static_cast<uint32_t>(16 * h) << 16), pk_p[h]);
+          tmem_st_16x128b_x4(xb + COL_X2 + (static_cast<uint32_t>(16 * h) << 16), pk_d[h]);
+        }
+      } else {
+        uint32_t x1[32], x2[32], pk_d[16], none;
+        tmem_ld_32x32b_x32(xb, x1);
+        tmem_ld_32x32b_x32(xb + COL_X2, x2);
         tmem_ld_wait();
-        tie32(b1);
-        tie32(b2);
-        half(EDGE, 32, b1, b2);
-      };
-      if (edge) tile_rows(std::true_type{});
-      else tile_rows(std::false_type{});
-      tmem_st_32x32b_x32(xb + COL_X2, pk_d);
-      if (DKV) tmem_st_32x32b_x32(xb, pk_p);
+        tie32(x1);
+        tie32(x2);
+        const float2 nl = make_float2(-row_lse, -row_lse), nd = make_float2(-row_delta, -row_delta);
+        const int pos = gblk * 128 + r;
+        auto rows = [&](auto EDGE) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i)
+            grad2(x1[2 * i], x1[2 * i + 1], x2[2 * i], x2[2 * i + 1], nl, nd,
+                  decltype(EDGE)::value && col0 + 2 * i > pos, decltype(EDGE)::value && col0 + 2 * i + 1 > pos, none,
+                  pk_d[i]);
+        };
+        if (edge) rows(std::true_type{});
+        else rows(std::false_type{});
+        tmem_st_32x32b_x16(xb + COL_X2, pk_d);
+      }
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&pd_ready[s]);
+      if (++ts == STAGES) { ts = 0; t_ph ^= 1; }
+      if (++t == t_first + t_count) t = t_first;   // dKV: the next head of the group
     }
-    // every row thread gets here (no early exit above), so the group barrier below is safe
+    // every row warp gets here, also one that gave up, so the group barrier below is safe
     ok = wait_all(acc_done, 0, p.status) && ok;
     // resident tiles are no longer read: reuse them as the staging for the TMA stores.
     // dKV: group 0 drains dK, group 1 drains dV.  dQ: each group drains 64 columns.
-    uint8_t* stage = smem + ((DKV && wg == 1) ? RB_OFF : RA_OFF);
+    uint8_t* out = smem + ((DKV && wg == 1) ? RB_OFF : RA_OFF);
     if (ok) {
       tc_fence_after();
-      const uint32_t col0 = (DKV && wg == 1) ? Cols<DKV>::ACC2 : Cols<DKV>::ACC1;
+      const uint32_t col0 = (DKV && wg == 1) ? COL_ACC2 : COL_ACC1;
       const int c_lo = DKV ? 0 : wg * 64, c_hi = DKV ? D : wg * 64 + 64;
 #pragma unroll 1
       for (int c = c_lo; c < c_hi; c += 32) {
@@ -761,7 +778,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
           // a key block with no local query at or after it gets an all-zero gradient
           for (int k = 0; k < 8; ++k) f[k] = n_it > 0 ? __uint_as_float(v[8 * i + k]) : 0.f;
           const int col = c + 8 * i;
-          st_swz(stage + (col >> 6) * 16384, r, (col & 63) >> 3, pack_bf16x8(f));
+          st_swz(out + (col >> 6) * 16384, r, (col & 63) >> 3, pack_bf16x8(f));
         }
       }
       fence_proxy_async_smem();
@@ -770,10 +787,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
       const int ox = (DKV ? g : hy) * D;
       if (DKV) {
         const CUtensorMap* tm = wg == 0 ? &tmO1 : &tmO2;
-        tma_store_3d(tm, stage, ox, row0, b);
-        tma_store_3d(tm, stage + 16384, ox + 64, row0, b);
+        tma_store_3d(tm, out, ox, row0, b);
+        tma_store_3d(tm, out + 16384, ox + 64, row0, b);
       } else {
-        tma_store_3d(&tmO1, stage + wg * 16384, ox + wg * 64, row0, b);
+        tma_store_3d(&tmO1, out + wg * 16384, ox + wg * 64, row0, b);
       }
       tma_store_commit();
       tma_store_wait<0>();
@@ -865,7 +882,7 @@ PB_API int pb_attn_fwd(const void* q, const void* k, const void* v, void* out, v
                         ldo, scale, status, st);
 }
 
-// Gradients of pb_attn_fwd_cp. delta: fp32 scratch [batch, heads, seq] (written here).
+// Gradients of pb_attn_fwd_cp. delta: fp32 scratch [batch, heads, ceil(seq / 64), 128] (written here), 16-byte aligned.
 // dq: [batch * seq, ldq]; dk, dv: [batch * seq_kv, ldkv] (all bf16, fully overwritten; key rows
 // that no local query sees get zeros).
 PB_API int pb_attn_bwd_cp(const void* q, const void* k, const void* v, const void* out,
@@ -875,7 +892,8 @@ PB_API int pb_attn_bwd_cp(const void* q, const void* k, const void* v, const voi
                           cudaStream_t st) {
   using namespace attn;
   if (bad_geometry(batch, seq, heads, kv_heads, ldq, ldkv) || ldo < heads * D || ldo % 8 != 0 ||
-      !(scale > 0.f) || q_off < 0 || q_off % 128 != 0 || seq_kv < q_off + seq)
+      !(scale > 0.f) || q_off < 0 || q_off % 128 != 0 || seq_kv < q_off + seq ||
+      (reinterpret_cast<uintptr_t>(delta) & 15) != 0)
     return PB_BAD_ARG;
   const long grid_q = grid_ctas(seq, 128, heads, batch), grid_kv = grid_ctas(seq_kv, 128, kv_heads, batch);
   if (grid_q < 0 || grid_kv < 0) return PB_BAD_ARG;
@@ -895,7 +913,7 @@ PB_API int pb_attn_bwd_cp(const void* q, const void* k, const void* v, const voi
   p.seq_kv = seq_kv; p.q_off = q_off;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;
   p.lse2 = static_cast<const float*>(lse2);
-  p.delta = static_cast<float*>(delta);
+  p.vec = static_cast<float*>(delta);
   p.status = status;
   int r = 0;
   {

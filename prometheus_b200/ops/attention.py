@@ -31,6 +31,12 @@ def causal_gqa_ref(q: Tensor, k: Tensor, v: Tensor, scale: float | None = None) 
     return (torch.softmax(logits, dim=-1) @ vf).transpose(1, 2).to(q.dtype)
 
 
+def backward_scratch(lse2: Tensor) -> Tensor:
+    """Scratch of ``pb_attn_bwd``: two floats of every query row, twice, in tiles of 64 rows."""
+    b, h, s = lse2.shape
+    return torch.empty((b, h, (s + 63) // 64, 128), dtype=torch.float32, device=lse2.device)
+
+
 class _AttnFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, scale, want_max):
@@ -62,7 +68,7 @@ class _AttnFn(torch.autograd.Function):
         hkv = k.shape[2]
         d_out = _tma_ready(d_out)
         dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-        delta = torch.empty_like(lse2)
+        delta = backward_scratch(lse2)
         call("pb_attn_bwd", ptr(q), ptr(k), ptr(v), ptr(out), ptr(d_out), ptr(lse2), ptr(delta),
              ptr(dq), ptr(dk), ptr(dv), b, s, hq, hkv, hq * d, hkv * d, hq * d, ctx.scale,
              ptr(status_word(q.device)), stream_ptr())
@@ -99,7 +105,7 @@ class _AttnCpFn(torch.autograd.Function):
         skv, hkv = k.shape[1], k.shape[2]
         d_out = d_out.contiguous()
         dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-        delta = torch.empty_like(lse2)
+        delta = backward_scratch(lse2)
         call("pb_attn_bwd_cp", ptr(q), ptr(k), ptr(v), ptr(out), ptr(d_out), ptr(lse2), ptr(delta), ptr(dq),
              ptr(dk), ptr(dv), b, s, skv, q_off, hq, hkv, hq * d, hkv * d, hq * d, scale,
              ptr(status_word(q.device)), stream_ptr())

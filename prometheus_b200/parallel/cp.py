@@ -465,6 +465,7 @@ class _ZigzagAttnFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, d_out):
         from ..ops._lib import call, ptr, stream_ptr
+        from ..ops.attention import backward_scratch
         from ..ops.functional import status_word
 
         q, kf, vf, out, lse2 = ctx.saved_tensors
@@ -475,7 +476,7 @@ class _ZigzagAttnFn(torch.autograd.Function):
         half_elems = L * hkv * d
         d_out = d_out.contiguous()
         dq = torch.empty_like(q)
-        delta = torch.empty_like(lse2)
+        delta = backward_scratch(lse2[0])     # one half after the other
         scale = 1.0 / math.sqrt(d)
         status = ptr(status_word(q.device))
         row_q, es = hq * d, q.element_size()
@@ -487,7 +488,7 @@ class _ZigzagAttnFn(torch.autograd.Function):
         for half, pos, dk, dv in ((1, far, dk_full, dv_full), (0, near, tmp_k, tmp_v)):
             off = half * L * row_q * es
             call("pb_attn_bwd_cp", q.data_ptr() + off, ptr(kf), ptr(vf), out.data_ptr() + off,
-                 d_out.data_ptr() + off, ptr(lse2[half]), ptr(delta[half]), dq.data_ptr() + off, ptr(dk),
+                 d_out.data_ptr() + off, ptr(lse2[half]), ptr(delta), dq.data_ptr() + off, ptr(dk),
                  ptr(dv), b, L, (pos + 1) * L, pos * L, hq, hkv, row_q, hkv * d, row_q, float(scale),
                  status, stream_ptr())
         dk_full[:tmp_k.numel()] += tmp_k
