@@ -586,6 +586,17 @@ __device__ __forceinline__ void umma_f16_words(uint32_t tmem_d, uint32_t a_lo, u
       : "memory");
 }
 
+// Both operands in 128-byte-swizzled tiles with 1024 bytes between groups of eight rows, given by their low words.
+__device__ __forceinline__ void umma_f16_lo(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc,
+                                            uint32_t accumulate) {
+  constexpr uint32_t HI = sdesc_hi_sw128(1024);
+  umma_f16_words(tmem_d, a_lo, HI, b_lo, HI, idesc, accumulate);
+}
+// Low word of step j (16 deep) of an operand whose first word is `lo`: K-major, tiles of 64 rows x 64 columns one after
+// the other; MN-major, 16 rows of 128 bytes a step.
+__device__ __forceinline__ uint32_t step_k(uint32_t lo, int j) { return lo + (((j >> 2) * 8192 + (j & 3) * 32) >> 4); }
+__device__ __forceinline__ uint32_t step_mn(uint32_t lo, int j) { return lo + ((j * 2048) >> 4); }
+
 // Pair form of umma_f16_words (cta_group::2, issued by the even CTA).
 __device__ __forceinline__ void umma_f16_pair_words(uint32_t tmem_d, uint32_t a_lo, uint32_t a_hi,
                                                     uint32_t b_lo, uint32_t b_hi, uint32_t idesc,

@@ -24,6 +24,8 @@
 // recurrence); the chunked WY algebra and this kernel are this library's own.
 #include <cuda.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace pb {
@@ -111,8 +113,9 @@ delta_prep_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   const uint32_t lane_addr = tmem + (static_cast<uint32_t>(warp * 32) << 16);
   const uint32_t id_kk64 = make_idesc(1, 1, 128, 64, 0, 0);    // A, B K-major, N = 64
   const uint32_t id_kn = make_idesc(1, 1, 128, 128, 0, 1);     // A K-major, B MN-major
-  const uint32_t kt = smem_u32(smem + KT), qt = smem_u32(smem + QT), vt = smem_u32(smem + VA);
-  const uint32_t ap = qt;
+  // descriptor words of the operands: an issue is one add for each
+  const uint32_t k_k = sdesc_lo(smem_u32(smem + KT), 16), q_k = sdesc_lo(smem_u32(smem + QT), 16), ap_k = q_k;
+  const uint32_t k_mn = sdesc_lo(smem_u32(smem + KT), 8192), v_mn = sdesc_lo(smem_u32(smem + VA), 8192);
 
   uint32_t ph = 0;
   for (int g = blockIdx.x; g < p.total; g += gridDim.x, ph ^= 1) {
@@ -141,12 +144,10 @@ delta_prep_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
         tc_fence_after();
 #pragma unroll
         for (int j = 0; j < 8; ++j)     // G = K K^T -> columns [0, 64)
-          umma_f16(tmem, make_sdesc_sw128(kt + (j >> 2) * 8192 + (j & 3) * 32, 16, 1024),
-                   make_sdesc_sw128(kt + (j >> 2) * 8192 + (j & 3) * 32, 16, 1024), id_kk64, j > 0);
+          umma_f16_lo(tmem, step_k(k_k, j), step_k(k_k, j), id_kk64, j > 0);
 #pragma unroll
         for (int j = 0; j < 8; ++j)     // Q K^T -> columns [64, 128)
-          umma_f16(tmem + 64, make_sdesc_sw128(qt + (j >> 2) * 8192 + (j & 3) * 32, 16, 1024),
-                   make_sdesc_sw128(kt + (j >> 2) * 8192 + (j & 3) * 32, 16, 1024), id_kk64, j > 0);
+          umma_f16_lo(tmem + 64, step_k(q_k, j), step_k(k_k, j), id_kk64, j > 0);
         umma_commit(mma1);
       }
     }
@@ -179,21 +180,30 @@ delta_prep_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
       tma_store_commit();
     }
 
-    // column r of T = (I + A)^-1 by forward substitution
+    // Column r of T = (I + A)^-1 by forward substitution. Every value of A that a warp reads costs a cycle of the SM's
+    // one shared-memory port, as many for the substitution as four schedulers need for its multiply-adds in four times
+    // the cycles; so the second warp, whose columns are zero down to row 32, leaves that half out.
     float t[64];
+    auto substitute = [&](auto FIRST) {
+      constexpr int i0 = decltype(FIRST)::value;
 #pragma unroll
-    for (int i = 0; i < 64; ++i) {
-      float a0 = (i == r) ? 1.f : 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
+      for (int i = 0; i < i0; ++i) t[i] = 0.f;
 #pragma unroll
-      for (int c = 0; c < (i + 3) / 4; ++c) {
-        const float4 a = af4[i * 16 + (c ^ (i & 15))];
-        if (4 * c + 0 < i) a0 = fmaf(-a.x, t[4 * c + 0], a0);
-        if (4 * c + 1 < i) a1 = fmaf(-a.y, t[4 * c + 1], a1);
-        if (4 * c + 2 < i) a2 = fmaf(-a.z, t[4 * c + 2], a2);
-        if (4 * c + 3 < i) a3 = fmaf(-a.w, t[4 * c + 3], a3);
+      for (int i = i0; i < 64; ++i) {
+        float a0 = (i == r) ? 1.f : 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
+#pragma unroll
+        for (int c = i0 / 4; c < (i + 3) / 4; ++c) {
+          const float4 a = af4[i * 16 + (c ^ (i & 15))];
+          if (4 * c + 0 < i) a0 = fmaf(-a.x, t[4 * c + 0], a0);
+          if (4 * c + 1 < i) a1 = fmaf(-a.y, t[4 * c + 1], a1);
+          if (4 * c + 2 < i) a2 = fmaf(-a.z, t[4 * c + 2], a2);
+          if (4 * c + 3 < i) a3 = fmaf(-a.w, t[4 * c + 3], a3);
+        }
+        t[i] = (a0 + a1) + (a2 + a3);
       }
-      t[i] = (a0 + a1) + (a2 + a3);
-    }
+    };
+    if (warp == 0) substitute(std::integral_constant<int, 0>{});
+    else substitute(std::integral_constant<int, 32>{});
     // A has been read and M has left: V comes into A's place, A' goes into M's
     if (r == 0) tma_store_wait_read<0>();
     fence_proxy_async_smem();
@@ -224,8 +234,7 @@ delta_prep_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
       tc_fence_after();
 #pragma unroll
       for (int j = 0; j < 4; ++j)       // W = A' K -> columns [0, 128)
-        umma_f16(tmem, make_sdesc_sw128(ap + j * 32, 16, 1024),
-                 make_sdesc_sw128(kt + j * 2048, 8192, 1024), id_kn, j > 0);
+        umma_f16_lo(tmem, step_k(ap_k, j), step_mn(k_mn, j), id_kn, j > 0);
       umma_commit(mma2);
       if (p.store_ta) {
         tma_store_3d(&tmT, smem + QT + 8192, 0, g * C, 0);
@@ -246,8 +255,7 @@ delta_prep_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
       tc_fence_after();
 #pragma unroll
       for (int j = 0; j < 4; ++j)       // U^ = A' V -> the same columns
-        umma_f16(tmem, make_sdesc_sw128(ap + j * 32, 16, 1024),
-                 make_sdesc_sw128(vt + j * 2048, 8192, 1024), id_kn, j > 0);
+        umma_f16_lo(tmem, step_k(ap_k, j), step_mn(v_mn, j), id_kn, j > 0);
       umma_commit(mma3);
       tma_store_3d(&tmW, smem + KT, 0, g * C, 0);
       tma_store_3d(&tmW, smem + KT + 8192, 64, g * C, 0);
@@ -397,15 +405,10 @@ delta_prep_bwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   const uint32_t id_mm64 = make_idesc(1, 1, 128, 64, 1, 1);
   const uint32_t id_kn = make_idesc(1, 1, 128, 128, 0, 1);
   const uint32_t id_mm = make_idesc(1, 1, 128, 128, 1, 1);
-  const uint32_t dw = smem_u32(smem + DW), ndu = smem_u32(smem + NDU), kt = smem_u32(smem + KTB);
-  const uint32_t vq = smem_u32(smem + VQ), ap = smem_u32(smem + APB), tt = smem_u32(smem + TT);
-  const uint32_t dm = smem_u32(smem + DM), tmp = smem_u32(smem + TMP);
-  // operand descriptors: 128-wide K-major (8 steps), 64-wide K-major (4), MN-major (4)
-  auto k128 = [](uint32_t base, int j) {
-    return make_sdesc_sw128(base + (j >> 2) * 8192 + (j & 3) * 32, 16, 1024);
-  };
-  auto k64 = [](uint32_t base, int j) { return make_sdesc_sw128(base + j * 32, 16, 1024); };
-  auto mn = [](uint32_t base, int j) { return make_sdesc_sw128(base + j * 2048, 8192, 1024); };
+  // operand descriptors, from words made once: K-major (8 steps over 128 columns, 4 over 64), MN-major (4 steps)
+  const uint32_t base_k = sdesc_lo(smem_u32(smem), 16), base_mn = sdesc_lo(smem_u32(smem), 8192);
+  auto kk = [&](int tile, int j) { return step_k(base_k + (tile >> 4), j); };
+  auto mn = [&](int tile, int j) { return step_mn(base_mn + (tile >> 4), j); };
 
   uint32_t ph = 0;
   for (int g = blockIdx.x; g < p.total; g += gridDim.x, ph ^= 1) {
@@ -442,11 +445,11 @@ delta_prep_bwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
       if (ok) {
         tc_fence_after();
 #pragma unroll
-        for (int j = 0; j < 8; ++j) umma_f16(tmem + 0, k128(dw, j), k128(kt, j), id_kk64, j > 0);
+        for (int j = 0; j < 8; ++j) umma_f16_lo(tmem + 0, kk(DW, j), kk(KTB, j), id_kk64, j > 0);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) umma_f16(tmem + 64, k128(ndu, j), k128(vq, j), id_kk64, j > 0);
+        for (int j = 0; j < 8; ++j) umma_f16_lo(tmem + 64, kk(NDU, j), kk(VQ, j), id_kk64, j > 0);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) umma_f16(tmem + 128, mn(ap, j), mn(ndu, j), id_mm, j > 0);
+        for (int j = 0; j < 4; ++j) umma_f16_lo(tmem + 128, mn(APB, j), mn(NDU, j), id_mm, j > 0);
         umma_commit(&mma[0]);
       }
     }
@@ -498,11 +501,11 @@ delta_prep_bwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
       tma_store_3d(&tmDV, smem + NDU + 8192, x0 + 64, t0, b);
       tma_store_commit();
 #pragma unroll
-      for (int j = 0; j < 4; ++j) umma_f16(tmem + 0, k64(tmp, j), k64(ap, j), id_kk64, j > 0);
+      for (int j = 0; j < 4; ++j) umma_f16_lo(tmem + 0, kk(TMP, j), kk(APB, j), id_kk64, j > 0);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) umma_f16(tmem + 64, mn(tmp, j), mn(tt, j), id_mm64, j > 0);
+      for (int j = 0; j < 4; ++j) umma_f16_lo(tmem + 64, mn(TMP, j), mn(TT, j), id_mm64, j > 0);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) umma_f16(tmem + 128, mn(ap, j), mn(dw, j), id_mm, j > 0);
+      for (int j = 0; j < 4; ++j) umma_f16_lo(tmem + 128, mn(APB, j), mn(DW, j), id_mm, j > 0);
       umma_commit(&mma[1]);
     }
     ok = mbar_wait_spin(&mma[1], ph, p.status);
@@ -539,9 +542,9 @@ delta_prep_bwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     if (lead) {
       tc_fence_after();
 #pragma unroll
-      for (int j = 0; j < 4; ++j) umma_f16(tmem + 0, mn(tt, j), mn(tmp, j), id_mm64, j > 0);
+      for (int j = 0; j < 4; ++j) umma_f16_lo(tmem + 0, mn(TT, j), mn(TMP, j), id_mm64, j > 0);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) umma_f16(tmem + 64, k128(kt, j), k128(kt, j), id_kk64, j > 0);
+      for (int j = 0; j < 8; ++j) umma_f16_lo(tmem + 64, kk(KTB, j), kk(KTB, j), id_kk64, j > 0);
       umma_commit(&mma[2]);
     }
     ok = mbar_wait_spin(&mma[2], ph, p.status);
@@ -579,13 +582,13 @@ delta_prep_bwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
       if (ok) {
         tc_fence_after();
 #pragma unroll
-        for (int j = 0; j < 4; ++j) umma_f16(tmem + 128, k64(tmp, j), mn(kt, j), id_kn, 1);
+        for (int j = 0; j < 4; ++j) umma_f16_lo(tmem + 128, kk(TMP, j), mn(KTB, j), id_kn, 1);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) umma_f16(tmem + 128, mn(tmp, j), mn(kt, j), id_mm, 1);
+        for (int j = 0; j < 4; ++j) umma_f16_lo(tmem + 128, mn(TMP, j), mn(KTB, j), id_mm, 1);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) umma_f16(tmem + 128, mn(dm, j), mn(vq, j), id_mm, 1);
+        for (int j = 0; j < 4; ++j) umma_f16_lo(tmem + 128, mn(DM, j), mn(VQ, j), id_mm, 1);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) umma_f16(tmem + 0, k64(dm, j), mn(kt, j), id_kn, j > 0);
+        for (int j = 0; j < 4; ++j) umma_f16_lo(tmem + 0, kk(DM, j), mn(KTB, j), id_kn, j > 0);
         umma_commit(&mma[3]);
       }
       tma_store_wait_read<0>();   // dV has left the tile dK is staged in

@@ -20,7 +20,7 @@
 // quarter, 64 columns each); the state update is issued before the output product and has its own
 // barrier; the output accumulator is double-buffered, so chunk n's output rows are staged while
 // chunk n + 1's Y product runs; the part of the backward's Y that does not need the state is issued
-// before the state image is ready. 64 sequences of 64 chunks: forward 115 us (1.8 us a chunk), backward 102 us;
+// before the state image is ready. 64 sequences of 64 chunks: forward 113 us (1.8 us a chunk), backward 101 us;
 // four row warps that did all of it in order, in one CTA a sequence, took 230 and 133 us.
 //
 // The columns of the state never mix (U, O and dU have the same columns), so when the sequences or
@@ -221,11 +221,14 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     if (lane == 0) {
       const uint32_t id_kn = make_idesc(1, 1, 128, S::CC, 0, 1);  // A K-major, B MN-major
       const uint32_t id_nn = make_idesc(1, 1, 128, S::CC, 1, 1);  // A MN-major, B MN-major
-      const uint32_t xb_a = smem_u32(xb), ub_a = smem_u32(ub);
+      // descriptor words made once: an issue is one add for each operand
+      const uint32_t xb_mn = sdesc_lo(smem_u32(xb), 16384), ub_mn = sdesc_lo(smem_u32(ub), 8192);
+      const uint32_t st_k = sdesc_lo(smem_u32(smem), 16), st_mn = sdesc_lo(smem_u32(smem), 8192);
       for (int it = 0; it < N; ++it) {
         const int s = it & 1;
         const uint32_t ph = (it >> 1) & 1, cph = it & 1;
-        const uint32_t st = smem_u32(smem + s * S::STAGE);
+        auto k_major = [&](int tile) { return st_k + ((s * S::STAGE + tile) >> 4); };
+        auto mn_major = [&](int tile) { return st_mn + ((s * S::STAGE + tile) >> 4); };
         const uint32_t col_o = tmem + COL_O + (it & 1) * 128;
         if (!mbar_wait_spin(&full[s], ph, p.status)) break;
         if (BWD) {
@@ -233,8 +236,7 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
           tc_fence_after();
 #pragma unroll
           for (int j = 0; j < 4; ++j)
-            umma_f16(tmem + COL_Y, make_sdesc_sw128(st + TILE_M + j * 2048, 8192, 1024),
-                     make_sdesc_sw128(st + TILE_DO + j * 2048, 8192, 1024), id_nn, j > 0);
+            umma_f16_lo(tmem + COL_Y, step_mn(mn_major(TILE_M), j), step_mn(mn_major(TILE_DO), j), id_nn, j > 0);
         }
         if (!mbar_wait_spin(x_ready, cph, p.status)) break;
         tc_fence_after();
@@ -242,47 +244,37 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
           // Y = W X ; O = Q X
 #pragma unroll
           for (int j = 0; j < 8; ++j)
-            umma_f16(tmem + COL_Y,
-                     make_sdesc_sw128(st + TILE_W + (j >> 2) * 8192 + (j & 3) * 32, 16, 1024),
-                     make_sdesc_sw128(xb_a + j * 2048, 16384, 1024), id_kn, j > 0);
+            umma_f16_lo(tmem + COL_Y, step_k(k_major(TILE_W), j), step_mn(xb_mn, j), id_kn, j > 0);
           umma_commit(y_done);
           if (!sum) {
             // the buffer's previous rows (chunk it - 2) were staged before this x_ready
 #pragma unroll
             for (int j = 0; j < 8; ++j)
-              umma_f16(col_o,
-                       make_sdesc_sw128(st + TILE_Q + (j >> 2) * 8192 + (j & 3) * 32, 16, 1024),
-                       make_sdesc_sw128(xb_a + j * 2048, 16384, 1024), id_kn, j > 0);
+              umma_f16_lo(col_o, step_k(k_major(TILE_Q), j), step_mn(xb_mn, j), id_kn, j > 0);
           }
         } else {
           // Y += K X
 #pragma unroll
           for (int j = 0; j < 8; ++j)
-            umma_f16(tmem + COL_Y,
-                     make_sdesc_sw128(st + TILE_K + (j >> 2) * 8192 + (j & 3) * 32, 16, 1024),
-                     make_sdesc_sw128(xb_a + j * 2048, 16384, 1024), id_kn, 1);
+            umma_f16_lo(tmem + COL_Y, step_k(k_major(TILE_K), j), step_mn(xb_mn, j), id_kn, 1);
           umma_commit(y_done);
           // X += Q^T dO   (independent of dU: keeps the tensor core busy meanwhile)
 #pragma unroll
           for (int j = 0; j < 4; ++j)
-            umma_f16(tmem + COL_X, make_sdesc_sw128(st + TILE_Q + j * 2048, 8192, 1024),
-                     make_sdesc_sw128(st + TILE_DO + j * 2048, 8192, 1024), id_nn, 1);
+            umma_f16_lo(tmem + COL_X, step_mn(mn_major(TILE_Q), j), step_mn(mn_major(TILE_DO), j), id_nn, 1);
         }
         if (!mbar_wait_spin(u_ready, cph, p.status)) break;
         tc_fence_after();
         // X += K^T U  (forward), X += W^T (-dU)  (backward): what the next chunk waits for
-        const uint32_t a_t = st + (BWD ? TILE_W : TILE_K);
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-          umma_f16(tmem + COL_X, make_sdesc_sw128(a_t + j * 2048, 8192, 1024),
-                   make_sdesc_sw128(ub_a + j * 2048, 8192, 1024), id_nn, 1);
+          umma_f16_lo(tmem + COL_X, step_mn(mn_major(BWD ? TILE_W : TILE_K), j), step_mn(ub_mn, j), id_nn, 1);
         umma_commit(x_done);
         if (!BWD && !sum) {
           // O += M U
 #pragma unroll
           for (int j = 0; j < 4; ++j)
-            umma_f16(col_o, make_sdesc_sw128(st + TILE_M + j * 32, 16, 1024),
-                     make_sdesc_sw128(ub_a + j * 2048, 8192, 1024), id_kn, 1);
+            umma_f16_lo(col_o, step_k(k_major(TILE_M), j), step_mn(ub_mn, j), id_kn, 1);
           umma_commit(o_done);
         }
         umma_commit(&empty[s]);
@@ -371,11 +363,6 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
       const uint32_t cph = it & 1;
       const int g = seq * NT + n;
       if (it > 0) wait(x_done, cph ^ 1);
-      // all earlier bulk stores have finished reading xb / ub / ob before they are rewritten
-      if (!sum) {
-        if (r == 0 && ch == 0) tma_store_wait_read<0>();
-        sync_rows();
-      }
       // bf16 image of the state entering this chunk
       {
         uint32_t v[WC];
@@ -394,6 +381,7 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
         }
       }
       if (!sum) {
+        if (r == 0 && ch == 0) tma_store_wait_read<0>();   // U of the previous chunk has left ub
         sync_rows();
         if (r == 0 && ch == 0) {
           if (!BWD && it > 0) {
@@ -409,10 +397,17 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
         }
       }
       if (tok_warp) {
+        uint8_t* ut = smem + (it & 1) * S::STAGE + TILE_DO;
+        constexpr bool EARLY = !BWD && !S::BOTH;   // two chains have no registers for it
+        bf16x8 uh[EARLY ? WC / 8 : 1];             // this lane's U^, read while Y is computed
+        if (EARLY && !lin) {
+          wait(&full[it & 1], (it >> 1) & 1);
+#pragma unroll
+          for (int i = 0; i < WC / 8; ++i) uh[EARLY ? i : 0] = *reinterpret_cast<const bf16x8*>(piece(ut, C, i));
+        }
         wait(y_done, cph);
         uint32_t v[WC];
         load_cols(COL_Y, v);
-        uint8_t* uh = smem + (it & 1) * S::STAGE + TILE_DO;
 #pragma unroll
         for (int i = 0; i < WC / 8; ++i) {
           float y[8];
@@ -420,7 +415,7 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
           for (int j = 0; j < 8; ++j) y[j] = __uint_as_float(v[8 * i + j]);
           if (!BWD && !lin) {
             float uhv[8];
-            unpack8(*reinterpret_cast<const bf16x8*>(piece(uh, C, i)), uhv);
+            unpack8(EARLY ? uh[EARLY ? i : 0] : *reinterpret_cast<const bf16x8*>(piece(ut, C, i)), uhv);
 #pragma unroll
             for (int j = 0; j < 8; ++j) y[j] = uhv[j] - y[j];  // U = U^ - W S
           } else {
@@ -438,6 +433,13 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
             tma_store_commit();
           }
         }
+      }
+      if (!sum) {   // while the state is updated: the bulk stores before U's have read xb and ob, which are rewritten next
+        if (r == 0 && ch == 0) {
+          if (store_ux) tma_store_wait_read<1>();
+          else tma_store_wait_read<0>();
+        }
+        sync_rows();
       }
     }
     // drain: last chunk's output rows and the final state
