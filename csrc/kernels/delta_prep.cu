@@ -8,14 +8,15 @@
 //
 // K, Q and V are read by TMA straight out of the projection outputs ([batch * seq,
 // heads * 128], no per-chunk copies); G and Q K^T are two tcgen05.mma products with their
-// accumulators in tensor memory; the unit-lower-triangular inverse is an fp32 forward
-// substitution with one column per thread (operand rows broadcast from shared memory as
-// 16-byte loads); A' goes back to shared memory as a 128-byte-swizzled bf16 operand for
+// accumulators in tensor memory; the unit-lower-triangular inverse is taken in fp32 by blocks (invert_unit_lower);
+// A' goes back to shared memory as a 128-byte-swizzled bf16 operand for
 // the two products W and U^; every result leaves by a TMA store. A chunk is one long chain of
 // waits in two warps, so what counts is how many chunks an SM has in flight: four CTAs of 64
-// threads, 49 KB and 128 tensor-memory columns each. V takes the place of the fp32 A once the
-// substitution has read it, A' that of M once M is stored, and U^ W's columns once W is in registers.
-// 4096 chunks: two CTAs with room for everything 165 us, three 141 us, four 129 us.
+// threads, 49 KB and 128 tensor-memory columns each. V takes the place of the fp32 T once it is
+// in registers, A' that of M once M is stored, U^ W's columns once W is in registers, and the next chunk's K and Q
+// arrive while U^ is converted and stored.
+// 4096 chunks: two CTAs with room for everything 165 us, three 141 us, four 129 us; with the inverse by blocks and
+// the early loads 89 us (4.8 TB/s).
 //
 // Sequences need not be a multiple of 64 tokens: the token tensors are mapped per batch entry, so the
 // rows the last chunk lacks load as zeros and are clipped from the stores; their beta counts as 0.
@@ -23,8 +24,6 @@
 // Reference semantics: kernels/__init__.py:357-376 of the reference (per-token delta-rule
 // recurrence); the chunked WY algebra and this kernel are this library's own.
 #include <cuda.h>
-
-#include <type_traits>
 
 #include "common.cuh"
 
@@ -78,6 +77,92 @@ __device__ __forceinline__ void row_to_tile(uint32_t taddr, uint8_t* tile, int r
   }
 }
 
+// The fp32 matrix that is inverted: 64 rows of 16 pieces of 16 bytes, piece p of row i at p ^ (i & 15).
+struct Square {
+  float4* base;
+  __device__ __forceinline__ float4& operator()(int row, int piece) const { return base[row * 16 + (piece ^ (row & 15))]; }
+};
+__device__ __forceinline__ void axpy(float4& acc, float a, const float4& b) {
+  acc.x = fmaf(a, b.x, acc.x); acc.y = fmaf(a, b.y, acc.y);
+  acc.z = fmaf(a, b.z, acc.z); acc.w = fmaf(a, b.w, acc.w);
+}
+// acc (R rows x 4 columns) = sum over k = 4 k_lo .. 4 k_hi - 1 of L(l_row + u, k from piece l_piece) R(r_row + k, r_piece)
+template <int R>
+__device__ __forceinline__ void block_mul(const Square m, float4 (&acc)[R], int l_row, int l_piece, int r_row,
+                                          int r_piece, int k_lo, int k_hi) {
+#pragma unroll
+  for (int u = 0; u < R; ++u) acc[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
+  for (int k4 = k_lo; k4 < k_hi; ++k4) {
+    float4 a[R], b[4];
+#pragma unroll
+    for (int u = 0; u < R; ++u) a[u] = m(l_row + u, l_piece + k4);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) b[j] = m(r_row + 4 * k4 + j, r_piece);
+#pragma unroll
+    for (int u = 0; u < R; ++u) {
+      axpy(acc[u], a[u].x, b[0]); axpy(acc[u], a[u].y, b[1]);
+      axpy(acc[u], a[u].z, b[2]); axpy(acc[u], a[u].w, b[3]);
+    }
+  }
+}
+// In place, 64 threads: the strictly lower A becomes T = (I + A)^-1. The 16 x 16 blocks on the diagonal by forward
+// substitution, a column to a thread, then twice T21 = -T22 (A21 T11), a few rows and columns to a thread. What bounds
+// it is the shared-memory port, 32 values a cycle whoever reads them: a substitution over all 64 rows, where a value
+// serves one column a lane, takes 2752 cycles of it a chunk (for 1008 of multiply-adds), the blocks 1650.
+__device__ __forceinline__ void invert_unit_lower(const Square m, int tid) {
+  const int warp = tid >> 5, lane = tid & 31;
+  {
+    const int blk = tid >> 4, c = tid & 15;
+    float t[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      float a0 = (i == c) ? 1.f : 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
+#pragma unroll
+      for (int q = 0; q < (i + 3) / 4; ++q) {
+        const float4 a = m(16 * blk + i, 4 * blk + q);
+        if (4 * q + 0 < i) a0 = fmaf(-a.x, t[4 * q + 0], a0);
+        if (4 * q + 1 < i) a1 = fmaf(-a.y, t[4 * q + 1], a1);
+        if (4 * q + 2 < i) a2 = fmaf(-a.z, t[4 * q + 2], a2);
+        if (4 * q + 3 < i) a3 = fmaf(-a.w, t[4 * q + 3], a3);
+      }
+      t[i] = (a0 + a1) + (a2 + a3);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 16; ++i) reinterpret_cast<float*>(&m(16 * blk + i, 4 * blk + (c >> 2)))[c & 3] = t[i];
+    __syncwarp();
+  }
+  {   // 16 -> 32: a warp has one pair of blocks, a thread two rows and four columns
+    const int row = 32 * warp + 16 + 2 * (lane >> 2), piece = 8 * warp + (lane & 3);
+    float4 x[2];
+    block_mul<2>(m, x, row, 8 * warp, 32 * warp, piece, 0, 4);
+    __syncwarp();
+    m(row, piece) = x[0]; m(row + 1, piece) = x[1];
+    __syncwarp();
+    block_mul<2>(m, x, row, 8 * warp + 4, 32 * warp + 16, piece, 0, 4);
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < 2; ++u) m(row + u, piece) = make_float4(-x[u].x, -x[u].y, -x[u].z, -x[u].w);
+  }
+  __syncthreads();
+  {   // 32 -> 64: four rows and four columns to a thread; the zeros of T11 and T22 are left out by halves
+    float4 x[4];
+    int row = 32 + 4 * (lane >> 2), piece = 4 * warp + (lane & 3);
+    block_mul<4>(m, x, row, 0, 0, piece, 4 * warp, 8);
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 4; ++u) m(row + u, piece) = x[u];
+    __syncthreads();
+    row = 32 + 16 * warp + 4 * (lane >> 3); piece = lane & 7;
+    block_mul<4>(m, x, row, 8, 32, piece, 0, 4 * warp + 4);
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 4; ++u) m(row + u, piece) = make_float4(-x[u].x, -x[u].y, -x[u].z, -x[u].w);
+  }
+  __syncthreads();
+}
+
 __global__ void __launch_bounds__(64, FWD_CTAS)
 delta_prep_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmQ,
                       const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmW,
@@ -95,6 +180,8 @@ delta_prep_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   uint64_t* fullv = bars + 4;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 5);
   float4* af4 = reinterpret_cast<float4*>(smem + VA);
+  __shared__ float4 betas_[C / 4];
+  float* betas = reinterpret_cast<float*>(betas_);
 
   const int r = threadIdx.x, warp = r >> 5;
   if (r == 0) {
@@ -117,20 +204,22 @@ delta_prep_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   const uint32_t k_k = sdesc_lo(smem_u32(smem + KT), 16), q_k = sdesc_lo(smem_u32(smem + QT), 16), ap_k = q_k;
   const uint32_t k_mn = sdesc_lo(smem_u32(smem + KT), 8192), v_mn = sdesc_lo(smem_u32(smem + VA), 8192);
 
+  auto load_kq = [&](int g) {
+    const int seq = g / p.n_chunks, t0 = (g - seq * p.n_chunks) * C;
+    const int b = seq / p.heads, x0 = (seq - b * p.heads) * D;
+    mbar_arrive_expect_tx(full, 2 * 16384);
+    tma_load_3d(smem + KT, &tmK, full, x0, t0, b);
+    tma_load_3d(smem + KT + 8192, &tmK, full, x0 + 64, t0, b);
+    tma_load_3d(smem + QT, &tmQ, full, x0, t0, b);
+    tma_load_3d(smem + QT + 8192, &tmQ, full, x0 + 64, t0, b);
+  };
+  if (r == 0 && static_cast<int>(blockIdx.x) < p.total) load_kq(blockIdx.x);
   uint32_t ph = 0;
   for (int g = blockIdx.x; g < p.total; g += gridDim.x, ph ^= 1) {
     const int seq = g / p.n_chunks, n = g - seq * p.n_chunks;
     const int b = seq / p.heads, h = seq - b * p.heads;
     const int t0 = n * C;                     // first token of the chunk
     const int x0 = h * D;
-    if (r == 0) {
-      tma_store_wait_read<0>();  // earlier stores have drained the tiles about to be refilled
-      mbar_arrive_expect_tx(full, 2 * 16384);
-      tma_load_3d(smem + KT, &tmK, full, x0, t0, b);
-      tma_load_3d(smem + KT + 8192, &tmK, full, x0 + 64, t0, b);
-      tma_load_3d(smem + QT, &tmQ, full, x0, t0, b);
-      tma_load_3d(smem + QT + 8192, &tmQ, full, x0 + 64, t0, b);
-    }
     float beta = 0.f;
     if (t0 + r < p.seq_len) {
       const size_t bidx = (static_cast<size_t>(b) * p.seq_len + t0 + r) * p.heads + h;
@@ -152,10 +241,12 @@ delta_prep_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
       }
     }
     ok = mbar_wait_spin(mma1, ph, p.status) && ok;
+    if (r == 0) tma_store_wait_read<0>();   // the previous chunk's U^ has left the tile that A goes into
     if (!__syncthreads_and(ok)) break;
     tc_fence_after();
 
-    // A = diag(beta) tril(G, -1), fp32, rows in 16-byte pieces at position (piece ^ (row & 15))
+    betas[r] = beta;
+    // A = diag(beta) tril(G, -1), fp32
 #pragma unroll 1
     for (int c = 0; c < 64; c += 32) {
       uint32_t v[32];
@@ -168,7 +259,7 @@ delta_prep_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
         a.y = (c + 4 * i + 1 < r) ? beta * __uint_as_float(v[4 * i + 1]) : 0.f;
         a.z = (c + 4 * i + 2 < r) ? beta * __uint_as_float(v[4 * i + 2]) : 0.f;
         a.w = (c + 4 * i + 3 < r) ? beta * __uint_as_float(v[4 * i + 3]) : 0.f;
-        af4[r * 16 + (((c >> 2) + i) ^ (r & 15))] = a;
+        Square{af4}(r, (c >> 2) + i) = a;
       }
     }
     // M = tril(Q K^T) -> the Q tile's first half (the products that read Q are complete)
@@ -180,31 +271,11 @@ delta_prep_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
       tma_store_commit();
     }
 
-    // Column r of T = (I + A)^-1 by forward substitution. Every value of A that a warp reads costs a cycle of the SM's
-    // one shared-memory port, as many for the substitution as four schedulers need for its multiply-adds in four times
-    // the cycles; so the second warp, whose columns are zero down to row 32, leaves that half out.
-    float t[64];
-    auto substitute = [&](auto FIRST) {
-      constexpr int i0 = decltype(FIRST)::value;
+    invert_unit_lower(Square{af4}, r);
+    float4 t[16];   // row r of T
 #pragma unroll
-      for (int i = 0; i < i0; ++i) t[i] = 0.f;
-#pragma unroll
-      for (int i = i0; i < 64; ++i) {
-        float a0 = (i == r) ? 1.f : 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-#pragma unroll
-        for (int c = i0 / 4; c < (i + 3) / 4; ++c) {
-          const float4 a = af4[i * 16 + (c ^ (i & 15))];
-          if (4 * c + 0 < i) a0 = fmaf(-a.x, t[4 * c + 0], a0);
-          if (4 * c + 1 < i) a1 = fmaf(-a.y, t[4 * c + 1], a1);
-          if (4 * c + 2 < i) a2 = fmaf(-a.z, t[4 * c + 2], a2);
-          if (4 * c + 3 < i) a3 = fmaf(-a.w, t[4 * c + 3], a3);
-        }
-        t[i] = (a0 + a1) + (a2 + a3);
-      }
-    };
-    if (warp == 0) substitute(std::integral_constant<int, 0>{});
-    else substitute(std::integral_constant<int, 32>{});
-    // A has been read and M has left: V comes into A's place, A' goes into M's
+    for (int q = 0; q < 16; ++q) t[q] = Square{af4}(r, q);
+    // T is in registers and M has left: V comes into T's place, A' goes into M's
     if (r == 0) tma_store_wait_read<0>();
     fence_proxy_async_smem();
     __syncthreads();
@@ -213,19 +284,16 @@ delta_prep_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
       tma_load_3d(smem + VA, &tmV, fullv, x0, t0, b);
       tma_load_3d(smem + VA + 8192, &tmV, fullv, x0 + 64, t0, b);
     }
-    // T -> the Q tile's second half, A' = T diag(beta) -> its first (element (i, r) each)
-    {
-      uint8_t* tt = smem + QT + 8192;
-      uint8_t* at = smem + QT;
-      const int sub = (r & 7) * 2, c16 = r >> 3;
+    // T -> the Q tile's second half, A' = T diag(beta) -> its first
 #pragma unroll
-      for (int i = 0; i < 64; ++i)
-        *reinterpret_cast<bf16*>(at + i * 128 + ((c16 ^ (i & 7)) << 4) + sub) = f32_to_bf16(t[i] * beta);
-      if (p.store_ta) {
-#pragma unroll
-        for (int i = 0; i < 64; ++i)
-          *reinterpret_cast<bf16*>(tt + i * 128 + ((c16 ^ (i & 7)) << 4) + sub) = f32_to_bf16(t[i]);
-      }
+    for (int q = 0; q < 8; ++q) {
+      const float4 lo = t[2 * q], hi = t[2 * q + 1];
+      const float4 bl = reinterpret_cast<const float4*>(betas)[2 * q], bh = reinterpret_cast<const float4*>(betas)[2 * q + 1];
+      const float ta[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+      const float aa[8] = {lo.x * bl.x, lo.y * bl.y, lo.z * bl.z, lo.w * bl.w,
+                           hi.x * bh.x, hi.y * bh.y, hi.z * bh.z, hi.w * bh.w};
+      st_swz(smem + QT, r, q, pack8(aa));
+      if (p.store_ta) st_swz(smem + QT + 8192, r, q, pack8(ta));
     }
     fence_proxy_async_smem();
     tc_fence_before();
@@ -264,6 +332,11 @@ delta_prep_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     ok = mbar_wait_spin(mma3, ph, p.status) && ok;
     if (!__syncthreads_and(ok)) break;
     tc_fence_after();
+    if (r == 0 && g + static_cast<int>(gridDim.x) < p.total) {
+      // nothing reads K, W, A' or T any more: the next chunk's K and Q arrive while U^ is converted and stored
+      tma_store_wait_read<0>();
+      load_kq(g + gridDim.x);
+    }
     // U^ -> V tile
     row_to_tile(lane_addr + 0, smem + VA, r, 63);
     row_to_tile(lane_addr + 64, smem + VA + 8192, r, 63);

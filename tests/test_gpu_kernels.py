@@ -814,6 +814,37 @@ def test_delta_compose(n_seq, n_seg, reverse):
             assert (p_tot.double() - tot).norm() <= 1e-5 * tot.norm()
 
 
+@pytest.mark.parametrize("S,close", [(1, False), (16, True), (17, True), (33, True), (64, True), (100, False), (640, True)])
+def test_delta_chunk_inverse(S, close):
+    """T = (I + diag(beta) tril(K K^T, -1))^-1 of every chunk, block by block, against float64. ``close``: keys that
+    nearly agree, so that A is far from small. An inverse taken from the blocks' products in fp32 is off by at most
+    n u |T| |I + A| |T| elementwise in each product, and T is then rounded to bf16."""
+    from prometheus_b200.ops._lib import call, ptr, stream_ptr
+    from prometheus_b200.ops.functional import status_word
+
+    B, H, n = 2, 3, -(-S // 64)
+    k = _r(B, S, H, 128, seed=S) + (4.0 * _r(B, 1, H, 128, seed=1) if close else 0)
+    k = torch.nn.functional.normalize(k.float(), dim=-1).to(BF16).contiguous()
+    beta = torch.sigmoid(_r(B, S, H, seed=2, dtype=torch.float32) + 1.0)
+    q, v = _r(B, S, H, 128, seed=3), _r(B, S, H, 128, seed=4)
+    g = B * H * n
+    w, u = (torch.empty(g, 64, 128, dtype=BF16, device="cuda") for _ in range(2))
+    m, ap, t = (torch.empty(g, 64, 64, dtype=BF16, device="cuda") for _ in range(3))
+    call("pb_delta_prep_fwd", ptr(q), ptr(k), ptr(v), ptr(beta), 1, ptr(w), ptr(u), ptr(m), ptr(ap), ptr(t), B, S, H,
+         H * 128, ptr(status_word(k.device)), 0, stream_ptr())
+    pad = n * 64 - S
+    kc = torch.nn.functional.pad(k, (0, 0, 0, 0, 0, pad)).reshape(B, n, 64, H, 128).permute(0, 3, 1, 2, 4).double()
+    bc = torch.nn.functional.pad(beta, (0, 0, 0, pad)).reshape(B, n, 64, H).permute(0, 3, 1, 2).double()
+    a = torch.tril(bc[..., None] * (kc @ kc.transpose(-1, -2)), -1).reshape(g, 64, 64)
+    ia = torch.eye(64, dtype=torch.float64, device="cuda") + a
+    ref = torch.linalg.inv(ia)
+    slack = 2 * 64 * 2.0 ** -24 * (ref.abs() @ ia.abs() @ ref.abs()) + 2.0 ** -133
+    err = (t.double() - ref).abs()
+    assert bool((err <= 2.0 ** -8 * ref.abs() + 2 * slack).all()), (err - 2.0 ** -8 * ref.abs() - 2 * slack).max().item()
+    err = (ap.double() - ref * bc.reshape(g, 1, 64)).abs()
+    assert bool((err <= 2.0 ** -8 * ref.abs() + 2 * slack).all())
+
+
 def test_delta_prep_bwd_kernel_matches_fp32_oracle():
     """The fused chunk-local backward against the same algebra in batched fp32 PyTorch."""
     from prometheus_b200.ops import delta as dl
