@@ -7,7 +7,8 @@
 // 128 x 128 block. Exactly the arithmetic of quantise -> dequantise -> fp32 matmul, with the
 // dequantisation applied to the 128-deep partial products instead of to the operands.
 //
-// One CTA per SM, persistent over 128 x 256 output tiles:
+// Two kernels: on CTA pairs (gemm_fp8_pair_kernel below) and on single CTAs, for small or finely grouped products and
+// for rows that are still arriving. The latter, one CTA per SM, persistent over 128 x 256 output tiles:
 //   warp 0   TMA producer: per K-block a 128 x 128 B tile of A and a 256 x 128 B tile of B
 //            (128 bytes per row = one swizzle atom), 4-stage ring
 //   warp 1   MMA issuer: four kind::f8f6f4 MMAs (M 128, N 256, K 32) per K-block into one of
@@ -301,6 +302,228 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     for (int i = 0; i < 2000; ++i) __nanosleep(1000);   // let copies in flight land
     __syncthreads();
   }
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 2 * BN);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// CTA-pair variant: a cluster of two CTAs computes a 256 x 256 tile with tcgen05.mma.cta_group::2, each loading its 128
+// rows of A and 128 of the tile's 256 rows of B. A K-block of the single-CTA tile writes 48 KB to shared memory and
+// reads them once, 768 clocks of it against 524 of tensor core; the pair's writes and reads 32 KB.
+// Bound by the promotion and by handing the accumulators over (about 1090 clocks a K-block). Sixteen promotion warps,
+// 64 columns each, so that a scheduler has four of them to hide tensor-memory reads, multiply-adds and waits behind one
+// another, with what that takes: 104 registers (at 96, spilled, 8192^3 takes 616 us), eight columns read at a
+// time (sixteen: 569 us), scales multiplied when they are used (as soon as they are asked for: 719 us), one arrival a
+// warp with the scope of its CTA (released to the cluster 1228 us; what is handed over is tensor memory, which
+// tcgen05.fence orders). Single-CTA / pair: 8192^3 705 / 555 us, 16384 x 2816 x 2048 154 / 124, 16384 x 2048 x 1408
+// 86 / 70, 5000 x 2816 x 2048 56 / 48, 129 x 2816 x 2048 23.5 / 21.5.
+// Row blocks of a pair may belong to two groups: then the pair makes two passes, one for each group's B, and in each the
+// CTA whose rows are not of that group drops its half (at most once a group).
+// Same arithmetic as the single-CTA kernel, bit for bit.
+// ---------------------------------------------------------------------------
+constexpr int P_STAGES = 5, P_OP = 128 * BK, P_STAGE = 2 * P_OP;      // A and B: 128 rows of 128 bytes each
+constexpr int P_WARPS = 16, P_COLS = 64, P_THREADS = (4 + P_WARPS) * 32;   // warps 0 loads, 1 MMA, 2 and 3 idle
+constexpr int P_EPI = P_STAGES * P_STAGE, P_BARS = P_EPI + P_WARPS * 4096, P_SMEM = P_BARS + 256 + 1024;
+static_assert(P_SMEM <= 227 * 1024, "one CTA's shared memory");
+
+__device__ __forceinline__ void umma_f8_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                             uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+__global__ void __launch_bounds__(P_THREADS, 1)
+gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                     const __grid_constant__ CUtensorMap tmC, const Params p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>(
+      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + P_BARS);
+  uint64_t* full = bars;                    // [P_STAGES], the even CTA's
+  uint64_t* empty = bars + P_STAGES;        // [P_STAGES], both
+  uint64_t* tfull = bars + 2 * P_STAGES;    // [2], both
+  uint64_t* tempty = tfull + 2;             // [2], the even CTA's
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = static_cast<int>(cluster_ctarank());   // 0: even CTA (issues the MMAs)
+  const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
+  const int num_m = (p.M + 255) / 256, num_n = (p.N + BN - 1) / BN;
+  const int nkb = p.K / BK;
+  const int total = num_m * num_n;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < P_STAGES; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(&tfull[a], 1);
+      mbar_init(&tempty[a], 2 * P_WARPS);
+    }
+    fence_barrier_init();
+    tma_prefetch_desc(&tmA);
+    tma_prefetch_desc(&tmB);
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, 2 * BN);   // all columns: one address serves both CTAs
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  cluster_sync_all();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  // column-major inside groups of 8 pair rows: B tiles stay in L2
+  auto coords = [&](int r, int& m_pair, int& n_blk) {
+    const int first = (r / (8 * num_n)) * 8;
+    const int gsz = min(num_m - first, 8);
+    m_pair = first + (r % (8 * num_n)) % gsz;
+    n_blk = (r % (8 * num_n)) / gsz;
+  };
+  const int n_blocks = (p.M + BM - 1) / BM;
+  auto group_of = [&](int blk) { return p.mblk_group == nullptr ? 0 : blk < n_blocks ? p.mblk_group[blk] : -1; };
+  // the groups whose B a pair of row blocks needs, in order, and this CTA's own (negative: padding)
+  struct Passes {
+    int first, second, n, own;
+    __device__ int operator[](int i) const { return i == 0 ? first : second; }
+  };
+  auto passes = [&](int m_pair) {
+    const int g0 = group_of(2 * m_pair), g1 = group_of(2 * m_pair + 1);
+    Passes q;
+    q.own = rank == 0 ? g0 : g1;
+    q.first = g0 >= 0 ? g0 : g1;
+    q.second = g1;
+    q.n = (g0 >= 0 ? 1 : 0) + (g1 >= 0 && g1 != g0 ? 1 : 0);
+    return q;
+  };
+
+  // 640 threads start with 96 registers: 128 x 56 + 512 x 104 are fewer than those 61440
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    if (warp == 0 && lane == 0) {
+      int s = 0;
+      uint32_t ph = 0;
+      bool ok = true;
+      for (int t = pair; t < total && ok; t += n_pairs) {
+        int m_pair, n_blk;
+        coords(t, m_pair, n_blk);
+        const Passes q = passes(m_pair);
+        const int m_blk = 2 * m_pair + rank;
+        for (int i = 0; i < q.n && ok; ++i)
+          for (int kb = 0; kb < nkb; ++kb) {
+            if (!mbar_wait(&empty[s], ph ^ 1, p.status)) { ok = false; break; }
+            if (rank == 0) mbar_arrive_expect_tx(&full[s], 2 * P_STAGE);
+            const uint32_t bar = cluster_map(smem_u32(&full[s]), 0);
+            uint8_t* st = smem + s * P_STAGE;
+            tma_load_3d_pair(st, &tmA, bar, kb * BK, m_blk * BM, 0);
+            tma_load_3d_pair(st + P_OP, &tmB, bar, kb * BK, n_blk * BN + rank * 128, q[i]);
+            if (++s == P_STAGES) { s = 0; ph ^= 1; }
+          }
+      }
+    }
+    if (warp == 1 && lane == 0 && rank == 0) {
+      const uint32_t idesc = make_idesc(0, 0, 256, BN, 0, 0);   // e4m3 x e4m3, both K-major
+      constexpr uint64_t HI = static_cast<uint64_t>(sdesc_hi_sw128(1024)) << 32;
+      const uint32_t lo0 = sdesc_lo(smem_u32(smem), 16);
+      int s = 0;
+      uint32_t ph = 0, it = 0;   // it: K-blocks issued so far, picks the accumulator and its phase
+      bool ok = true;
+      for (int t = pair; t < total && ok; t += n_pairs) {
+        int m_pair, n_blk;
+        coords(t, m_pair, n_blk);
+        const Passes q = passes(m_pair);
+        for (int kb = 0; kb < q.n * nkb; ++kb, ++it) {
+          const int acc = it & 1;
+          if (!mbar_wait_spin(&tempty[acc], ((it >> 1) & 1) ^ 1, p.status) ||
+              !mbar_wait_spin(&full[s], ph, p.status)) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t a_lo = lo0 + s * (P_STAGE >> 4), b_lo = a_lo + (P_OP >> 4);
+#pragma unroll
+          for (int j = 0; j < BK / 32; ++j)
+            umma_f8_pair(tmem_base + acc * BN, HI | (a_lo + 2 * j), HI | (b_lo + 2 * j), idesc, j > 0 ? 1u : 0u);
+          umma_commit_pair(&empty[s], 3);
+          umma_commit_pair(&tfull[acc], 3);
+          if (++s == P_STAGES) { s = 0; ph ^= 1; }
+        }
+      }
+    }
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+    const int q4 = warp & 3, cg = (warp - 4) >> 2;   // tensor-memory lane quarter, 64-column group
+    const int n_sb_rows = (p.N + HALF - 1) / HALF;
+    const uint32_t tempty0 = cluster_map(smem_u32(&tempty[0]), 0);
+    uint8_t* buf = smem + P_EPI + (warp - 4) * 4096;
+    uint32_t it = 0;
+    bool ok = true;
+    for (int t = pair; t < total && ok; t += n_pairs) {
+      int m_pair, n_blk;
+      coords(t, m_pair, n_blk);
+      const Passes q = passes(m_pair);
+      const int y0 = (2 * m_pair + rank) * BM + q4 * 32;
+      const float* sa_row = p.sa + min(y0 + lane, p.M - 1);
+      for (int i = 0; i < q.n && ok; ++i) {
+        const bool mine = q[i] == q.own;
+        const float* sb = p.sb + (static_cast<size_t>(q[i]) * n_sb_rows + min(n_blk * 2 + (cg >> 1), n_sb_rows - 1)) * nkb;
+        float acc[P_COLS];
+#pragma unroll
+        for (int c = 0; c < P_COLS; ++c) acc[c] = 0.f;
+        float sa_next = 0.f, sb_next = 0.f;   // scales, one K-block ahead
+        if (mine) { sa_next = __ldcg(sa_row); sb_next = __ldg(sb); }
+        for (int kb = 0; kb < nkb; ++kb, ++it) {
+          const int a = it & 1;
+          if (!mbar_wait_warp(&tfull[a], (it >> 1) & 1, p.status)) { ok = false; break; }
+          tc_fence_after();
+          if (mine) {
+            const float scale = sa_next * sb_next;
+            if (kb + 1 < nkb) {
+              sa_next = __ldcg(sa_row + static_cast<size_t>(kb + 1) * p.M);
+              sb_next = __ldg(sb + kb + 1);
+            }
+            const uint32_t t_addr = tmem_base + a * BN + cg * P_COLS + (static_cast<uint32_t>(q4 * 32) << 16);
+#pragma unroll
+            for (int c = 0; c < P_COLS; c += 8) {
+              uint32_t v[8];
+              tmem_ld_32x32b_x8(t_addr + c, v);
+              tmem_ld_wait();
+#pragma unroll
+              for (int e = 0; e < 8; e += 2) fma2(acc[c + e], acc[c + e + 1], scale, v[e], v[e + 1]);
+            }
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0)
+            asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(tempty0 + a * 8) : "memory");
+        }
+        if (!ok || !mine) continue;
+        if (lane == 0) tma_store_wait_read<0>();
+        __syncwarp();
+        uint8_t* rowp = buf + lane * 128;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) *reinterpret_cast<bf16x8*>(rowp + ((c ^ (lane & 7)) << 4)) = pack8(acc + 8 * c);
+        fence_proxy_async_smem();
+        __syncwarp();
+        const int x0 = n_blk * BN + cg * P_COLS;
+        if (lane == 0 && x0 < p.N && y0 < p.M) tma_store_3d(&tmC, buf, x0, y0, 0);
+        if (lane == 0) tma_store_commit();
+      }
+    }
+    if (lane == 0) tma_store_wait<0>();
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != PB_OK) {
+    for (int i = 0; i < 2000; ++i) __nanosleep(1000);   // let copies in flight land
+  }
+  // neither CTA leaves while its peer may still signal its barriers or read its operands
+  cluster_sync_all();
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 2 * BN);
@@ -620,6 +843,49 @@ PB_API int pb_fp8_fakequant_blocks(const void* w, long ld, int rows, int K, void
   return static_cast<int>(cudaGetLastError());
 }
 
+namespace pb {
+namespace f8 {
+// Whether a product runs on CTA pairs. Ungrouped they are the faster way at every size beyond one tile of the other
+// kernel, equal within a microsecond where the contraction is 512 or less (above, and 1000 x 2816 x 2048 24.6 / 23.5 us,
+// 4096 x 2048 x 1408 31.8 / 27.6, 1024 x 1024 x 512 13.4 / 14.4, 4096 x 512 x 256 13.2 / 13.2). With groups, every
+// second group boundary costs a pass of which half is dropped; single / pair at row blocks a group, N = 2816,
+// K = 2048: 3.9 blocks 290 / 309 us, 6.2 133 / 135, 8.2 584 / 534, 16 159 / 136. Rows that peers are still
+// storing, and limited grids, stay on one CTA.
+static bool takes_pairs(int M, int N, int groups, const Params& p, int max_ctas) {
+  return M > BM && N > HALF && (max_ctas <= 0 || max_ctas >= num_sms()) && p.blk_arrived == nullptr &&
+         (p.mblk_group == nullptr || (M + BM - 1) / BM >= 8L * groups);
+}
+static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const Params& p,
+                       cudaStream_t st) {
+  static pb::DeviceOnce attr_once;   // per device: the attribute belongs to the current GPU
+  static int max_pairs = 0;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  cfg.blockDim = dim3(P_THREADS, 1, 1);
+  cfg.dynamicSmemBytes = P_SMEM;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (attr_once.need()) {
+    cudaError_t e = cudaFuncSetAttribute(gemm_fp8_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    cfg.gridDim = dim3(num_sms() & ~1, 1, 1);
+    int n = 0;
+    e = cudaOccupancyMaxActiveClusters(&n, gemm_fp8_pair_kernel, &cfg);
+    if (e != cudaSuccess) { cudaGetLastError(); n = num_sms() / 2; }
+    max_pairs = n > 0 && n < num_sms() / 2 ? n : num_sms() / 2;
+    attr_once.done();
+  }
+  const long tiles = static_cast<long>((p.M + 255) / 256) * ((p.N + BN - 1) / BN);
+  cfg.gridDim = dim3(static_cast<unsigned>(2 * (tiles < max_pairs ? tiles : max_pairs)), 1, 1);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_fp8_pair_kernel, tmA, tmB, tmC, p);
+  return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
+}
+}  // namespace f8
+}  // namespace pb
+
 // C [M, N] bf16 = block-scaled Aq [M, K] x Bq [groups, N, K]^T. K % 128 == 0, N % 8 == 0.
 // sa [K / 128, M]; sb [groups, ceil(N / 128), K / 128]; mblk_group null (groups == 1) or one
 // int per 128-row block of A / C.
@@ -692,18 +958,20 @@ static int gemm_fp8_launch(const void* Aq, const float* sa, const void* Bq, cons
     if (e != cudaSuccess) return static_cast<int>(e);
     attr_once.done();
   }
-  CUtensorMap tmA, tmB, tmC;
-  int r = make_tmap_3d(&tmA, Aq, 1, K, M, 1, K, 0, BK, BM);
-  if (r != 0) return 1000 + r;
-  r = make_tmap_3d(&tmB, Bq, 1, K, N, groups, K, static_cast<uint64_t>(N) * K, BK, BN);
-  if (r != 0) return 2000 + r;
-  r = make_tmap_3d(&tmC, C, 2, N, M, 1, ldc, 0, 64, 32);
-  if (r != 0) return 3000 + r;
   Params p;
   p.M = M; p.N = N; p.K = K;
   p.sa = sa; p.sb = sb; p.mblk_group = mblk_group; p.status = status;
   p.blk_arrived = blk_arrived; p.blk_expect = blk_expect;
   p.wait_budget_ns = static_cast<uint64_t>(budget_ns);
+  const bool pair = PROBE == 0 && takes_pairs(M, N, groups, p, max_ctas);
+  CUtensorMap tmA, tmB, tmC;
+  int r = make_tmap_3d(&tmA, Aq, 1, K, M, 1, K, 0, BK, BM);
+  if (r != 0) return 1000 + r;
+  r = make_tmap_3d(&tmB, Bq, 1, K, N, groups, K, static_cast<uint64_t>(N) * K, BK, pair ? 128 : BN);
+  if (r != 0) return 2000 + r;
+  r = make_tmap_3d(&tmC, C, 2, N, M, 1, ldc, 0, 64, 32);
+  if (r != 0) return 3000 + r;
+  if (pair) return launch_pair(tmA, tmB, tmC, p, st);
   const long tiles = static_cast<long>((M + BM - 1) / BM) * ((N + BN - 1) / BN);
   int grid = num_sms();
   if (max_ctas > 0 && max_ctas < grid) grid = max_ctas;

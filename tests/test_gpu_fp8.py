@@ -99,6 +99,41 @@ def test_fp8_gemm_equals_dequantised_matmul(M, N, K):
     assert rel < 0.06, rel
 
 
+@pytest.mark.parametrize("N,K", [(136, 128), (200, 384), (512, 1408)])
+@pytest.mark.parametrize("blocks", [129, 256, 300, 1000, [3, 2, 1, 4], [40, 23, -2, 17], [33, -1, 32, -3], [17, 25, 9, 31]])
+def test_fp8_pair_kernel_equals_single_cta(N, K, blocks):
+    """The CTA-pair product against the single-CTA one, bit for bit: row and column remainders, pairs of row blocks of two
+    groups, of one group and padding (negative counts), padding only. A grid limit selects the single-CTA kernel."""
+    from prometheus_b200.ops import fp8
+    from prometheus_b200.ops import functional as ops
+    from prometheus_b200.ops._lib import call, ptr, stream_ptr
+
+    grouped = isinstance(blocks, list)
+    if grouped:
+        N = -(-N // 128) * 128
+        ids = [g for i, c in enumerate(blocks) for g in [i if c > 0 else -1] * abs(c)]
+        rows, groups = 128 * len(ids), len(blocks)
+        mg = torch.tensor(ids, dtype=torch.int32, device="cuda")
+    else:
+        rows, groups, mg = blocks, 1, None
+    x, w = _r(rows, K, seed=rows), _r(groups * N, K, seed=2, scale=0.05)
+    xq, sx = fp8.quantize_rows(x)
+    wq, sw = fp8.quantize_blocks(w)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    outs = []
+    for limit in (0, sms - 1):
+        c = torch.full((rows, N), 7.0, dtype=BF16, device="cuda")
+        call("pb_gemm_fp8_blockscaled", ptr(xq), ptr(sx), ptr(wq), ptr(sw), ptr(c), rows, N, K, groups, N, ptr(mg),
+             ptr(ops.status_word("cuda")), limit, stream_ptr())
+        outs.append(c)
+    torch.cuda.synchronize()
+    ops.check_status("cuda")
+    assert torch.equal(outs[0], outs[1])
+    if not grouped:
+        ref = fp8.dequantize_rows(xq, sx) @ fp8.dequantize_blocks(wq, sw).t()
+        assert (outs[0].float() - ref).abs().max().item() <= 1e-2 * ref.abs().max().item()
+
+
 def test_fp8_linear_and_grouped_gemm():
     from prometheus_b200 import kernels
     from prometheus_b200.ops import fp8, moe
