@@ -199,6 +199,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  after_previous_kernel();
 
   if (warp == 10) {
     if (lane == 0) {
@@ -511,6 +512,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  after_previous_kernel();
 
   if (warp == 11) {
     if (lane == 0) {
@@ -871,7 +873,7 @@ PB_API int pb_attn_fwd_cp(const void* q, const void* k, const void* v, void* out
   p.lse2 = static_cast<float*>(lse2);
   p.rowmax = static_cast<float*>(rowmax);
   p.status = status;
-  fwd::attn_fwd_kernel<<<static_cast<unsigned>(grid), 352, fwd::SMEM, st>>>(tQ, tK, tV, tO, p);
+  pb::launch(fwd::attn_fwd_kernel, static_cast<unsigned>(grid), 352, fwd::SMEM, st, tQ, tK, tV, tO, p);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -927,7 +929,7 @@ PB_API int pb_attn_bwd_cp(const void* q, const void* k, const void* v, const voi
     r |= tok_map(&tDQ, dq, qi, seq, batch, ldq, 128);
     if (r != 0) return 1000 + r;
     p.n_blk = (seq + 127) / 128;
-    bwd::attn_bwd_kernel<false><<<static_cast<unsigned>(grid_q), 384, bwd::SMEM, st>>>(
+    pb::launch(bwd::attn_bwd_kernel<false>, static_cast<unsigned>(grid_q), 384, bwd::SMEM, st, 
         tQ, tDO, tK, tV, tDQ, tDQ, tO, p);
   }
   {
@@ -941,7 +943,7 @@ PB_API int pb_attn_bwd_cp(const void* q, const void* k, const void* v, const voi
     r |= tok_map(&tDV, dv, ki, seq_kv, batch, ldkv, 128);
     if (r != 0) return 2000 + r;
     p.n_blk = (seq_kv + 127) / 128;
-    bwd::attn_bwd_kernel<true><<<static_cast<unsigned>(grid_kv), 384, bwd::SMEM, st>>>(
+    pb::launch(bwd::attn_bwd_kernel<true>, static_cast<unsigned>(grid_kv), 384, bwd::SMEM, st, 
         tK, tV, tQ, tDO, tDK, tDV, tK, p);
   }
   return static_cast<int>(cudaGetLastError());

@@ -38,6 +38,28 @@ struct DeviceOnce {
   }
 };
 
+// Launch in stream order whose start overlaps the end of the kernel before it (programmatic stream serialisation): the
+// grid is set up while the other one's results are made visible, and its threads wait in after_previous_kernel(),
+// which every kernel launched this way calls before it touches global memory. A launch costs 2 us less on
+// the device: 2048 x 8 x 1024 product 10.4 -> 8.7 us, 1024^3 x 4 16.5 -> 14.6, launches back to back. (Letting the next grid
+// start earlier than at the end of this one gave nothing more.)
+template <typename... Params, typename... Args>
+static inline void launch(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<Args&&>(args)...);   // callers read cudaGetLastError
+}
+// Every kernel before this one in its stream has ended and its writes are visible.
+__device__ __forceinline__ void after_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 typedef __nv_bfloat16 bf16;
 typedef __nv_bfloat162 bf162;
 

@@ -76,6 +76,7 @@ delta_chunk_kernel(const __grid_constant__ CUtensorMap tmNDU, const __grid_const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  after_previous_kernel();
 
   if (warp == 2) {
     if (lane == 0) {
@@ -216,6 +217,6 @@ PB_API int pb_delta_chunk_products(const void* ndU, const void* dO, const void* 
   r |= make_tmap_3d(&tM, dM, 2, C, rows, 1, C, 0, 64, C);
   if (r != 0) return 1000 + r;
   const int grid = p.total < num_sms() ? p.total : num_sms();
-  delta_chunk_kernel<<<grid, THREADS, SMEM, st>>>(tN, tO, tU, tS, tD, tW, tQ, tK, tM, p);
+  pb::launch(delta_chunk_kernel, grid, THREADS, SMEM, st, tN, tO, tU, tS, tD, tW, tQ, tK, tM, p);
   return static_cast<int>(cudaGetLastError());
 }

@@ -197,6 +197,7 @@ delta_prep_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  after_previous_kernel();
   const uint32_t lane_addr = tmem + (static_cast<uint32_t>(warp * 32) << 16);
   const uint32_t id_kk64 = make_idesc(1, 1, 128, 64, 0, 0);    // A, B K-major, N = 64
   const uint32_t id_kn = make_idesc(1, 1, 128, 128, 0, 1);     // A K-major, B MN-major
@@ -472,6 +473,7 @@ delta_prep_bwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  after_previous_kernel();
   const uint32_t lane_addr = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
   const int c32 = half * 32, c64 = half * 64;
   const uint32_t id_kk64 = make_idesc(1, 1, 128, 64, 0, 0);
@@ -749,7 +751,7 @@ PB_API int pb_delta_prep_fwd(const void* q, const void* k, const void* v, const 
   int grid = FWD_CTAS * sms;
   if (max_ctas > 0 && max_ctas < grid) grid = max_ctas;
   if (grid > p.total) grid = p.total;
-  delta_prep_fwd_kernel<<<grid, 64, SMEM_BYTES, st>>>(tK, tQ, tV, tW, tU, tM, tA, tT, p);
+  pb::launch(delta_prep_fwd_kernel, grid, 64, SMEM_BYTES, st, tK, tQ, tV, tW, tU, tM, tA, tT, p);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -805,7 +807,7 @@ PB_API int pb_delta_prep_bwd(const void* q, const void* k, const void* v, const 
   int grid = 2 * sms;
   if (max_ctas > 0 && max_ctas < grid) grid = max_ctas;
   if (grid > p.total) grid = p.total;
-  delta_prep_bwd_kernel<<<grid, bwd::THREADS_BWD, bwd::SMEM_BWD, st>>>(tK, tQ, tV, tDW, tNDU, tDM, tA, tT, tDQ,
+  pb::launch(delta_prep_bwd_kernel, grid, bwd::THREADS_BWD, bwd::SMEM_BWD, st, tK, tQ, tV, tDW, tNDU, tDM, tA, tT, tDQ,
                                                            tDK, tDV, tAQ, tAK, p);
   return static_cast<int>(cudaGetLastError());
 }

@@ -179,6 +179,7 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot + chain * 128;
+  after_previous_kernel();
 
   if (warp == TMA_WARP) {
     // ------------------------------- TMA producer -------------------------------
@@ -502,7 +503,7 @@ int launch_cols(const CUtensorMap& tW, const CUtensorMap& tQ, const CUtensorMap&
     if (e != cudaSuccess) return static_cast<int>(e);
     attr_once.done();
   }
-  delta_scan_kernel<BWD, NC><<<ctas, Shape<NC>::THREADS, Shape<NC>::TOTAL, st>>>(tW, tQ, tK, tM, tD, tXB, tU, tO, p);
+  pb::launch(delta_scan_kernel<BWD, NC>, ctas, Shape<NC>::THREADS, Shape<NC>::TOTAL, st, tW, tQ, tK, tM, tD, tXB, tU, tO, p);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -678,6 +679,7 @@ __global__ void __launch_bounds__(256)
 compose_kernel(const float* __restrict__ P, const float* __restrict__ R,
                const float* __restrict__ s0, float* __restrict__ s_in, float* __restrict__ s_fin,
                float* __restrict__ p_tot, int n_seg, int reverse, int slabs_state) {
+  after_previous_kernel();
   extern __shared__ float sm[];
   float* cur = sm + 2 * D * LDP;                                    // cur[row * LDC + column]
   const int seq = blockIdx.y;
@@ -772,7 +774,7 @@ PB_API int pb_delta_compose(const void* P, const void* R, const void* s0, void* 
     if (e != cudaSuccess) return static_cast<int>(e);
     attr_once.done();
   }
-  pb::dcomp::compose_kernel<<<grid, 256, pb::dcomp::SMEM, st>>>(
+  pb::launch(pb::dcomp::compose_kernel, grid, 256, pb::dcomp::SMEM, st, 
       static_cast<const float*>(P), static_cast<const float*>(R), static_cast<const float*>(s0),
       static_cast<float*>(s_in), static_cast<float*>(s_fin), static_cast<float*>(p_tot), n_seg,
       reverse, slabs);

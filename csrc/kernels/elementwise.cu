@@ -23,6 +23,7 @@ __global__ void __launch_bounds__(128) rmsnorm_fwd_kernel(const bf16* __restrict
                                                           bf16* __restrict__ y, bf16* h_out,
                                                           float* __restrict__ rstd_out, int rows,
                                                           int d, float eps) {
+  after_previous_kernel();
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows) return;
@@ -79,6 +80,7 @@ __global__ void __launch_bounds__(128) rmsnorm_fwd_reg_kernel(
     const bf16* __restrict__ x, const bf16* __restrict__ res, const float* __restrict__ w,
     bf16* __restrict__ y, bf16* h_out, float* __restrict__ rstd_out, int rows, float eps,
     uint8_t* __restrict__ q_out, float* __restrict__ s_out) {
+  after_previous_kernel();
   constexpr int d = NV * 256;
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -167,6 +169,7 @@ __global__ void __launch_bounds__(256, 2) rmsnorm_bwd_kernel(
     const bf16* __restrict__ dy, const bf16* __restrict__ h, const float* __restrict__ w,
     const float* __restrict__ rstd_in, const bf16* __restrict__ dres, bf16* __restrict__ dx,
     float* __restrict__ dw_partial, int rows, int d) {
+  after_previous_kernel();
   constexpr int R = RMS_BWD_ROWS;
   extern __shared__ __align__(16) uint8_t rms_stage[];   // [2][R][3][256] x 16 bytes
   __shared__ float red[2][R][8];
@@ -272,6 +275,7 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_generic_kernel(
     const bf16* __restrict__ dy, const bf16* __restrict__ h, const float* __restrict__ w,
     const float* __restrict__ rstd_in, const bf16* __restrict__ dres, bf16* __restrict__ dx,
     float* __restrict__ dw_partial, int rows, int d) {
+  after_previous_kernel();
   extern __shared__ float sm[];  // [d] dw + 33 scratch
   float* sdw = sm;
   float* scratch = sm + d;
@@ -307,6 +311,7 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_generic_kernel(
 __global__ void __launch_bounds__(256) fold_partials_kernel(const float* __restrict__ partial,
                                                             float* __restrict__ out, int nparts, int d,
                                                             int accumulate) {
+  after_previous_kernel();
   __shared__ float sums[8][32];
   const int g = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int c = blockIdx.x * 32 + lane;
@@ -339,6 +344,7 @@ __global__ void __launch_bounds__(256) fold_partials_kernel(const float* __restr
 __global__ void rope_kernel(bf16* __restrict__ x, const int* __restrict__ pos, long tokens,
                             int heads, int D, int rot_pairs, int seq_len, float base,
                             int inverse) {
+  after_previous_kernel();
   // One thread per (token, group of four pairs): the angles depend on the token and the pair
   // only, so sine and cosine are computed once and reused for every head of the token.
   const int vec_per_head = D >> 3;
@@ -408,6 +414,7 @@ __global__ void rope_kernel(bf16* __restrict__ x, const int* __restrict__ pos, l
 template <typename Index>
 __global__ void __launch_bounds__(256) swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict__ out,
                                                          long rows, int H, const int* __restrict__ rows_dev) {
+  after_previous_kernel();
   if (rows_dev != nullptr) rows = min(rows, static_cast<long>(*rows_dev));
   const Index vph = static_cast<Index>(H >> 3);
   const Index total = static_cast<Index>(rows) * vph;
@@ -428,6 +435,7 @@ template <typename Index>
 __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const bf16* __restrict__ dout, const bf16* __restrict__ gu,
                                                          bf16* __restrict__ dgu, long rows, int H,
                                                          const int* __restrict__ rows_dev) {
+  after_previous_kernel();
   if (rows_dev != nullptr) rows = min(rows, static_cast<long>(*rows_dev));
   const Index vph = static_cast<Index>(H >> 3);
   const Index total = static_cast<Index>(rows) * vph;
@@ -459,6 +467,7 @@ __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const bf16* __restrict_
 // ---------------------------------------------------------------------------
 __global__ void l2norm_fwd_kernel(bf16* __restrict__ x, float* __restrict__ inv_norm, long nvec,
                                   int D, float eps) {
+  after_previous_kernel();
   const int lane = threadIdx.x & 31;
   const long vec = blockIdx.x * static_cast<long>(blockDim.x >> 5) + (threadIdx.x >> 5);
   if (vec >= nvec) return;
@@ -482,6 +491,7 @@ __global__ void l2norm_fwd_kernel(bf16* __restrict__ x, float* __restrict__ inv_
 }
 __global__ void l2norm_bwd_kernel(bf16* __restrict__ dxn, const bf16* __restrict__ xn,
                                   const float* __restrict__ inv_norm, long nvec, int D) {
+  after_previous_kernel();
   const int lane = threadIdx.x & 31;
   const long vec = blockIdx.x * static_cast<long>(blockDim.x >> 5) + (threadIdx.x >> 5);
   if (vec >= nvec) return;
@@ -520,6 +530,7 @@ __device__ __forceinline__ float half_warp_sum(float v) {
 __global__ void __launch_bounds__(256) l2norm128_fwd_kernel(bf16* __restrict__ x,
                                                             float* __restrict__ inv_norm,
                                                             long nvec, float eps) {
+  after_previous_kernel();
   const int lane = threadIdx.x & 31, half = lane >> 4, l16 = lane & 15;
   const long wstride = static_cast<long>(gridDim.x) * (blockDim.x >> 5) * 8;
   for (long v0 = (blockIdx.x * static_cast<long>(blockDim.x >> 5) + (threadIdx.x >> 5)) * 8;
@@ -556,6 +567,7 @@ __global__ void __launch_bounds__(256) l2norm128_bwd_kernel(bf16* __restrict__ d
                                                             const bf16* __restrict__ xn,
                                                             const float* __restrict__ inv_norm,
                                                             long nvec) {
+  after_previous_kernel();
   const int lane = threadIdx.x & 31, half = lane >> 4, l16 = lane & 15;
   const long wstride = static_cast<long>(gridDim.x) * (blockDim.x >> 5) * 8;
   for (long v0 = (blockIdx.x * static_cast<long>(blockDim.x >> 5) + (threadIdx.x >> 5)) * 8;
@@ -615,6 +627,7 @@ __global__ void __launch_bounds__(512) softcap_ce_kernel(bf16* __restrict__ logi
                                                          float* __restrict__ lse_rows, int V,
                                                          float cap, int write_grad,
                                                          const float* __restrict__ sums) {
+  after_previous_kernel();
   __shared__ float scratch[33];
   const long row = blockIdx.x;
   bf16* p = logits + row * V;
@@ -696,6 +709,7 @@ __global__ void __launch_bounds__(512) softcap_ce_kernel(bf16* __restrict__ logi
 // as two library passes 976 us -> 223 us (1.6 GB).
 __global__ void __launch_bounds__(256) scale_cast_kernel(const float* __restrict__ x, const float* __restrict__ g,
                                                          bf16* __restrict__ out, long n) {
+  after_previous_kernel();
   const float s = *g;
   const long i = (blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x) * 8;
   if (i + 8 <= n) {
@@ -709,6 +723,7 @@ __global__ void __launch_bounds__(256) scale_cast_kernel(const float* __restrict
 
 // out[i] = sigmoid(x[i]) (bf16 -> bf16), dx = dy * s * (1 - s)
 __global__ void sigmoid_fwd_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, long n) {
+  after_previous_kernel();
   for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<long>(gridDim.x) * blockDim.x)
     y[i] = f32_to_bf16(sigmoidf_(bf16_to_f32(x[i])));
@@ -776,10 +791,10 @@ static int rmsnorm_fwd_impl(const void* x, const void* res, const void* w, void*
 #define PB_CASE(NV)                                                                              \
   case NV:                                                                                       \
     if (q_ != nullptr)                                                                           \
-      rmsnorm_fwd_reg_kernel<NV, true><<<grid, wpb * 32, 0, st>>>(x_, r_, w_, y_, h_, s_, rows,  \
+      pb::launch(rmsnorm_fwd_reg_kernel<NV, true>, grid, wpb * 32, 0, st, x_, r_, w_, y_, h_, s_, rows,  \
                                                                   eps, q_, sc_);                 \
     else                                                                                         \
-      rmsnorm_fwd_reg_kernel<NV, false><<<grid, wpb * 32, 0, st>>>(x_, r_, w_, y_, h_, s_, rows, \
+      pb::launch(rmsnorm_fwd_reg_kernel<NV, false>, grid, wpb * 32, 0, st, x_, r_, w_, y_, h_, s_, rows, \
                                                                    eps, nullptr, nullptr);       \
     break;
       PB_CASE(1) PB_CASE(2) PB_CASE(3) PB_CASE(4) PB_CASE(5) PB_CASE(6) PB_CASE(7) PB_CASE(8)
@@ -787,7 +802,7 @@ static int rmsnorm_fwd_impl(const void* x, const void* res, const void* w, void*
     }
     return cudaGetLastError();
   }
-  rmsnorm_fwd_kernel<<<(rows + wpb - 1) / wpb, wpb * 32, 0, st>>>(
+  pb::launch(rmsnorm_fwd_kernel, (rows + wpb - 1) / wpb, wpb * 32, 0, st, 
       static_cast<const bf16*>(x), static_cast<const bf16*>(res), static_cast<const float*>(w),
       static_cast<bf16*>(y), static_cast<bf16*>(h_out), static_cast<float*>(rstd), rows, d, eps);
   return cudaGetLastError();
@@ -821,15 +836,15 @@ PB_API int pb_rmsnorm_bwd(const void* dy, const void* h, const void* w, const vo
                            RMS_BWD_SMEM);
       attr_once.done();
     }
-    rmsnorm_bwd_kernel<<<grid, 256, RMS_BWD_SMEM, st>>>(dy_, h_, w_, r_, dr_, dx_, part, rows, d);
+    pb::launch(rmsnorm_bwd_kernel, grid, 256, RMS_BWD_SMEM, st, dy_, h_, w_, r_, dr_, dx_, part, rows, d);
   } else {
     const size_t smem = (d + 33) * sizeof(float);
     if (smem > 48 * 1024)
       cudaFuncSetAttribute(rmsnorm_bwd_generic_kernel,
                            cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    rmsnorm_bwd_generic_kernel<<<grid, 256, smem, st>>>(dy_, h_, w_, r_, dr_, dx_, part, rows, d);
+    pb::launch(rmsnorm_bwd_generic_kernel, grid, 256, smem, st, dy_, h_, w_, r_, dr_, dx_, part, rows, d);
   }
-  fold_partials_kernel<<<(d + 31) / 32, 256, 0, st>>>(part, static_cast<float*>(dw), grid, d,
+  pb::launch(fold_partials_kernel, (d + 31) / 32, 256, 0, st, part, static_cast<float*>(dw), grid, d,
                                                         accumulate);
   return cudaGetLastError();
 }
@@ -839,7 +854,7 @@ PB_API int pb_rope(void* x, const void* pos, long tokens, int heads, int D, int 
   if (D % 8 != 0) return PB_BAD_ARG;
   const long total = tokens * ((rot_pairs + 3) / 4);
   if (total <= 0) return 0;
-  rope_kernel<<<grid_for(total, 128), 128, 0, st>>>(static_cast<bf16*>(x),
+  pb::launch(rope_kernel, grid_for(total, 128), 128, 0, st, static_cast<bf16*>(x),
                                                     static_cast<const int*>(pos), tokens, heads,
                                                     D, rot_pairs, seq_len, base, inverse);
   return cudaGetLastError();
@@ -850,8 +865,8 @@ static int swiglu_fwd_launch(const void* gu, void* out, long rows, int H, const 
   bf16* o_ = static_cast<bf16*>(out);
   const int grid = grid_for(rows * (H / 8), 256);
   // a grid stride past the end must not wrap either
-  if (rows * (H / 8) < (1L << 31)) swiglu_fwd_kernel<uint32_t><<<grid, 256, 0, st>>>(g_, o_, rows, H, rows_dev);
-  else swiglu_fwd_kernel<uint64_t><<<grid, 256, 0, st>>>(g_, o_, rows, H, rows_dev);
+  if (rows * (H / 8) < (1L << 31)) pb::launch(swiglu_fwd_kernel<uint32_t>, grid, 256, 0, st, g_, o_, rows, H, rows_dev);
+  else pb::launch(swiglu_fwd_kernel<uint64_t>, grid, 256, 0, st, g_, o_, rows, H, rows_dev);
   return cudaGetLastError();
 }
 static int swiglu_bwd_launch(const void* dout, const void* gu, void* dgu, long rows, int H, const int* rows_dev,
@@ -859,8 +874,8 @@ static int swiglu_bwd_launch(const void* dout, const void* gu, void* dgu, long r
   const bf16 *d_ = static_cast<const bf16*>(dout), *g_ = static_cast<const bf16*>(gu);
   bf16* o_ = static_cast<bf16*>(dgu);
   const int grid = grid_for(rows * (H / 8), 256);
-  if (rows * (H / 8) < (1L << 31)) swiglu_bwd_kernel<uint32_t><<<grid, 256, 0, st>>>(d_, g_, o_, rows, H, rows_dev);
-  else swiglu_bwd_kernel<uint64_t><<<grid, 256, 0, st>>>(d_, g_, o_, rows, H, rows_dev);
+  if (rows * (H / 8) < (1L << 31)) pb::launch(swiglu_bwd_kernel<uint32_t>, grid, 256, 0, st, d_, g_, o_, rows, H, rows_dev);
+  else pb::launch(swiglu_bwd_kernel<uint64_t>, grid, 256, 0, st, d_, g_, o_, rows, H, rows_dev);
   return cudaGetLastError();
 }
 PB_API int pb_swiglu_fwd(const void* gu, void* out, long rows, int H, cudaStream_t st) {
@@ -885,6 +900,7 @@ __global__ void __launch_bounds__(256) copy_rows_dyn_kernel(const uint4* __restr
                                                             uint4* __restrict__ dst, long vec_per_row,
                                                             long max_rows,
                                                             const int* __restrict__ rows_dev) {
+  after_previous_kernel();
   const long rows = min(max_rows, static_cast<long>(*rows_dev));
   const long total = rows * vec_per_row;
   const long stride = static_cast<long>(gridDim.x) * blockDim.x;
@@ -900,7 +916,7 @@ PB_API int pb_copy_rows_dyn(const void* src, void* dst, long row_bytes, long max
   if (row_bytes <= 0 || row_bytes % 16 != 0 || max_rows <= 0 || rows_dev == nullptr ||
       ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) != 0)
     return PB_BAD_ARG;
-  copy_rows_dyn_kernel<<<grid_for(max_rows * (row_bytes / 16), 256 * 4), 256, 0, st>>>(
+  pb::launch(copy_rows_dyn_kernel, grid_for(max_rows * (row_bytes / 16), 256 * 4), 256, 0, st, 
       static_cast<const uint4*>(src), static_cast<uint4*>(dst), row_bytes / 16, max_rows, rows_dev);
   return cudaGetLastError();
 }
@@ -914,12 +930,12 @@ PB_API int pb_l2norm_fwd(void* x, void* inv_norm, long nvec, int D, float eps, c
   if (D % 4 != 0) return PB_BAD_ARG;
   if (D == 128 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
     const long warps = (nvec + 7) / 8;
-    l2norm128_fwd_kernel<<<grid_for((warps + 7) / 8, 1, 148 * 8), 256, 0, st>>>(
+    pb::launch(l2norm128_fwd_kernel, grid_for((warps + 7) / 8, 1, 148 * 8), 256, 0, st, 
         static_cast<bf16*>(x), static_cast<float*>(inv_norm), nvec, eps);
     return cudaGetLastError();
   }
   const int wpb = 8;
-  l2norm_fwd_kernel<<<static_cast<unsigned>((nvec + wpb - 1) / wpb), wpb * 32, 0, st>>>(
+  pb::launch(l2norm_fwd_kernel, static_cast<unsigned>((nvec + wpb - 1) / wpb), wpb * 32, 0, st, 
       static_cast<bf16*>(x), static_cast<float*>(inv_norm), nvec, D, eps);
   return cudaGetLastError();
 }
@@ -928,13 +944,13 @@ PB_API int pb_l2norm_bwd(void* dxn, const void* xn, const void* inv_norm, long n
   if (D % 4 != 0) return PB_BAD_ARG;
   if (D == 128 && ((reinterpret_cast<uintptr_t>(dxn) | reinterpret_cast<uintptr_t>(xn)) & 15) == 0) {
     const long warps = (nvec + 7) / 8;
-    l2norm128_bwd_kernel<<<grid_for((warps + 7) / 8, 1, 148 * 8), 256, 0, st>>>(
+    pb::launch(l2norm128_bwd_kernel, grid_for((warps + 7) / 8, 1, 148 * 8), 256, 0, st, 
         static_cast<bf16*>(dxn), static_cast<const bf16*>(xn),
         static_cast<const float*>(inv_norm), nvec);
     return cudaGetLastError();
   }
   const int wpb = 8;
-  l2norm_bwd_kernel<<<static_cast<unsigned>((nvec + wpb - 1) / wpb), wpb * 32, 0, st>>>(
+  pb::launch(l2norm_bwd_kernel, static_cast<unsigned>((nvec + wpb - 1) / wpb), wpb * 32, 0, st, 
       static_cast<bf16*>(dxn), static_cast<const bf16*>(xn),
       static_cast<const float*>(inv_norm), nvec, D);
   return cudaGetLastError();
@@ -944,7 +960,7 @@ PB_API int pb_softcap_ce(void* logits, const void* targets, const void* wt, void
                          void* lse_rows, long rows, int V, float cap, int write_grad,
                          cudaStream_t st) {
   if (V % 8 != 0 || rows <= 0) return PB_BAD_ARG;
-  softcap_ce_kernel<<<static_cast<unsigned>(rows), 512, 0, st>>>(
+  pb::launch(softcap_ce_kernel, static_cast<unsigned>(rows), 512, 0, st, 
       static_cast<bf16*>(logits), static_cast<const int*>(targets),
       static_cast<const float*>(wt), static_cast<float*>(loss_rows),
       static_cast<float*>(lse_rows), V, cap, write_grad, nullptr);
@@ -956,7 +972,7 @@ PB_API int pb_softcap_ce(void* logits, const void* targets, const void* wt, void
 PB_API int pb_softcap_ce_sums(void* logits, const void* targets, const void* wt, void* loss_rows, const void* sums,
                               long rows, int V, float cap, int write_grad, cudaStream_t st) {
   if (V % 8 != 0 || rows <= 0 || !(cap > 0.f) || sums == nullptr) return PB_BAD_ARG;
-  softcap_ce_kernel<<<static_cast<unsigned>(rows), 512, 0, st>>>(
+  pb::launch(softcap_ce_kernel, static_cast<unsigned>(rows), 512, 0, st, 
       static_cast<bf16*>(logits), static_cast<const int*>(targets), static_cast<const float*>(wt),
       static_cast<float*>(loss_rows), nullptr, V, cap, write_grad, static_cast<const float*>(sums));
   return cudaGetLastError();
@@ -965,13 +981,13 @@ PB_API int pb_softcap_ce_sums(void* logits, const void* targets, const void* wt,
 // x fp32 [n], g fp32 [1], out bf16 [n]; x and out 16-byte aligned.
 PB_API int pb_scale_cast(const void* x, const void* g, void* out, long n, cudaStream_t st) {
   if (n <= 0 || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15)) return PB_BAD_ARG;
-  scale_cast_kernel<<<static_cast<unsigned>((n + 2047) / 2048), 256, 0, st>>>(
+  pb::launch(scale_cast_kernel, static_cast<unsigned>((n + 2047) / 2048), 256, 0, st, 
       static_cast<const float*>(x), static_cast<const float*>(g), static_cast<bf16*>(out), n);
   return cudaGetLastError();
 }
 
 PB_API int pb_sigmoid(const void* x, void* y, long n, cudaStream_t st) {
-  sigmoid_fwd_kernel<<<grid_for(n, 256), 256, 0, st>>>(static_cast<const bf16*>(x),
+  pb::launch(sigmoid_fwd_kernel, grid_for(n, 256), 256, 0, st, static_cast<const bf16*>(x),
                                                        static_cast<bf16*>(y), n);
   return cudaGetLastError();
 }

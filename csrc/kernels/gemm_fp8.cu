@@ -125,6 +125,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  after_previous_kernel();
 
   // n-major inside groups of 8 row blocks, like the bf16 kernel: B tiles stay in L2
   auto coords = [&](long t, int& m_blk, int& n_blk) {
@@ -379,6 +380,7 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
   cluster_sync_all();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  after_previous_kernel();
 
   // column-major inside groups of 8 pair rows: B tiles stay in L2
   auto coords = [&](int r, int& m_pair, int& n_blk) {
@@ -645,6 +647,7 @@ __global__ void __launch_bounds__(256) quant_rows_kernel(const bf16* __restrict_
                                                          int K, uint8_t* __restrict__ q,
                                                          float* __restrict__ scales,
                                                          const int* __restrict__ rows_dev) {
+  after_previous_kernel();
   const int lane = threadIdx.x & 31;
   const int m_eff = rows_dev != nullptr ? min(M, *rows_dev) : M;
   int row0, c;
@@ -668,6 +671,7 @@ __global__ void __launch_bounds__(256) swiglu_quant_kernel(const bf16* __restric
                                                            uint8_t* __restrict__ q,
                                                            float* __restrict__ scales,
                                                            const int* __restrict__ rows_dev) {
+  after_previous_kernel();
   const int lane = threadIdx.x & 31;
   const int m_eff = rows_dev != nullptr ? min(M, *rows_dev) : M;
   int row0, c;
@@ -704,6 +708,7 @@ __global__ void __launch_bounds__(256) dequant_rows_kernel(const uint8_t* __rest
                                                            long ld_s, int M, int K,
                                                            bf16* __restrict__ y,
                                                            const int* __restrict__ rows_dev) {
+  after_previous_kernel();
   const int lane = threadIdx.x & 31;
   const int m_eff = rows_dev != nullptr ? min(M, *rows_dev) : M;
   int row0, c;
@@ -733,6 +738,7 @@ __global__ void __launch_bounds__(256) dequant_rows_kernel(const uint8_t* __rest
 __global__ void __launch_bounds__(256, 4)
 quant_blocks_kernel(const bf16* __restrict__ w, long ld, int N, int K, uint8_t* __restrict__ q,
                     float* __restrict__ scales, bf16* __restrict__ deq) {
+  after_previous_kernel();
   __shared__ float red[33];
   const int nb = blockIdx.y, kb = blockIdx.x;
   const int r0 = nb * 128 + (threadIdx.x >> 4), c = kb * 128 + (threadIdx.x & 15) * 8;
@@ -785,7 +791,7 @@ PB_API int pb_fp8_quant_rows(const void* x, long ld, int M, int K, void* q, floa
                              cudaStream_t st) {
   if (M <= 0 || K <= 0 || K % 128 != 0 || ld % 8 != 0 || (reinterpret_cast<uintptr_t>(x) & 15) != 0)
     return PB_BAD_ARG;
-  f8::quant_rows_kernel<<<f8::tile_grid(f8::QR, M, K), 256, 0, st>>>(
+  pb::launch(f8::quant_rows_kernel, f8::tile_grid(f8::QR, M, K), 256, 0, st, 
       static_cast<const bf16*>(x), ld, M, K, static_cast<uint8_t*>(q), scales, nullptr);
   return static_cast<int>(cudaGetLastError());
 }
@@ -794,7 +800,7 @@ PB_API int pb_fp8_quant_rows_dyn(const void* x, long ld, int M, int K, void* q, 
                                  const int* rows_dev, cudaStream_t st) {
   if (M <= 0 || K <= 0 || K % 128 != 0 || ld % 8 != 0 || (reinterpret_cast<uintptr_t>(x) & 15) != 0)
     return PB_BAD_ARG;
-  f8::quant_rows_kernel<<<f8::tile_grid(f8::QR, M, K), 256, 0, st>>>(
+  pb::launch(f8::quant_rows_kernel, f8::tile_grid(f8::QR, M, K), 256, 0, st, 
       static_cast<const bf16*>(x), ld, M, K, static_cast<uint8_t*>(q), scales, rows_dev);
   return static_cast<int>(cudaGetLastError());
 }
@@ -804,7 +810,7 @@ PB_API int pb_fp8_quant_rows_dyn(const void* x, long ld, int M, int K, void* q, 
 PB_API int pb_swiglu_quant(const void* gu, void* h, int M, int H, void* q, float* scales,
                            const int* rows_dev, cudaStream_t st) {
   if (M <= 0 || H <= 0 || H % 128 != 0) return PB_BAD_ARG;
-  f8::swiglu_quant_kernel<<<f8::tile_grid(f8::QR_SWI, M, H), 256, 0, st>>>(
+  pb::launch(f8::swiglu_quant_kernel, f8::tile_grid(f8::QR_SWI, M, H), 256, 0, st, 
       static_cast<const bf16*>(gu), static_cast<bf16*>(h), M, H, static_cast<uint8_t*>(q), scales,
       rows_dev);
   return static_cast<int>(cudaGetLastError());
@@ -815,7 +821,7 @@ PB_API int pb_swiglu_quant(const void* gu, void* h, int M, int H, void* q, float
 PB_API int pb_fp8_dequant_rows(const void* q, const float* scales, long ld_s, int M, int K, void* y,
                                const int* rows_dev, cudaStream_t st) {
   if (M <= 0 || K <= 0 || K % 128 != 0 || ld_s < M) return PB_BAD_ARG;
-  f8::dequant_rows_kernel<<<f8::tile_grid(f8::QR, M, K), 256, 0, st>>>(
+  pb::launch(f8::dequant_rows_kernel, f8::tile_grid(f8::QR, M, K), 256, 0, st, 
       static_cast<const uint8_t*>(q), scales, ld_s, M, K, static_cast<bf16*>(y), rows_dev);
   return static_cast<int>(cudaGetLastError());
 }
@@ -826,7 +832,7 @@ PB_API int pb_fp8_quant_blocks(const void* w, long ld, int rows, int K, void* q,
                                cudaStream_t st) {
   if (rows <= 0 || K <= 0 || K % 128 != 0 || ld % 4 != 0) return PB_BAD_ARG;
   dim3 grid(K / 128, (rows + 127) / 128);
-  f8::quant_blocks_kernel<<<grid, 256, 0, st>>>(static_cast<const bf16*>(w), ld, rows, K,
+  pb::launch(f8::quant_blocks_kernel, grid, 256, 0, st, static_cast<const bf16*>(w), ld, rows, K,
                                                 static_cast<uint8_t*>(q), scales, nullptr);
   return static_cast<int>(cudaGetLastError());
 }
@@ -838,7 +844,7 @@ PB_API int pb_fp8_fakequant_blocks(const void* w, long ld, int rows, int K, void
                                    cudaStream_t st) {
   if (rows <= 0 || K <= 0 || K % 128 != 0 || ld % 4 != 0 || out == nullptr) return PB_BAD_ARG;
   dim3 grid(K / 128, (rows + 127) / 128);
-  f8::quant_blocks_kernel<<<grid, 256, 0, st>>>(static_cast<const bf16*>(w), ld, rows, K, nullptr,
+  pb::launch(f8::quant_blocks_kernel, grid, 256, 0, st, static_cast<const bf16*>(w), ld, rows, K, nullptr,
                                                 nullptr, static_cast<bf16*>(out));
   return static_cast<int>(cudaGetLastError());
 }
@@ -860,14 +866,16 @@ static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUt
   static pb::DeviceOnce attr_once;   // per device: the attribute belongs to the current GPU
   static int max_pairs = 0;
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // as pb::launch
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.blockDim = dim3(P_THREADS, 1, 1);
   cfg.dynamicSmemBytes = P_SMEM;
   cfg.stream = st;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   if (attr_once.need()) {
     cudaError_t e = cudaFuncSetAttribute(gemm_fp8_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM);
     if (e != cudaSuccess) return static_cast<int>(e);
@@ -976,6 +984,6 @@ static int gemm_fp8_launch(const void* Aq, const float* sa, const void* Bq, cons
   int grid = num_sms();
   if (max_ctas > 0 && max_ctas < grid) grid = max_ctas;
   if (tiles < grid) grid = static_cast<int>(tiles);
-  gemm_fp8_kernel<PROBE><<<grid, THREADS, SMEM_TOTAL, st>>>(tmA, tmB, tmC, p);
+  pb::launch(gemm_fp8_kernel<PROBE>, grid, THREADS, SMEM_TOTAL, st, tmA, tmB, tmC, p);
   return static_cast<int>(cudaGetLastError());
 }

@@ -16,6 +16,7 @@ namespace pb {
 // one warp per gathered row; d % 8 == 0
 __global__ void latent_gather_kernel(const bf16* __restrict__ src, bf16* __restrict__ rows, int B,
                                      int S, int d, int start, int K) {
+  after_previous_kernel();
   const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (w >= B * K) return;
   const int b = w / K, j = w % K;
@@ -27,6 +28,7 @@ __global__ void latent_gather_kernel(const bf16* __restrict__ src, bf16* __restr
 // rows (B*K, d) added into / written to positions start .. start+K of a zero or existing tensor
 __global__ void latent_scatter_kernel(const bf16* __restrict__ rows, bf16* __restrict__ dst, int B,
                                       int S, int d, int start, int K) {
+  after_previous_kernel();
   const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (w >= B * K) return;
   const int b = w / K, j = w % K;
@@ -40,6 +42,7 @@ __global__ void latent_norm_scatter_kernel(const bf16* __restrict__ a, const flo
                                            const bf16* __restrict__ embeds, bf16* __restrict__ out,
                                            float* __restrict__ rstd, int B, int S, int d, int start,
                                            int K, float eps) {
+  after_previous_kernel();
   const long row = (static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (row >= static_cast<long>(B) * S) return;
@@ -72,6 +75,7 @@ __global__ void latent_norm_scatter_kernel(const bf16* __restrict__ a, const flo
 }
 
 __global__ void silu_fwd_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, long n8) {
+  after_previous_kernel();
   for (long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n8;
        i += static_cast<long>(gridDim.x) * blockDim.x) {
     float f[8];
@@ -83,6 +87,7 @@ __global__ void silu_fwd_kernel(const bf16* __restrict__ x, bf16* __restrict__ y
 }
 __global__ void silu_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x,
                                 bf16* __restrict__ dx, long n8) {
+  after_previous_kernel();
   for (long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n8;
        i += static_cast<long>(gridDim.x) * blockDim.x) {
     float f[8], g[8];
@@ -109,7 +114,7 @@ static bool bad_slots(int B, int S, int d, int start, int K) {
 PB_API int pb_latent_gather(const void* src, void* rows, int B, int S, int d, int start, int K,
                             cudaStream_t st) {
   if (bad_slots(B, S, d, start, K)) return PB_BAD_ARG;
-  latent_gather_kernel<<<(B * K * 32 + 255) / 256, 256, 0, st>>>(
+  pb::launch(latent_gather_kernel, (B * K * 32 + 255) / 256, 256, 0, st, 
       static_cast<const bf16*>(src), static_cast<bf16*>(rows), B, S, d, start, K);
   return static_cast<int>(cudaGetLastError());
 }
@@ -118,7 +123,7 @@ PB_API int pb_latent_gather(const void* src, void* rows, int B, int S, int d, in
 PB_API int pb_latent_scatter(const void* rows, void* dst, int B, int S, int d, int start, int K,
                              cudaStream_t st) {
   if (bad_slots(B, S, d, start, K)) return PB_BAD_ARG;
-  latent_scatter_kernel<<<(B * K * 32 + 255) / 256, 256, 0, st>>>(
+  pb::launch(latent_scatter_kernel, (B * K * 32 + 255) / 256, 256, 0, st, 
       static_cast<const bf16*>(rows), static_cast<bf16*>(dst), B, S, d, start, K);
   return static_cast<int>(cudaGetLastError());
 }
@@ -129,7 +134,7 @@ PB_API int pb_latent_norm_scatter(const void* a, const void* w, const void* embe
                                   cudaStream_t st) {
   if (bad_slots(B, S, d, start, K)) return PB_BAD_ARG;
   const long warps = static_cast<long>(B) * S;
-  latent_norm_scatter_kernel<<<static_cast<unsigned>((warps * 32 + 255) / 256), 256, 0, st>>>(
+  pb::launch(latent_norm_scatter_kernel, static_cast<unsigned>((warps * 32 + 255) / 256), 256, 0, st, 
       static_cast<const bf16*>(a), static_cast<const float*>(w), static_cast<const bf16*>(embeds),
       static_cast<bf16*>(out), static_cast<float*>(rstd), B, S, d, start, K, eps);
   return static_cast<int>(cudaGetLastError());
@@ -139,14 +144,14 @@ PB_API int pb_silu_fwd(const void* x, void* y, long n, cudaStream_t st) {
   if (n <= 0 || n % 8 != 0) return PB_BAD_ARG;
   const long n8 = n / 8;
   const int grid = static_cast<int>(n8 / 256 + 1 < 148 * 8 ? n8 / 256 + 1 : 148 * 8);
-  silu_fwd_kernel<<<grid, 256, 0, st>>>(static_cast<const bf16*>(x), static_cast<bf16*>(y), n8);
+  pb::launch(silu_fwd_kernel, grid, 256, 0, st, static_cast<const bf16*>(x), static_cast<bf16*>(y), n8);
   return static_cast<int>(cudaGetLastError());
 }
 PB_API int pb_silu_bwd(const void* dy, const void* x, void* dx, long n, cudaStream_t st) {
   if (n <= 0 || n % 8 != 0) return PB_BAD_ARG;
   const long n8 = n / 8;
   const int grid = static_cast<int>(n8 / 256 + 1 < 148 * 8 ? n8 / 256 + 1 : 148 * 8);
-  silu_bwd_kernel<<<grid, 256, 0, st>>>(static_cast<const bf16*>(dy), static_cast<const bf16*>(x),
+  pb::launch(silu_bwd_kernel, grid, 256, 0, st, static_cast<const bf16*>(dy), static_cast<const bf16*>(x),
                                         static_cast<bf16*>(dx), n8);
   return static_cast<int>(cudaGetLastError());
 }

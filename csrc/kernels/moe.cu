@@ -31,6 +31,7 @@ template <int PER>
 __global__ void route_kernel(const float* __restrict__ logits, const float* __restrict__ bias,
                              int T, int E, int k, float* __restrict__ probs, int* __restrict__ ids,
                              float* __restrict__ gates) {
+  after_previous_kernel();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (warp >= T) return;
   const float* row = logits + static_cast<size_t>(warp) * E;
@@ -84,6 +85,7 @@ __global__ void route_kernel(const float* __restrict__ logits, const float* __re
 __global__ void route_bwd_kernel(const float* __restrict__ dgates, const float* __restrict__ gates,
                                  const float* __restrict__ probs, const int* __restrict__ ids, int T,
                                  int E, int k, float* __restrict__ dlogits) {
+  after_previous_kernel();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (warp >= T) return;
   float* drow = dlogits + static_cast<size_t>(warp) * E;
@@ -110,6 +112,7 @@ __global__ void route_bwd_kernel(const float* __restrict__ dgates, const float* 
 // per-block histogram of expert ids. block_counts: [nblocks, E]
 __global__ void count_kernel(const int* __restrict__ ids, int n_pairs, int pairs_per_block, int E,
                              int* __restrict__ block_counts) {
+  after_previous_kernel();
   __shared__ int hist[MAX_E];
   for (int e = threadIdx.x; e < E; e += blockDim.x) hist[e] = 0;
   __syncthreads();
@@ -163,6 +166,7 @@ __device__ __forceinline__ void write_segments(const int* tot, int* off, int E, 
 __global__ void scan_kernel(int* __restrict__ block_counts, int nblocks, int E,
                             int* __restrict__ expert_off, int* __restrict__ totals,
                             int* __restrict__ k_len, int* __restrict__ mblk_group, int max_mblk) {
+  after_previous_kernel();
   __shared__ int tot[MAX_E];
   __shared__ int off[MAX_E + 1];
   for (int e = threadIdx.x; e < E; e += blockDim.x) {
@@ -201,6 +205,7 @@ __device__ __forceinline__ void place_pairs(const int* __restrict__ ids, int lo,
 __global__ void place_kernel(const int* __restrict__ ids, int n_pairs, int pairs_per_block, int E,
                              const int* __restrict__ block_base, const int* __restrict__ expert_off,
                              int* __restrict__ row_of) {
+  after_previous_kernel();
   __shared__ int run[MAX_E];
   const int lane = threadIdx.x;
   for (int e = lane; e < E; e += 32)
@@ -221,6 +226,7 @@ __global__ void __launch_bounds__(SORT_WARPS * 32) sort_small_kernel(const int* 
                                                                      int* __restrict__ totals,
                                                                      int* __restrict__ k_len,
                                                                      int* __restrict__ mblk_group, int max_mblk) {
+  after_previous_kernel();
   __shared__ int run[SORT_WARPS][MAX_E];
   __shared__ int tot[MAX_E];
   __shared__ int off[MAX_E + 1];
@@ -261,6 +267,7 @@ __device__ __forceinline__ void zero_pad_rows(bf16* __restrict__ buf, int d, int
 }
 __global__ void __launch_bounds__(256) zero_pad_kernel(bf16* __restrict__ buf, int d, const int* __restrict__ expert_off,
                                                        const int* __restrict__ totals) {
+  after_previous_kernel();
   zero_pad_rows(buf, d, blockIdx.x, blockIdx.y, gridDim.y, expert_off, totals);
 }
 // the same rows of a quantised buffer: zero bytes, scale 1 (what the row quantiser makes of zeros)
@@ -283,6 +290,7 @@ __global__ void __launch_bounds__(256) permute_kernel(const bf16* __restrict__ s
                                                       long ld_src, bf16* __restrict__ dst, long dst_rows,
                                                       int pair_blocks, const int* __restrict__ expert_off,
                                                       const int* __restrict__ totals) {
+  after_previous_kernel();
   if (static_cast<int>(blockIdx.x) >= pair_blocks) {   // the blocks after the pairs' clear the padding rows
     const int i = blockIdx.x - pair_blocks;
     zero_pad_rows(dst, d, i / PAD_SPLIT, i % PAD_SPLIT, PAD_SPLIT, expert_off, totals);
@@ -324,6 +332,7 @@ __global__ void __launch_bounds__(256) permute_q_kernel(const uint8_t* __restric
                                                         float* __restrict__ dscales, long dst_rows, int pair_blocks,
                                                         const int* __restrict__ expert_off,
                                                         const int* __restrict__ totals) {
+  after_previous_kernel();
   if (static_cast<int>(blockIdx.x) >= pair_blocks) {
     const int i = blockIdx.x - pair_blocks;
     zero_pad_q_rows(dq, dscales, K, dst_rows, i / PAD_SPLIT, i % PAD_SPLIT, expert_off, totals);
@@ -355,6 +364,7 @@ __global__ void __launch_bounds__(256) permute_q_kernel(const uint8_t* __restric
 __global__ void __launch_bounds__(256) combine_kernel(const bf16* __restrict__ y, const int* __restrict__ row_of,
                                                       const float* __restrict__ gates, const bf16* __restrict__ add,
                                                       int T, int k, int d, bf16* __restrict__ out, long y_rows) {
+  after_previous_kernel();
   const long w = (static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31, parts = (d + 511) / 512;
   const long t = w / parts;
@@ -397,6 +407,7 @@ __global__ void __launch_bounds__(256) combine_kernel(const bf16* __restrict__ y
 __global__ void combine_bwd_kernel(const bf16* __restrict__ y, const bf16* __restrict__ dout,
                                    const int* __restrict__ row_of, int n_pairs, int k, int d,
                                    float* __restrict__ dgates) {
+  after_previous_kernel();
   const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (w >= n_pairs) return;
   const bf16* a = y + static_cast<size_t>(row_of[w]) * d;
@@ -427,17 +438,17 @@ PB_API int pb_moe_route(const float* logits, const float* bias, int T, int E, in
   if (T <= 0 || E <= 0 || E > moe::MAX_E || k <= 0 || k > moe::MAX_K || k > E) return PB_BAD_ARG;
   const int per = (E + 31) / 32;
   const int grid = warps_grid(T, 256);
-  if (per <= 2) moe::route_kernel<2><<<grid, 256, 0, st>>>(logits, bias, T, E, k, probs, ids, gates);
-  else if (per <= 4) moe::route_kernel<4><<<grid, 256, 0, st>>>(logits, bias, T, E, k, probs, ids, gates);
-  else if (per <= 8) moe::route_kernel<8><<<grid, 256, 0, st>>>(logits, bias, T, E, k, probs, ids, gates);
-  else moe::route_kernel<moe::MAX_E / 32><<<grid, 256, 0, st>>>(logits, bias, T, E, k, probs, ids, gates);
+  if (per <= 2) pb::launch(moe::route_kernel<2>, grid, 256, 0, st, logits, bias, T, E, k, probs, ids, gates);
+  else if (per <= 4) pb::launch(moe::route_kernel<4>, grid, 256, 0, st, logits, bias, T, E, k, probs, ids, gates);
+  else if (per <= 8) pb::launch(moe::route_kernel<8>, grid, 256, 0, st, logits, bias, T, E, k, probs, ids, gates);
+  else pb::launch(moe::route_kernel<moe::MAX_E / 32>, grid, 256, 0, st, logits, bias, T, E, k, probs, ids, gates);
   return static_cast<int>(cudaGetLastError());
 }
 
 PB_API int pb_moe_route_bwd(const float* dgates, const float* gates, const float* probs,
                             const int* ids, int T, int E, int k, float* dlogits, cudaStream_t st) {
   if (T <= 0 || E <= 0 || k <= 0) return PB_BAD_ARG;
-  moe::route_bwd_kernel<<<warps_grid(T, 256), 256, 0, st>>>(dgates, gates, probs, ids, T, E, k, dlogits);
+  pb::launch(moe::route_bwd_kernel, warps_grid(T, 256), 256, 0, st, dgates, gates, probs, ids, T, E, k, dlogits);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -454,16 +465,16 @@ PB_API int pb_moe_sort(const int* ids, int n_pairs, int k, int E, int* scratch, 
                        cudaStream_t st) {
   if (n_pairs <= 0 || E <= 0 || E > moe::MAX_E || k <= 0) return PB_BAD_ARG;
   if (n_pairs <= moe::SORT_MAX) {
-    moe::sort_small_kernel<<<1, moe::SORT_WARPS * 32, 0, st>>>(ids, n_pairs, E, row_of, expert_off, totals, k_len,
+    pb::launch(moe::sort_small_kernel, 1, moe::SORT_WARPS * 32, 0, st, ids, n_pairs, E, row_of, expert_off, totals, k_len,
                                                                mblk_group, max_mblk);
     return static_cast<int>(cudaGetLastError());
   }
   const int per = moe::TOK_PER_BLOCK * k;
   const int nblocks = (n_pairs + per - 1) / per;
-  moe::count_kernel<<<nblocks, 256, 0, st>>>(ids, n_pairs, per, E, scratch);
-  moe::scan_kernel<<<1, 512, 0, st>>>(scratch, nblocks, E, expert_off, totals, k_len, mblk_group,
+  pb::launch(moe::count_kernel, nblocks, 256, 0, st, ids, n_pairs, per, E, scratch);
+  pb::launch(moe::scan_kernel, 1, 512, 0, st, scratch, nblocks, E, expert_off, totals, k_len, mblk_group,
                                       max_mblk);
-  moe::place_kernel<<<nblocks, 32, 0, st>>>(ids, n_pairs, per, E, scratch, expert_off, row_of);
+  pb::launch(moe::place_kernel, nblocks, 32, 0, st, ids, n_pairs, per, E, scratch, expert_off, row_of);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -475,7 +486,7 @@ PB_API int pb_moe_permute(const void* src, const int* row_of, const float* scale
   const long dst_rows = (static_cast<long>(n_pairs) + static_cast<long>(E > 0 ? E : 1) * 127 + 127) / 128 * 128;
   const int pair_blocks = warps_grid(n_pairs, 256);
   const int pad_blocks = expert_off != nullptr ? E * moe::PAD_SPLIT : 0;
-  moe::permute_kernel<<<pair_blocks + pad_blocks, 256, 0, st>>>(static_cast<const bf16*>(src), row_of, scale, n_pairs, k,
+  pb::launch(moe::permute_kernel, pair_blocks + pad_blocks, 256, 0, st, static_cast<const bf16*>(src), row_of, scale, n_pairs, k,
                                                                 d, ld_src, static_cast<bf16*>(dst), dst_rows,
                                                                 pair_blocks, expert_off, totals);
   return static_cast<int>(cudaGetLastError());
@@ -489,7 +500,7 @@ PB_API int pb_moe_permute_q(const void* q, const float* scales, const int* row_o
   if (T <= 0 || k <= 0 || K <= 0 || K % 128 != 0 || E <= 0) return PB_BAD_ARG;
   const int n_pairs = T * k;
   const int pair_blocks = warps_grid(n_pairs, 256);
-  moe::permute_q_kernel<<<pair_blocks + E * moe::PAD_SPLIT, 256, 0, st>>>(
+  pb::launch(moe::permute_q_kernel, pair_blocks + E * moe::PAD_SPLIT, 256, 0, st, 
       static_cast<const uint8_t*>(q), scales, row_of, n_pairs, k, K, T, static_cast<uint8_t*>(dq), dscales, rows,
       pair_blocks, expert_off, totals);
   return static_cast<int>(cudaGetLastError());
@@ -498,7 +509,7 @@ PB_API int pb_moe_permute_q(const void* q, const float* scales, const int* row_o
 PB_API int pb_moe_zero_pad(void* buf, int d, const int* expert_off, const int* totals, int E,
                            cudaStream_t st) {
   if (E <= 0 || d % 8 != 0) return PB_BAD_ARG;
-  moe::zero_pad_kernel<<<dim3(E, moe::PAD_SPLIT), 256, 0, st>>>(static_cast<bf16*>(buf), d, expert_off, totals);
+  pb::launch(moe::zero_pad_kernel, dim3(E, moe::PAD_SPLIT), 256, 0, st, static_cast<bf16*>(buf), d, expert_off, totals);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -506,7 +517,7 @@ PB_API int pb_moe_zero_pad(void* buf, int d, const int* expert_off, const int* t
 PB_API int pb_moe_combine(const void* y, const int* row_of, const float* gates, const void* add,
                           int T, int k, int d, void* out, long y_rows, cudaStream_t st) {
   if (T <= 0 || d % 8 != 0) return PB_BAD_ARG;
-  moe::combine_kernel<<<warps_grid(static_cast<long>(T) * ((d + 511) / 512), 256), 256, 0, st>>>(
+  pb::launch(moe::combine_kernel, warps_grid(static_cast<long>(T) * ((d + 511) / 512), 256), 256, 0, st, 
       static_cast<const bf16*>(y), row_of, gates, static_cast<const bf16*>(add), T, k, d,
       static_cast<bf16*>(out), y_rows > 0 ? y_rows : (1L << 62));
   return static_cast<int>(cudaGetLastError());
@@ -515,7 +526,7 @@ PB_API int pb_moe_combine(const void* y, const int* row_of, const float* gates, 
 PB_API int pb_moe_combine_bwd(const void* y, const void* dout, const int* row_of, int n_pairs, int k,
                               int d, float* dgates, cudaStream_t st) {
   if (n_pairs <= 0 || d % 8 != 0) return PB_BAD_ARG;
-  moe::combine_bwd_kernel<<<warps_grid(n_pairs, 256), 256, 0, st>>>(
+  pb::launch(moe::combine_bwd_kernel, warps_grid(n_pairs, 256), 256, 0, st, 
       static_cast<const bf16*>(y), static_cast<const bf16*>(dout), row_of, n_pairs, k, d, dgates);
   return static_cast<int>(cudaGetLastError());
 }

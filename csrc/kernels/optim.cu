@@ -12,6 +12,7 @@ namespace pb {
 // partial[b] = sum over this block's grid-stride slice of x^2
 __global__ void __launch_bounds__(256) sumsq_partial_kernel(const float* __restrict__ x, long n,
                                                             float* __restrict__ partial) {
+  after_previous_kernel();
   __shared__ float scratch[33];
   float s = 0.f;
   const long n4 = n >> 2;
@@ -29,6 +30,7 @@ __global__ void __launch_bounds__(256) sumsq_partial_kernel(const float* __restr
 __global__ void __launch_bounds__(256) sumsq_partial_bf16_kernel(const bf16* __restrict__ x,
                                                                  long n,
                                                                  float* __restrict__ partial) {
+  after_previous_kernel();
   __shared__ float scratch[33];
   float s = 0.f;
   for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < n;
@@ -42,6 +44,7 @@ __global__ void __launch_bounds__(256) sumsq_partial_bf16_kernel(const bf16* __r
 // out[0] (+)= sum_b partial[b], fixed order, one warp.
 __global__ void fold_scalar_kernel(const float* __restrict__ partial, int nparts,
                                    float* __restrict__ out, int accumulate) {
+  after_previous_kernel();
   float s = 0.f;
   for (int b = threadIdx.x; b < nparts; b += 32) s += partial[b];
   // fixed-shape butterfly: deterministic for a fixed nparts
@@ -53,6 +56,7 @@ __global__ void fold_scalar_kernel(const float* __restrict__ partial, int nparts
 // same fixed order as fold_scalar_kernel.
 __global__ void fold_rows_kernel(const float* __restrict__ partial, int nparts,
                                  float* __restrict__ out) {
+  after_previous_kernel();
   const float* p = partial + static_cast<long>(blockIdx.x) * nparts;
   float s = 0.f;
   for (int b = threadIdx.x; b < nparts; b += 32) s += p[b];
@@ -75,6 +79,7 @@ __global__ void __launch_bounds__(256) adamw_kernel(float* __restrict__ p,
                                                     float inv_bc1, float inv_bc2,
                                                     const float* __restrict__ gnorm_sq,
                                                     float clip, float gscale) {
+  after_previous_kernel();
   const float s = clip_scale(gnorm_sq, clip) * gscale;
   for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<long>(gridDim.x) * blockDim.x) {
@@ -99,6 +104,7 @@ __global__ void __launch_bounds__(256) muon_momentum_kernel(const float* __restr
                                                             const float* __restrict__ gnorm_sq,
                                                             float clip, float gscale,
                                                             float* __restrict__ partial) {
+  after_previous_kernel();
   __shared__ float scratch[33];
   const float s = clip_scale(gnorm_sq, clip) * gscale;
   g += static_cast<long>(blockIdx.y) * n;
@@ -124,6 +130,7 @@ __global__ void __launch_bounds__(256) muon_normalize_kernel(const float* __rest
                                                              const float* __restrict__ gnorm_sq,
                                                              float clip, float gscale,
                                                              const float* __restrict__ nes_sq) {
+  after_previous_kernel();
   const float s = clip_scale(gnorm_sq, clip) * gscale;
   g += static_cast<long>(blockIdx.y) * n;
   m += static_cast<long>(blockIdx.y) * n;
@@ -141,6 +148,7 @@ __global__ void __launch_bounds__(256) muon_apply_kernel(float* __restrict__ p,
                                                          const bf16* __restrict__ o,
                                                          bf16* __restrict__ p_lp, long n, float lr,
                                                          float scale, float wd) {
+  after_previous_kernel();
   for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<long>(gridDim.x) * blockDim.x) {
     const float pi = p[i];
@@ -153,6 +161,7 @@ __global__ void __launch_bounds__(256) muon_apply_kernel(float* __restrict__ p,
 // y = bf16(x * scale) ; plain cast helpers for the flat buffers
 __global__ void cast_f32_bf16_kernel(const float* __restrict__ x, bf16* __restrict__ y, long n,
                                      float scale) {
+  after_previous_kernel();
   for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<long>(gridDim.x) * blockDim.x)
     y[i] = f32_to_bf16(x[i] * scale);
@@ -160,6 +169,7 @@ __global__ void cast_f32_bf16_kernel(const float* __restrict__ x, bf16* __restri
 // acc_f32 += scale * x_bf16
 __global__ void axpy_bf16_f32_kernel(const bf16* __restrict__ x, float* __restrict__ acc, long n,
                                      float scale) {
+  after_previous_kernel();
   for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<long>(gridDim.x) * blockDim.x)
     acc[i] += scale * bf16_to_f32(x[i]);
@@ -167,6 +177,7 @@ __global__ void axpy_bf16_f32_kernel(const bf16* __restrict__ x, float* __restri
 // out[c][r] = in[r][c] (bf16), 32x32 tiles through shared memory
 __global__ void transpose_bf16_kernel(const bf16* __restrict__ in, bf16* __restrict__ out,
                                       int rows, int cols) {
+  after_previous_kernel();
   __shared__ bf16 tile[32][33];
   const int bx = blockIdx.x * 32, by = blockIdx.y * 32;
   const size_t boff = static_cast<size_t>(blockIdx.z) * rows * cols;
@@ -194,6 +205,7 @@ __global__ void __launch_bounds__(256) qk_clip_rescale_kernel(float* __restrict_
                                                               int n_q_heads, int is_k, long row0,
                                                               const float* __restrict__ max_logit,
                                                               float tau) {
+  after_previous_kernel();
   const long r = blockIdx.x;
   if (r >= rows) return;
   const int head = static_cast<int>((row0 + r) / dh);
@@ -227,6 +239,7 @@ __global__ void __launch_bounds__(256) qk_clip_rescale_kernel(float* __restrict_
 // integer adds, so the result does not depend on the grid.
 __global__ void __launch_bounds__(256) checksum_u32_kernel(const uint32_t* __restrict__ x, long n,
                                                            unsigned long long* __restrict__ out) {
+  after_previous_kernel();
   unsigned long long acc = 0ull;
   for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<long>(gridDim.x) * blockDim.x) {
@@ -259,18 +272,18 @@ PB_API int pb_sumsq_nparts(long n) {
 PB_API int pb_sumsq_f32(const void* x, long n, void* scratch, void* out, int accumulate,
                         cudaStream_t st) {
   const int g = pb_sumsq_nparts(n);
-  sumsq_partial_kernel<<<g, 256, 0, st>>>(static_cast<const float*>(x), n,
+  pb::launch(sumsq_partial_kernel, g, 256, 0, st, static_cast<const float*>(x), n,
                                           static_cast<float*>(scratch));
-  fold_scalar_kernel<<<1, 32, 0, st>>>(static_cast<const float*>(scratch), g,
+  pb::launch(fold_scalar_kernel, 1, 32, 0, st, static_cast<const float*>(scratch), g,
                                        static_cast<float*>(out), accumulate);
   return cudaGetLastError();
 }
 PB_API int pb_sumsq_bf16(const void* x, long n, void* scratch, void* out, int accumulate,
                          cudaStream_t st) {
   const int g = pb_sumsq_nparts(n);
-  sumsq_partial_bf16_kernel<<<g, 256, 0, st>>>(static_cast<const bf16*>(x), n,
+  pb::launch(sumsq_partial_bf16_kernel, g, 256, 0, st, static_cast<const bf16*>(x), n,
                                                static_cast<float*>(scratch));
-  fold_scalar_kernel<<<1, 32, 0, st>>>(static_cast<const float*>(scratch), g,
+  pb::launch(fold_scalar_kernel, 1, 32, 0, st, static_cast<const float*>(scratch), g,
                                        static_cast<float*>(out), accumulate);
   return cudaGetLastError();
 }
@@ -281,7 +294,7 @@ PB_API int pb_adamw(void* p, const void* g, void* m, void* v, void* p_lp, long n
   if (step < 1) return PB_BAD_ARG;
   const float inv_bc1 = 1.f / (1.f - powf(b1, static_cast<float>(step)));
   const float inv_bc2 = 1.f / (1.f - powf(b2, static_cast<float>(step)));
-  adamw_kernel<<<ogrid(n), 256, 0, st>>>(
+  pb::launch(adamw_kernel, ogrid(n), 256, 0, st, 
       static_cast<float*>(p), static_cast<const float*>(g), static_cast<float*>(m),
       static_cast<float*>(v), static_cast<bf16*>(p_lp), n, lr, b1, b2, eps, wd, inv_bc1, inv_bc2,
       static_cast<const float*>(gnorm_sq), clip, gscale);
@@ -296,12 +309,12 @@ PB_API int pb_muon_prepare(const void* g, void* m, void* x0, long n, float beta,
   const int parts = pb_sumsq_nparts(n);
   float* part = static_cast<float*>(scratch);
   float* nes_sq = part + parts;
-  muon_momentum_kernel<<<parts, 256, 0, st>>>(static_cast<const float*>(g),
+  pb::launch(muon_momentum_kernel, parts, 256, 0, st, static_cast<const float*>(g),
                                               static_cast<float*>(m), n, beta,
                                               static_cast<const float*>(gnorm_sq), clip, gscale,
                                               part);
-  fold_scalar_kernel<<<1, 32, 0, st>>>(part, parts, nes_sq, 0);
-  muon_normalize_kernel<<<ogrid(n), 256, 0, st>>>(
+  pb::launch(fold_scalar_kernel, 1, 32, 0, st, part, parts, nes_sq, 0);
+  pb::launch(muon_normalize_kernel, ogrid(n), 256, 0, st, 
       static_cast<const float*>(g), static_cast<const float*>(m), static_cast<bf16*>(x0), n, beta,
       static_cast<const float*>(gnorm_sq), clip, gscale, nes_sq);
   return cudaGetLastError();
@@ -323,11 +336,11 @@ PB_API int pb_muon_prepare_batched(const void* g, void* m, void* x0, long n, int
     float* mj = static_cast<float*>(m) + static_cast<long>(j0) * n;
     bf16* xj = static_cast<bf16*>(x0) + static_cast<long>(j0) * n;
     float* pj = part + static_cast<long>(j0) * parts;
-    muon_momentum_kernel<<<dim3(parts, cnt), 256, 0, st>>>(gj, mj, n, beta,
+    pb::launch(muon_momentum_kernel, dim3(parts, cnt), 256, 0, st, gj, mj, n, beta,
                                                          static_cast<const float*>(gnorm_sq),
                                                          clip, gscale, pj);
-    fold_rows_kernel<<<cnt, 32, 0, st>>>(pj, parts, nes_sq + j0);
-    muon_normalize_kernel<<<dim3(ogrid(n), cnt), 256, 0, st>>>(
+    pb::launch(fold_rows_kernel, cnt, 32, 0, st, pj, parts, nes_sq + j0);
+    pb::launch(muon_normalize_kernel, dim3(ogrid(n), cnt), 256, 0, st, 
         gj, mj, xj, n, beta, static_cast<const float*>(gnorm_sq), clip, gscale, nes_sq + j0);
   }
   return cudaGetLastError();
@@ -335,7 +348,7 @@ PB_API int pb_muon_prepare_batched(const void* g, void* m, void* x0, long n, int
 
 PB_API int pb_muon_apply(void* p, const void* o, void* p_lp, long n, float lr, float scale,
                          float wd, cudaStream_t st) {
-  muon_apply_kernel<<<ogrid(n), 256, 0, st>>>(static_cast<float*>(p), static_cast<const bf16*>(o),
+  pb::launch(muon_apply_kernel, ogrid(n), 256, 0, st, static_cast<float*>(p), static_cast<const bf16*>(o),
                                               static_cast<bf16*>(p_lp), n, lr, scale, wd);
   return cudaGetLastError();
 }
@@ -349,7 +362,7 @@ PB_API int pb_qk_clip_rescale(void* master, void* lp, int rows, int cols, int dh
   if (cols <= 0 || dh <= 0 || group <= 0 || n_q_heads <= 0 || tau <= 0.f || max_logit == nullptr ||
       (master == nullptr && lp == nullptr))
     return PB_BAD_ARG;
-  qk_clip_rescale_kernel<<<rows, 256, 0, st>>>(static_cast<float*>(master), static_cast<bf16*>(lp),
+  pb::launch(qk_clip_rescale_kernel, rows, 256, 0, st, static_cast<float*>(master), static_cast<bf16*>(lp),
                                                rows, cols, dh, group, n_q_heads, is_k, row0,
                                                static_cast<const float*>(max_logit), tau);
   return cudaGetLastError();
@@ -360,25 +373,25 @@ PB_API int pb_checksum_u32(const void* x, long n, void* out, cudaStream_t st) {
   cudaError_t e = cudaMemsetAsync(out, 0, 8, st);
   if (e != cudaSuccess) return static_cast<int>(e);
   if (n > 0)
-    checksum_u32_kernel<<<ogrid(n), 256, 0, st>>>(static_cast<const uint32_t*>(x), n,
+    pb::launch(checksum_u32_kernel, ogrid(n), 256, 0, st, static_cast<const uint32_t*>(x), n,
                                                   static_cast<unsigned long long*>(out));
   return cudaGetLastError();
 }
 
 PB_API int pb_cast_f32_bf16(const void* x, void* y, long n, float scale, cudaStream_t st) {
-  cast_f32_bf16_kernel<<<ogrid(n), 256, 0, st>>>(static_cast<const float*>(x),
+  pb::launch(cast_f32_bf16_kernel, ogrid(n), 256, 0, st, static_cast<const float*>(x),
                                                  static_cast<bf16*>(y), n, scale);
   return cudaGetLastError();
 }
 PB_API int pb_axpy_bf16_f32(const void* x, void* acc, long n, float scale, cudaStream_t st) {
-  axpy_bf16_f32_kernel<<<ogrid(n), 256, 0, st>>>(static_cast<const bf16*>(x),
+  pb::launch(axpy_bf16_f32_kernel, ogrid(n), 256, 0, st, static_cast<const bf16*>(x),
                                                  static_cast<float*>(acc), n, scale);
   return cudaGetLastError();
 }
 PB_API int pb_transpose_bf16(const void* in, void* out, int batch, int rows, int cols,
                              cudaStream_t st) {
   dim3 grid((cols + 31) / 32, (rows + 31) / 32, batch);
-  transpose_bf16_kernel<<<grid, dim3(32, 8), 0, st>>>(static_cast<const bf16*>(in),
+  pb::launch(transpose_bf16_kernel, grid, dim3(32, 8), 0, st, static_cast<const bf16*>(in),
                                                       static_cast<bf16*>(out), rows, cols);
   return cudaGetLastError();
 }
