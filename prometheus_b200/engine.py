@@ -1360,20 +1360,7 @@ class Trainer:
         m = min(rows, cols)
         g = self.ns_g[0][: nb * m * m].view(nb, m, m)
         pm = self.ns_g[1][: nb * m * m].view(nb, m, m)
-        a, b, c = T._NS_A, T._NS_B, T._NS_C
-        wide = rows <= cols
-        for _ in range(steps):
-            if wide:
-                ops.gemm(x, x, out=g)                                     # G = X X^T
-            else:
-                ops.gemm(x, x, a_mn=True, b_mn=True, out=g)               # G = X^T X
-            ops.gemm(g, g, out=pm, d=g, alpha=c, beta=b)                  # P = b G + c G^2
-            if wide:
-                ops.gemm(pm, x, b_mn=True, out=y, d=x, alpha=1.0, beta=a)  # aX + P X
-            else:
-                ops.gemm(x, pm, out=y, d=x, alpha=1.0, beta=a)            # aX + X P
-            x, y = y, x
-        return x
+        return ops.newton_schulz(x, y, g, pm, steps, T._NS_A, T._NS_B, T._NS_C)
 
     def optimizer_step(self, lr_mult: float, gscale: float = 1.0) -> None:
         """Clip, AdamW slabs, batched Muon on the owned matrices; refreshes the bf16 working

@@ -128,6 +128,20 @@ def _gemm_2d(a: Tensor, b: Tensor, a_mn: bool, b_mn: bool, out: Tensor | None, o
     return out
 
 
+def newton_schulz(x: Tensor, y: Tensor, g: Tensor, pm: Tensor, steps: int, a: float, b: float, c: float) -> Tensor:
+    """``steps`` quintic Newton-Schulz iterations over a batch of matrices ``x`` (nb, rows, cols) bf16: the products
+    ``gemm`` would be called for, issued by one call. ``y`` like ``x``, ``g`` and ``pm`` (nb, m, m) with m the smaller
+    side are overwritten; returns ``x`` or ``y``, whichever holds the result."""
+    nb, rows, cols = x.shape
+    m = min(rows, cols)
+    assert y.shape == x.shape and g.shape == pm.shape == (nb, m, m)
+    assert all(t.dtype == BF16 and t.is_cuda and t.is_contiguous() for t in (x, y, g, pm))
+    call("pb_newton_schulz", ptr(x), ptr(y), ptr(g), ptr(pm), rows, cols, nb, int(steps), float(a), float(b), float(c),
+         ptr(status_word(x.device)), stream_ptr())
+    _lib.launch_count += 3 * int(steps) - 1
+    return y if steps % 2 else x
+
+
 def gemm_ref(a, b, *, a_mn=False, b_mn=False, d=None, alpha=1.0, beta=0.0):
     af = a.float().transpose(-1, -2) if a_mn else a.float()
     bf = b.float().transpose(-1, -2) if b_mn else b.float()

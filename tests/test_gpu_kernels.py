@@ -814,6 +814,24 @@ def test_delta_compose(n_seq, n_seg, reverse):
             assert (p_tot.double() - tot).norm() <= 1e-5 * tot.norm()
 
 
+@pytest.mark.parametrize("rows,cols,nb,steps", [(64, 64, 1, 1), (128, 264, 3, 5), (264, 128, 2, 5), (256, 1024, 3, 4), (8, 1024, 2, 0)])
+def test_newton_schulz_is_its_products(rows, cols, nb, steps):
+    """One call against the products it stands for, bit for bit: both orientations, odd and even step counts."""
+    from prometheus_b200 import train
+    from prometheus_b200.ops import functional as ops
+
+    x = _r(nb, rows, cols, seed=rows + cols, scale=(rows * cols) ** -0.5)
+    m, wide = min(rows, cols), rows <= cols
+    a, b, c = train._NS_A, train._NS_B, train._NS_C
+    ref = x.clone()
+    for _ in range(steps):
+        g = ops.gemm(ref, ref) if wide else ops.gemm(ref, ref, a_mn=True, b_mn=True)
+        p = ops.gemm(g, g, d=g, alpha=c, beta=b)
+        ref = ops.gemm(p, ref, b_mn=True, d=ref, beta=a) if wide else ops.gemm(ref, p, d=ref, beta=a)
+    g, p = (torch.empty(nb, m, m, dtype=BF16, device="cuda") for _ in range(2))
+    assert torch.equal(ops.newton_schulz(x, torch.empty_like(x), g, p, steps, a, b, c), ref)
+
+
 @pytest.mark.parametrize("S,close", [(1, False), (16, True), (17, True), (33, True), (64, True), (100, False), (640, True)])
 def test_delta_chunk_inverse(S, close):
     """T = (I + diag(beta) tril(K K^T, -1))^-1 of every chunk, block by block, against float64. ``close``: keys that
