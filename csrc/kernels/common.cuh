@@ -360,6 +360,15 @@ __device__ __forceinline__ void tma_store_3d_hint(const void* tmap, const void* 
       "r"(smem_u32(smem_src)), "r"(x), "r"(y), "r"(z), "l"(policy)
       : "memory");
 }
+// Adds the fp32 tile to the matrix instead of storing it.
+__device__ __forceinline__ void tma_add_3d_hint(const void* tmap, const void* smem_src, int32_t x, int32_t y, int32_t z,
+                                                uint64_t policy) {
+  asm volatile(
+      "cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group.L2::cache_hint [%0, {%2, %3, %4}], "
+      "[%1], %5;" ::"l"(reinterpret_cast<uint64_t>(tmap)),
+      "r"(smem_u32(smem_src)), "r"(x), "r"(y), "r"(z), "l"(policy)
+      : "memory");
+}
 __device__ __forceinline__ void tma_store_commit() {
   asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
@@ -456,28 +465,10 @@ __device__ __forceinline__ uint32_t cluster_map(uint32_t local_smem_addr, uint32
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_smem_addr), "r"(cta));
   return r;
 }
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr)
-               : "memory");
-}
-// Bounded wait that also acquires what CTAs of the whole cluster released before arriving.
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, int* status) {
-  for (uint32_t it = 0; it < PB_MBAR_SPIN_LIMIT; ++it) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    if (ok) return true;
-    if ((it & 1023u) == 1023u && status != nullptr &&
-        *reinterpret_cast<volatile int*>(status) != PB_OK)
-      return false;
-  }
-  if (status != nullptr) atomicCAS(status, PB_OK, PB_TIMEOUT_MBAR);
-  return false;
+// Arrival on a barrier of a CTA of the cluster, with the scope of this CTA: for handing over tensor memory, which the
+// tcgen05 fences order. Released to the cluster an arrival waits about 1800 clocks for the thread's earlier writes.
+__device__ __forceinline__ void mbar_arrive_peer(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 // Tile load of a CTA pair: the bytes land in this CTA's shared memory, the completion is
 // counted on the barrier at `bar_cluster_addr`, which may live in the peer CTA.

@@ -500,8 +500,7 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
           }
           tc_fence_before();
           __syncwarp();
-          if (lane == 0)
-            asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(tempty0 + a * 8) : "memory");
+          if (lane == 0) mbar_arrive_peer(tempty0 + a * 8);
         }
         if (!ok || !mine) continue;
         if (lane == 0) tma_store_wait_read<0>();

@@ -814,6 +814,22 @@ def test_delta_compose(n_seq, n_seg, reverse):
             assert (p_tot.double() - tot).norm() <= 1e-5 * tot.norm()
 
 
+@pytest.mark.parametrize("M,N,K,batch", [(8, 1024, 64, 1), (136, 264, 200, 1), (264, 1000, 72, 3), (1024, 1152, 136, 2), (4736, 512, 128, 1),
+                                         (4744, 512, 128, 1)])
+def test_gemm_accumulates_in_place_as_with_a_copy(M, N, K, batch):
+    """fp32 C += A^T B by adding stores against the same product with D elsewhere, which the epilogue reads: the same
+    bits, on tiles of 128 (up to 148 of them: 4736 x 512) and on pairs, with rows and columns cut off."""
+    from prometheus_b200.ops import functional as ops
+
+    a, b = _r(batch, K, M, seed=1), _r(batch, K, N, seed=2)
+    c = _r(batch, M, N, seed=3, dtype=torch.float32)
+    want = ops.gemm(a, b, a_mn=True, b_mn=True, out=torch.empty_like(c), d=c.clone(), beta=1.0)
+    got = ops.gemm(a, b, a_mn=True, b_mn=True, out=c, d=c, beta=1.0)
+    assert torch.equal(got, want)
+    ref = (a.double().transpose(1, 2) @ b.double()) + _r(batch, M, N, seed=3, dtype=torch.float32).double()
+    assert ((got.double() - ref).norm() / ref.norm()).item() < 1e-6
+
+
 @pytest.mark.parametrize("rows,cols,nb,steps", [(64, 64, 1, 1), (128, 264, 3, 5), (264, 128, 2, 5), (256, 1024, 3, 4), (8, 1024, 2, 0)])
 def test_newton_schulz_is_its_products(rows, cols, nb, steps):
     """One call against the products it stands for, bit for bit: both orientations, odd and even step counts."""
