@@ -88,6 +88,7 @@ _SIGS = {
     "pb_attn_bwd_cp": [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, F, P, P],
     "pb_attn_bwd": [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, F, P, P],
     "pb_delta_prep_fwd": [P, P, P, P, I, P, P, P, P, P, I, I, I, I, P, I, P],
+    "pb_delta_bwd": [P, P, P, P, I, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, P, P],
     "pb_delta_prep_bwd": [P, P, P, P, I, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, P, I, P],
     "pb_gemm_bf16_grouped": [P, P, P, I, I, I, I, L, L, L, L, I, P, P, I, P],
     "pb_gemm_bf16_grouped_wgrad": [P, P, P, P, I, I, I, I, L, L, L, L, I, I, F, P, P, P, I, P],

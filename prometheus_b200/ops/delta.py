@@ -222,7 +222,7 @@ class _DeltaFusedFn(torch.autograd.Function):
     state walk. q, k, v are read in place from their ``[B, S, H, 128]`` layout and the output
     is written in that layout; the rows a last partial chunk lacks read as zeros with beta = 0,
     which leaves the state untouched, and are not written. The chunk-local part of the backward is
-    one kernel of batched products (``pb_delta_chunk_products``) and ``pb_delta_prep_bwd``.
+    one kernel (``pb_delta_bwd``).
     ``keep``: something will run backward, so A', T, the walk's U and the bf16 states are stored.
 
     The walk is affine in the state, ``S_out = P S_in + R`` per run of chunks. When the batch
@@ -303,8 +303,7 @@ class _DeltaFusedFn(torch.autograd.Function):
         seg, cp = ctx.seg, ctx.cp
         rows, square, st128 = bh * n * 8192, bh * n * 4096, bh * n * 16384
         w, m, ap, t, u, sb = _addresses(work, rows, square, square, square, rows, st128)
-        # -dU (the walk writes it), dS', dW, the walk's dQ and dK, dM
-        grads, (ndu, dsb, d_w, d_qs, d_ks, d_m) = _carve(dev, rows, st128, rows, rows, rows, square)
+        grads, (ndu, dsb) = _carve(dev, rows, st128)     # -dU and the gradients of the states, which the walk writes
         d_out = torch.zeros_like(q) if d_out is None else _tma_ready(d_out)
         ds0 = torch.empty((bh, 128, 128), dtype=torch.float32, device=dev)
         dfin = None if d_sfin is None else d_sfin.reshape(bh, d, d).float().contiguous()
@@ -326,15 +325,10 @@ class _DeltaFusedFn(torch.autograd.Function):
                  bh, seg, 1, stream_ptr())
             call("pb_delta_scan_bwd_seg", w, ptr(q), ptr(k), m, ptr(d_out), ndu,
                  dsb, ptr(g_in), None, bh, n, seg, h, s, h * d, status, stream_ptr())
-        # dW = -dU S^T, the walk's dQ = dO S^T and dK = U dS'^T, dM = dO U^T (masked in the kernel)
-        call("pb_delta_chunk_products", ndu, ptr(d_out), u, sb, dsb, d_w, d_qs,
-             d_ks, d_m, b, s, h, h * d, status, stream_ptr())
         d_q, d_k, d_v = torch.empty_like(q), torch.empty_like(q), torch.empty_like(q)
         d_beta = torch.empty_like(beta)
-        call("pb_delta_prep_bwd", ptr(q), ptr(k), ptr(v), ptr(beta),
-             1 if beta.dtype == torch.float32 else 0, ap, t, d_w, ndu, d_m,
-             d_qs, d_ks, ptr(d_q), ptr(d_k), ptr(d_v), ptr(d_beta), b, s, h, h * d,
-             status, 0, stream_ptr())
+        call("pb_delta_bwd", ptr(q), ptr(k), ptr(v), ptr(beta), 1 if beta.dtype == torch.float32 else 0, ap, t, ndu,
+             ptr(d_out), u, sb, dsb, ptr(d_q), ptr(d_k), ptr(d_v), ptr(d_beta), b, s, h, h * d, status, stream_ptr())
         return (d_q, d_k, d_v, d_beta, (ds0.reshape(b, h, d, d) if ctx.has_s0 else None), None, None, None)
 
 

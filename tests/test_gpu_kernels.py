@@ -924,6 +924,43 @@ def test_delta_prep_bwd_kernel_matches_fp32_oracle():
     _close(db, rb, 3e-2)
 
 
+@pytest.mark.parametrize("B,S,H,fp32", [(1, 1, 1, 1), (2, 63, 3, 0), (1, 64, 2, 1), (2, 65, 1, 0), (1, 300, 80, 0), (1, 300, 80, 1)])
+def test_delta_bwd_kernel_matches_fp32_oracle(B, S, H, fp32):
+    """The chunk-local backward in one kernel against its algebra in batched fp32 PyTorch: one token, the edges of a
+    chunk, more chunks than SMs (400), both types of beta. dW, dM, dA', X and dG are rounded to bf16 once each and a
+    result once more: 2^-9 of their largest values, through at most four products whose weights have row sums of a few
+    units (|T|, |A'|, |K K^T| of 64 random unit keys), stays under 3e-2 of the result's scale."""
+    from prometheus_b200.ops import delta as dl
+    from prometheus_b200.ops import functional as ops
+    from prometheus_b200.ops._lib import call, ptr, stream_ptr
+
+    D, n = 128, -(-S // 64)
+    G, pad = B * H * n, n * 64 - S
+    q, k = (torch.nn.functional.normalize(_r(B, S, H, D, seed=i).float(), dim=-1).to(BF16) for i in (1, 2))
+    v, d_out = _r(B, S, H, D, seed=3), _r(B, S, H, D, seed=5, scale=0.5)
+    beta = torch.sigmoid(_r(B, S, H, seed=4).float()).to(torch.float32 if fp32 else BF16)
+    ap, t = (torch.empty(G, 64, 64, dtype=BF16, device="cuda") for _ in range(2))
+    w, uh = (torch.empty(G, 64, D, dtype=BF16, device="cuda") for _ in range(2))
+    m, st = torch.empty_like(ap), ptr(ops.status_word("cuda"))
+    call("pb_delta_prep_fwd", ptr(q), ptr(k), ptr(v), ptr(beta), fp32, ptr(w), ptr(uh), ptr(m), ptr(ap), ptr(t), B, S, H,
+         H * D, st, 0, stream_ptr())
+    ndu, u = _r(G, 64, D, seed=11, scale=0.5), _r(G, 64, D, seed=12, scale=0.5)
+    sb, dsb = _r(G, D, D, seed=13, scale=0.1), _r(G, D, D, seed=14, scale=0.1)
+    dq, dk, dv = (torch.full_like(q, float("nan")) for _ in range(3))
+    db = torch.full_like(beta, float("nan"))
+    call("pb_delta_bwd", ptr(q), ptr(k), ptr(v), ptr(beta), fp32, ptr(ap), ptr(t), ptr(ndu), ptr(d_out), ptr(u), ptr(sb),
+         ptr(dsb), ptr(dq), ptr(dk), ptr(dv), ptr(db), B, S, H, H * D, st, stream_ptr())
+    torch.cuda.synchronize()
+    ops.check_status("cuda")
+    full = lambda x: torch.nn.functional.pad(x, (0, 0) * (x.dim() - 2) + (0, pad))
+    doc = dl._to_chunks(full(d_out), n).float()
+    d_w, d_m = ndu.float() @ sb.float().transpose(1, 2), doc @ u.float().transpose(1, 2)
+    d_qs, d_ks = doc @ sb.float().transpose(1, 2), u.float() @ dsb.float().transpose(1, 2)
+    want = dl.delta_prep_backward_ref(full(q), full(k), full(v), full(beta), ap, t, d_w, ndu, d_m, d_qs, d_ks)
+    for got, ref in zip((dq, dk, dv, db), want):
+        _close(got, ref[:, :S], 3e-2)
+
+
 def test_debug_bounds_build_records_and_skips_a_bad_index():
     """The -DPB_DEBUG_BOUNDS library: an index that comes from data and leaves its range is
     recorded as (kernel, index, limit) and the access is skipped; the kernel finishes and the
