@@ -518,6 +518,45 @@ def test_softcap_ce_accumulator_from_saved_tensor_hooks(form):
         assert torch.equal(got, want)
 
 
+@pytest.mark.parametrize("rows,form", [(1, ""), (63, ""), (256, ""), (257, ""), (130, "h rewritten"), (130, "bf16 double"),
+                                       (130, "shifted"), (130, "transposed"), (130, "batched"), (130, "graph")])
+def test_softcap_ce_unembedding_gradient_in_the_backward(rows, form):
+    """One chunk of at most 2 d rows (256 here): dU is a product of the backward, scaled in its epilogue. fp32 sums times
+    the factor, rounded once, are bit for bit the accumulating form's buffer times the factor. The saved
+    tensors in other forms, an h that was reused, and batched or differentiated upstream gradients give the same."""
+    from prometheus_b200.ops import functional as ops
+
+    d, V, cap = 128, 1032, 30.0
+    h, U = _r(rows, d, seed=3), _r(V, d, seed=4, scale=0.1)
+    tgt = torch.randint(0, V, (rows,), device="cuda", dtype=torch.int32)
+    wt = torch.full((rows,), 1.0 / rows, device="cuda")
+    Um = U.clone().requires_grad_(True)
+    Um.main_grad = torch.zeros(V, d, device="cuda")
+    ops.softcap_cross_entropy(h, Um, tgt, wt, cap)
+    want = (Um.main_grad * 2.5).to(BF16)
+
+    def unpack(t):
+        if form == "bf16 double":
+            return t.double()
+        if form == "transposed":
+            return t.t().contiguous().t()
+        return torch.empty(t.numel() + 1, dtype=t.dtype, device="cuda")[1:].view(t.shape).copy_(t)
+
+    Ug, hg = U.clone().requires_grad_(True), h.clone()
+    hooks = form in ("bf16 double", "shifted", "transposed")
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, unpack if hooks else (lambda t: t)):
+        loss = ops.softcap_cross_entropy(hg, Ug, tgt, wt, cap)
+    if form == "h rewritten":
+        hg.zero_()
+    if form == "batched":
+        (gU,) = torch.autograd.grad(loss, (Ug,), torch.tensor([2.5, 1.0], device="cuda"), is_grads_batched=True)
+        assert torch.equal(gU[1], Um.main_grad.to(BF16))
+        gU = gU[0]
+    else:
+        (gU,) = torch.autograd.grad(2.5 * loss, (Ug,), create_graph=form == "graph")
+    assert torch.equal(gU.detach(), want)
+
+
 def test_optimizer_kernels():
     from prometheus_b200 import train
     from prometheus_b200.ops import _lib
