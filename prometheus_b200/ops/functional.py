@@ -489,7 +489,7 @@ class _SoftcapCeFn(torch.autograd.Function):
     during the forward. Where one chunk is all and d(loss)/d(logits) is no larger than an fp32 dU (rows <= 2 d), that is what
     waits for the backward instead: dU is then one product that takes the upstream gradient as a factor and stores bf16,
     and neither an fp32 dU nor the pass that scales and rounds it moves (forward + backward of 64 / 512 / 4096 rows
-    x 2048 x 131072: 1328 / 1417 / 5891 us -> 821 / 1095 / 5569). Under a cap, and where
+    x 2048 x 131072: 889 / 1183 / 5900 us -> 382 / 861 / 5580). Under a cap, and where
     it is the faster way (``pb_gemm_softcap_pays``), the product's epilogue adds up each row's
     exponentials, so the CE kernel reads the logits once instead of twice."""
 

@@ -557,6 +557,37 @@ def test_softcap_ce_unembedding_gradient_in_the_backward(rows, form):
     assert torch.equal(gU.detach(), want)
 
 
+@pytest.mark.parametrize("M,N,K,batch,a_mn,b_mn,out,d", [
+    (1, 8, 1024, 1, 0, 0, "bf16", ""), (129, 128, 1088, 1, 0, 0, "f32", "bf16"), (64, 1, 1032, 1, 0, 0, "bf16", "f32"),
+    (72, 520, 2048, 1, 1, 1, "f32", "same"), (300, 700, 4104, 1, 0, 0, "bf16", "bf16"), (128, 264, 1024, 9, 0, 1, "bf16", "f32"),
+    (1024, 1152, 1536, 1, 1, 1, "f32", "same"), (1024, 1160, 1536, 1, 1, 0, "bf16", ""), (1152, 1024, 1024, 1, 0, 0, "f32", "f32")])
+def test_gemm_split_contraction(M, N, K, batch, a_mn, b_mn, out, d):
+    """Products with few tiles and a long contraction, shared out over clusters of two to eight CTAs: one element, ragged
+    edges and unaligned rows, contractions that do not divide evenly, batches, 72 tiles (split), 80 (not), every kind of D.
+    fp32 sums: each product K u of its absolute terms, then the output's rounding. Two runs give the same bits."""
+    from prometheus_b200.ops import functional as ops
+
+    a = _r(batch, *((K, M) if a_mn else (M, K)), seed=1)
+    b = _r(batch, *((K, N) if b_mn else (N, K)), seed=2)
+    ty = BF16 if out == "bf16" else torch.float32
+    dt = {"": None, "bf16": BF16, "f32": torch.float32, "same": ty}[d]
+    dd = None if dt is None else _r(batch, M, N, seed=3).to(dt)
+    runs = []
+    for _ in range(2):
+        c = dd.clone() if d == "same" else torch.full((batch, M, N), float("nan"), dtype=ty, device="cuda")
+        add = c if d == "same" else dd
+        runs.append(ops.gemm(a, b, a_mn=bool(a_mn), b_mn=bool(b_mn), out=c, d=add, alpha=0.5, beta=0.75 if d != "same" else 1.0))
+    assert torch.equal(runs[0], runs[1])
+    ad = a.double().transpose(1, 2) if a_mn else a.double()
+    bd = b.double() if b_mn else b.double().transpose(1, 2)
+    ref, slack = 0.5 * ad @ bd, 0.5 * ad.abs() @ bd.abs()
+    if dd is not None:
+        ref = ref + (0.75 if d != "same" else 1.0) * dd.double()
+        slack = slack + dd.double().abs()
+    tol = (K + 8) * 2.0 ** -24 * slack + (2.0 ** -8 if out == "bf16" else 0.0) * ref.abs()
+    assert bool(((runs[0].double() - ref).abs() <= tol).all())
+
+
 def test_optimizer_kernels():
     from prometheus_b200 import train
     from prometheus_b200.ops import _lib
