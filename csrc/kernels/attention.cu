@@ -66,7 +66,7 @@ __device__ __forceinline__ float ex2(float x) {
 }
 // 16-byte store of 8 bf16 into a [rows][64] 128B-swizzled chunk (row pitch 128 bytes).
 __device__ __forceinline__ void st_swz(uint8_t* chunk_base, int row, int c16, const bf16x8& v) {
-  *reinterpret_cast<bf16x8*>(chunk_base + row * 128 + ((c16 ^ (row & 7)) << 4)) = v;
+  st_shared8(chunk_base + row * 128 + ((c16 ^ (row & 7)) << 4), v);
 }
 __device__ __forceinline__ bf16x8 pack_bf16x8(const float* f) {
   bf16x8 pk;
@@ -634,8 +634,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
         auto lanes = [&](const int i) -> float2 {   // 16-byte piece i: two lanes' partial sums
           const int off = (i >> 3) * 16384 + r * 128 + (((i & 7) ^ (r & 7)) << 4);
           float x[8], y[8];
-          unpack8(*reinterpret_cast<const bf16x8*>(smem + RB_OFF + off), x);
-          unpack8(*reinterpret_cast<const bf16x8*>(stage(O_STAGE) + off), y);
+          unpack8(ld_shared8(smem + RB_OFF + off), x);
+          unpack8(ld_shared8(stage(O_STAGE) + off), y);
           float t[4];   // products of bf16 values are exact
 #pragma unroll
           for (int e = 0; e < 4; ++e) t[e] = fmaf(x[2 * e], y[2 * e], x[2 * e + 1] * y[2 * e + 1]);

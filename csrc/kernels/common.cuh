@@ -146,6 +146,28 @@ __device__ __forceinline__ bf16x8 pack8(const float* f) {
   return p;
 }
 
+// Eight bf16 from and to shared memory in one 16-byte access. Through a pointer to the struct the compiler may make four
+// of 4 bytes of it, and lanes that each own a 128-byte row then meet four at a bank.
+__device__ __forceinline__ bf16x8 ld_shared8(const void* p) {
+  uint32_t w[4];
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3])
+               : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(p)))
+               : "memory");
+  bf16x8 v;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) v.v[i] = *reinterpret_cast<const bf162*>(&w[i]);
+  return v;
+}
+__device__ __forceinline__ void st_shared8(void* p, const bf16x8& v) {
+  uint32_t w[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) w[i] = *reinterpret_cast<const uint32_t*>(&v.v[i]);
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(p))),
+               "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3])
+               : "memory");
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

@@ -64,7 +64,7 @@ __device__ __forceinline__ void tie(float (&f)[N]) {
                       "+f"(f[i + 6]), "+f"(f[i + 7]));
 }
 __device__ __forceinline__ void put8(uint8_t* tile, int row, int col, const float* f) {
-  *reinterpret_cast<bf16x8*>(tile + (col >> 6) * 8192 + row * 128 + ((((col & 63) >> 3) ^ (row & 7)) << 4)) = pack8(f);
+  st_shared8(tile + (col >> 6) * 8192 + row * 128 + ((((col & 63) >> 3) ^ (row & 7)) << 4), pack8(f));
 }
 
 __global__ void __launch_bounds__(THREADS, 1)

@@ -148,7 +148,7 @@ delta_chunk_kernel(const __grid_constant__ CUtensorMap tmNDU, const __grid_const
 #pragma unroll
           for (int j = 0; j < 4; ++j)
             pk.v[j] = __floats2bfloat162_rn(__uint_as_float(v[8 * i + 2 * j]), __uint_as_float(v[8 * i + 2 * j + 1]));
-          *reinterpret_cast<bf16x8*>(out + (c >> 6) * 8192 + r * 128 + ((i ^ (r & 7)) << 4)) = pk;
+          st_shared8(out + (c >> 6) * 8192 + r * 128 + ((i ^ (r & 7)) << 4), pk);
         }
       }
       tc_fence_before();

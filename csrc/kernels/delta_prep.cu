@@ -56,7 +56,7 @@ struct Params {
 };
 
 __device__ __forceinline__ void st_swz(uint8_t* tile, int row, int c16, const bf16x8& v) {
-  *reinterpret_cast<bf16x8*>(tile + row * 128 + ((c16 ^ (row & 7)) << 4)) = v;
+  st_shared8(tile + row * 128 + ((c16 ^ (row & 7)) << 4), v);
 }
 
 // Row `row` of a 64-column fp32 accumulator block -> bf16 [64][64] swizzled tile, keeping
@@ -423,7 +423,7 @@ __device__ __forceinline__ void row64_to_tile(uint32_t taddr, uint8_t* tiles, in
       for (int j = 0; j < 8; ++j) o[j] = sign * f[8 * i + j];
       if (add) {
         float a[8];
-        unpack8(*reinterpret_cast<const bf16x8*>(tile + row * 128 + ((c16 ^ (row & 7)) << 4)), a);
+        unpack8(ld_shared8(tile + row * 128 + ((c16 ^ (row & 7)) << 4)), a);
 #pragma unroll
         for (int j = 0; j < 8; ++j) o[j] += a[j];
       }
@@ -556,13 +556,13 @@ delta_prep_bwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int c16 = (c32 >> 3) + i;
-        bf16x8* cell = reinterpret_cast<bf16x8*>(smem + DM + r * 128 + ((c16 ^ (r & 7)) << 4));
+        uint8_t* cell = smem + DM + r * 128 + ((c16 ^ (r & 7)) << 4);
         if (8 * c16 + 7 > r) {
           float f[8];
-          unpack8(*cell, f);
+          unpack8(ld_shared8(cell), f);
 #pragma unroll
           for (int j = 0; j < 8; ++j) if (8 * c16 + j > r) f[j] = 0.f;
-          *cell = pack8(f);
+          st_shared8(cell, pack8(f));
         }
       }
     }

@@ -323,16 +323,10 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     auto put_cols = [&](uint8_t* tile, int rows, const uint32_t (&v)[WC]) {
 #pragma unroll
       for (int i = 0; i < WC / 8; ++i) {
-        uint32_t pk[4];
+        float f[8];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(v[8 * i + 2 * j]), __uint_as_float(v[8 * i + 2 * j + 1]));
-          pk[j] = *reinterpret_cast<const uint32_t*>(&h);
-        }
-        // one 16-byte store: as four of 4 bytes, which the compiler may make of a struct, each is a
-        // four-way bank conflict
-        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(smem_u32(piece(tile, rows, i))), "r"(pk[0]),
-                     "r"(pk[1]), "r"(pk[2]), "r"(pk[3]) : "memory");
+        for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(v[8 * i + j]);
+        st_shared8(piece(tile, rows, i), pack8(f));
       }
     };
     {
@@ -404,7 +398,7 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
         if (EARLY && !lin) {
           wait(&full[it & 1], (it >> 1) & 1);
 #pragma unroll
-          for (int i = 0; i < WC / 8; ++i) uh[EARLY ? i : 0] = *reinterpret_cast<const bf16x8*>(piece(ut, C, i));
+          for (int i = 0; i < WC / 8; ++i) uh[EARLY ? i : 0] = ld_shared8(piece(ut, C, i));
         }
         wait(y_done, cph);
         uint32_t v[WC];
@@ -416,14 +410,14 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
           for (int j = 0; j < 8; ++j) y[j] = __uint_as_float(v[8 * i + j]);
           if (!BWD && !lin) {
             float uhv[8];
-            unpack8(EARLY ? uh[EARLY ? i : 0] : *reinterpret_cast<const bf16x8*>(piece(ut, C, i)), uhv);
+            unpack8(EARLY ? uh[EARLY ? i : 0] : ld_shared8(piece(ut, C, i)), uhv);
 #pragma unroll
             for (int j = 0; j < 8; ++j) y[j] = uhv[j] - y[j];  // U = U^ - W S
           } else {
 #pragma unroll
             for (int j = 0; j < 8; ++j) y[j] = -y[j];          // operand (and output) is -dU
           }
-          *reinterpret_cast<bf16x8*>(piece(ub, C, i)) = pack8(y);
+          st_shared8(piece(ub, C, i), pack8(y));
         }
         arrive(u_ready);
         if (store_ux) {

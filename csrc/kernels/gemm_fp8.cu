@@ -285,7 +285,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 #pragma unroll
           for (int j = 0; j < 4; ++j)
             pk.v[j] = __floats2bfloat162_rn(acc[sl * 64 + 8 * i + 2 * j], acc[sl * 64 + 8 * i + 2 * j + 1]);
-          *reinterpret_cast<bf16x8*>(rowp + ((i ^ (lane & 7)) << 4)) = pk;
+          st_shared8(rowp + ((i ^ (lane & 7)) << 4), pk);
         }
         fence_proxy_async_smem();
         __syncwarp();
@@ -507,7 +507,7 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         __syncwarp();
         uint8_t* rowp = buf + lane * 128;
 #pragma unroll
-        for (int c = 0; c < 8; ++c) *reinterpret_cast<bf16x8*>(rowp + ((c ^ (lane & 7)) << 4)) = pack8(acc + 8 * c);
+        for (int c = 0; c < 8; ++c) st_shared8(rowp + ((c ^ (lane & 7)) << 4), pack8(acc + 8 * c));
         fence_proxy_async_smem();
         __syncwarp();
         const int x0 = n_blk * BN + cg * P_COLS;
