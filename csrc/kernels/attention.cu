@@ -168,7 +168,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint64_t* o_done = bars + 17;    // [tile][buf]: P V of the block whose scores that buffer held
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 22);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   // blocks start in index order, so the row block is the slowest index: the longest rows of all heads and
   // batch entries first, the shortest fill the gaps at the end. One grid dimension for all three: the others end
   // at 65535 blocks
@@ -222,7 +222,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
     }
   } else if (warp >= 8) {
-    if (lane == 0) {
+    {
       const int t = warp - 8;                                     // the tile this thread issues for
       const int nj = nj1 - (t == 0 ? 2 : 0);
       const uint32_t id_s = make_idesc(1, 1, 128, 64, 0, 0);     // S = Q K^T, N = 64 keys
@@ -232,21 +232,21 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const uint32_t q_lo = sdesc_lo(smem_u32(smem + Q_OFF + t * 32768), 16);
       const uint32_t kv0 = smem_u32(smem + KV_OFF);
       const uint32_t d_o = tmem + COL_O + t * 128;
-      bool ok = mbar_wait_spin(q_full, 0, p.status);
+      bool ok = mbar_wait_spin_warp(q_full, 0, p.status);
       auto issue_s = [&](int j) -> bool {
         const int s = j % KV_STAGES;
         const int sb = t * 2 + (j & 1);
-        if (!mbar_wait_spin(&kv_full[s], (j / KV_STAGES) & 1, p.status)) return false;
+        if (!mbar_wait_spin_warp(&kv_full[s], (j / KV_STAGES) & 1, p.status)) return false;
         // the buffer still holds P of block j - 2 until its P V product is done
-        if (j >= 2 && !mbar_wait_spin(&o_done[sb], ((j - 2) >> 1) & 1, p.status)) return false;
+        if (j >= 2 && !mbar_wait_spin_warp(&o_done[sb], ((j - 2) >> 1) & 1, p.status)) return false;
         tc_fence_after();
         const uint32_t k_lo = sdesc_lo(kv0 + s * KV_STAGE, 16);
         const uint32_t d = tmem + COL_S + sb * 64;
 #pragma unroll
         for (int jj = 0; jj < 8; ++jj)
-          umma_f16_words(d, q_lo + (((jj >> 2) * 16384 + (jj & 3) * 32) >> 4), HI,
+          umma_f16_words_warp(d, q_lo + (((jj >> 2) * 16384 + (jj & 3) * 32) >> 4), HI,
                          k_lo + (((jj >> 2) * 8192 + (jj & 3) * 32) >> 4), HI, id_s, jj > 0);
-        umma_commit(&s_done[sb]);
+        umma_commit_warp(&s_done[sb]);
         return true;
       };
       // the scores run two blocks ahead of the P V products, so neither the row warps nor
@@ -255,17 +255,17 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       if (ok && nj > 1) ok = issue_s(1);
       for (int j = 0; j < nj && ok; ++j) {
         const int s = j % KV_STAGES;
-        if (!mbar_wait_spin(&p_ready[t], j & 1, p.status)) break;
+        if (!mbar_wait_spin_warp(&p_ready[t], j & 1, p.status)) break;
         tc_fence_after();
         const uint32_t v_lo = sdesc_lo(kv0 + s * KV_STAGE + 16384, 8192);
         // 16 values of a bf16 operand row are eight tensor-memory columns
         const uint32_t p_col = tmem + COL_S + (t * 2 + (j & 1)) * 64;
 #pragma unroll
         for (int jj = 0; jj < 4; ++jj)
-          umma_f16_ts(d_o, p_col + jj * 8, (static_cast<uint64_t>(HI) << 32) | (v_lo + ((jj * 2048) >> 4)), id_o,
+          umma_f16_ts_warp(d_o, p_col + jj * 8, (static_cast<uint64_t>(HI) << 32) | (v_lo + ((jj * 2048) >> 4)), id_o,
                       (j > 0) || (jj > 0));
-        umma_commit(&o_done[t * 2 + (j & 1)]);
-        umma_commit(&kv_empty[s]);   // needs both tiles' commits (tile 0 skips the last two blocks,
+        umma_commit_warp(&o_done[t * 2 + (j & 1)]);
+        umma_commit_warp(&kv_empty[s]);   // needs both tiles' commits (tile 0 skips the last two blocks,
                                      // whose stages are never refilled)
         if (j + 2 < nj && !issue_s(j + 2)) break;
       }
@@ -472,7 +472,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
   constexpr int STAGES = Ring<DKV>::STAGES, O_STAGE = 3;
   auto stage = [&](int s) { return smem + Ring<DKV>::off(s); };
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int group = p.heads / p.kv_heads;
   // dQ: heavy blocks are the late query blocks; dKV: the early key blocks. Heavy blocks of all heads and
   // batch entries come first, in one grid dimension, as in the forward.
@@ -553,20 +553,20 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
     }
   } else if (warp == 8 || warp == 9) {
     // score products: warp 8 issues X1 = RA T1^T, warp 9 issues X2 = RB T2^T
-    if (lane == 0) {
+    {
       const int which = warp - 8;
       const uint32_t id_x = make_idesc(1, 1, 128, 64, 0, 0);     // A K-major, B K-major, N = 64
       constexpr uint32_t HI = sdesc_hi_sw128(1024);
       const uint32_t r_lo = sdesc_lo(smem_u32(smem + (which == 0 ? RA_OFF : RB_OFF)), 16);
       const uint32_t r_col = tmem + COL_R + which * 64;
       const uint32_t col = which == 0 ? 0 : COL_X2;
-      bool ok = n_it == 0 || mbar_wait_spin(DKV ? r_full : r_read, 0, p.status);
+      bool ok = n_it == 0 || mbar_wait_spin_warp(DKV ? r_full : r_read, 0, p.status);
       int ts = 0;
       uint32_t ph = 0;
       for (int it = 0; it < n_it && ok; ++it) {
         const int s = it & 1;
-        if (!mbar_wait_spin(&t_full[ts], ph, p.status)) break;
-        if (!mbar_wait_spin(&x_free[s], ((it >> 1) & 1) ^ 1, p.status)) break;
+        if (!mbar_wait_spin_warp(&t_full[ts], ph, p.status)) break;
+        if (!mbar_wait_spin_warp(&x_free[s], ((it >> 1) & 1) ^ 1, p.status)) break;
         tc_fence_after();
         const uint32_t t_lo = sdesc_lo(smem_u32(stage(ts)) + which * 16384, 16);
         const uint32_t d = tmem + col + s * 128;
@@ -574,23 +574,23 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
         for (int jj = 0; jj < 8; ++jj) {
           const uint32_t b_lo = t_lo + (((jj >> 2) * 8192 + (jj & 3) * 32) >> 4);
           if (DKV)
-            umma_f16_words(d, r_lo + (((jj >> 2) * 16384 + (jj & 3) * 32) >> 4), HI, b_lo, HI, id_x, jj > 0);
+            umma_f16_words_warp(d, r_lo + (((jj >> 2) * 16384 + (jj & 3) * 32) >> 4), HI, b_lo, HI, id_x, jj > 0);
           else
-            umma_f16_ts(d, r_col + jj * 8, (static_cast<uint64_t>(HI) << 32) | b_lo, id_x, jj > 0);
+            umma_f16_ts_warp(d, r_col + jj * 8, (static_cast<uint64_t>(HI) << 32) | b_lo, id_x, jj > 0);
         }
-        umma_commit(&x_done[s]);
+        umma_commit_warp(&x_done[s]);
         if (++ts == STAGES) { ts = 0; ph ^= 1; }
       }
     }
   } else if (warp == 10) {
-    // gradient accumulations, all from this one thread so that they stay ordered
-    if (lane == 0) {
+    // gradient accumulations, all from this one warp so that they stay ordered
+    {
       const uint32_t id_acc = make_idesc(1, 1, 128, 128, 0, 1);  // A from tensor memory, B MN-major
       constexpr uint64_t HI = static_cast<uint64_t>(sdesc_hi_sw128(1024)) << 32;
       int it = 0, ts = 0;
       for (; it < n_it; ++it) {
         const int s = it & 1;
-        if (!mbar_wait_spin(&pd_ready[s], (it >> 1) & 1, p.status)) break;
+        if (!mbar_wait_spin_warp(&pd_ready[s], (it >> 1) & 1, p.status)) break;
         tc_fence_after();
         // the streamed tiles again, now as MN-major B operands (64-wide chunks 8 KB apart); 16
         // values of a bf16 operand row are eight tensor-memory columns, 32 of them to a warpgroup's part
@@ -599,21 +599,21 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
         auto a_col = [](const int jj) { return static_cast<uint32_t>((jj >> 1) * 32 + (jj & 1) * 8); };
 #pragma unroll
         for (int jj = 0; jj < 4; ++jj)
-          umma_f16_ts(tmem + COL_ACC1, xb + COL_X2 + a_col(jj), HI | (t1_mn + ((jj * 2048) >> 4)), id_acc,
+          umma_f16_ts_warp(tmem + COL_ACC1, xb + COL_X2 + a_col(jj), HI | (t1_mn + ((jj * 2048) >> 4)), id_acc,
                       (it > 0) || (jj > 0));
         if (DKV) {
 #pragma unroll
           for (int jj = 0; jj < 4; ++jj)
-            umma_f16_ts(tmem + COL_ACC2, xb + a_col(jj), HI | (t2_mn + ((jj * 2048) >> 4)), id_acc,
+            umma_f16_ts_warp(tmem + COL_ACC2, xb + a_col(jj), HI | (t2_mn + ((jj * 2048) >> 4)), id_acc,
                         (it > 0) || (jj > 0));
         }
         // the score products of this tile finished before the row warps could signal pd_ready,
         // so the completion of these MMAs releases the whole stage and the score buffer
-        umma_commit(&t_empty[ts]);
-        umma_commit(&x_free[s]);
+        umma_commit_warp(&t_empty[ts]);
+        umma_commit_warp(&x_free[s]);
         if (++ts == STAGES) ts = 0;
       }
-      if (it == n_it) umma_commit(acc_done);
+      if (it == n_it) umma_commit_warp(acc_done);
     }
   } else {
     const int wg = warp >> 2;          // warpgroup = half of a tile's columns

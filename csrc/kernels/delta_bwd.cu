@@ -99,7 +99,7 @@ delta_bwd_kernel(const __grid_constant__ CUtensorMap tmNDU, const __grid_constan
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
   __shared__ float dbeta_part[4][C];
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     mbar_init(full0, 2);
     for (int i = 1; i < 10; ++i) mbar_init(bars + i, 1);
@@ -169,7 +169,7 @@ delta_bwd_kernel(const __grid_constant__ CUtensorMap tmNDU, const __grid_constan
       if (ok && mbar_wait(mv, ph, p.status)) load_q(g - step);   // the last chunk's (the grid is at most the chunks)
     }
   } else if (warp == 3) {
-    if (lane == 0) {
+    {
       const uint32_t id_kk = make_idesc(1, 1, 128, 128, 0, 0), id_kk64 = make_idesc(1, 1, 128, 64, 0, 0);
       const uint32_t id_mm = make_idesc(1, 1, 128, 128, 1, 1), id_mm64 = make_idesc(1, 1, 128, 64, 1, 1);
       const uint32_t id_kn = make_idesc(1, 1, 128, 128, 0, 1);
@@ -180,67 +180,67 @@ delta_bwd_kernel(const __grid_constant__ CUtensorMap tmNDU, const __grid_constan
       auto kk128 = [&](int tile, int j) { return base_k + ((tile + (j >> 2) * 16384 + (j & 3) * 32) >> 4); };
       auto first_products = [&] {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) umma_f16_lo(tmem + COL_W, kk(NDU, j), kk128(ST, j), id_kk, j > 0);
+        for (int j = 0; j < 8; ++j) umma_f16_lo_warp(tmem + COL_W, kk(NDU, j), kk128(ST, j), id_kk, j > 0);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) umma_f16_lo(tmem + COL_A, kk(DO, j), kk(UT, j), id_kk64, j > 0);
-        umma_commit(m0);
+        for (int j = 0; j < 8; ++j) umma_f16_lo_warp(tmem + COL_A, kk(DO, j), kk(UT, j), id_kk64, j > 0);
+        umma_commit_warp(m0);
       };
       uint32_t ph = 0;
-      if (static_cast<int>(blockIdx.x) < p.total && mbar_wait_spin(full0, 0, p.status)) {
+      if (static_cast<int>(blockIdx.x) < p.total && mbar_wait_spin_warp(full0, 0, p.status)) {
         tc_fence_after();
         first_products();
         for (int g = blockIdx.x; g < p.total; g += step, ph ^= 1) {
-          if (!mbar_wait_spin(acc_read, ph ^ 1, p.status)) break;
+          if (!mbar_wait_spin_warp(acc_read, ph ^ 1, p.status)) break;
           tc_fence_after();
 #pragma unroll
-          for (int j = 0; j < 8; ++j) umma_f16_lo(tmem + COL_Q, kk(DO, j), kk128(ST, j), id_kk, j > 0);
+          for (int j = 0; j < 8; ++j) umma_f16_lo_warp(tmem + COL_Q, kk(DO, j), kk128(ST, j), id_kk, j > 0);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) umma_f16_lo(tmem + COL_K, kk(UT, j), kk128(DS, j), id_kk, j > 0);
-          umma_commit(states);
-          if (!mbar_wait_spin(full1, ph, p.status)) break;
+          for (int j = 0; j < 8; ++j) umma_f16_lo_warp(tmem + COL_K, kk(UT, j), kk128(DS, j), id_kk, j > 0);
+          umma_commit_warp(states);
+          if (!mbar_wait_spin_warp(full1, ph, p.status)) break;
           tc_fence_after();
 #pragma unroll
-          for (int j = 0; j < 8; ++j) umma_f16_lo(tmem + COL_B, kk(NDU, j), kk(VQ, j), id_kk64, j > 0);
-          if (!mbar_wait_spin(c0, ph, p.status)) break;
+          for (int j = 0; j < 8; ++j) umma_f16_lo_warp(tmem + COL_B, kk(NDU, j), kk(VQ, j), id_kk64, j > 0);
+          if (!mbar_wait_spin_warp(c0, ph, p.status)) break;
           tc_fence_after();
 #pragma unroll
-          for (int j = 0; j < 8; ++j) umma_f16_lo(tmem + COL_A, kk(DW, j), kk(KT, j), id_kk64, j > 0);
-          umma_commit(m1);
+          for (int j = 0; j < 8; ++j) umma_f16_lo_warp(tmem + COL_A, kk(DW, j), kk(KT, j), id_kk64, j > 0);
+          umma_commit_warp(m1);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) umma_f16_lo(tmem + COL_W, mn(AP, j), mn(NDU, j), id_mm, j > 0);
-          umma_commit(mv);
-          if (!mbar_wait_spin(c1, ph, p.status)) break;
+          for (int j = 0; j < 4; ++j) umma_f16_lo_warp(tmem + COL_W, mn(AP, j), mn(NDU, j), id_mm, j > 0);
+          umma_commit_warp(mv);
+          if (!mbar_wait_spin_warp(c1, ph, p.status)) break;
           tc_fence_after();
 #pragma unroll
-          for (int j = 0; j < 4; ++j) umma_f16_lo(tmem + COL_A, kk(TMP, j), kk(AP, j), id_kk64, j > 0);
-          umma_commit(m2);
+          for (int j = 0; j < 4; ++j) umma_f16_lo_warp(tmem + COL_A, kk(TMP, j), kk(AP, j), id_kk64, j > 0);
+          umma_commit_warp(m2);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) umma_f16_lo(tmem + COL_B, mn(TMP, j), mn(TT, j), id_mm64, j > 0);
+          for (int j = 0; j < 4; ++j) umma_f16_lo_warp(tmem + COL_B, mn(TMP, j), mn(TT, j), id_mm64, j > 0);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) umma_f16_lo(tmem + COL_K, mn(AP, j), mn(DW, j), id_mm, 1);
-          if (!mbar_wait_spin(dv_read, ph, p.status)) break;
+          for (int j = 0; j < 4; ++j) umma_f16_lo_warp(tmem + COL_K, mn(AP, j), mn(DW, j), id_mm, 1);
+          if (!mbar_wait_spin_warp(dv_read, ph, p.status)) break;
           tc_fence_after();
 #pragma unroll
-          for (int j = 0; j < 8; ++j) umma_f16_lo(tmem + COL_W, kk(KT, j), kk(KT, j), id_kk64, j > 0);
-          if (!mbar_wait_spin(c2, ph, p.status)) break;
+          for (int j = 0; j < 8; ++j) umma_f16_lo_warp(tmem + COL_W, kk(KT, j), kk(KT, j), id_kk64, j > 0);
+          if (!mbar_wait_spin_warp(c2, ph, p.status)) break;
           tc_fence_after();
 #pragma unroll
-          for (int j = 0; j < 4; ++j) umma_f16_lo(tmem + COL_A, mn(TT, j), mn(OUTK, j), id_mm64, j > 0);
-          umma_commit(m3);
-          if (!mbar_wait_spin(fullq, ph, p.status) || !mbar_wait_spin(c3, ph, p.status)) break;
+          for (int j = 0; j < 4; ++j) umma_f16_lo_warp(tmem + COL_A, mn(TT, j), mn(OUTK, j), id_mm64, j > 0);
+          umma_commit_warp(m3);
+          if (!mbar_wait_spin_warp(fullq, ph, p.status) || !mbar_wait_spin_warp(c3, ph, p.status)) break;
           tc_fence_after();
 #pragma unroll
-          for (int j = 0; j < 4; ++j) umma_f16_lo(tmem + COL_K, kk(TMP, j), mn(KT, j), id_kn, 1);
+          for (int j = 0; j < 4; ++j) umma_f16_lo_warp(tmem + COL_K, kk(TMP, j), mn(KT, j), id_kn, 1);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) umma_f16_lo(tmem + COL_K, mn(TMP, j), mn(KT, j), id_mm, 1);
+          for (int j = 0; j < 4; ++j) umma_f16_lo_warp(tmem + COL_K, mn(TMP, j), mn(KT, j), id_mm, 1);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) umma_f16_lo(tmem + COL_K, mn(DM, j), mn(VQ, j), id_mm, 1);
+          for (int j = 0; j < 4; ++j) umma_f16_lo_warp(tmem + COL_K, mn(DM, j), mn(VQ, j), id_mm, 1);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) umma_f16_lo(tmem + COL_Q, kk(DM, j), mn(KT, j), id_kn, 1);
-          umma_commit(m4);
+          for (int j = 0; j < 4; ++j) umma_f16_lo_warp(tmem + COL_Q, kk(DM, j), mn(KT, j), id_kn, 1);
+          umma_commit_warp(m4);
           if (g + step < p.total) {
             // the next chunk's dW and dM: the row warps have read what those columns held
-            if (!mbar_wait_spin(full0, ph ^ 1, p.status)) break;
+            if (!mbar_wait_spin_warp(full0, ph ^ 1, p.status)) break;
             tc_fence_after();
             first_products();
           }

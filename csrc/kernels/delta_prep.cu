@@ -183,7 +183,7 @@ delta_prep_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
   __shared__ float4 betas_[C / 4];
   float* betas = reinterpret_cast<float*>(betas_);
 
-  const int r = threadIdx.x, warp = r >> 5;
+  const int r = threadIdx.x, warp = warp_index();
   if (r == 0) {
     mbar_init(full, 1); mbar_init(mma1, 1); mbar_init(mma2, 1); mbar_init(mma3, 1); mbar_init(fullv, 1);
     fence_barrier_init();
@@ -228,17 +228,17 @@ delta_prep_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
                         : bf16_to_f32(static_cast<const bf16*>(p.beta)[bidx]);
     }
     bool ok = true;
-    if (r == 0) {
-      ok = mbar_wait(full, ph, p.status);
+    if (warp == 0) {
+      ok = mbar_wait_warp(full, ph, p.status);
       if (ok) {
         tc_fence_after();
 #pragma unroll
         for (int j = 0; j < 8; ++j)     // G = K K^T -> columns [0, 64)
-          umma_f16_lo(tmem, step_k(k_k, j), step_k(k_k, j), id_kk64, j > 0);
+          umma_f16_lo_warp(tmem, step_k(k_k, j), step_k(k_k, j), id_kk64, j > 0);
 #pragma unroll
         for (int j = 0; j < 8; ++j)     // Q K^T -> columns [64, 128)
-          umma_f16_lo(tmem + 64, step_k(q_k, j), step_k(k_k, j), id_kk64, j > 0);
-        umma_commit(mma1);
+          umma_f16_lo_warp(tmem + 64, step_k(q_k, j), step_k(k_k, j), id_kk64, j > 0);
+        umma_commit_warp(mma1);
       }
     }
     ok = mbar_wait_spin(mma1, ph, p.status) && ok;
@@ -299,13 +299,13 @@ delta_prep_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     fence_proxy_async_smem();
     tc_fence_before();
     __syncthreads();
-    if (r == 0) {
+    if (warp == 0) {
       tc_fence_after();
 #pragma unroll
       for (int j = 0; j < 4; ++j)       // W = A' K -> columns [0, 128)
-        umma_f16_lo(tmem, step_k(ap_k, j), step_mn(k_mn, j), id_kn, j > 0);
-      umma_commit(mma2);
-      if (p.store_ta) {
+        umma_f16_lo_warp(tmem, step_k(ap_k, j), step_mn(k_mn, j), id_kn, j > 0);
+      umma_commit_warp(mma2);
+      if (r == 0 && p.store_ta) {
         tma_store_3d(&tmT, smem + QT + 8192, 0, g * C, 0);
         tma_store_3d(&tmAP, smem + QT, 0, g * C, 0);
         tma_store_commit();
@@ -320,15 +320,17 @@ delta_prep_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     fence_proxy_async_smem();
     tc_fence_before();
     __syncthreads();
-    if (r == 0 && (ok = mbar_wait_spin(fullv, ph, p.status))) {
+    if (warp == 0 && (ok = mbar_wait_spin_warp(fullv, ph, p.status))) {
       tc_fence_after();
 #pragma unroll
       for (int j = 0; j < 4; ++j)       // U^ = A' V -> the same columns
-        umma_f16_lo(tmem, step_k(ap_k, j), step_mn(v_mn, j), id_kn, j > 0);
-      umma_commit(mma3);
-      tma_store_3d(&tmW, smem + KT, 0, g * C, 0);
-      tma_store_3d(&tmW, smem + KT + 8192, 64, g * C, 0);
-      tma_store_commit();
+        umma_f16_lo_warp(tmem, step_k(ap_k, j), step_mn(v_mn, j), id_kn, j > 0);
+      umma_commit_warp(mma3);
+      if (r == 0) {
+        tma_store_3d(&tmW, smem + KT, 0, g * C, 0);
+        tma_store_3d(&tmW, smem + KT + 8192, 64, g * C, 0);
+        tma_store_commit();
+      }
     }
     ok = mbar_wait_spin(mma3, ph, p.status) && ok;
     if (!__syncthreads_and(ok)) break;

@@ -121,7 +121,7 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int chain = !S::BOTH ? 0 : (warp < MMA_WARP ? warp >> 3 : warp == MMA_WARP + 1);
   uint8_t* xb = smem + S::XB + chain * 32768;
   uint8_t* ub = smem + S::UB + chain * 16384;
@@ -219,7 +219,7 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     }
   } else if (warp >= MMA_WARP) {
     // -------------------------------- MMA issuer --------------------------------
-    if (lane == 0) {
+    {
       const uint32_t id_kn = make_idesc(1, 1, 128, S::CC, 0, 1);  // A K-major, B MN-major
       const uint32_t id_nn = make_idesc(1, 1, 128, S::CC, 1, 1);  // A MN-major, B MN-major
       // descriptor words made once: an issue is one add for each operand
@@ -231,54 +231,54 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
         auto k_major = [&](int tile) { return st_k + ((s * S::STAGE + tile) >> 4); };
         auto mn_major = [&](int tile) { return st_mn + ((s * S::STAGE + tile) >> 4); };
         const uint32_t col_o = tmem + COL_O + (it & 1) * 128;
-        if (!mbar_wait_spin(&full[s], ph, p.status)) break;
+        if (!mbar_wait_spin_warp(&full[s], ph, p.status)) break;
         if (BWD) {
           // Y = M^T dO: the previous Y was in registers before its u_ready
           tc_fence_after();
 #pragma unroll
           for (int j = 0; j < 4; ++j)
-            umma_f16_lo(tmem + COL_Y, step_mn(mn_major(TILE_M), j), step_mn(mn_major(TILE_DO), j), id_nn, j > 0);
+            umma_f16_lo_warp(tmem + COL_Y, step_mn(mn_major(TILE_M), j), step_mn(mn_major(TILE_DO), j), id_nn, j > 0);
         }
-        if (!mbar_wait_spin(x_ready, cph, p.status)) break;
+        if (!mbar_wait_spin_warp(x_ready, cph, p.status)) break;
         tc_fence_after();
         if (!BWD) {
           // Y = W X ; O = Q X
 #pragma unroll
           for (int j = 0; j < 8; ++j)
-            umma_f16_lo(tmem + COL_Y, step_k(k_major(TILE_W), j), step_mn(xb_mn, j), id_kn, j > 0);
-          umma_commit(y_done);
+            umma_f16_lo_warp(tmem + COL_Y, step_k(k_major(TILE_W), j), step_mn(xb_mn, j), id_kn, j > 0);
+          umma_commit_warp(y_done);
           if (!sum) {
             // the buffer's previous rows (chunk it - 2) were staged before this x_ready
 #pragma unroll
             for (int j = 0; j < 8; ++j)
-              umma_f16_lo(col_o, step_k(k_major(TILE_Q), j), step_mn(xb_mn, j), id_kn, j > 0);
+              umma_f16_lo_warp(col_o, step_k(k_major(TILE_Q), j), step_mn(xb_mn, j), id_kn, j > 0);
           }
         } else {
           // Y += K X
 #pragma unroll
           for (int j = 0; j < 8; ++j)
-            umma_f16_lo(tmem + COL_Y, step_k(k_major(TILE_K), j), step_mn(xb_mn, j), id_kn, 1);
-          umma_commit(y_done);
+            umma_f16_lo_warp(tmem + COL_Y, step_k(k_major(TILE_K), j), step_mn(xb_mn, j), id_kn, 1);
+          umma_commit_warp(y_done);
           // X += Q^T dO   (independent of dU: keeps the tensor core busy meanwhile)
 #pragma unroll
           for (int j = 0; j < 4; ++j)
-            umma_f16_lo(tmem + COL_X, step_mn(mn_major(TILE_Q), j), step_mn(mn_major(TILE_DO), j), id_nn, 1);
+            umma_f16_lo_warp(tmem + COL_X, step_mn(mn_major(TILE_Q), j), step_mn(mn_major(TILE_DO), j), id_nn, 1);
         }
-        if (!mbar_wait_spin(u_ready, cph, p.status)) break;
+        if (!mbar_wait_spin_warp(u_ready, cph, p.status)) break;
         tc_fence_after();
         // X += K^T U  (forward), X += W^T (-dU)  (backward): what the next chunk waits for
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-          umma_f16_lo(tmem + COL_X, step_mn(mn_major(BWD ? TILE_W : TILE_K), j), step_mn(ub_mn, j), id_nn, 1);
-        umma_commit(x_done);
+          umma_f16_lo_warp(tmem + COL_X, step_mn(mn_major(BWD ? TILE_W : TILE_K), j), step_mn(ub_mn, j), id_nn, 1);
+        umma_commit_warp(x_done);
         if (!BWD && !sum) {
           // O += M U
 #pragma unroll
           for (int j = 0; j < 4; ++j)
-            umma_f16_lo(col_o, step_k(k_major(TILE_M), j), step_mn(ub_mn, j), id_kn, 1);
-          umma_commit(o_done);
+            umma_f16_lo_warp(col_o, step_k(k_major(TILE_M), j), step_mn(ub_mn, j), id_kn, 1);
+          umma_commit_warp(o_done);
         }
-        umma_commit(&empty[s]);
+        umma_commit_warp(&empty[s]);
       }
     }
   } else {

@@ -99,7 +99,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   uint64_t* tempty = bars + 2 * STAGES + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int num_m = (p.M + BM - 1) / BM, num_n = (p.N + BN - 1) / BN;
   const int nkb = p.K / BK;
   const long total = static_cast<long>(num_m) * num_n;
@@ -168,7 +168,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
       const uint32_t idesc = make_idesc(0, 0, BM, BN, 0, 0);   // e4m3 x e4m3, both K-major
       int s = 0;
       uint32_t ph = 0;
@@ -180,18 +180,18 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         if (group_of(m_blk) < 0) continue;
         for (int kb = 0; kb < nkb; it += (PROBE == 2 ? (kb == nkb - 1) : 1), ++kb) {
           const int acc = it & 1;
-          if ((PROBE != 2 || kb == 0) && !mbar_wait(&tempty[acc], ((it >> 1) & 1) ^ 1, p.status)) { ok = false; break; }
-          if (!mbar_wait(&full[s], ph, p.status)) { ok = false; break; }
+          if ((PROBE != 2 || kb == 0) && !mbar_wait_warp(&tempty[acc], ((it >> 1) & 1) ^ 1, p.status)) { ok = false; break; }
+          if (!mbar_wait_warp(&full[s], ph, p.status)) { ok = false; break; }
           tc_fence_after();
           const uint32_t a_addr = smem_u32(smA + s * A_BYTES);
           const uint32_t b_addr = smem_u32(smB + s * B_BYTES);
 #pragma unroll
           for (int j = 0; j < BK / 32; ++j)
-            umma_f8(tmem_base + acc * BN, make_sdesc_sw128(a_addr + j * 32, 16, 1024),
+            umma_f8_warp(tmem_base + acc * BN, make_sdesc_sw128(a_addr + j * 32, 16, 1024),
                     make_sdesc_sw128(b_addr + j * 32, 16, 1024), idesc,
                     (j > 0 || (PROBE == 2 && kb > 0)) ? 1u : 0u);
-          umma_commit(&empty[s]);
-          if (PROBE != 2 || kb == nkb - 1) umma_commit(&tfull[acc]);
+          umma_commit_warp(&empty[s]);
+          if (PROBE != 2 || kb == nkb - 1) umma_commit_warp(&tfull[acc]);
           if (++s == STAGES) { s = 0; ph ^= 1; }
         }
       }
@@ -329,16 +329,6 @@ constexpr int P_WARPS = 16, P_COLS = 64, P_THREADS = (4 + P_WARPS) * 32;   // wa
 constexpr int P_EPI = P_STAGES * P_STAGE, P_BARS = P_EPI + P_WARPS * 4096, P_SMEM = P_BARS + 256 + 1024;
 static_assert(P_SMEM <= 227 * 1024, "one CTA's shared memory");
 
-__device__ __forceinline__ void umma_f8_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                             uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
 __global__ void __launch_bounds__(P_THREADS, 1)
 gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                      const __grid_constant__ CUtensorMap tmC, const Params p) {
@@ -352,7 +342,7 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
   uint64_t* tempty = tfull + 2;             // [2], the even CTA's
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int rank = static_cast<int>(cluster_ctarank());   // 0: even CTA (issues the MMAs)
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
   const int num_m = (p.M + 255) / 256, num_n = (p.N + BN - 1) / BN;
@@ -430,7 +420,7 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
           }
       }
     }
-    if (warp == 1 && lane == 0 && rank == 0) {
+    if (warp == 1 && rank == 0) {
       const uint32_t idesc = make_idesc(0, 0, 256, BN, 0, 0);   // e4m3 x e4m3, both K-major
       constexpr uint64_t HI = static_cast<uint64_t>(sdesc_hi_sw128(1024)) << 32;
       const uint32_t lo0 = sdesc_lo(smem_u32(smem), 16);
@@ -443,15 +433,15 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         const Passes q = passes(m_pair);
         for (int kb = 0; kb < q.n * nkb; ++kb, ++it) {
           const int acc = it & 1;
-          if (!mbar_wait_spin(&tempty[acc], ((it >> 1) & 1) ^ 1, p.status) ||
-              !mbar_wait_spin(&full[s], ph, p.status)) { ok = false; break; }
+          if (!mbar_wait_spin_warp(&tempty[acc], ((it >> 1) & 1) ^ 1, p.status) ||
+              !mbar_wait_spin_warp(&full[s], ph, p.status)) { ok = false; break; }
           tc_fence_after();
           const uint32_t a_lo = lo0 + s * (P_STAGE >> 4), b_lo = a_lo + (P_OP >> 4);
 #pragma unroll
           for (int j = 0; j < BK / 32; ++j)
-            umma_f8_pair(tmem_base + acc * BN, HI | (a_lo + 2 * j), HI | (b_lo + 2 * j), idesc, j > 0 ? 1u : 0u);
-          umma_commit_pair(&empty[s], 3);
-          umma_commit_pair(&tfull[acc], 3);
+            umma_f8_pair_warp(tmem_base + acc * BN, HI | (a_lo + 2 * j), HI | (b_lo + 2 * j), idesc, j > 0 ? 1u : 0u);
+          umma_commit_pair_warp(&empty[s], 3);
+          umma_commit_pair_warp(&tfull[acc], 3);
           if (++s == P_STAGES) { s = 0; ph ^= 1; }
         }
       }
