@@ -20,8 +20,10 @@
 // quarter, 64 columns each); the state update is issued before the output product and has its own
 // barrier; the output accumulator is double-buffered, so chunk n's output rows are staged while
 // chunk n + 1's Y product runs; the part of the backward's Y that does not need the state is issued
-// before the state image is ready. 64 sequences of 64 chunks: forward 113 us (1.8 us a chunk), backward 101 us;
-// four row warps that did all of it in order, in one CTA a sequence, took 230 and 133 us.
+// before the state image is ready. 64 sequences of 64 chunks: forward 105 us (1.6 us a chunk), backward 98 us, which is 4.7 and 5.0 TB/s;
+// 16 of 256 chunks 287 and 283 us. Four row warps that did all of it in order, in one CTA a sequence, took 230 and 133 us. Extra
+// warps for the output rows and the bulk stores gave nothing: what a chunk takes is the products' chain and the
+// shared memory that they and the conversions share.
 //
 // The columns of the state never mix (U, O and dU have the same columns), so when the sequences or
 // segments take at most half of the SMs, two CTAs walk each of them with 64 columns: the conversions
@@ -32,13 +34,13 @@
 // A forward summary walks every segment twice, once per map, over the same W and K. When the two CTAs a
 // segment that takes are more than the SMs, one CTA does both, as two independent chains whose conversions
 // and products fall into each other's waits: one wave and half of the operand reads. 16 sequences x 8
-// segments x 32 chunks: 86 us, against 104 us as two waves of a CTA for each map. (One chain of 256 columns:
+// segments x 32 chunks: 69 us (86 us when it was built, against 104 us as two waves of a CTA for each map). (One chain of 256 columns:
 // 120 us, its conversions and products take turns.) With a CTA for each map on SMs of their own a chain is the
 // shorter, so up to half of the SMs it stays so: 72 segments of 32 chunks 62 us, 80 segments in a CTA each 87 us.
 // The initial state is read 16 bytes at a time: element by element the walk of those segments, 70 us, takes 6 us more.
 //
 // warps 0-7: tensor-memory <-> registers <-> shared/global (lane = state row or token)
-// warp 8   : MMA issue (one lane)          warp 9: TMA producer (one lane)
+// warp 8   : MMA issue                     warp 9: TMA producer (one lane)
 // (two chains: 0-15 rows, 16 and 17 MMA issue, 18 TMA)
 //
 // Reference semantics: kernels/__init__.py:357-376 (per-token recurrence, post-update
@@ -353,6 +355,25 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
       }
       tmem_st_wait();
     }
+    // Rows of the previous chunk's output: tensor memory -> staging tile. Q S takes 512 clocks of shared-memory reads with
+    // 128 columns, in which stores to it hardly pass: there the rows are staged behind U, while the state is updated. With
+    // 64 columns they are while Y is computed. Late / early, us: 80 sequences x 64 chunks (128 columns) 107 / 127,
+    // 128 segments x 32 chunks 68.9 / 71.7, 16 sequences x 256 chunks (64 columns) 290 / 285.
+    constexpr bool LATE = NC == 128;
+    auto stage_rows = [&](uint32_t buf) {
+      if (BWD || sum) return;
+      wait(o_done, buf);
+      if (tok_warp) {
+        uint32_t v[WC];
+        load_cols(COL_O + buf * 128, v);
+        put_cols(ob, C, v);
+        fence_proxy_async_smem();
+      }
+    };
+    auto store_rows = [&](int n) {
+#pragma unroll
+      for (int hf = 0; hf < HALVES; ++hf) tma_store_3d(&tmO, ob + hf * 8192, tx + col0 + hf * 64, tok0 + n * C, tb);
+    };
     for (int it = 0; it < N; ++it) {
       const int n = n0 + (BWD ? (N - 1 - it) : it);
       const uint32_t cph = it & 1;
@@ -365,25 +386,12 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
         put_cols(xb, D, v);
       }
       arrive(x_ready);
-      if (!BWD && !sum && it > 0) {
-        // rows of the previous chunk's output: tensor memory -> staging tile, while Y is computed
-        wait(o_done, cph ^ 1);
-        if (tok_warp) {
-          uint32_t v[WC];
-          load_cols(COL_O + (cph ^ 1) * 128, v);
-          put_cols(ob, C, v);
-          fence_proxy_async_smem();
-        }
-      }
+      if (!LATE && it > 0) stage_rows(cph ^ 1);
       if (!sum) {
         if (r == 0 && ch == 0) tma_store_wait_read<0>();   // U of the previous chunk has left ub
         sync_rows();
         if (r == 0 && ch == 0) {
-          if (!BWD && it > 0) {
-            const int prow = tok0 + (n - 1) * C;
-#pragma unroll
-            for (int hf = 0; hf < HALVES; ++hf) tma_store_3d(&tmO, ob + hf * 8192, tx + col0 + hf * 64, prow, tb);
-          }
+          if (!BWD && !LATE && it > 0) store_rows(n - 1);
           if (store_ux) {
 #pragma unroll
             for (int hf = 0; hf < HALVES; ++hf) tma_store_3d(&tmXB, xb + hf * 16384, col0 + hf * 64, g * D, 0);
@@ -393,31 +401,36 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
       }
       if (tok_warp) {
         uint8_t* ut = smem + (it & 1) * S::STAGE + TILE_DO;
-        constexpr bool EARLY = !BWD && !S::BOTH;   // two chains have no registers for it
-        bf16x8 uh[EARLY ? WC / 8 : 1];             // this lane's U^, read while Y is computed
-        if (EARLY && !lin) {
+        bf16x8 uh[BWD ? 1 : WC / 8];   // this lane's U^, read while Y is computed
+        if (!BWD && !lin) {
           wait(&full[it & 1], (it >> 1) & 1);
 #pragma unroll
-          for (int i = 0; i < WC / 8; ++i) uh[EARLY ? i : 0] = ld_shared8(piece(ut, C, i));
+          for (int i = 0; i < WC / 8; ++i) uh[BWD ? 0 : i] = ld_shared8(piece(ut, C, i));
         }
         wait(y_done, cph);
-        uint32_t v[WC];
-        load_cols(COL_Y, v);
+        constexpr int PART = S::BOTH ? 32 : WC;   // columns at a time: what the registers of two chains hold
 #pragma unroll
-        for (int i = 0; i < WC / 8; ++i) {
-          float y[8];
+        for (int c = 0; c < WC; c += PART) {
+          uint32_t v[PART];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) y[j] = __uint_as_float(v[8 * i + j]);
-          if (!BWD && !lin) {
-            float uhv[8];
-            unpack8(EARLY ? uh[EARLY ? i : 0] : ld_shared8(piece(ut, C, i)), uhv);
+          for (int k = 0; k < PART; k += 32) tmem_ld_32x32b_x32(lane_addr + COL_Y + c + k, v + k);
+          tmem_ld_wait();
 #pragma unroll
-            for (int j = 0; j < 8; ++j) y[j] = uhv[j] - y[j];  // U = U^ - W S
-          } else {
+          for (int i = 0; i < PART / 8; ++i) {
+            float y[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) y[j] = -y[j];          // operand (and output) is -dU
+            for (int j = 0; j < 8; ++j) y[j] = __uint_as_float(v[8 * i + j]);
+            if (!BWD && !lin) {
+              float uhv[8];
+              unpack8(uh[BWD ? 0 : c / 8 + i], uhv);
+#pragma unroll
+              for (int j = 0; j < 8; ++j) y[j] = uhv[j] - y[j];  // U = U^ - W S
+            } else {
+#pragma unroll
+              for (int j = 0; j < 8; ++j) y[j] = -y[j];          // operand (and output) is -dU
+            }
+            st_shared8(piece(ub, C, c / 8 + i), pack8(y));
           }
-          st_shared8(piece(ub, C, i), pack8(y));
         }
         arrive(u_ready);
         if (store_ux) {
@@ -429,12 +442,17 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
           }
         }
       }
+      if (LATE && it > 0) stage_rows(cph ^ 1);
       if (!sum) {   // while the state is updated: the bulk stores before U's have read xb and ob, which are rewritten next
         if (r == 0 && ch == 0) {
           if (store_ux) tma_store_wait_read<1>();
           else tma_store_wait_read<0>();
         }
         sync_rows();
+        if (!BWD && LATE && it > 0 && r == 0 && ch == 0) {   // read by the next chunk's first wait, before rows are staged again
+          store_rows(n - 1);
+          tma_store_commit();
+        }
       }
     }
     // drain: last chunk's output rows and the final state
@@ -452,9 +470,7 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
         }
         sync_rows();
         if (r == 0 && ch == 0) {
-          const int prow = tok0 + (n0 + N - 1) * C;
-#pragma unroll
-          for (int hf = 0; hf < HALVES; ++hf) tma_store_3d(&tmO, ob + hf * 8192, tx + col0 + hf * 64, prow, tb);
+          store_rows(n0 + N - 1);
           tma_store_commit();
         }
       }
