@@ -20,7 +20,10 @@
 namespace pb {
 namespace moe {
 
-constexpr int TOK_PER_BLOCK = 256;   // tokens per block of the counting sort
+// Tokens per block of the counting sort. One warp walks a block's pairs in order, 32 at a time, so more blocks are shorter
+// walks, and more counts for the scan. 32 / 64 / 128 of them, us for the three kernels: 8192 tokens top-6 of 64 11.0 / 11.6 /
+// 14.2, 32768 20.8 / 16.4 / 17.4, 4097 top-1 of 512 26.5 / 23.3 / 22.4 (256, and a scan of one thread an expert: 26.6, 39.1, 23.6).
+constexpr int TOK_PER_BLOCK = 64;
 constexpr int MAX_E = 512;
 constexpr int MAX_K = 32;
 
@@ -162,6 +165,8 @@ __device__ __forceinline__ void write_segments(const int* tot, int* off, int E, 
   }
 }
 
+constexpr int SCAN_THREADS = 512;
+static_assert(SCAN_THREADS >= MAX_E, "a thread for every expert");
 // One block. Turns block_counts into exclusive per-block bases and writes the segments.
 __global__ void scan_kernel(int* __restrict__ block_counts, int nblocks, int E,
                             int* __restrict__ expert_off, int* __restrict__ totals,
@@ -169,25 +174,46 @@ __global__ void scan_kernel(int* __restrict__ block_counts, int nblocks, int E,
   after_previous_kernel();
   __shared__ int tot[MAX_E];
   __shared__ int off[MAX_E + 1];
-  for (int e = threadIdx.x; e < E; e += blockDim.x) {
-    int run = 0;
-    for (int b = 0; b < nblocks; ++b) {
-      const int c = block_counts[static_cast<size_t>(b) * E + e];
-      block_counts[static_cast<size_t>(b) * E + e] = run;
-      run += c;
+  // A thread has one expert and a share of the blocks, eight counts in flight at a time: one thread an expert that
+  // waited for each count took 10 us of 8192 tokens' 27.
+  __shared__ int part[SCAN_THREADS];
+  const int groups = SCAN_THREADS / E;   // at least one
+  const int e = threadIdx.x % E, g = threadIdx.x / E;
+  const int b0 = g < groups ? nblocks * g / groups : 0, b1 = g < groups ? nblocks * (g + 1) / groups : 0;
+  int* mine = block_counts + e;
+  auto walk = [&](int run, bool store) {
+    for (int b = b0; b < b1; b += 8) {
+      int c[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) c[u] = b + u < b1 ? mine[static_cast<size_t>(b + u) * E] : 0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        if (store && b + u < b1) mine[static_cast<size_t>(b + u) * E] = run;
+        run += c[u];
+      }
     }
-    tot[e] = run;
+    return run;
+  };
+  int base = 0;
+  if (groups > 1) {
+    part[threadIdx.x] = walk(0, false);
+    __syncthreads();
+    for (int q = 0; q < g && g < groups; ++q) base += part[q * E + e];
   }
+  base = walk(base, true);
+  if (g == groups - 1) tot[e] = base;
   write_segments(tot, off, E, expert_off, totals, k_len, mblk_group, max_mblk);
 }
 
 // One warp walks the pairs [lo, hi) in order; run[e] is the next row of expert e for them.
 __device__ __forceinline__ void place_pairs(const int* __restrict__ ids, int lo, int hi, int* run,
                                             int* __restrict__ row_of, int lane) {
+  int next = lo + lane < hi ? ids[lo + lane] : 0;
   for (int base = lo; base < hi; base += 32) {
     const int i = base + lane;
     const bool on = i < hi;
-    const int e = on ? ids[i] : -1 - lane;
+    const int e = on ? next : -1 - lane;
+    if (i + 32 < hi) next = ids[i + 32];   // arrives while these are placed
     const unsigned same = __match_any_sync(0xffffffffu, e);
     const int rank = __popc(same & ((1u << lane) - 1u));
     int start = 0;
@@ -217,8 +243,7 @@ __global__ void place_kernel(const int* __restrict__ ids, int n_pairs, int pairs
 
 // The whole sort in one block, each warp an eighth of the pairs: three launches less two for inputs whose
 // kernels are shorter than a launch. Same placement (stable in the pair index).
-// 1024 pairs, 8 experts: 10 us in three kernels -> 3.1 us in one; SORT_MAX pairs are where its walk takes as long
-// as the three together.
+// One / three, us: 1024 pairs of 8 experts 2.9 / 6.3, 2046 of 64 5.9 / 9.9, 4096 of 8 4.6 / 6.4, 4092 of 64 8.2 / 10.2.
 constexpr int SORT_WARPS = 8, SORT_MAX = 4096;
 __global__ void __launch_bounds__(SORT_WARPS * 32) sort_small_kernel(const int* __restrict__ ids, int n_pairs, int E,
                                                                      int* __restrict__ row_of,
@@ -472,7 +497,7 @@ PB_API int pb_moe_sort(const int* ids, int n_pairs, int k, int E, int* scratch, 
   const int per = moe::TOK_PER_BLOCK * k;
   const int nblocks = (n_pairs + per - 1) / per;
   pb::launch(moe::count_kernel, nblocks, 256, 0, st, ids, n_pairs, per, E, scratch);
-  pb::launch(moe::scan_kernel, 1, 512, 0, st, scratch, nblocks, E, expert_off, totals, k_len, mblk_group,
+  pb::launch(moe::scan_kernel, 1, moe::SCAN_THREADS, 0, st, scratch, nblocks, E, expert_off, totals, k_len, mblk_group,
                                       max_mblk);
   pb::launch(moe::place_kernel, nblocks, 32, 0, st, ids, n_pairs, per, E, scratch, expert_off, row_of);
   return static_cast<int>(cudaGetLastError());

@@ -52,6 +52,24 @@ def test_route_and_placement(T, E, k):
         assert off[mg[m]] <= m * 128 < off[mg[m] + 1]
 
 
+@pytest.mark.parametrize("T,E,k,skew", [(683, 64, 6, 0), (4097, 512, 1, 0), (64 * 9 + 1, 300, 8, 0), (8200, 5, 3, 0), (4160, 64, 1, 1)])
+def test_placement_over_many_blocks(T, E, k, skew):
+    """The three-kernel sort: one pair more than the one-block sort takes, a thread or several to an expert in the scan, shares of
+    blocks that do not divide, a last block of one token, and all pairs on one expert. Rows are those of a stable sort."""
+    from prometheus_b200.ops import moe
+
+    ids = torch.randint(0, 1 if skew else E, (T, k), generator=torch.Generator().manual_seed(T), dtype=torch.int32)
+    pl = moe.place(ids.cuda(), E)
+    flat = ids.reshape(-1).long()
+    counts = torch.bincount(flat, minlength=E)
+    off = torch.cat([torch.zeros(1, dtype=torch.long), ((counts + 127) // 128 * 128).cumsum(0)])
+    order = torch.argsort(flat, stable=True)
+    want = torch.empty_like(flat)
+    want[order] = torch.arange(flat.numel()) - (counts.cumsum(0) - counts)[flat[order]] + off[flat[order]]
+    assert torch.equal(pl.row_of.cpu().long(), want)
+    assert torch.equal(pl.expert_off.cpu().long(), off) and torch.equal(pl.totals.cpu().long(), counts)
+
+
 def test_grouped_gemms_match_per_expert_products():
     from prometheus_b200.ops import functional as ops
     from prometheus_b200.ops import moe
