@@ -12,7 +12,7 @@
 // M = 128, N = its columns; the bf16 image of the state and of U that the MMAs consume as
 // their B operand is rewritten in shared memory each chunk in the 128-byte-swizzled
 // layout TMA itself produces; Q/K/W/M and U^ (or dO) tiles arrive by TMA through a
-// two-stage ring, and every output leaves by a TMA store from shared memory. Tiles with 64 token rows are used as 128-row A operands: the upper 64
+// ring of two or three stages, and every output leaves by a TMA store from shared memory. Tiles with 64 token rows are used as 128-row A operands: the upper 64
 // accumulator rows are then meaningless and are never read.
 //
 // The walk is a serial chain per chunk (state image -> Y -> U -> state update), so its length is
@@ -20,8 +20,8 @@
 // quarter, 64 columns each); the state update is issued before the output product and has its own
 // barrier; the output accumulator is double-buffered, so chunk n's output rows are staged while
 // chunk n + 1's Y product runs; the part of the backward's Y that does not need the state is issued
-// before the state image is ready. 64 sequences of 64 chunks: forward 105 us (1.6 us a chunk), backward 98 us, which is 4.7 and 5.0 TB/s;
-// 16 of 256 chunks 287 and 283 us. Four row warps that did all of it in order, in one CTA a sequence, took 230 and 133 us. Extra
+// before the state image is ready. 64 sequences of 64 chunks: forward 96 us (1.5 us a chunk), backward 86 us, which is 5.1 and 5.7 TB/s;
+// 16 of 256 chunks 287 and 256 us. Four row warps that did all of it in order, in one CTA a sequence, took 230 and 133 us. Extra
 // warps for the output rows and the bulk stores gave nothing: what a chunk takes is the products' chain and the
 // shared memory that they and the conversions share.
 //
@@ -87,7 +87,7 @@ struct Params {
 // NC: state columns of a CTA. 128, or 64 (then two CTAs per segment, not in summary mode), or 256: both
 // maps of a forward summary as two chains of 128 columns (0: R, 1: P), each with its own row warps, MMA
 // warp and barriers, over the same W and K tiles; no Q, M and output staging.
-template <int NC>
+template <int NC, int ST>
 struct Shape {
   static constexpr bool BOTH = NC == 256;
   static constexpr int CHAINS = BOTH ? 2 : 1;
@@ -99,23 +99,24 @@ struct Shape {
   // a stage: W, Q, K (16 KB each), M (8 KB), U^ or dO (16 KB). W's second half is followed by at
   // least 8 KB of the stage: as a 128-row A operand its upper rows are read from there.
   static constexpr int TILE_W = 0, TILE_Q = 16384, TILE_K = BOTH ? 16384 : 32768, TILE_M = 49152,
-                       TILE_DO = BOTH ? 32768 : 57344, STAGE = TILE_DO + 16384;
-  static constexpr int XB = 2 * STAGE;
-  static constexpr int UB = XB + (BOTH ? 65536 : 32768);
-  static constexpr int OB = UB + (BOTH ? 32768 : 16384);
-  static constexpr int BARS = OB + (BOTH ? 0 : 16384);
+                       TILE_DO = BOTH ? 32768 : 57344, STAGE = TILE_DO + (NC == 64 ? 8192 : 16384);
+  static constexpr int STAGES = ST;
+  static constexpr int XB = STAGES * STAGE;
+  static constexpr int UB = XB + 256 * NC;                  // state image, U and output staging: 128, 64 and 64 rows of NC
+  static constexpr int OB = UB + 128 * NC;
+  static constexpr int BARS = OB + (BOTH ? 0 : 128 * NC);
   static constexpr int TOTAL = BARS + 256 + 1024;
   static_assert(TOTAL <= 227 * 1024, "shared memory of a CTA");
 };
 
-template <bool BWD, int NC>
-__global__ void __launch_bounds__(Shape<NC>::THREADS, 1)
+template <bool BWD, int NC, int ST>
+__global__ void __launch_bounds__(Shape<NC, ST>::THREADS, 1)
 delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmQ,
                   const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmM,
                   const __grid_constant__ CUtensorMap tmDO, const __grid_constant__ CUtensorMap tmXB,
                   const __grid_constant__ CUtensorMap tmU, const __grid_constant__ CUtensorMap tmO,
                   const Params p) {
-  using S = Shape<NC>;
+  using S = Shape<NC, ST>;
   static_assert(!(BWD && S::BOTH), "both maps at once: forward summary only");
   constexpr int TILE_W = S::TILE_W, TILE_Q = S::TILE_Q, TILE_K = S::TILE_K, TILE_M = S::TILE_M, TILE_DO = S::TILE_DO;
   constexpr uint32_t COL_Y = S::COL_Y, COL_O = S::COL_O;
@@ -129,15 +130,16 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
   uint8_t* ub = smem + S::UB + chain * 16384;
   uint8_t* ob = smem + S::OB;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::BARS);
-  uint64_t* full = bars;          // [2]
-  uint64_t* empty = bars + 2;     // [2]
-  uint64_t* chain_bars = bars + 4 + 5 * chain;
+  constexpr int STAGES = S::STAGES;
+  uint64_t* full = bars;          // [STAGES]
+  uint64_t* empty = bars + 3;     // [STAGES]
+  uint64_t* chain_bars = bars + 6 + 5 * chain;
   uint64_t* x_ready = chain_bars;
   uint64_t* y_done = chain_bars + 1;
   uint64_t* u_ready = chain_bars + 2;
   uint64_t* x_done = chain_bars + 3;    // the state update of a chunk
   uint64_t* o_done = chain_bars + 4;    // its output product (forward)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4 + 5 * S::CHAINS);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 6 + 5 * S::CHAINS);
 
   const int n_units = p.n_seq * p.n_seg;
   constexpr int HALVES = NC == 64 ? 1 : 2;   // 64-column chunks of U^, dO and the outputs
@@ -160,11 +162,11 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
   const int tx = tokmaj ? (seq % p.heads) * D : 0;
 
   if (threadIdx.x == 0) {
-    mbar_init(&full[0], 1); mbar_init(&full[1], 1);
-    mbar_init(&empty[0], S::CHAINS); mbar_init(&empty[1], S::CHAINS);
+#pragma unroll
+    for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], S::CHAINS); }
 #pragma unroll
     for (int c = 0; c < S::CHAINS; ++c) {
-      uint64_t* b = bars + 4 + 5 * c;
+      uint64_t* b = bars + 6 + 5 * c;
       mbar_init(b, 8); mbar_init(b + 2, 4);   // x_ready, u_ready: one arrival per warp that takes part
       mbar_init(b + 1, 1); mbar_init(b + 3, 1); mbar_init(b + 4, 1);
     }
@@ -192,8 +194,8 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
       const uint32_t stage_tx = 32768u + (need_qm ? 24576u : 0u) + (need_fifth ? HALVES * 8192u : 0u);
       for (int it = 0; it < N; ++it) {
         const int n = n0 + (BWD ? (N - 1 - it) : it);
-        const int s = it & 1;
-        const uint32_t ph = (it >> 1) & 1;
+        const int s = it % STAGES;
+        const uint32_t ph = (it / STAGES) & 1;
         if (!mbar_wait(&empty[s], ph ^ 1, p.status)) break;
         mbar_arrive_expect_tx(&full[s], stage_tx);
         uint8_t* st = smem + s * S::STAGE;
@@ -228,8 +230,8 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
       const uint32_t xb_mn = sdesc_lo(smem_u32(xb), 16384), ub_mn = sdesc_lo(smem_u32(ub), 8192);
       const uint32_t st_k = sdesc_lo(smem_u32(smem), 16), st_mn = sdesc_lo(smem_u32(smem), 8192);
       for (int it = 0; it < N; ++it) {
-        const int s = it & 1;
-        const uint32_t ph = (it >> 1) & 1, cph = it & 1;
+        const int s = it % STAGES;
+        const uint32_t ph = (it / STAGES) & 1, cph = it & 1;
         auto k_major = [&](int tile) { return st_k + ((s * S::STAGE + tile) >> 4); };
         auto mn_major = [&](int tile) { return st_mn + ((s * S::STAGE + tile) >> 4); };
         const uint32_t col_o = tmem + COL_O + (it & 1) * 128;
@@ -400,10 +402,10 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
         }
       }
       if (tok_warp) {
-        uint8_t* ut = smem + (it & 1) * S::STAGE + TILE_DO;
+        uint8_t* ut = smem + it % STAGES * S::STAGE + TILE_DO;
         bf16x8 uh[BWD ? 1 : WC / 8];   // this lane's U^, read while Y is computed
         if (!BWD && !lin) {
-          wait(&full[it & 1], (it >> 1) & 1);
+          wait(&full[it % STAGES], (it / STAGES) & 1);
 #pragma unroll
           for (int i = 0; i < WC / 8; ++i) uh[BWD ? 0 : i] = ld_shared8(piece(ut, C, i));
         }
@@ -501,19 +503,19 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
   }
 }
 
-template <bool BWD, int NC>
+template <bool BWD, int NC, int ST = 2>
 int launch_cols(const CUtensorMap& tW, const CUtensorMap& tQ, const CUtensorMap& tK, const CUtensorMap& tM,
                 const CUtensorMap& tD, const CUtensorMap& tXB, const CUtensorMap& tU, const CUtensorMap& tO,
                 const Params& p, int ctas, cudaStream_t st) {
   static pb::DeviceOnce attr_once;   // per device: the attribute belongs to the current GPU
   if (attr_once.need()) {
-    cudaError_t e = cudaFuncSetAttribute(delta_scan_kernel<BWD, NC>,
+    cudaError_t e = cudaFuncSetAttribute(delta_scan_kernel<BWD, NC, ST>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         Shape<NC>::TOTAL);
+                                         Shape<NC, ST>::TOTAL);
     if (e != cudaSuccess) return static_cast<int>(e);
     attr_once.done();
   }
-  pb::launch(delta_scan_kernel<BWD, NC>, ctas, Shape<NC>::THREADS, Shape<NC>::TOTAL, st, tW, tQ, tK, tM, tD, tXB, tU, tO, p);
+  pb::launch(delta_scan_kernel<BWD, NC, ST>, ctas, Shape<NC, ST>::THREADS, Shape<NC, ST>::TOTAL, st, tW, tQ, tK, tM, tD, tXB, tU, tO, p);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -545,8 +547,15 @@ int launch(const void* W, const void* Q, const void* K, const void* M, const voi
   else r |= tok_map(&tO, o_out);
   if (r != 0) return 1000 + r;
   const int units = p.n_seq * p.n_seg;
-  if (!p.summary && 2 * units <= num_sms())
-    return launch_cols<BWD, 64>(tW, tQ, tK, tM, tD, tXB, tU, tO, p, 2 * units, st);
+  if (!p.summary && 2 * units <= num_sms()) {
+    // Three stages hide the latency that memory has when many CTAs read and write it. A forward walk of few CTAs, or one
+    // that keeps nothing for the backward, does not wait for memory, and there the earlier arrivals cost more in shared
+    // memory than they save. Two / three, 64 chunks, us: forward 16 sequences 76 / 83, 32 80 / 84, 40 85 / 84, 48 92 / 84..90, 64
+    // 105 / 96; nothing kept 48 76 / 79, 64 81 / 80; backward 16 74 / 68, 40 83 / 69, 64 99 / 86.
+    if (BWD || (p.store_ux != 0 && units > 36))
+      return launch_cols<BWD, 64, 3>(tW, tQ, tK, tM, tD, tXB, tU, tO, p, 2 * units, st);
+    if constexpr (!BWD) return launch_cols<BWD, 64>(tW, tQ, tK, tM, tD, tXB, tU, tO, p, 2 * units, st);
+  }
   if constexpr (!BWD) {
     // both maps in one CTA where a CTA for each would be a second wave
     if (p.summary && 2 * units > num_sms())

@@ -837,6 +837,25 @@ def test_delta_summary_maps(n_seq, n_chunks, n_seg, cut):
         assert err.max() <= 2e-2, err.max()
 
 
+@pytest.mark.parametrize("H,S", [(36, 448), (37, 64), (37, 129), (37, 256), (37, 448), (74, 300)])
+def test_delta_walk_stages(H, S):
+    """64-column walks with two stages (forward up to 36 sequences) and with three (more of them, and backward), of one chunk to
+    more than twice the stages, against the same heads among 80, whose walk has 128 columns: the columns of the
+    state never mix and each sum is over the same terms in the same order, so all outputs are the same bits."""
+    from prometheus_b200.ops.delta import delta_rule_fused
+
+    q, k, v, do = (_r(1, S, 80, 128, seed=i, scale=0.08) for i in (1, 2, 3, 5))
+    beta = torch.sigmoid(_r(1, S, 80, seed=4, dtype=torch.float32))
+
+    def run(h):
+        leaves = [t[:, :, :h].contiguous().requires_grad_(True) for t in (q, k, v, beta)]
+        out, fin = delta_rule_fused(*leaves, None, n_seg=1)
+        return [t[:, :, :H] for t in (out, *torch.autograd.grad(out, leaves, do[:, :, :h].contiguous()))] + [fin[:, :H]]
+
+    for few, many in zip(run(H), run(80)):
+        assert torch.equal(few, many)
+
+
 @pytest.mark.parametrize("H", [4, 80])          # 64- and 128-column walks
 def test_delta_initial_state_at_any_float(H):
     """An initial state and a final-state gradient whose storage starts 4 bytes off a 16-byte boundary
