@@ -12,18 +12,19 @@
 // M = 128, N = its columns; the bf16 image of the state and of U that the MMAs consume as
 // their B operand is rewritten in shared memory each chunk in the 128-byte-swizzled
 // layout TMA itself produces; Q/K/W/M and U^ (or dO) tiles arrive by TMA through a
-// ring of two or three stages, and every output leaves by a TMA store from shared memory. Tiles with 64 token rows are used as 128-row A operands: the upper 64
-// accumulator rows are then meaningless and are never read.
+// ring of two or three stages, and every output leaves by a TMA store from shared memory. Tiles with 64 token rows
+// are used as 128-row A operands: the upper 64 accumulator rows are then meaningless and are never read. In the forward
+// walk they are Q: W and Q are one operand of 128 rows, so that Y and O take eight products instead of sixteen (16
+// sequences of 256 chunks 288 -> 272 us, 283 -> 259 where nothing is kept), and the warps without rows of Y stage O's.
 //
 // The walk is a serial chain per chunk (state image -> Y -> U -> state update), so its length is
 // what counts, not throughput. Eight row warps share the conversions (two per tensor-memory lane
 // quarter, 64 columns each); the state update is issued before the output product and has its own
 // barrier; the output accumulator is double-buffered, so chunk n's output rows are staged while
 // chunk n + 1's Y product runs; the part of the backward's Y that does not need the state is issued
-// before the state image is ready. 64 sequences of 64 chunks: forward 96 us (1.5 us a chunk), backward 86 us, which is 5.1 and 5.7 TB/s;
-// 16 of 256 chunks 287 and 256 us. Four row warps that did all of it in order, in one CTA a sequence, took 230 and 133 us. Extra
-// warps for the output rows and the bulk stores gave nothing: what a chunk takes is the products' chain and the
-// shared memory that they and the conversions share.
+// before the state image is ready. 64 sequences of 64 chunks: forward 96 us (1.5 us a chunk), backward 86 us, which is 5.1
+// and 5.7 TB/s; 16 of 256 chunks 272 and 256 us. Four row warps that did all of it in order, in one CTA a sequence, took
+// 230 and 133 us. What a chunk takes is the products' chain and the shared memory that they and the conversions share.
 //
 // The columns of the state never mix (U, O and dU have the same columns), so when the sequences or
 // segments take at most half of the SMs, two CTAs walk each of them with 64 columns: the conversions
@@ -34,8 +35,8 @@
 // A forward summary walks every segment twice, once per map, over the same W and K. When the two CTAs a
 // segment that takes are more than the SMs, one CTA does both, as two independent chains whose conversions
 // and products fall into each other's waits: one wave and half of the operand reads. 16 sequences x 8
-// segments x 32 chunks: 69 us (86 us when it was built, against 104 us as two waves of a CTA for each map). (One chain of 256 columns:
-// 120 us, its conversions and products take turns.) With a CTA for each map on SMs of their own a chain is the
+// segments x 32 chunks: 69 us; when it was built 86 us, against 104 us as two waves of a CTA for each map and 120 us as
+// one chain of 256 columns, whose conversions and products take turns. With a CTA for each map on SMs of their own a chain is the
 // shorter, so up to half of the SMs it stays so: 72 segments of 32 chunks 62 us, 80 segments in a CTA each 87 us.
 // The initial state is read 16 bytes at a time: element by element the walk of those segments, 70 us, takes 6 us more.
 //
@@ -87,7 +88,7 @@ struct Params {
 // NC: state columns of a CTA. 128, or 64 (then two CTAs per segment, not in summary mode), or 256: both
 // maps of a forward summary as two chains of 128 columns (0: R, 1: P), each with its own row warps, MMA
 // warp and barriers, over the same W and K tiles; no Q, M and output staging.
-template <int NC, int ST>
+template <int NC>
 struct Shape {
   static constexpr bool BOTH = NC == 256;
   static constexpr int CHAINS = BOTH ? 2 : 1;
@@ -96,11 +97,14 @@ struct Shape {
   static constexpr int ROW_WARPS = 8 * CHAINS;
   static constexpr int THREADS = (ROW_WARPS + CHAINS + 1) * 32;
   static constexpr uint32_t COL_Y = BOTH ? 256 : 128, COL_O = 256;   // COL_O: two buffers of 128
+  // Tiles sized for 64 columns leave room for a third stage, which hides the latency that memory has when many CTAs read
+  // and write it. Two / three, 64 chunks, us: forward 16 sequences 79 / 72, 48 98 / 80, 64 112 / 98; backward 74 / 68, 88 / 73,
+  // 99 / 86.
   // a stage: W, Q, K (16 KB each), M (8 KB), U^ or dO (16 KB). W's second half is followed by at
   // least 8 KB of the stage: as a 128-row A operand its upper rows are read from there.
   static constexpr int TILE_W = 0, TILE_Q = 16384, TILE_K = BOTH ? 16384 : 32768, TILE_M = 49152,
                        TILE_DO = BOTH ? 32768 : 57344, STAGE = TILE_DO + (NC == 64 ? 8192 : 16384);
-  static constexpr int STAGES = ST;
+  static constexpr int STAGES = NC == 64 ? 3 : 2;
   static constexpr int XB = STAGES * STAGE;
   static constexpr int UB = XB + 256 * NC;                  // state image, U and output staging: 128, 64 and 64 rows of NC
   static constexpr int OB = UB + 128 * NC;
@@ -109,17 +113,21 @@ struct Shape {
   static_assert(TOTAL <= 227 * 1024, "shared memory of a CTA");
 };
 
-template <bool BWD, int NC, int ST>
-__global__ void __launch_bounds__(Shape<NC, ST>::THREADS, 1)
+template <bool BWD, int NC>
+__global__ void __launch_bounds__(Shape<NC>::THREADS, 1)
 delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmQ,
                   const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmM,
                   const __grid_constant__ CUtensorMap tmDO, const __grid_constant__ CUtensorMap tmXB,
                   const __grid_constant__ CUtensorMap tmU, const __grid_constant__ CUtensorMap tmO,
                   const Params p) {
-  using S = Shape<NC, ST>;
+  using S = Shape<NC>;
   static_assert(!(BWD && S::BOTH), "both maps at once: forward summary only");
   constexpr int TILE_W = S::TILE_W, TILE_Q = S::TILE_Q, TILE_K = S::TILE_K, TILE_M = S::TILE_M, TILE_DO = S::TILE_DO;
   constexpr uint32_t COL_Y = S::COL_Y, COL_O = S::COL_O;
+  // Forward walk: W and Q of a 64-column half lie one behind the other, 128 rows of one A operand, so that Y and O are one
+  // product: Y in lanes 0 .. 63 and O in lanes 64 .. 127 of the output's buffer. (The backward's K, and W alone where a
+  // summary wants no O, run as 128-row operands whose upper lanes are never read.)
+  constexpr bool STACK = !BWD && !S::BOTH;
   constexpr int MMA_WARP = S::ROW_WARPS, TMA_WARP = MMA_WARP + S::CHAINS;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(
@@ -133,13 +141,15 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
   constexpr int STAGES = S::STAGES;
   uint64_t* full = bars;          // [STAGES]
   uint64_t* empty = bars + 3;     // [STAGES]
-  uint64_t* chain_bars = bars + 6 + 5 * chain;
+  uint64_t* chain_bars = bars + 6 + 4 * chain;
   uint64_t* x_ready = chain_bars;
   uint64_t* y_done = chain_bars + 1;
   uint64_t* u_ready = chain_bars + 2;
   uint64_t* x_done = chain_bars + 3;    // the state update of a chunk
-  uint64_t* o_done = chain_bars + 4;    // its output product (forward)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 6 + 5 * S::CHAINS);
+  // [2], by output buffer: a chunk's output product (forward). One barrier for both would be two phases ahead of a warp that
+  // stages rows after U.
+  uint64_t* o_done = bars + 6 + 4 * S::CHAINS;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 2);
 
   const int n_units = p.n_seq * p.n_seg;
   constexpr int HALVES = NC == 64 ? 1 : 2;   // 64-column chunks of U^, dO and the outputs
@@ -166,10 +176,11 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], S::CHAINS); }
 #pragma unroll
     for (int c = 0; c < S::CHAINS; ++c) {
-      uint64_t* b = bars + 6 + 5 * c;
+      uint64_t* b = bars + 6 + 4 * c;
       mbar_init(b, 8); mbar_init(b + 2, 4);   // x_ready, u_ready: one arrival per warp that takes part
-      mbar_init(b + 1, 1); mbar_init(b + 3, 1); mbar_init(b + 4, 1);
+      mbar_init(b + 1, 1); mbar_init(b + 3, 1);
     }
+    mbar_init(&o_done[0], 1); mbar_init(&o_done[1], 1);
     fence_barrier_init();
     tma_prefetch_desc(&tmW); tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK);
     tma_prefetch_desc(&tmM);
@@ -202,12 +213,12 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
         const int row = (seq * NT + n) * C;
         const int trow = tok0 + n * C;
         tma_load_3d(st + TILE_W, &tmW, &full[s], 0, row, 0);
-        tma_load_3d(st + TILE_W + 8192, &tmW, &full[s], 64, row, 0);
+        tma_load_3d(st + TILE_W + (STACK ? 16384 : 8192), &tmW, &full[s], 64, row, 0);
         tma_load_3d(st + TILE_K, &tmK, &full[s], tx, trow, tb);
         tma_load_3d(st + TILE_K + 8192, &tmK, &full[s], tx + 64, trow, tb);
         if (need_qm) {
-          tma_load_3d(st + TILE_Q, &tmQ, &full[s], tx, trow, tb);
-          tma_load_3d(st + TILE_Q + 8192, &tmQ, &full[s], tx + 64, trow, tb);
+          tma_load_3d(st + (STACK ? TILE_W + 8192 : TILE_Q), &tmQ, &full[s], tx, trow, tb);
+          tma_load_3d(st + (STACK ? TILE_W + 24576 : TILE_Q + 8192), &tmQ, &full[s], tx + 64, trow, tb);
           tma_load_3d(st + TILE_M, &tmM, &full[s], 0, row, 0);
         }
         if (BWD) {
@@ -246,17 +257,14 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
         if (!mbar_wait_spin_warp(x_ready, cph, p.status)) break;
         tc_fence_after();
         if (!BWD) {
-          // Y = W X ; O = Q X
+          // Y = W X, and with W and Q stacked O = Q X too. The buffer's previous rows (chunk it - 2) were staged before
+          // this x_ready
 #pragma unroll
           for (int j = 0; j < 8; ++j)
-            umma_f16_lo_warp(tmem + COL_Y, step_k(k_major(TILE_W), j), step_mn(xb_mn, j), id_kn, j > 0);
+            umma_f16_lo_warp(STACK ? col_o : tmem + COL_Y,
+                             STACK ? k_major(TILE_W) + (((j >> 2) * 16384 + (j & 3) * 32) >> 4) : step_k(k_major(TILE_W), j),
+                             step_mn(xb_mn, j), id_kn, j > 0);
           umma_commit_warp(y_done);
-          if (!sum) {
-            // the buffer's previous rows (chunk it - 2) were staged before this x_ready
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-              umma_f16_lo_warp(col_o, step_k(k_major(TILE_Q), j), step_mn(xb_mn, j), id_kn, j > 0);
-          }
         } else {
           // Y += K X
 #pragma unroll
@@ -276,11 +284,11 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
           umma_f16_lo_warp(tmem + COL_X, step_mn(mn_major(BWD ? TILE_W : TILE_K), j), step_mn(ub_mn, j), id_nn, 1);
         umma_commit_warp(x_done);
         if (!BWD && !sum) {
-          // O += M U
+          // O += M U: M in the upper 64 rows; what the lower ones add to Y's lanes is never read
 #pragma unroll
           for (int j = 0; j < 4; ++j)
-            umma_f16_lo_warp(col_o, step_k(k_major(TILE_M), j), step_mn(ub_mn, j), id_kn, 1);
-          umma_commit_warp(o_done);
+            umma_f16_lo_warp(col_o, step_k(k_major(TILE_M) - (8192 >> 4), j), step_mn(ub_mn, j), id_kn, 1);
+          umma_commit_warp(&o_done[it & 1]);
         }
         umma_commit_warp(&empty[s]);
       }
@@ -357,20 +365,16 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
       }
       tmem_st_wait();
     }
-    // Rows of the previous chunk's output: tensor memory -> staging tile. Q S takes 512 clocks of shared-memory reads with
-    // 128 columns, in which stores to it hardly pass: there the rows are staged behind U, while the state is updated. With
-    // 64 columns they are while Y is computed. Late / early, us: 80 sequences x 64 chunks (128 columns) 107 / 127,
-    // 128 segments x 32 chunks 68.9 / 71.7, 16 sequences x 256 chunks (64 columns) 290 / 285.
-    constexpr bool LATE = NC == 128;
-    auto stage_rows = [&](uint32_t buf) {
-      if (BWD || sum) return;
-      wait(o_done, buf);
-      if (tok_warp) {
-        uint32_t v[WC];
-        load_cols(COL_O + buf * 128, v);
-        put_cols(ob, C, v);
-        fence_proxy_async_smem();
-      }
+    // Rows of the previous chunk's output: tensor memory -> staging tile, by the warps that have no token rows of Y, while
+    // the others make U.
+    auto stage_rows = [&](int chunk) {   // the walk's chunk-th
+      if (BWD || sum || tok_warp) return;
+      const uint32_t buf = chunk & 1;
+      wait(&o_done[buf], (chunk >> 1) & 1);
+      uint32_t v[WC];
+      load_cols(COL_O + buf * 128, v);
+      put_cols(ob - C * 128, C, v);   // lanes 64 .. 127 are its rows
+      fence_proxy_async_smem();
     };
     auto store_rows = [&](int n) {
 #pragma unroll
@@ -388,12 +392,10 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
         put_cols(xb, D, v);
       }
       arrive(x_ready);
-      if (!LATE && it > 0) stage_rows(cph ^ 1);
       if (!sum) {
         if (r == 0 && ch == 0) tma_store_wait_read<0>();   // U of the previous chunk has left ub
         sync_rows();
         if (r == 0 && ch == 0) {
-          if (!BWD && !LATE && it > 0) store_rows(n - 1);
           if (store_ux) {
 #pragma unroll
             for (int hf = 0; hf < HALVES; ++hf) tma_store_3d(&tmXB, xb + hf * 16384, col0 + hf * 64, g * D, 0);
@@ -415,7 +417,7 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
         for (int c = 0; c < WC; c += PART) {
           uint32_t v[PART];
 #pragma unroll
-          for (int k = 0; k < PART; k += 32) tmem_ld_32x32b_x32(lane_addr + COL_Y + c + k, v + k);
+          for (int k = 0; k < PART; k += 32) tmem_ld_32x32b_x32(lane_addr + (STACK ? COL_O + cph * 128 : COL_Y) + c + k, v + k);
           tmem_ld_wait();
 #pragma unroll
           for (int i = 0; i < PART / 8; ++i) {
@@ -444,14 +446,14 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
           }
         }
       }
-      if (LATE && it > 0) stage_rows(cph ^ 1);
+      if (it > 0) stage_rows(it - 1);
       if (!sum) {   // while the state is updated: the bulk stores before U's have read xb and ob, which are rewritten next
         if (r == 0 && ch == 0) {
           if (store_ux) tma_store_wait_read<1>();
           else tma_store_wait_read<0>();
         }
         sync_rows();
-        if (!BWD && LATE && it > 0 && r == 0 && ch == 0) {   // read by the next chunk's first wait, before rows are staged again
+        if (!BWD && it > 0 && r == 0 && ch == 0) {   // read by the next chunk's first wait, before rows are staged again
           store_rows(n - 1);
           tma_store_commit();
         }
@@ -461,15 +463,9 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     if (N > 0) {
       wait(x_done, (N - 1) & 1);
       if (!BWD && !sum) {
-        wait(o_done, (N - 1) & 1);
         if (r == 0 && ch == 0) tma_store_wait_read<0>();
         sync_rows();
-        if (tok_warp) {
-          uint32_t v[WC];
-          load_cols(COL_O + ((N - 1) & 1) * 128, v);
-          put_cols(ob, C, v);
-          fence_proxy_async_smem();
-        }
+        stage_rows(N - 1);
         sync_rows();
         if (r == 0 && ch == 0) {
           store_rows(n0 + N - 1);
@@ -503,19 +499,19 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
   }
 }
 
-template <bool BWD, int NC, int ST = 2>
+template <bool BWD, int NC>
 int launch_cols(const CUtensorMap& tW, const CUtensorMap& tQ, const CUtensorMap& tK, const CUtensorMap& tM,
                 const CUtensorMap& tD, const CUtensorMap& tXB, const CUtensorMap& tU, const CUtensorMap& tO,
                 const Params& p, int ctas, cudaStream_t st) {
   static pb::DeviceOnce attr_once;   // per device: the attribute belongs to the current GPU
   if (attr_once.need()) {
-    cudaError_t e = cudaFuncSetAttribute(delta_scan_kernel<BWD, NC, ST>,
+    cudaError_t e = cudaFuncSetAttribute(delta_scan_kernel<BWD, NC>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         Shape<NC, ST>::TOTAL);
+                                         Shape<NC>::TOTAL);
     if (e != cudaSuccess) return static_cast<int>(e);
     attr_once.done();
   }
-  pb::launch(delta_scan_kernel<BWD, NC, ST>, ctas, Shape<NC, ST>::THREADS, Shape<NC, ST>::TOTAL, st, tW, tQ, tK, tM, tD, tXB, tU, tO, p);
+  pb::launch(delta_scan_kernel<BWD, NC>, ctas, Shape<NC>::THREADS, Shape<NC>::TOTAL, st, tW, tQ, tK, tM, tD, tXB, tU, tO, p);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -547,15 +543,8 @@ int launch(const void* W, const void* Q, const void* K, const void* M, const voi
   else r |= tok_map(&tO, o_out);
   if (r != 0) return 1000 + r;
   const int units = p.n_seq * p.n_seg;
-  if (!p.summary && 2 * units <= num_sms()) {
-    // Three stages hide the latency that memory has when many CTAs read and write it. A forward walk of few CTAs, or one
-    // that keeps nothing for the backward, does not wait for memory, and there the earlier arrivals cost more in shared
-    // memory than they save. Two / three, 64 chunks, us: forward 16 sequences 76 / 83, 32 80 / 84, 40 85 / 84, 48 92 / 84..90, 64
-    // 105 / 96; nothing kept 48 76 / 79, 64 81 / 80; backward 16 74 / 68, 40 83 / 69, 64 99 / 86.
-    if (BWD || (p.store_ux != 0 && units > 36))
-      return launch_cols<BWD, 64, 3>(tW, tQ, tK, tM, tD, tXB, tU, tO, p, 2 * units, st);
-    if constexpr (!BWD) return launch_cols<BWD, 64>(tW, tQ, tK, tM, tD, tXB, tU, tO, p, 2 * units, st);
-  }
+  if (!p.summary && 2 * units <= num_sms())
+    return launch_cols<BWD, 64>(tW, tQ, tK, tM, tD, tXB, tU, tO, p, 2 * units, st);
   if constexpr (!BWD) {
     // both maps in one CTA where a CTA for each would be a second wave
     if (p.summary && 2 * units > num_sms())
