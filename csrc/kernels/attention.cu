@@ -20,7 +20,7 @@
 // All tensors are token-major: Q/O/dO/dQ [batch * seq, ldq] with head h at columns 128 h,
 // K/V/dK/dV [batch * seq, ldkv] with KV head g at columns 128 g. Any seq: the tensor maps are per batch entry,
 // so the rows a last tile lacks read as zeros (no real query sees a key after itself, and a zero
-// query with zero dO adds nothing) and are clipped from the stores. 3 x 1000 x 16/4 forward: 24.6 us; with
+// query with zero dO adds nothing) and are clipped from the stores. 3 x 1000 x 16/4 forward: 19.0 us; with
 // padded copies of q, k, v and a cut of the result it took 48 us more.
 //
 // Reference semantics: model/__init__.py gqa/mla attention (softmax(q k^T / sqrt(d)) v with a
@@ -147,11 +147,12 @@ struct Params {
 // (warps 0-3 and 4-7) so that one group's exponentials overlap the other's tensor-core work.
 // Keys and values arrive in blocks of 64. P goes back to tensor memory, over the scores it was made of, as the A
 // operand of P V: 32 KB less shared-memory traffic per block and tile than an operand tile written and read
-// there, and room for five K/V stages instead of three. The rows bound it (about 1800 of 2100 clocks a block: 1024 of
-// exponentials for the two tiles, and the latencies around them); 4 x 4096 x 16/4: 294 -> 280 us. One exponential in
-// eight as a polynomial on the FMA pipe: the same time; one in four: 304.
-// warps 8 and 9: MMA issue for tile 0 and tile 1 (a
-// single issuing thread cannot keep up with 24 small MMAs per block), warp 10: TMA producer.
+// there, and room for five K/V stages instead of three. A block of both tiles takes about 1650
+// clocks: 1280 of products (Q K^T at N = 64 reads 6 KB of shared memory a step) and 1024 of exponentials, which overlap but for
+// the latencies around them. P in tensor memory 4 x 4096 x 16/4 294 -> 280 us, products issued by a warp 280 -> 259 (1 x
+// 8192 x 4/1 132.8 -> 112.7). Taken back: one exponential in eight as a polynomial on the FMA pipe, the same time, one in four
+// slower; the next block's scores read before this one's exponentials 117; the groups' exponentials in turns 120.
+// warps 8 and 9: MMA issue for tile 0 and tile 1, warp 10: TMA producer.
 __global__ void __launch_bounds__(352, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
@@ -447,8 +448,9 @@ struct Params {
 // log-sum-exp and delta come with their tile, and a lane of the dK / dV rows reads 8 columns of them instead of 64.
 // dS is rounded to bf16 once, with the softmax scale in it: P (dP - delta) scale costs two multiplications an
 // element, so the rows' arithmetic is packed two elements to an instruction.
-// 4 x 4096 x 16/4, clocks a 128 x 64 tile: dQ 1157 -> 1081 (768 of them MMAs), dK and dV 1908 -> 1644 (1280);
-// together 909 -> 835 us, under the power cap 1045 -> 956.
+// 4 x 4096 x 16/4, clocks a 128 x 64 tile: dQ 1157 -> 1081 (768 of them MMAs), dK and dV 1908 -> 1500 (1280; 1644
+// before a warp issued them); together 909 -> 811 us. A dQ block spends 10500 of 45600 clocks outside its loop: its
+// resident tiles' arrival, delta, and the stores.
 template <bool DKV>
 __global__ void __launch_bounds__(384, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant__ CUtensorMap tmRB,
@@ -495,7 +497,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
     mbar_init(r_full, 1);
     for (int i = 0; i < STAGES; ++i) { mbar_init(&t_full[i], 1); mbar_init(&t_empty[i], 1); }
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&x_done[i], 2); mbar_init(&x_free[i], 1);    // two issuing threads
+      mbar_init(&x_done[i], 2); mbar_init(&x_free[i], 1);    // two issuing warps
       mbar_init(&pd_ready[i], 8);                            // one arrival per row warp
     }
     mbar_init(acc_done, 1);

@@ -587,8 +587,8 @@ __device__ __forceinline__ uint64_t make_sdesc_sw128(uint32_t saddr, uint32_t lb
 }
 
 // The same descriptor split into its two 32-bit words. Only the low word (start address,
-// leading byte offset) changes between the MMAs of a tile, and only by a constant, so an
-// issuing thread that keeps `lo` in a register spends one add per operand per MMA:
+// leading byte offset) changes between the MMAs of a tile, and only by a constant, so
+// code that keeps `lo` in a register spends one add per operand per MMA:
 //   lo' = lo + (byte_offset >> 4)      (valid inside the 256 KB shared-memory window)
 __device__ __forceinline__ uint32_t sdesc_lo(uint32_t saddr, uint32_t lbo_bytes) {
   return ((saddr & 0x3FFFFu) >> 4) | (((lbo_bytes >> 4) & 0x3FFFu) << 16);

@@ -17,7 +17,7 @@
 // taken out of it: the next chunk's S, dS', dO, U and -dU arrive in a region of their own while this one is worked on,
 // its dW and dM are multiplied during this chunk's last products, and the state products of dQ and dK run
 // beside the conversion of dW.
-//   warp 2: TMA producer   warp 3: MMA issue (one lane)
+//   warp 2: TMA producer   warp 3: MMA issue
 //   warps 0, 1, 4, 5, 8, 9, 12, 13: rows 0..31 and 32..63 of the accumulators (a warp reads the tensor-memory lanes of its
 //   quarter; the 64-row operands run as 128-row ones, whose upper rows are never read), a quarter of the columns each
 //
