@@ -449,7 +449,7 @@ struct Params {
 // dS is rounded to bf16 once, with the softmax scale in it: P (dP - delta) scale costs two multiplications an
 // element, so the rows' arithmetic is packed two elements to an instruction.
 // 4 x 4096 x 16/4, clocks a 128 x 64 tile: dQ 1157 -> 1081 (768 of them MMAs), dK and dV 1908 -> 1500 (1280; 1644
-// before a warp issued them); together 909 -> 811 us. A dQ block spends 10500 of 45600 clocks outside its loop: its
+// before a warp issued them); together 909 -> 811 us. A dQ block spends 10000 of 45000 clocks outside its loop: its
 // resident tiles' arrival, delta, and the stores.
 template <bool DKV>
 __global__ void __launch_bounds__(384, 1)
@@ -469,8 +469,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
   uint64_t* pd_ready = bars + 17; // [2] its P^T and dS
   uint64_t* acc_done = bars + 19;
   uint64_t* o_full = bars + 20;   // dQ: the forward's output tile, in the last of the first four stages
-  uint64_t* r_read = bars + 21;   // dQ: delta is taken from it and the resident tiles are in tensor memory
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 22);
+  uint64_t* r_read = bars + 21;   // dQ: delta is taken from it and from the resident dO
+  uint64_t* r_copied = bars + 22; // dQ: the resident tiles are in tensor memory
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 23);
   constexpr int STAGES = Ring<DKV>::STAGES, O_STAGE = 3;
   auto stage = [&](int s) { return smem + Ring<DKV>::off(s); };
 
@@ -501,7 +502,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
       mbar_init(&pd_ready[i], 8);                            // one arrival per row warp
     }
     mbar_init(acc_done, 1);
-    mbar_init(o_full, 1); mbar_init(r_read, 8);
+    mbar_init(o_full, 1); mbar_init(r_read, 8); mbar_init(r_copied, 8);
     fence_barrier_init();
     tma_prefetch_desc(&tmRA); tma_prefetch_desc(&tmRB);
     tma_prefetch_desc(&tmT1); tma_prefetch_desc(&tmT2);
@@ -562,7 +563,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
       const uint32_t r_lo = sdesc_lo(smem_u32(smem + (which == 0 ? RA_OFF : RB_OFF)), 16);
       const uint32_t r_col = tmem + COL_R + which * 64;
       const uint32_t col = which == 0 ? 0 : COL_X2;
-      bool ok = n_it == 0 || mbar_wait_spin_warp(DKV ? r_full : r_read, 0, p.status);
+      bool ok = n_it == 0 || mbar_wait_spin_warp(DKV ? r_full : r_copied, 0, p.status);
       int ts = 0;
       uint32_t ph = 0;
       for (int it = 0; it < n_it && ok; ++it) {
@@ -628,8 +629,26 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
       const size_t bh = static_cast<size_t>(b) * p.heads + hy;
       if (q < p.seq) row_lse = p.lse2[bh * p.seq + q];
       // delta of the row from the resident dO and the forward's output: a kernel of its own read both
-      // again (268 MB, 45 us at 4 x 4096 x 16). Both groups need it.
-      ok = wait_all(r_full, 0, p.status) && wait_all(o_full, 0, p.status);
+      // again (268 MB, 45 us at 4 x 4096 x 16). Both groups need it, and add up half of it each.
+      ok = wait_all(r_full, 0, p.status);
+      if (ok) {
+        // group 0 puts Q, group 1 dO where the score products read them, so that these run while delta is added up (3 x 1000 x 16/4,
+        // both kernels: 91.6 -> 89.6 us, and 88.6 with delta halved): a row is 64 columns of bf16 pairs
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          uint32_t w[32];
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            *reinterpret_cast<uint4*>(w + 4 * i) = *reinterpret_cast<const uint4*>(
+                smem + (wg == 0 ? RA_OFF : RB_OFF) + c * 16384 + r * 128 + ((i ^ (r & 7)) << 4));
+          tmem_st_32x32b_x32(lane_addr + COL_R + wg * 64 + c * 32, w);
+        }
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(r_copied);
+        ok = wait_all(o_full, 0, p.status);
+      }
       if (ok) {
         // Columns are added as a warp with four of them to a lane adds its lanes up (halves, quarters, ..):
         // dS, and with it the gradients' bf16 roundings, depend on the sum's last bit.
@@ -645,28 +664,24 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmRA, const __grid_constant_
         };
         auto half_sum = [&](const int i) { return add2(lanes(i), lanes(i + 8)); };
         auto quarter_sum = [&](const int i) { return add2(half_sum(i), half_sum(i + 4)); };
-        const float2 even = add2(quarter_sum(0), quarter_sum(2)), odd = add2(quarter_sum(1), quarter_sum(3));
-        const float2 sum = add2(even, odd);
+        // a group adds up half of the pieces and takes the other half from the other group
+        float2* const swap = reinterpret_cast<float2*>(smem + VEC_OFF);   // 2 KB, unused by dQ
+        const float2 mine = wg == 0 ? add2(quarter_sum(0), quarter_sum(2)) : add2(quarter_sum(1), quarter_sum(3));
+        swap[threadIdx.x] = mine;
+      }
+      ok = bar_sync_and(3, 256, ok);
+      if (ok) {
+        const float2* const swap = reinterpret_cast<const float2*>(smem + VEC_OFF);
+        const float2 mine = swap[threadIdx.x], theirs = swap[threadIdx.x ^ 128];
+        const float2 sum = wg == 0 ? add2(mine, theirs) : add2(theirs, mine);
         row_delta = __fadd_rn(sum.x, sum.y);
         if (q < (p.seq + 63) / 64 * 64) {   // rows past seq have zeros in all four
           float* v = p.vec + (bh * ((p.seq + 63) / 64) + (q >> 6)) * 128 + ((q & 63) >> 1) * 4 + (q & 1);
           if (wg == 0) v[0] = -row_lse;
           else v[2] = -row_delta;
         }
-        // group 0 puts Q, group 1 dO where the score products read them: a row is 64 columns of bf16 pairs
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          uint32_t w[32];
-#pragma unroll
-          for (int i = 0; i < 8; ++i)
-            *reinterpret_cast<uint4*>(w + 4 * i) = *reinterpret_cast<const uint4*>(
-                smem + (wg == 0 ? RA_OFF : RB_OFF) + c * 16384 + r * 128 + ((i ^ (r & 7)) << 4));
-          tmem_st_32x32b_x32(lane_addr + COL_R + wg * 64 + c * 32, w);
-        }
-        tmem_st_wait();
       }
       fence_proxy_async_smem();   // the producer's next loads go over what was read here
-      tc_fence_before();
       __syncwarp();
       if (ok && lane == 0) mbar_arrive(r_read);
     }
