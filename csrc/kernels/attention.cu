@@ -165,9 +165,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint64_t* kv_full = bars + 1;    // [KV_STAGES]
   uint64_t* kv_empty = bars + 6;   // [KV_STAGES]
   uint64_t* s_done = bars + 11;    // [tile][buf]
-  uint64_t* p_ready = bars + 15;   // [tile]
-  uint64_t* o_done = bars + 17;    // [tile][buf]: P V of the block whose scores that buffer held
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 22);
+  // [tile][buf], like the scores: these run two blocks ahead, so a warp may be done with block j + 1 while another still
+  // rescales O in block j. With one barrier for both, its two arrivals and two of the others would complete block j's phase,
+  // and P V would read the slow warp's raw scores as its P. Block j + 2 of a buffer comes after P V of j, that is after all.
+  uint64_t* p_ready = bars + 15;
+  uint64_t* o_done = bars + 19;    // [tile][buf]: P V of the block whose scores that buffer held
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 23);
 
   const int warp = warp_index(), lane = threadIdx.x & 31;
   // blocks start in index order, so the row block is the slowest index: the longest rows of all heads and
@@ -187,8 +190,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     for (int i = 0; i < KV_STAGES; ++i) { mbar_init(&kv_full[i], 1); mbar_init(&kv_empty[i], 2); }
     for (int i = 0; i < 4; ++i) {
       mbar_init(&s_done[i], 1); mbar_init(&o_done[i], 1);
+      mbar_init(&p_ready[i], 4);   // one arrival per warp
     }
-    mbar_init(&p_ready[0], 4); mbar_init(&p_ready[1], 4);   // one arrival per warp
     fence_barrier_init();
     tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
   }
@@ -256,7 +259,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       if (ok && nj > 1) ok = issue_s(1);
       for (int j = 0; j < nj && ok; ++j) {
         const int s = j % KV_STAGES;
-        if (!mbar_wait_spin_warp(&p_ready[t], j & 1, p.status)) break;
+        if (!mbar_wait_spin_warp(&p_ready[t * 2 + (j & 1)], (j >> 1) & 1, p.status)) break;
         tc_fence_after();
         const uint32_t v_lo = sdesc_lo(kv0 + s * KV_STAGE + 16384, 8192);
         // 16 values of a bf16 operand row are eight tensor-memory columns
@@ -347,7 +350,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&p_ready[t]);
+      if (lane == 0) mbar_arrive(&p_ready[sb]);
       PB_PROF(5)
 #ifdef PB_ATTN_PROF
       if (r == 0) atomicAdd(&g_attn_prof[6], 1ull);

@@ -60,6 +60,27 @@ def test_attention_large_logits_exercise_the_rescale_path():
     assert _rel(out, ref) < 1.5e-2
 
 
+@pytest.mark.parametrize("slow", [1, 2, 4])
+def test_rows_that_rescale_in_every_block_beside_rows_that_never_do(slow):
+    """``slow`` of the four warps of a tile see scores that grow by 2^12 a block of keys, so they rescale O in each, and the
+    others, whose scores stay small, wait for none of it. P is rounded to bf16 once (2^-9 of a value) and so is the result."""
+    from prometheus_b200.ops import attention
+
+    s, hq = 2048, 32
+    q, k, v = _rand(1, s, hq, 1, 5, 0.5)
+    row, head = torch.arange(s, device="cuda"), torch.arange(hq, device="cuda")
+    quarter = (row[:, None] // 32 + head) % 4             # which warps are slow differs from head to head
+    step = 12 * math.log(2.0) * math.sqrt(128) / 16
+    q[0, ..., 0] = torch.where(quarter < slow, 16.0, 0.0).to(BF16)
+    k[0, :, 0, 0] = (row // 64 * step).to(BF16)
+    out, top = attention.causal_gqa(q, k, v, return_max_logit=True)
+    again = attention.causal_gqa(q, k, v)
+    ref = attention.causal_gqa_ref(q.float(), k.float(), v.float())
+    assert torch.equal(out, again)
+    assert (out.float() - ref).abs().max() <= 2.0 ** -7 * v.float().abs().max()
+    assert torch.isfinite(top).all()
+
+
 def test_attention_is_deterministic_and_matches_library_kernel():
     import torch.nn.functional as F
 

@@ -5,6 +5,7 @@ gave up one by one would leave the others at an instruction that never completes
 reported would become a kernel that never returns. So a wait either belongs to a single thread, or it is one of
 the warp-uniform forms, or its result goes through ``__syncthreads_and`` before anybody acts on it; and where a
 named barrier follows a wait, either the barrier carries the result (``bar_sync_and``) or nobody leaves the loop."""
+import random
 import re
 from pathlib import Path
 
@@ -67,3 +68,44 @@ def test_the_reader_of_sources_sees_a_wait_that_splits_a_warp():
     text = _text("gemm.cu")
     assert "mbar_wait_warp(&tfull" in text
     assert per_thread_waits(text.replace("mbar_wait_warp(&tfull", "mbar_wait(&tfull"))
+
+
+def miscounted_blocks(text, blocks=12, schedules=200):
+    """Blocks of the attention forward whose P V product is issued before all four row warps of the tile have stored P, or never,
+    over random schedules of the warps and the issuer. Barriers, their indexes and parities are the source's; the scores of block j
+    are there once P V of block j - 2 is issued, and a warp that has to raise its maximum may take any time over a block."""
+    wait = re.search(r"mbar_wait_spin_warp\(&p_ready\[(.+?)\], (.+?), p\.status\)", text)
+    arrive = re.search(r"mbar_arrive\(&p_ready\[(\w+)\]\)", text)
+    sb = re.search(r"const int sb = (t \* 2 \+ \(j & 1\));\s+const uint32_t ph", text)
+    assert wait and arrive and sb and re.search(r"mbar_init\(&p_ready\[\w+\], 4\)", text)
+    value = lambda expr, j: eval(expr, {"t": 0, "j": j, "sb": eval(sb.group(1), {"t": 0, "j": j})})
+    bad = set()
+    for seed in range(schedules):
+        rng = random.Random(seed)
+        pending, phase, at, done = [4] * 4, [0] * 4, [0] * 4, 0
+        for _ in range(200 * blocks):
+            actor = rng.choice((0, 0, 0, 1, 1, 1, 2, 2, 2, 3, "issuer"))      # warp 3 is the slow one
+            if done == blocks:
+                break
+            if actor == "issuer":
+                if phase[value(wait.group(1), done)] != value(wait.group(2), done):
+                    if min(at) <= done:
+                        bad.add(done)
+                    done += 1
+            elif at[actor] < min(done + 2, blocks):
+                i = value(arrive.group(1), at[actor])
+                at[actor] += 1
+                pending[i] -= 1
+                if pending[i] == 0:
+                    pending[i], phase[i] = 4, phase[i] ^ 1
+        if done < blocks:
+            bad.add(done)
+    return bad
+
+
+def test_attention_forward_counts_each_block_of_every_row_warp():
+    text = _text("attention.cu")
+    assert miscounted_blocks(text) == set()
+    # one barrier for both score buffers: a fast warp's next block stands in for a slow warp's
+    one = re.sub(r"(mbar_wait_spin_warp\(&p_ready\[).+?\], .+?,", r"\1t], j & 1,", text)
+    assert miscounted_blocks(one.replace("mbar_arrive(&p_ready[sb])", "mbar_arrive(&p_ready[t])"))
