@@ -24,6 +24,7 @@ from __future__ import annotations
 
 import argparse
 import json
+import math
 import os
 import statistics
 import subprocess
@@ -333,7 +334,20 @@ def measure(args, config: str, world: int, rank: int, local_rank: int, dev, step
 
     gc.collect()
     torch.cuda.empty_cache()
-    return result
+    return without_broken_runs(result)
+
+
+def without_broken_runs(result: dict) -> dict:
+    """The result without the rates of a region whose training was broken when it ended: steps on NaN operands draw
+    less power and run faster than the real ones. (NaN is not JSON either.)"""
+    out = dict(result)
+    if not math.isfinite(out["e2e_loss"]):
+        out["e2e"] = {"value": None, "unit": "tokens/s", "unavailable": "the loss at the end of the region is not finite"}
+        out["e2e_loss"] = None
+    if not math.isfinite(out["loss"]):
+        out["unavailable"] = "the loss at the end of the timed region is not finite"
+        out.update(value=None, mfu=None, loss=None)
+    return out
 
 
 def main() -> int:
@@ -384,6 +398,8 @@ def main() -> int:
             secondary["moe16b"] = {k: sec[k] for k in ("value", "ms_per_step", "mfu", "config",
                                                        "gpu_launches", "loss")}
             secondary["moe16b"]["unit"] = "tokens/s"
+            if "unavailable" in sec:
+                secondary["moe16b"]["unavailable"] = sec["unavailable"]
     if rank == 0:
         value = main_res["value"]
         line = {
@@ -396,6 +412,8 @@ def main() -> int:
             "exposed_comm_ms": main_res["exposed_comm_ms"],
             "loss": main_res["loss"], "e2e_loss": main_res["e2e_loss"], "impl": "ours",
         }
+        if "unavailable" in main_res:
+            line["unavailable"] = main_res["unavailable"]
         if secondary:
             line["secondary"] = secondary
         print(json.dumps(line), flush=True)
@@ -408,7 +426,7 @@ def vs_baseline(value: float, world: int, args):
     """value / the baseline number recorded for this GPU count. The reference publishes no
     throughput; the recorded baseline is this repository's own NCCL-only gradient path
     (``--grad-sync nccl``) on the same configuration, kept in ``baseline/nccl_only.json``."""
-    if args.config != "dense" or args.layers:
+    if args.config != "dense" or args.layers or value is None:
         return None
     try:
         table = json.loads((ROOT / "baseline" / "nccl_only.json").read_text())
