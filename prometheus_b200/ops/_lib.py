@@ -116,6 +116,7 @@ _SIGS = {
     "pb_gemm_fp8_probe": [P, P, P, P, P, I, I, I, L, I, P, P],       # debug build only
     "pb_gemm_set_variant": [I],
     "pb_newton_schulz": [P, P, P, P, I, I, I, I, F, F, F, P, P],
+    "pb_gemm_f32_in_order": [P, P, P, I, I, I, L, L, L, P, P],
     "pb_gemm_bf16_scaled": [P, P, P, I, I, I, L, L, L, I, I, P, P, P],
     "pb_gemm_bf16": [P, P, P, P, I, I, I, I, L, L, L, L, L, L, L, L, I, I, I, I, F, F, P, I, P],
 }

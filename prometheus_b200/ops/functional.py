@@ -128,6 +128,18 @@ def _gemm_2d(a: Tensor, b: Tensor, a_mn: bool, b_mn: bool, out: Tensor | None, o
     return out
 
 
+def router_logits(x: Tensor, w: Tensor) -> Tensor:
+    """fp32 ``x @ w^T`` whose rows do not depend on how many of them there are: ``gemm`` shares long contractions of
+    products with few tiles between CTAs, and a token near a tie would choose other experts in a short call than in a long
+    one."""
+    assert x.dtype == w.dtype == BF16 and x.is_cuda and x.shape[1] == w.shape[1]
+    x, w = (t if t.stride(1) == 1 and t.stride(0) % 8 == 0 else t.contiguous() for t in (x, w))
+    out = torch.empty((x.shape[0], w.shape[0]), dtype=torch.float32, device=x.device)
+    call("pb_gemm_f32_in_order", ptr(x), ptr(w), ptr(out), x.shape[0], w.shape[0], x.shape[1], x.stride(0), w.stride(0),
+         out.stride(0), ptr(status_word(x.device)), stream_ptr())
+    return out
+
+
 def newton_schulz(x: Tensor, y: Tensor, g: Tensor, pm: Tensor, steps: int, a: float, b: float, c: float) -> Tensor:
     """``steps`` quintic Newton-Schulz iterations over a batch of matrices ``x`` (nb, rows, cols) bf16: the products
     ``gemm`` would be called for, issued by one call. ``y`` like ``x``, ``g`` and ``pm`` (nb, m, m) with m the smaller

@@ -147,7 +147,7 @@ def _acc_grad(w: Tensor, shape3, fn):
 class _MoeFfnFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, router_w, router_bias, w_gu_p, w_down_p, top_k, n_shared, shapes, fp8=False):
-        from .functional import gemm
+        from .functional import router_logits
 
         ctx.set_materialize_grads(False)   # the scores' and logits' gradients are often absent
         w_gu = w_gu_p.view(shapes[0]) if shapes is not None else w_gu_p
@@ -155,7 +155,7 @@ class _MoeFfnFn(torch.autograd.Function):
         T, d = x.shape
         E, two_h, _ = w_gu.shape          # routed + shared
         h = two_h // 2
-        logits = gemm(x, router_w, out_dtype=torch.float32)
+        logits = router_logits(x, router_w)
         probs, ids_r, gates_r = route(logits, router_bias, top_k)
         if n_shared:
             # shared experts: every token, gate 1, appended as extra slots

@@ -158,7 +158,7 @@ class _EpMoeFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, router_w, router_bias, w_gu_p, w_down_p, top_k, ep, shapes, fp8=False):
         from ..ops import fp8 as F8
-        from ..ops.functional import gemm
+        from ..ops.functional import router_logits
 
         w_gu = w_gu_p.view(shapes[0]) if shapes is not None else w_gu_p      # [El, 2h, d]
         w_down = w_down_p.view(shapes[1]) if shapes is not None else w_down_p
@@ -166,7 +166,7 @@ class _EpMoeFn(torch.autograd.Function):
         h = w_gu.shape[1] // 2
         sym = ep.sym
         use_fp8 = bool(fp8) and ep.fp8_ok and h % 128 == 0
-        logits = gemm(x, router_w, out_dtype=torch.float32)
+        logits = router_logits(x, router_w)
         probs, ids, gates = M.route(logits, router_bias, top_k)
         local = M.place(ids, ep.E)
         ep.counts_local.copy_(local.totals)

@@ -52,6 +52,23 @@ def test_route_and_placement(T, E, k):
         assert off[mg[m]] <= m * 128 < off[mg[m] + 1]
 
 
+@pytest.mark.parametrize("d,E", [(2048, 64), (1024, 8), (2056, 160), (1024, 512)])
+def test_a_token_chooses_its_experts_whatever_the_call_holds_beside_it(d, E):
+    """Router logits of the first rows alone and among 8192, bit for bit: 1 to 256 tiles, contractions that an ordinary product
+    shares out between 8, 2 or no CTAs, and the last of them on CTA pairs."""
+    from prometheus_b200.ops import functional as ops
+
+    x, w = _r(8192, d, seed=1), _r(E, d, seed=2, scale=d ** -0.5)
+    full = ops.router_logits(x, w)
+    _close(full, x.float() @ w.float().t(), 1e-4)
+    for n in (1, 100, 512, 2500, 4736):
+        assert torch.equal(ops.router_logits(x[:n], w), full[:n]), n
+    wide = torch.zeros(100, d + 5, dtype=BF16, device="cuda")        # rows that do not start on 16 bytes
+    wide[:, 3:3 + d] = x[:100]
+    assert torch.equal(ops.router_logits(wide[:, 3:3 + d], w), full[:100])
+    ops.check_status("cuda")
+
+
 @pytest.mark.parametrize("T,E,k,skew", [(683, 64, 6, 0), (4097, 512, 1, 0), (64 * 9 + 1, 300, 8, 0), (8200, 5, 3, 0), (4160, 64, 1, 1)])
 def test_placement_over_many_blocks(T, E, k, skew):
     """The three-kernel sort: one pair more than the one-block sort takes, a thread or several to an expert in the scan, shares of
