@@ -42,6 +42,7 @@ _SIGS = {
     "pb_l2norm_bwd": [P, P, P, L, I, P],
     "pb_softcap_ce": [P, P, P, P, P, L, I, F, I, P],
     "pb_softcap_ce_sums": [P, P, P, P, P, L, I, F, I, P],
+    "pb_gemm_on_pairs": [I, I, I],
     "pb_gemm_softcap_ok": [I, I, I],
     "pb_gemm_softcap_pays": [I, I, I],
     "pb_gemm_softcap_logits": [P, P, P, I, I, I, L, L, L, F, P, P, P, P],

@@ -133,7 +133,7 @@ def test_gemm_c_and_d_at_any_base(M, N, c_f32, d_f32):
     a, b = _r(2, M, 192, seed=1), _r(2, N, 192, seed=2)
     d = _r(2, M, N, seed=3, dtype=dts[d_f32])
     try:
-        for variant in (0, 8):         # CTA pairs where they apply, the single-CTA kernel
+        for variant in (0, 8):         # single CTAs, tiles of 128 x 128 and of 128 x 256
             call("pb_gemm_set_variant", variant)
             kw = dict(out_dtype=dts[c_f32], alpha=0.5, beta=-2.0)
             want = ops.gemm(a, b, d=d, **kw)
@@ -159,7 +159,7 @@ def test_gemm_c_and_d_at_any_base(M, N, c_f32, d_f32):
 def test_gemm_d_at_remainders_against_fp32(M, N, c_f32, d_f32):
     """alpha A B^T + beta D where a row's D is read partly in whole slabs ahead of the accumulator and partly by
     column chunks: every combination of the types of C and D, a contiguous D and a column slice of a wider one, on
-    CTA pairs and on single CTAs, alone and batched."""
+    single CTAs with 128 x 128 and 128 x 256 tiles, alone and batched."""
     from prometheus_b200.ops import functional as ops
     from prometheus_b200.ops._lib import call
 
@@ -179,6 +179,38 @@ def test_gemm_d_at_remainders_against_fp32(M, N, c_f32, d_f32):
                     assert (err <= tol * ref.abs() + 1e-3).all(), (variant, float(err.max()))
     finally:
         call("pb_gemm_set_variant", 0)
+    ops.check_status("cuda")
+
+
+# beyond one wave of 128 x 128 tiles: the same remainders as above where CTA pairs run the product
+@pytest.mark.parametrize("M,N,batch", [(200, 328, 40), (456, 264, 14), (520, 264, 26), (4296, 1288, 1)])
+@pytest.mark.parametrize("c_f32", [False, True])
+@pytest.mark.parametrize("d_f32", [False, True])
+def test_gemm_c_and_d_on_pairs_at_remainders_and_any_base(M, N, batch, c_f32, d_f32):
+    """alpha A B^T + beta D on CTA pairs at row remainders 200, 8 and column remainders 8 and 72: a contiguous D, column slices
+    that start on and off 16 bytes, destinations and D's an element off, against fp32 and the aligned call."""
+    from prometheus_b200.ops import functional as ops
+    from prometheus_b200.ops._lib import query
+
+    assert query("pb_gemm_on_pairs", M, N, batch) == 1 and query("pb_gemm_on_pairs", 200, 328, 2) == 0
+    ty = {False: BF16, True: torch.float32}
+    a, b = _r(batch, M, 192, seed=1), _r(batch, N, 192, seed=2)
+    wide = _r(batch, M, N + 24, seed=3, dtype=ty[d_f32], scale=8.0)      # D as large as the product
+    kw = dict(alpha=0.5, beta=-2.0)
+    tol = 1e-5 if c_f32 else 2.0 ** -8      # fp32 sums of 192 products, one rounding of the result
+    aligned = None
+    for d in (wide[:, :, 8:8 + N], wide[:, :, 8:8 + N].contiguous(), wide[:, :, 1:1 + N]):
+        ref = ops.gemm_ref(a, b, d=d, **kw)
+        got = ops.gemm(a, b, d=d, out_dtype=ty[c_f32], **kw)
+        assert ((got.float() - ref).abs() <= tol * ref.abs() + 1e-3).all()
+        aligned = got if aligned is None else aligned
+    d = wide[:, :, 8:8 + N]
+    for off_c, off_d in ((0, 1), (1, 0), (1, 1)):
+        buf = torch.full((batch * M * N + 16,), 7.0, dtype=ty[c_f32], device="cuda")
+        out = buf[off_c:off_c + batch * M * N].view(batch, M, N)
+        shifted = torch.empty(batch * M * N + 1, dtype=ty[d_f32], device="cuda")[off_d:off_d + batch * M * N].view(d.shape).copy_(d)
+        assert torch.equal(ops.gemm(a, b, out=out, d=shifted, **kw), aligned), (off_c, off_d)
+        assert (buf[:off_c] == 7).all() and (buf[off_c + out.numel():] == 7).all()
     ops.check_status("cuda")
 
 
