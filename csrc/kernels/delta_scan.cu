@@ -28,9 +28,10 @@
 //
 // The columns of the state never mix (U, O and dU have the same columns), so when the sequences or
 // segments take at most half of the SMs, two CTAs walk each of them with 64 columns: the conversions
-// and products between two waits are half as long. On both sides of the line, 64 chunks each: 74 sequences with
-// 64 columns a CTA 79 us forward (nothing kept) and 104 us backward, 75 sequences with 128 columns 105 and 110 us. With
-// more CTAs than SMs it would be two waves of a chain that is not half as long.
+// and products between two waits are half as long. A forward walk that keeps the states stops eight sequences earlier, at 66 on
+// 148 SMs, where its stores are what it waits for (figures at the rule in launch()). On both sides of the line, 64 chunks
+// each: 74 sequences with 64 columns a CTA 79 us forward (nothing kept) and 104 us backward, 75 sequences with 128 columns 105
+// and 110 us. With more CTAs than SMs it would be two waves of a chain that is not half as long.
 //
 // A forward summary walks every segment twice, once per map, over the same W and K. When the two CTAs a
 // segment that takes are more than the SMs, one CTA does both, as two independent chains whose conversions
@@ -544,7 +545,7 @@ int launch(const void* W, const void* Q, const void* K, const void* M, const voi
   if (r != 0) return 1000 + r;
   const int units = p.n_seq * p.n_seg;
   // A forward walk that keeps the states stays on 128 columns from 67 sequences on: with the last SMs writing too its stores
-  // back up. 64 / 128 columns, 64 chunks, us: 60 sequences 91 / 120, 64 98 / 125, 68 141 / 127..131, 72 150 / 136, 74 150 / 129; nothing
+  // back up (seen on 148 SMs; the line is a measured one). 64 / 128 columns, 64 chunks, us: 60 sequences 91 / 120, 64 98 / 125, 68 141 / 127..131, 72 150 / 136, 74 150 / 129; nothing
   // kept 74 79 / 104, backward 74 104 / 109.
   const int most = BWD || p.store_ux == 0 ? num_sms() : num_sms() - 16;
   if (!p.summary && 2 * units <= most)

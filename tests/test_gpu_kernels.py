@@ -872,7 +872,7 @@ def test_delta_summary_maps(n_seq, n_chunks, n_seg, cut):
 @pytest.mark.parametrize("H,S", [(3, 448), (37, 64), (37, 129), (37, 256), (37, 448), (74, 300)])
 def test_delta_walk_stages(H, S):
     """64-column walks, which have three stages, of one chunk to more than twice as many, against the same heads among 80,
-    whose walk has 128 columns: the columns of the state never mix and each sum is over the same terms in the same
+    whose walk has 128 columns (from 67 on the forward has 128 too, since it keeps the states; the backward has 64 up to 74): the columns of the state never mix and each sum is over the same terms in the same
     order, so all outputs are the same bits."""
     from prometheus_b200.ops.delta import delta_rule_fused
 
@@ -886,6 +886,46 @@ def test_delta_walk_stages(H, S):
 
     for few, many in zip(run(H), run(80)):
         assert torch.equal(few, many)
+
+
+@pytest.mark.parametrize("H,grad", [(66, True), (67, True), (74, False), (75, False)])
+def test_delta_walk_columns_at_their_lines(H, grad):
+    """The last sequence counts of 64-column walks and the first of 128-column ones, on 148 SMs: 66 and 67 for a forward that
+    keeps the states (74 and 75 for its backward), 74 and 75 for one that keeps nothing. The same heads among 80, bit for bit."""
+    from prometheus_b200.ops.delta import delta_rule_fused
+
+    q, k, v, do = (_r(1, 300, 80, 128, seed=i, scale=0.08) for i in (1, 2, 3, 5))
+    beta = torch.sigmoid(_r(1, 300, 80, seed=4, dtype=torch.float32))
+
+    def run(h):
+        leaves = [t[:, :, :h].contiguous().requires_grad_(grad) for t in (q, k, v, beta)]
+        out, fin = delta_rule_fused(*leaves, None, n_seg=1)
+        grads = torch.autograd.grad(out, leaves, do[:, :, :h].contiguous()) if grad else ()
+        return [t[:, :, :H] for t in (out, *grads)] + [fin[:, :H]]
+
+    for few, many in zip(run(H), run(80)):
+        assert torch.equal(few, many)
+
+
+def test_delta_layer_over_128_sequences_of_64_chunks():
+    """The walks with 128 columns and the states kept, two stages deep over 64 chunks, as a training run at 8 x 4096 tokens and 16
+    heads has them, against the fp32 scan. Images of the state and of U, W, U^, M and the gradients' operands are bf16:
+    each rounds by 2^-9 of its size, about ten of them between an input and a result."""
+    from prometheus_b200.ops import delta as dl
+
+    B, S, H = 8, 4096, 16
+    q, k = (torch.nn.functional.normalize(_r(B, S, H, 128, seed=i).float(), dim=-1).to(BF16) for i in (1, 2))
+    v, do = _r(B, S, H, 128, seed=3), _r(B, S, H, 128, seed=5)
+    beta = torch.sigmoid(_r(B, S, H, seed=4))
+    leaves = [t.requires_grad_(True) for t in (q, k, v, beta)]
+    out, fin = dl.delta_rule_fused(*leaves, None)
+    got = [out, fin, *torch.autograd.grad(out, leaves, do)]
+    for b in range(0, B, 3):
+        ref = [t[b:b + 1].detach().float().requires_grad_(True) for t in leaves]
+        r_out, r_fin = dl.delta_rule_scan(*ref, None)
+        want = [r_out, r_fin, *torch.autograd.grad(r_out, ref, do[b:b + 1].float())]
+        for g, w in zip(got, want):
+            assert ((g[b:b + 1].float() - w).norm() / w.norm()).item() < 10 * 2.0 ** -9
 
 
 @pytest.mark.parametrize("H", [4, 80])          # 64- and 128-column walks
@@ -933,6 +973,23 @@ def test_delta_compose(n_seq, n_seg, reverse):
         assert (s_fin.double() - cur).norm() <= 1e-5 * cur.norm()
         if not reverse:
             assert (p_tot.double() - tot).norm() <= 1e-5 * tot.norm()
+
+
+def test_gemm_accumulates_sums_below_the_normal_range():
+    """Adding stores flush sums below 2^-126 to zero, the epilogue's addition does not: 32 products added into one buffer stay
+    within 32 x 2^-126 of the exact sum there, and above it differ from the epilogue's by no bit."""
+    from prometheus_b200.ops import functional as ops
+
+    tiny = 2.0 ** -126
+    a, b = _r(64, 256, seed=1), _r(64, 512, seed=2)
+    a[:, :128] *= 2.0 ** -63
+    b[:, :256] *= 2.0 ** -66
+    got, want = (torch.zeros(256, 512, device="cuda") for _ in range(2))
+    for _ in range(32):
+        ops.gemm(a, b, a_mn=True, b_mn=True, out=got, d=got, beta=1.0)
+        want = ops.gemm(a, b, a_mn=True, b_mn=True, out_dtype=torch.float32, d=want, beta=1.0)
+    assert ((got.double() - want.double()).abs() <= 32 * tiny).all()
+    assert torch.equal(got[128:], want[128:]) and torch.equal(got[:, 256:], want[:, 256:])
 
 
 @pytest.mark.parametrize("M,N,K,batch", [(8, 1024, 64, 1), (136, 264, 200, 1), (264, 1000, 72, 3), (1024, 1152, 136, 2), (4736, 512, 128, 1),
@@ -1080,6 +1137,16 @@ def test_delta_bwd_kernel_matches_fp32_oracle(B, S, H, fp32):
     want = dl.delta_prep_backward_ref(full(q), full(k), full(v), full(beta), ap, t, d_w, ndu, d_m, d_qs, d_ks)
     for got, ref in zip((dq, dk, dv, db), want):
         _close(got, ref[:, :S], 3e-2)
+    # and against the two kernels that do it in parts, which round dW, dM and the state products to bf16 in between
+    d_w, d_qs, d_ks = (torch.empty_like(u) for _ in range(3))
+    d_m, parts = torch.empty_like(ap), [torch.empty_like(q) for _ in range(3)] + [torch.empty_like(beta)]
+    call("pb_delta_chunk_products", ptr(ndu), ptr(d_out), ptr(u), ptr(sb), ptr(dsb), ptr(d_w), ptr(d_qs), ptr(d_ks), ptr(d_m),
+         B, S, H, H * D, st, stream_ptr())
+    call("pb_delta_prep_bwd", ptr(q), ptr(k), ptr(v), ptr(beta), fp32, ptr(ap), ptr(t), ptr(d_w), ptr(ndu), ptr(d_m), ptr(d_qs),
+         ptr(d_ks), *(ptr(x) for x in parts), B, S, H, H * D, st, 0, stream_ptr())
+    for got, ref in zip((dq, dk, dv, db), parts):
+        _close(got, ref, 2.0 ** -7)
+    ops.check_status("cuda")
 
 
 def test_debug_bounds_build_records_and_skips_a_bad_index():

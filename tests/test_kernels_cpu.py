@@ -155,3 +155,15 @@ def test_affine_scan_delta_matches_recurrent():
     o, st = delta.delta_rule_scan(q, k, v, beta, s0, chunk=16)
     torch.testing.assert_close(o, o_ref, rtol=1e-4, atol=1e-4)
     torch.testing.assert_close(st, s_ref, rtol=1e-4, atol=1e-4)
+
+
+@pytest.mark.parametrize("b,h,s", [(1, 1, 1), (2, 3, 63), (1, 2, 64), (3, 4, 65), (2, 16, 4096)])
+def test_attention_backward_scratch_holds_whole_tiles_of_rows(b, h, s):
+    """Every 64-row tile of a head is written and read as 512 bytes (16-byte aligned), the last one too when it is cut off; the
+    zig-zag halves, whose log-sum-exps are one tensor, take a half's scratch each."""
+    from prometheus_b200.ops.attention import backward_scratch
+
+    for lse2 in (torch.zeros(b, h, s), torch.zeros(2, b, h, s)[0], torch.zeros(2, b, h, s)[1]):
+        x = backward_scratch(lse2)
+        assert x.dtype == torch.float32 and x.is_contiguous() and x.data_ptr() % 16 == 0
+        assert x.numel() * 4 == b * h * -(-s // 64) * 512
