@@ -70,6 +70,17 @@ def test_the_reader_of_sources_sees_a_wait_that_splits_a_warp():
     assert per_thread_waits(text.replace("mbar_wait_warp(&tfull", "mbar_wait(&tfull"))
 
 
+def test_split_products_read_no_row_of_a_peer_that_they_do_not_store():
+    """The cluster barrier at the end of a split product is relaxed: it waits for a read of a peer's shared memory only because the
+    value read is stored before it. So the reads stop at the same row as the stores."""
+    text = _text("gemm.cu")
+    rows = text[text.index("void split_rows("):text.index("gemm_split_kernel(")]
+    read, store = rows.index("ld_cluster_f4("), rows.index("static_cast<float*>(p.C)")
+    stops = [m.start() for m in re.finditer(r"if \(r0 \+ i >= hi\) break;", rows)]
+    assert rows.count("ld_cluster_f4(") == 1 and len(stops) == 2 and stops[0] < read < stops[1] < store
+    assert "barrier.cluster.arrive.relaxed" in text
+
+
 def miscounted_blocks(text, blocks=12, schedules=200):
     """Blocks of the attention forward whose P V product is issued before all four row warps of the tile have stored P, or never,
     over random schedules of the warps and the issuer. Barriers, their indexes and parities are the source's; the scores of block j
