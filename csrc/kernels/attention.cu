@@ -227,7 +227,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     }
   } else if (warp >= 8) {
     {
-      const int t = warp - 8;                                     // the tile this thread issues for
+      const int t = warp - 8;                                     // the tile this warp issues for
       const int nj = nj1 - (t == 0 ? 2 : 0);
       const uint32_t id_s = make_idesc(1, 1, 128, 64, 0, 0);     // S = Q K^T, N = 64 keys
       const uint32_t id_o = make_idesc(1, 1, 128, 128, 0, 1);    // O += P V, V MN-major
@@ -439,9 +439,10 @@ struct Params {
 // DKV = true : resident K, V (one KV head); streams Q, dO tiles of the group; outputs dK, dV.
 // Two warpgroups (warps 0-3, 4-7) share every streamed tile, half of its columns each: what a tile waits for is its
 // score products, the rows' work on them and its gradient products one after the other, with two tiles on the
-// way, and the rows' part of that chain halves.  MMA issue is spread over three warps because one thread cannot issue
-// 20+ small MMAs per tile fast enough: warp 8 the first score product, warp 9 the second,
-// warp 10 the gradient accumulations; warp 11: TMA producer.
+// way, and the rows' part of that chain halves.  MMA issue is spread over three warps, so that each
+// waits only for what its own products need: warp 8 the first score product, warp 9 the second, warp 10 the gradient
+// accumulations; warp 11: TMA producer. (One lane could not issue all 20+ products of a tile in time; whether one warp can
+// was not measured.)
 //
 // Shared-memory bandwidth is what the products compete for: a 128 x 64 score product with both operands there reads
 // 6 KB per 16-deep step, half as much again as the tensor core can use. So what can be kept off it is: P^T
@@ -949,7 +950,7 @@ PB_API int pb_attn_bwd_cp(const void* q, const void* k, const void* v, const voi
     r |= tok_map(&tDQ, dq, qi, seq, batch, ldq, 128);
     if (r != 0) return 1000 + r;
     p.n_blk = (seq + 127) / 128;
-    pb::launch(bwd::attn_bwd_kernel<false>, static_cast<unsigned>(grid_q), 384, bwd::SMEM, st, 
+    pb::launch(bwd::attn_bwd_kernel<false>, static_cast<unsigned>(grid_q), 384, bwd::SMEM, st,
         tQ, tDO, tK, tV, tDQ, tDQ, tO, p);
   }
   {
@@ -963,7 +964,7 @@ PB_API int pb_attn_bwd_cp(const void* q, const void* k, const void* v, const voi
     r |= tok_map(&tDV, dv, ki, seq_kv, batch, ldkv, 128);
     if (r != 0) return 2000 + r;
     p.n_blk = (seq_kv + 127) / 128;
-    pb::launch(bwd::attn_bwd_kernel<true>, static_cast<unsigned>(grid_kv), 384, bwd::SMEM, st, 
+    pb::launch(bwd::attn_bwd_kernel<true>, static_cast<unsigned>(grid_kv), 384, bwd::SMEM, st,
         tK, tV, tQ, tDO, tDK, tDV, tK, p);
   }
   return static_cast<int>(cudaGetLastError());

@@ -3,6 +3,9 @@
 //
 //   dW  = (-dU) S^T        dQ_s = dO S^T        dK_s = U dS'^T        dM = dO U^T
 //
+// The layer's backward runs delta_bwd.cu, which does this and pb_delta_prep_bwd's part in one kernel. These two are what its test
+// compares it with, stage by stage.
+//
 // S is the bf16 state entering the chunk, dS' the gradient of the state leaving it, both
 // [128, 128]; U, -dU and dO are [64, 128], dO read in place from its token-major layout.
 //

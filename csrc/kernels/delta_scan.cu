@@ -787,7 +787,7 @@ PB_API int pb_delta_compose(const void* P, const void* R, const void* s0, void* 
     if (e != cudaSuccess) return static_cast<int>(e);
     attr_once.done();
   }
-  pb::launch(pb::dcomp::compose_kernel, grid, 256, pb::dcomp::SMEM, st, 
+  pb::launch(pb::dcomp::compose_kernel, grid, 256, pb::dcomp::SMEM, st,
       static_cast<const float*>(P), static_cast<const float*>(R), static_cast<const float*>(s0),
       static_cast<float*>(s_in), static_cast<float*>(s_fin), static_cast<float*>(p_tot), n_seg,
       reverse, slabs);

@@ -802,7 +802,7 @@ static int rmsnorm_fwd_impl(const void* x, const void* res, const void* w, void*
     }
     return cudaGetLastError();
   }
-  pb::launch(rmsnorm_fwd_kernel, (rows + wpb - 1) / wpb, wpb * 32, 0, st, 
+  pb::launch(rmsnorm_fwd_kernel, (rows + wpb - 1) / wpb, wpb * 32, 0, st,
       static_cast<const bf16*>(x), static_cast<const bf16*>(res), static_cast<const float*>(w),
       static_cast<bf16*>(y), static_cast<bf16*>(h_out), static_cast<float*>(rstd), rows, d, eps);
   return cudaGetLastError();
@@ -916,7 +916,7 @@ PB_API int pb_copy_rows_dyn(const void* src, void* dst, long row_bytes, long max
   if (row_bytes <= 0 || row_bytes % 16 != 0 || max_rows <= 0 || rows_dev == nullptr ||
       ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) != 0)
     return PB_BAD_ARG;
-  pb::launch(copy_rows_dyn_kernel, grid_for(max_rows * (row_bytes / 16), 256 * 4), 256, 0, st, 
+  pb::launch(copy_rows_dyn_kernel, grid_for(max_rows * (row_bytes / 16), 256 * 4), 256, 0, st,
       static_cast<const uint4*>(src), static_cast<uint4*>(dst), row_bytes / 16, max_rows, rows_dev);
   return cudaGetLastError();
 }
@@ -930,12 +930,12 @@ PB_API int pb_l2norm_fwd(void* x, void* inv_norm, long nvec, int D, float eps, c
   if (D % 4 != 0) return PB_BAD_ARG;
   if (D == 128 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
     const long warps = (nvec + 7) / 8;
-    pb::launch(l2norm128_fwd_kernel, grid_for((warps + 7) / 8, 1, 148 * 8), 256, 0, st, 
+    pb::launch(l2norm128_fwd_kernel, grid_for((warps + 7) / 8, 1, 148 * 8), 256, 0, st,
         static_cast<bf16*>(x), static_cast<float*>(inv_norm), nvec, eps);
     return cudaGetLastError();
   }
   const int wpb = 8;
-  pb::launch(l2norm_fwd_kernel, static_cast<unsigned>((nvec + wpb - 1) / wpb), wpb * 32, 0, st, 
+  pb::launch(l2norm_fwd_kernel, static_cast<unsigned>((nvec + wpb - 1) / wpb), wpb * 32, 0, st,
       static_cast<bf16*>(x), static_cast<float*>(inv_norm), nvec, D, eps);
   return cudaGetLastError();
 }
@@ -944,13 +944,13 @@ PB_API int pb_l2norm_bwd(void* dxn, const void* xn, const void* inv_norm, long n
   if (D % 4 != 0) return PB_BAD_ARG;
   if (D == 128 && ((reinterpret_cast<uintptr_t>(dxn) | reinterpret_cast<uintptr_t>(xn)) & 15) == 0) {
     const long warps = (nvec + 7) / 8;
-    pb::launch(l2norm128_bwd_kernel, grid_for((warps + 7) / 8, 1, 148 * 8), 256, 0, st, 
+    pb::launch(l2norm128_bwd_kernel, grid_for((warps + 7) / 8, 1, 148 * 8), 256, 0, st,
         static_cast<bf16*>(dxn), static_cast<const bf16*>(xn),
         static_cast<const float*>(inv_norm), nvec);
     return cudaGetLastError();
   }
   const int wpb = 8;
-  pb::launch(l2norm_bwd_kernel, static_cast<unsigned>((nvec + wpb - 1) / wpb), wpb * 32, 0, st, 
+  pb::launch(l2norm_bwd_kernel, static_cast<unsigned>((nvec + wpb - 1) / wpb), wpb * 32, 0, st,
       static_cast<bf16*>(dxn), static_cast<const bf16*>(xn),
       static_cast<const float*>(inv_norm), nvec, D);
   return cudaGetLastError();
@@ -960,7 +960,7 @@ PB_API int pb_softcap_ce(void* logits, const void* targets, const void* wt, void
                          void* lse_rows, long rows, int V, float cap, int write_grad,
                          cudaStream_t st) {
   if (V % 8 != 0 || rows <= 0) return PB_BAD_ARG;
-  pb::launch(softcap_ce_kernel, static_cast<unsigned>(rows), 512, 0, st, 
+  pb::launch(softcap_ce_kernel, static_cast<unsigned>(rows), 512, 0, st,
       static_cast<bf16*>(logits), static_cast<const int*>(targets),
       static_cast<const float*>(wt), static_cast<float*>(loss_rows),
       static_cast<float*>(lse_rows), V, cap, write_grad, nullptr);
@@ -972,7 +972,7 @@ PB_API int pb_softcap_ce(void* logits, const void* targets, const void* wt, void
 PB_API int pb_softcap_ce_sums(void* logits, const void* targets, const void* wt, void* loss_rows, const void* sums,
                               long rows, int V, float cap, int write_grad, cudaStream_t st) {
   if (V % 8 != 0 || rows <= 0 || !(cap > 0.f) || sums == nullptr) return PB_BAD_ARG;
-  pb::launch(softcap_ce_kernel, static_cast<unsigned>(rows), 512, 0, st, 
+  pb::launch(softcap_ce_kernel, static_cast<unsigned>(rows), 512, 0, st,
       static_cast<bf16*>(logits), static_cast<const int*>(targets), static_cast<const float*>(wt),
       static_cast<float*>(loss_rows), nullptr, V, cap, write_grad, static_cast<const float*>(sums));
   return cudaGetLastError();
@@ -981,7 +981,7 @@ PB_API int pb_softcap_ce_sums(void* logits, const void* targets, const void* wt,
 // x fp32 [n], g fp32 [1], out bf16 [n]; x and out 16-byte aligned.
 PB_API int pb_scale_cast(const void* x, const void* g, void* out, long n, cudaStream_t st) {
   if (n <= 0 || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15)) return PB_BAD_ARG;
-  pb::launch(scale_cast_kernel, static_cast<unsigned>((n + 2047) / 2048), 256, 0, st, 
+  pb::launch(scale_cast_kernel, static_cast<unsigned>((n + 2047) / 2048), 256, 0, st,
       static_cast<const float*>(x), static_cast<const float*>(g), static_cast<bf16*>(out), n);
   return cudaGetLastError();
 }

@@ -780,7 +780,7 @@ PB_API int pb_fp8_quant_rows(const void* x, long ld, int M, int K, void* q, floa
                              cudaStream_t st) {
   if (M <= 0 || K <= 0 || K % 128 != 0 || ld % 8 != 0 || (reinterpret_cast<uintptr_t>(x) & 15) != 0)
     return PB_BAD_ARG;
-  pb::launch(f8::quant_rows_kernel, f8::tile_grid(f8::QR, M, K), 256, 0, st, 
+  pb::launch(f8::quant_rows_kernel, f8::tile_grid(f8::QR, M, K), 256, 0, st,
       static_cast<const bf16*>(x), ld, M, K, static_cast<uint8_t*>(q), scales, nullptr);
   return static_cast<int>(cudaGetLastError());
 }
@@ -789,7 +789,7 @@ PB_API int pb_fp8_quant_rows_dyn(const void* x, long ld, int M, int K, void* q, 
                                  const int* rows_dev, cudaStream_t st) {
   if (M <= 0 || K <= 0 || K % 128 != 0 || ld % 8 != 0 || (reinterpret_cast<uintptr_t>(x) & 15) != 0)
     return PB_BAD_ARG;
-  pb::launch(f8::quant_rows_kernel, f8::tile_grid(f8::QR, M, K), 256, 0, st, 
+  pb::launch(f8::quant_rows_kernel, f8::tile_grid(f8::QR, M, K), 256, 0, st,
       static_cast<const bf16*>(x), ld, M, K, static_cast<uint8_t*>(q), scales, rows_dev);
   return static_cast<int>(cudaGetLastError());
 }
@@ -799,7 +799,7 @@ PB_API int pb_fp8_quant_rows_dyn(const void* x, long ld, int M, int K, void* q, 
 PB_API int pb_swiglu_quant(const void* gu, void* h, int M, int H, void* q, float* scales,
                            const int* rows_dev, cudaStream_t st) {
   if (M <= 0 || H <= 0 || H % 128 != 0) return PB_BAD_ARG;
-  pb::launch(f8::swiglu_quant_kernel, f8::tile_grid(f8::QR_SWI, M, H), 256, 0, st, 
+  pb::launch(f8::swiglu_quant_kernel, f8::tile_grid(f8::QR_SWI, M, H), 256, 0, st,
       static_cast<const bf16*>(gu), static_cast<bf16*>(h), M, H, static_cast<uint8_t*>(q), scales,
       rows_dev);
   return static_cast<int>(cudaGetLastError());
@@ -810,7 +810,7 @@ PB_API int pb_swiglu_quant(const void* gu, void* h, int M, int H, void* q, float
 PB_API int pb_fp8_dequant_rows(const void* q, const float* scales, long ld_s, int M, int K, void* y,
                                const int* rows_dev, cudaStream_t st) {
   if (M <= 0 || K <= 0 || K % 128 != 0 || ld_s < M) return PB_BAD_ARG;
-  pb::launch(f8::dequant_rows_kernel, f8::tile_grid(f8::QR, M, K), 256, 0, st, 
+  pb::launch(f8::dequant_rows_kernel, f8::tile_grid(f8::QR, M, K), 256, 0, st,
       static_cast<const uint8_t*>(q), scales, ld_s, M, K, static_cast<bf16*>(y), rows_dev);
   return static_cast<int>(cudaGetLastError());
 }

@@ -114,7 +114,7 @@ static bool bad_slots(int B, int S, int d, int start, int K) {
 PB_API int pb_latent_gather(const void* src, void* rows, int B, int S, int d, int start, int K,
                             cudaStream_t st) {
   if (bad_slots(B, S, d, start, K)) return PB_BAD_ARG;
-  pb::launch(latent_gather_kernel, (B * K * 32 + 255) / 256, 256, 0, st, 
+  pb::launch(latent_gather_kernel, (B * K * 32 + 255) / 256, 256, 0, st,
       static_cast<const bf16*>(src), static_cast<bf16*>(rows), B, S, d, start, K);
   return static_cast<int>(cudaGetLastError());
 }
@@ -123,7 +123,7 @@ PB_API int pb_latent_gather(const void* src, void* rows, int B, int S, int d, in
 PB_API int pb_latent_scatter(const void* rows, void* dst, int B, int S, int d, int start, int K,
                              cudaStream_t st) {
   if (bad_slots(B, S, d, start, K)) return PB_BAD_ARG;
-  pb::launch(latent_scatter_kernel, (B * K * 32 + 255) / 256, 256, 0, st, 
+  pb::launch(latent_scatter_kernel, (B * K * 32 + 255) / 256, 256, 0, st,
       static_cast<const bf16*>(rows), static_cast<bf16*>(dst), B, S, d, start, K);
   return static_cast<int>(cudaGetLastError());
 }
@@ -134,7 +134,7 @@ PB_API int pb_latent_norm_scatter(const void* a, const void* w, const void* embe
                                   cudaStream_t st) {
   if (bad_slots(B, S, d, start, K)) return PB_BAD_ARG;
   const long warps = static_cast<long>(B) * S;
-  pb::launch(latent_norm_scatter_kernel, static_cast<unsigned>((warps * 32 + 255) / 256), 256, 0, st, 
+  pb::launch(latent_norm_scatter_kernel, static_cast<unsigned>((warps * 32 + 255) / 256), 256, 0, st,
       static_cast<const bf16*>(a), static_cast<const float*>(w), static_cast<const bf16*>(embeds),
       static_cast<bf16*>(out), static_cast<float*>(rstd), B, S, d, start, K, eps);
   return static_cast<int>(cudaGetLastError());

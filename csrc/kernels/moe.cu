@@ -525,7 +525,7 @@ PB_API int pb_moe_permute_q(const void* q, const float* scales, const int* row_o
   if (T <= 0 || k <= 0 || K <= 0 || K % 128 != 0 || E <= 0) return PB_BAD_ARG;
   const int n_pairs = T * k;
   const int pair_blocks = warps_grid(n_pairs, 256);
-  pb::launch(moe::permute_q_kernel, pair_blocks + E * moe::PAD_SPLIT, 256, 0, st, 
+  pb::launch(moe::permute_q_kernel, pair_blocks + E * moe::PAD_SPLIT, 256, 0, st,
       static_cast<const uint8_t*>(q), scales, row_of, n_pairs, k, K, T, static_cast<uint8_t*>(dq), dscales, rows,
       pair_blocks, expert_off, totals);
   return static_cast<int>(cudaGetLastError());
@@ -542,7 +542,7 @@ PB_API int pb_moe_zero_pad(void* buf, int d, const int* expert_off, const int* t
 PB_API int pb_moe_combine(const void* y, const int* row_of, const float* gates, const void* add,
                           int T, int k, int d, void* out, long y_rows, cudaStream_t st) {
   if (T <= 0 || d % 8 != 0) return PB_BAD_ARG;
-  pb::launch(moe::combine_kernel, warps_grid(static_cast<long>(T) * ((d + 511) / 512), 256), 256, 0, st, 
+  pb::launch(moe::combine_kernel, warps_grid(static_cast<long>(T) * ((d + 511) / 512), 256), 256, 0, st,
       static_cast<const bf16*>(y), row_of, gates, static_cast<const bf16*>(add), T, k, d,
       static_cast<bf16*>(out), y_rows > 0 ? y_rows : (1L << 62));
   return static_cast<int>(cudaGetLastError());
@@ -551,7 +551,7 @@ PB_API int pb_moe_combine(const void* y, const int* row_of, const float* gates, 
 PB_API int pb_moe_combine_bwd(const void* y, const void* dout, const int* row_of, int n_pairs, int k,
                               int d, float* dgates, cudaStream_t st) {
   if (n_pairs <= 0 || d % 8 != 0) return PB_BAD_ARG;
-  pb::launch(moe::combine_bwd_kernel, warps_grid(n_pairs, 256), 256, 0, st, 
+  pb::launch(moe::combine_bwd_kernel, warps_grid(n_pairs, 256), 256, 0, st,
       static_cast<const bf16*>(y), static_cast<const bf16*>(dout), row_of, n_pairs, k, d, dgates);
   return static_cast<int>(cudaGetLastError());
 }

@@ -294,7 +294,7 @@ PB_API int pb_adamw(void* p, const void* g, void* m, void* v, void* p_lp, long n
   if (step < 1) return PB_BAD_ARG;
   const float inv_bc1 = 1.f / (1.f - powf(b1, static_cast<float>(step)));
   const float inv_bc2 = 1.f / (1.f - powf(b2, static_cast<float>(step)));
-  pb::launch(adamw_kernel, ogrid(n), 256, 0, st, 
+  pb::launch(adamw_kernel, ogrid(n), 256, 0, st,
       static_cast<float*>(p), static_cast<const float*>(g), static_cast<float*>(m),
       static_cast<float*>(v), static_cast<bf16*>(p_lp), n, lr, b1, b2, eps, wd, inv_bc1, inv_bc2,
       static_cast<const float*>(gnorm_sq), clip, gscale);
@@ -314,7 +314,7 @@ PB_API int pb_muon_prepare(const void* g, void* m, void* x0, long n, float beta,
                                               static_cast<const float*>(gnorm_sq), clip, gscale,
                                               part);
   pb::launch(fold_scalar_kernel, 1, 32, 0, st, part, parts, nes_sq, 0);
-  pb::launch(muon_normalize_kernel, ogrid(n), 256, 0, st, 
+  pb::launch(muon_normalize_kernel, ogrid(n), 256, 0, st,
       static_cast<const float*>(g), static_cast<const float*>(m), static_cast<bf16*>(x0), n, beta,
       static_cast<const float*>(gnorm_sq), clip, gscale, nes_sq);
   return cudaGetLastError();
@@ -340,7 +340,7 @@ PB_API int pb_muon_prepare_batched(const void* g, void* m, void* x0, long n, int
                                                          static_cast<const float*>(gnorm_sq),
                                                          clip, gscale, pj);
     pb::launch(fold_rows_kernel, cnt, 32, 0, st, pj, parts, nes_sq + j0);
-    pb::launch(muon_normalize_kernel, dim3(ogrid(n), cnt), 256, 0, st, 
+    pb::launch(muon_normalize_kernel, dim3(ogrid(n), cnt), 256, 0, st,
         gj, mj, xj, n, beta, static_cast<const float*>(gnorm_sq), clip, gscale, nes_sq + j0);
   }
   return cudaGetLastError();

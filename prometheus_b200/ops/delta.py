@@ -173,13 +173,22 @@ def scan_segments(n_seq: int, n_chunks: int, ctas: int = 148) -> int:
         waves(2 n_seq seg) * 0.6 n_chunks / seg  +  waves(n_seq seg) * n_chunks / seg  +  24
 
     The smallest power of two (at least four chunks per segment) whose estimate beats the single
-    pass's by a fifth is taken; 1 means the plain single-pass walk. The kernels differ from the model: walks
-    that take at most half of the SMs run as two CTAs each, and a summary whose CTAs do not fit runs both
-    maps in one (``csrc/kernels/delta_scan.cu``), so the choice is near the best and not always the best. Measured,
-    forward us at 1 / 4 / 8 / 16 segments (the rule's choice in parentheses): 16 sequences x 256 chunks
-    492 / 359 / 316 / 404 (8), 16 x 128 252 / 201 / 193 / 241 (8), 16 x 64 134 / 123 / 127 / 176 (4), 8 x 256
-    431 / 300 / 216 / 223 (16, 3 % slower than 8), 32 x 128 314 / 319 / 419 / 471 (4, 2 % slower than uncut),
-    32 x 64 163 / 194 / 241 / 334 (1). The backward, which uses the same segments, was not measured apart."""
+    pass's by a fifth is taken; 1 means the plain single-pass walk. The model's constants are older than the kernels, which
+    differ from it: walks that take at most half of the SMs run as two CTAs each, a summary whose CTAs do not fit runs both
+    maps in one (``csrc/kernels/delta_scan.cu``), and an uncut walk now takes a third less time than when they were fitted.
+    Measured, us of the layer's forward, and of forward and backward together, which use the same segments:
+
+        sequences x chunks    uncut         4             8             16            chosen
+        16 x 256              338 / 784     266 / 655     257 / 643     299 / 723     8
+        16 x 128              176 / 407     153 / 369     159 / 379     204 / 471     8, 4 % slower than 4
+        16 x 64               93 / 215      94 / 221      105 / 243     152 / 341     4, 1 to 3 % slower than uncut
+        8 x 256               298 / 659     227 / 496     168 / 400     189 / 443     16, 11 to 13 % slower than 8
+        8 x 64                81 / 181      82 / 177      78 / 174      106 / 233     8
+        4 x 256               277 / 590     206 / 429     145 / 314     136 / 313     16
+        32 x 128              212 / 528     258 / 646     298 / 726     391 / 908     4, 21 % slower than uncut
+        32 x 64               114 / 282     160 / 384     207 / 477     299 / 657     uncut
+        64 x 64               153 / 440     303 / 730     394 / 913     551 / 1237    uncut
+    """
     def waves(c):
         return -(-c // ctas)
 
