@@ -975,21 +975,21 @@ def test_delta_compose(n_seq, n_seg, reverse):
             assert (p_tot.double() - tot).norm() <= 1e-5 * tot.norm()
 
 
-def test_gemm_accumulates_sums_below_the_normal_range():
-    """Adding stores flush sums below 2^-126 to zero, the epilogue's addition does not: 32 products added into one buffer stay
-    within 32 x 2^-126 of the exact sum there, and above it differ from the epilogue's by no bit."""
+@pytest.mark.parametrize("M,N,K", [(256, 512, 64), (2048, 4096, 128)])      # one wave of 128 x 128 tiles, CTA pairs
+def test_gemm_accumulates_sums_below_the_normal_range(M, N, K):
+    """Four products of about 2^-126 added into one buffer by adding stores: the bits of the epilogue's addition, below the normal
+    range and beside it."""
     from prometheus_b200.ops import functional as ops
 
-    tiny = 2.0 ** -126
-    a, b = _r(64, 256, seed=1), _r(64, 512, seed=2)
-    a[:, :128] *= 2.0 ** -63
-    b[:, :256] *= 2.0 ** -66
-    got, want = (torch.zeros(256, 512, device="cuda") for _ in range(2))
-    for _ in range(32):
+    a, b = _r(K, M, seed=1), _r(K, N, seed=2)
+    a[:, :M // 2] *= 2.0 ** -65
+    b[:, :N // 2] *= 2.0 ** -65
+    got, want = (torch.zeros(M, N, device="cuda") for _ in range(2))
+    for _ in range(4):
         ops.gemm(a, b, a_mn=True, b_mn=True, out=got, d=got, beta=1.0)
         want = ops.gemm(a, b, a_mn=True, b_mn=True, out_dtype=torch.float32, d=want, beta=1.0)
-    assert ((got.double() - want.double()).abs() <= 32 * tiny).all()
-    assert torch.equal(got[128:], want[128:]) and torch.equal(got[:, 256:], want[:, 256:])
+    assert ((want != 0) & (want.abs() < 2.0 ** -126)).any()
+    assert torch.equal(got, want)
 
 
 @pytest.mark.parametrize("M,N,K,batch", [(8, 1024, 64, 1), (136, 264, 200, 1), (264, 1000, 72, 3), (1024, 1152, 136, 2), (4736, 512, 128, 1),
